@@ -202,6 +202,7 @@ struct wb_cosx {
     double* f64_P = nullptr;
     double* f64_E = nullptr;
     double* f64_boys = nullptr;
+    double* f64_fine = nullptr;      // the fine-node Boys table (fp64_boys.cuh)
     long long f64_ebase[wb::NCLASS] = {0};
     double* f64_alpha = nullptr;     // bra exponent per primitive pair
     double* f64_vsxyz = nullptr;     // virtual shell centres (3 each)
@@ -662,21 +663,31 @@ int ensure_fp64(wb_cosx* h) {
         if (B) cudaFree(B);
         return cuda_fail(e, "FP64 pair tables");
     }
+    // the same for every handle: formed once in the process
+    static const std::vector<double> fine = [] {
+        std::vector<double> t((size_t)wb::kBoysFineNodes * wb::kBoysFineCols);
+        for (int k = 0; k < wb::kBoysFineNodes; ++k)
+            wb::boys_f64(wb::kBoysFineCols - 1, k / 32.0,
+                         t.data() + (size_t)k * wb::kBoysFineCols);
+        return t;
+    }();
     std::vector<double> vxyz;
     std::vector<int> vat;
     for (const wb::VShell& v : h->hp.vsh) {
         for (int x = 0; x < 3; ++x) vxyz.push_back(v.A[x]);
         vat.push_back(v.atom);
     }
-    double *AL = nullptr, *VX = nullptr;
+    double *AL = nullptr, *VX = nullptr, *FI = nullptr;
     int* VA = nullptr;
     e = upload(&AL, hp64.alpha);
+    if (e == cudaSuccess) e = upload(&FI, fine);
     if (e == cudaSuccess) e = upload(&VX, vxyz);
     if (e == cudaSuccess) e = cudaMalloc(&VA, sizeof(int) * std::max<size_t>(vat.size(), 1));
     if (e == cudaSuccess && !vat.empty())
         e = cudaMemcpy(VA, vat.data(), sizeof(int) * vat.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
-        for (void* q : {(void*)P, (void*)E, (void*)B, (void*)AL, (void*)VX, (void*)VA})
+        for (void* q : {(void*)P, (void*)E, (void*)B, (void*)AL, (void*)VX, (void*)FI,
+                        (void*)VA})
             if (q) cudaFree(q);
         return cuda_fail(e, "FP64 pair tables");
     }
@@ -684,6 +695,7 @@ int ensure_fp64(wb_cosx* h) {
     h->f64_E = E;
     h->f64_boys = B;
     h->f64_alpha = AL;
+    h->f64_fine = FI;
     h->f64_vsxyz = VX;
     h->vs_atom = VA;
     for (int c = 0; c < wb::NCLASS; ++c) h->f64_ebase[c] = hp64.e_base[c];
@@ -774,7 +786,7 @@ int64_t hartree_ndh(const wb::HostPairs& hp) {
 
 struct WsLayout64 {
     WsLayout base;                  // counters, work, block statistics
-    size_t X = 0, F64 = 0, F32 = 0, G64 = 0, WG = 0, total = 0;
+    size_t X = 0, F64 = 0, F32 = 0, G64 = 0, WG = 0, rec = 0, total = 0;
 };
 
 WsLayout64 ws_layout_fp64(const wb_cosx* h, int64_t ld) {
@@ -799,6 +811,7 @@ WsLayout64 ws_layout_fp64(const wb_cosx* h, int64_t ld) {
     L.F32 = take(sizeof(float) * n);
     L.G64 = take(sizeof(double) * n);
     L.WG = take(sizeof(double) * n);
+    L.rec = take(sizeof(double) * wb::kF64Rec * (size_t)std::max(h->hp.npp, 1));
     L.total = off;
     return L;
 }
@@ -1119,6 +1132,7 @@ int wb_cosx_destroy(wb_cosx* h) {
     if (h->f64_P) cudaFree(h->f64_P);
     if (h->f64_E) cudaFree(h->f64_E);
     if (h->f64_boys) cudaFree(h->f64_boys);
+    if (h->f64_fine) cudaFree(h->f64_fine);
     if (h->f64_alpha) cudaFree(h->f64_alpha);
     if (h->f64_vsxyz) cudaFree(h->f64_vsxyz);
     if (h->vs_atom) cudaFree(h->vs_atom);
@@ -1486,11 +1500,10 @@ int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
         a.pp_begin[c] = h->hp.cls[c].pp_begin;
         a.e_base[c] = h->f64_ebase[c];
     }
-    a.P = h->f64_P;
-    a.p = h->p;
-    a.pref = h->pref;
+    double* rec = at<double>(workspace, L.rec);
+    a.rec = rec;
     a.E = h->f64_E;
-    a.boys = h->f64_boys;
+    a.boys = h->f64_fine;
     a.c2s = h->f64_boys + (size_t)wb::kBoys64Nodes * wb::kBoys64Cols;
     a.pflops = h->pflops;
     a.pnint = h->pnint;
@@ -1498,10 +1511,11 @@ int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
     a.work = at<int>(workspace, L.base.work);
     int64_t ntasks = 0;
     for (int j = 0; j < nomega; ++j) {
-        a.omega = omegas[j];
+        WB_CUDA(wb::launch_f64_records(h->hp.npp, h->f64_P, h->p, h->pref, h->f64_alpha,
+                                       omegas[j], rec, s));
         WB_CUDA(cudaMemsetAsync(G64, 0, sizeof(double) * (size_t)nao * ld, s));
         WB_CUDA(cudaMemsetAsync(a.work, 0, sizeof(int) * wb::NCLASS, s));
-        launches += 2;
+        launches += 3;
         for (int c = 0; c < wb::NCLASS; ++c) {
             const int pb = h->hp.cls[c].pair_begin, pe = h->hp.cls[c].pair_end;
             if (pe <= pb) continue;
@@ -1902,14 +1916,40 @@ int wb_cosx_batch_destroy(wb_cosx_batch* b) {
     return WB_OK;
 }
 
+namespace {
+// the FP64 form's layout, then the AO values and their x, y, z gradients
+// (4, nao, ld), the point columns of the gradient (3 natm, ld), the d/dQ of
+// the Hermite coefficients and the AO sums
+struct GradLayout {
+    WsLayout64 f64;
+    size_t X = 0, gpt = 0, dE = 0, aodot = 0, total = 0;
+};
+
+GradLayout grad_layout(const wb_cosx* h, int64_t ld, int natm) {
+    GradLayout L;
+    L.f64 = ws_layout_fp64(h, ld);
+    int64_t ne = 0;
+    for (int la = 0; la <= wb::LMAX; ++la)
+        for (int lb = 0; lb <= la; ++lb) {
+            const wb::ClassRange& r = h->hp.cls[wb::class_of(la, lb)];
+            ne += (int64_t)(r.pp_end - r.pp_begin) * 3 * wb::e64_axis(la, lb);
+        }
+    const size_t sizes[4] = {4 * (size_t)h->hp.nao * ld, 3 * (size_t)natm * ld, (size_t)ne,
+                             3 * (size_t)h->hp.nao};
+    size_t* offs[4] = {&L.X, &L.gpt, &L.dE, &L.aodot};
+    size_t off = L.f64.total;
+    for (int i = 0; i < 4; ++i) {
+        *offs[i] = off;
+        off = align256(off + sizeof(double) * sizes[i]);
+    }
+    L.total = off;
+    return L;
+}
+}  // namespace
+
 size_t wb_cosx_k_grad_workspace_bytes(const wb_cosx* h, int64_t npts, int natm) {
     if (!h || npts < 0 || natm < 1) return 0;
-    const int64_t ld = round32(std::max<int64_t>(npts, 1));
-    const WsLayout64 L = ws_layout_fp64(h, ld);
-    const size_t n = (size_t)h->hp.nao * ld;
-    return align256(L.total + sizeof(double) * 4 * n) +
-           align256(sizeof(double) * (size_t)(ld / 32) * natm * 3) +
-           align256(sizeof(double) * 3 * (size_t)h->hp.nao);
+    return grad_layout(h, round32(std::max<int64_t>(npts, 1)), natm).total;
 }
 
 int wb_cosx_k_grad(wb_cosx* h, const double* coords, const double* weights,
@@ -1934,15 +1974,14 @@ int wb_cosx_k_grad(wb_cosx* h, const double* coords, const double* weights,
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int nao = h->hp.nao;
     const size_t n = (size_t)nao * ld;
-    // the FP64 form's layout, then the AO values and their x, y, z
-    // gradients (4, nao, ld), the per-block gradient rows and the AO sums
-    const WsLayout64 L = ws_layout_fp64(h, ld);
-    char* base = static_cast<char*>(workspace);
-    double* Xd = reinterpret_cast<double*>(base + L.total);     // (4, nao, ld)
-    double* gbuf = reinterpret_cast<double*>(base + align256(L.total + sizeof(double) * 4 * n));
+    const GradLayout GL = grad_layout(h, ld, natm);
+    const WsLayout64& L = GL.f64;
+    double* Xd = at<double>(workspace, GL.X);       // (4, nao, ld)
+    double* gpt = at<double>(workspace, GL.gpt);
+    double* dE = at<double>(workspace, GL.dE);
+    double* aodot = at<double>(workspace, GL.aodot);
+    double* rec = at<double>(workspace, L.rec);
     const int nblk = (int)(ld / 32);
-    double* aodot = reinterpret_cast<double*>(
-        reinterpret_cast<char*>(gbuf) + align256(sizeof(double) * (size_t)nblk * natm * 3));
     double* F64 = at<double>(workspace, L.F64);
     float* F32 = at<float>(workspace, L.F32);
     double* G64 = at<double>(workspace, L.G64);
@@ -1974,19 +2013,21 @@ int wb_cosx_k_grad(wb_cosx* h, const double* coords, const double* weights,
     wb::CosxF64Args a;
     std::memset(&a, 0, sizeof(a));
     a.F = F64; a.G = G64; a.coords = coords; a.ld = ld; a.npts = (int)npts;
-    a.omega = omega; a.khdr = h->khdr; a.pshell = h->pshell; a.ptau = h->ptau;
+    a.khdr = h->khdr; a.pshell = h->pshell; a.ptau = h->ptau;
     a.bnd = h->bnd; a.bpref = h->bpref; a.blk_cr = bo.cr[0]; a.blk_msh = bo.msh[0];
     a.nblk = nblk; a.nvshell = h->hp.nvshell; a.tol = tol;
     for (int c = 0; c < wb::NCLASS; ++c) {
         a.pp_begin[c] = h->hp.cls[c].pp_begin;
         a.e_base[c] = h->f64_ebase[c];
     }
-    a.P = h->f64_P; a.p = h->p; a.pref = h->pref; a.E = h->f64_E; a.boys = h->f64_boys;
+    a.rec = rec; a.E = h->f64_E; a.boys = h->f64_fine;
     a.c2s = h->f64_boys + (size_t)wb::kBoys64Nodes * wb::kBoys64Cols;
     a.pflops = h->pflops; a.pnint = h->pnint;
     a.counters = at<unsigned long long>(workspace, L.base.counters);
     a.work = work;
     WB_CUDA(cudaMemsetAsync(a.counters, 0, sizeof(unsigned long long) * kCounterWords, s));
+    WB_CUDA(wb::launch_f64_records(h->hp.npp, h->f64_P, h->p, h->pref, h->f64_alpha, omega,
+                                   rec, s));
     WB_CUDA(cudaMemsetAsync(G64, 0, sizeof(double) * n, s));
     WB_CUDA(cudaMemsetAsync(work, 0, sizeof(int) * wb::NCLASS, s));
     for (int c = 0; c < wb::NCLASS; ++c) {
@@ -2003,21 +2044,27 @@ int wb_cosx_k_grad(wb_cosx* h, const double* coords, const double* weights,
     // integral side
     wb::CosxGradArgs g;
     std::memset(&g, 0, sizeof(g));
-    g.F = F64; g.coords = coords; g.weights = weights; g.ld = ld; g.npts = (int)npts;
-    g.omega = omega; g.khdr = h->khdr; g.pshell = h->pshell; g.ptau = h->ptau;
+    g.F = F64; g.coords = coords; g.ld = ld; g.npts = (int)npts;
+    g.khdr = h->khdr; g.pshell = h->pshell; g.ptau = h->ptau;
     g.bnd = h->bnd; g.bpref = h->bpref; g.blk_cr = bo.cr[0]; g.blk_msh = bo.msh[0];
     g.nblk = nblk; g.nvshell = h->hp.nvshell; g.tol = tol;
-    for (int c = 0; c < wb::NCLASS; ++c) g.pp_begin[c] = h->hp.cls[c].pp_begin;
-    g.P = h->f64_P; g.p = h->p; g.pref = h->pref; g.alpha = h->f64_alpha;
-    g.vs_xyz = h->f64_vsxyz; g.vs_atom = h->vs_atom; g.boys = h->f64_boys;
-    g.c2s = a.c2s; g.gbuf = gbuf; g.natm = natm; g.work = work;
-    WB_CUDA(cudaMemsetAsync(gbuf, 0, sizeof(double) * (size_t)nblk * natm * 3, s));
+    g.rec = rec; g.E = h->f64_E; g.dE = dE; g.vs_atom = h->vs_atom; g.boys = h->f64_fine;
+    g.c2s = a.c2s; g.gpt = gpt; g.work = work;
+    wb::GradEArgs ge;
+    ge.npairs = h->hp.npairs; ge.pclass = h->pclass; ge.hdr = h->hdr; ge.pshell = h->pshell;
+    ge.p = h->p; ge.alpha = h->f64_alpha; ge.vs_xyz = h->f64_vsxyz; ge.dE = dE;
+    for (int c = 0; c < wb::NCLASS; ++c) {
+        g.pp_begin[c] = ge.pp_begin[c] = h->hp.cls[c].pp_begin;
+        g.e_base[c] = ge.e_base[c] = h->f64_ebase[c];
+    }
+    WB_CUDA(wb::launch_grad_e(ge, s));
+    WB_CUDA(cudaMemsetAsync(gpt, 0, sizeof(double) * 3 * (size_t)natm * ld, s));
     WB_CUDA(cudaMemsetAsync(work, 0, sizeof(int) * wb::NCLASS, s));
     for (int c = 0; c < wb::NCLASS; ++c) {
         const int pb = h->hp.cls[c].pair_begin, pe = h->hp.cls[c].pair_end;
         if (pe > pb) WB_CUDA(wb::launch_cosx_grad64_class(c, g, pb, pe, h->nsm, s));
     }
-    WB_CUDA(wb::launch_grad_rows_sum(gbuf, nblk, natm, grad_out, s));
+    WB_CUDA(wb::launch_grad_points_sum(gpt, weights, npts, ld, natm, grad_out, s));
     return WB_OK;
 }
 

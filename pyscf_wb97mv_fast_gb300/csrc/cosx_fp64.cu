@@ -29,7 +29,46 @@ __global__ void weight_g64_kernel(const double* __restrict__ G,
         out[i] = g < npts ? w[g] * G[i] : 0.0;
     }
 }
+
+// the lane-independent factors of a primitive pair, once per omega: in the
+// class kernels the division and the square root would take 30 FP64
+// instructions of every (primitive pair, point)
+__global__ void f64_records_kernel(const int npp, const double* __restrict__ P,
+                                   const double* __restrict__ p,
+                                   const double* __restrict__ pref,
+                                   const double* __restrict__ alpha, const double om2,
+                                   double* __restrict__ rec) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= npp) return;
+    double* r = rec + (int64_t)q * kF64Rec;
+    const double pq = p[q];
+    double th = 1.0, sth = 1.0;
+    if (om2 > 0.0) {
+        th = om2 / (om2 + pq);
+        sth = sqrt(th);
+    }
+    const double pth = pq * th;
+    r[0] = P[3 * (int64_t)q];
+    r[1] = P[3 * (int64_t)q + 1];
+    r[2] = P[3 * (int64_t)q + 2];
+    r[3] = pth;
+    double c = pref[q] * sth;
+    for (int n = 0; n < 8; ++n) {
+        r[4 + n] = c;
+        c *= -2.0 * pth;
+    }
+    r[12] = alpha[q] / pq;
+}
 }  // namespace
+
+cudaError_t launch_f64_records(int npp, const double* P, const double* p,
+                               const double* pref, const double* alpha, double omega,
+                               double* rec, cudaStream_t s) {
+    if (npp <= 0) return cudaSuccess;
+    f64_records_kernel<<<(npp + 127) / 128, 128, 0, s>>>(npp, P, p, pref, alpha,
+                                                         omega * omega, rec);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_weight_g64(const double* G, const double* w, int64_t npts,
                               int64_t ld, int nao, double* out, cudaStream_t s) {

@@ -10,26 +10,38 @@
 // One warp owns one 32-point block (one point per lane) and walks its
 // class's shell pairs in order; 32 pairs at a time each lane evaluates one
 // pair's bound and a ballot keeps the warp on the kept ones.  Per task and
-// point: F_A, F_B -> Cartesian (c2s^T F), per primitive pair the Boys
-// values (FP64 Taylor table + downward recursion, or the asymptotic form
-// with upward recursion), R_tuv in place, the Hermite sums, and the
-// F-first accumulation ya += A fb, yb += A^T fa; the task ends with
-// G_A += c2s ya and G_B += c2s yb (diagonal pairs: G_A += (c2s ya + c2s
-// yb) / 2, the symmetrised block).  Each lane owns its point's column of G
-// and the classes run one after another on one stream, so every element of
-// G has one writer and a fixed summation order.
+// point: the Boys values (fp64_boys.cuh), R_tuv in place, the Hermite sums
+// axis by axis into the Cartesian block A_ab, summed over the primitive
+// pairs; then G_A += c2s (A c2s^T F_B) and G_B += c2s (A^T c2s^T F_A)
+// (diagonal pairs: G_A += c2s (A + A^T) / 2 c2s^T F_A).  F_A and the sums of
+// G_A stay in registers over a run of pairs with one bra shell.  Each lane
+// owns its point's column of G and the classes run one after another on one
+// stream, so every element of G has one writer and a fixed summation order.
+//
+// What bounds it: the FP64 pipe, 2 lanes per clock and SM, 64 times below
+// FP32.  Everything is arranged to spend few FP64 instructions, the other
+// pipes being idle: factors that depend on the primitive pair alone come
+// from a record formed once per omega (f64_records_kernel) instead of a
+// division and a square root a lane, E^{00} = 1 and the zeros of the c2s
+// tables are skipped, the block A is summed over the primitive pairs before
+// F meets it, G_A and G_B are added by reductions in the L2 (no FP64
+// instruction on the SM; one writer lane an element, so program order).
+// Eight to sixteen warps an SM fill the pipe, so one CTA an SM with the
+// whole register file and the Boys table in shared memory is enough.
+// Measured on 8 waters (192 AOs, 70,478 points, both omegas): class kernels
+// 165 -> 63 ms, at 82-88 % of the FP64 pipe's issue rate.
 #pragma once
 #include <algorithm>
 #include <cuda_runtime.h>
 
 #include "cosx_kernels.cuh"
 #include "cosx_fp64.hpp"
+#include "fp64_boys.cuh"
 
 namespace wb {
 namespace f64 {
 
-constexpr int kF64Threads = 128;
-constexpr int kTaylor = 12;              // terms of the Boys Taylor series
+constexpr int kTaylor = 12;              // terms of the 1/4-node Boys series
 
 constexpr __host__ __device__ int ncart_c(int l) { return (l + 1) * (l + 2) / 2; }
 constexpr __host__ __device__ int nr_c(int L) { return (L + 1) * (L + 2) * (L + 3) / 6; }
@@ -73,21 +85,39 @@ constexpr __host__ __device__ int eaxis(int la, int lb) {
     return eoff(lb, la + 1, 0);
 }
 
+// position of the Cartesian component x^i y^j z^(l-i-j) (libcint order)
+constexpr __host__ __device__ int cidx(int l, int i, int j) {
+    return (l - i) * (l - i + 1) / 2 + (l - i - j);
+}
+// whether Cartesian component c enters the real solid harmonic m = -l + s
+constexpr __host__ __device__ bool c2s_nz(int l, int c, int s) {
+    // one bit per component: 6 bits a column (d), 10 bits a column (f)
+    return l <= 1 ? c == s
+           : l == 2 ? ((0x02ull | 0x10ull << 6 | 0x29ull << 12 | 0x04ull << 18 |
+                        0x09ull << 24) >> (6 * s + c)) & 1
+           : s < 4 ? ((0x042ull | 0x010ull << 10 | 0x142ull << 20 | 0x284ull << 30) >>
+                      (10 * s + c)) & 1
+                   : ((0x029ull | 0x084ull << 10 | 0x009ull << 20) >> (10 * (s - 4) + c)) & 1;
+}
+
 // c2s^T v (Cartesian components of a spherical vector) and c2s y
 template<int L>
 __device__ __forceinline__ void to_cart(const double* __restrict__ c2s,
                                         const double* s, double* c) {
-    if constexpr (L <= 1) {
 #pragma unroll
-        for (int i = 0; i < ncart_c(L); ++i) c[i] = s[i];
-    } else {
-#pragma unroll
-        for (int i = 0; i < ncart_c(L); ++i) {
-            double a = 0.0;
+    for (int i = 0; i < ncart_c(L); ++i) {
+        if constexpr (L <= 1) {
+            c[i] = s[i];
+        } else {
+            bool first = true;
+            c[i] = 0.0;
 #pragma unroll
             for (int m = 0; m < 2 * L + 1; ++m)
-                a = fma(c2s[(L - 2) * 30 + i * (2 * L + 1) + m], s[m], a);
-            c[i] = a;
+                if (c2s_nz(L, i, m)) {
+                    const double t = c2s[(L - 2) * 30 + i * (2 * L + 1) + m];
+                    c[i] = first ? t * s[m] : fma(t, s[m], c[i]);
+                    first = false;
+                }
         }
     }
 }
@@ -97,10 +127,15 @@ __device__ __forceinline__ double to_sph(const double* __restrict__ c2s,
     if constexpr (L <= 1) {
         return y[m];
     } else {
+        bool first = true;
         double a = 0.0;
 #pragma unroll
         for (int i = 0; i < ncart_c(L); ++i)
-            a = fma(c2s[(L - 2) * 30 + i * (2 * L + 1) + m], y[i], a);
+            if (c2s_nz(L, i, m)) {
+                const double t = c2s[(L - 2) * 30 + i * (2 * L + 1) + m];
+                a = first ? t * y[i] : fma(t, y[i], a);
+                first = false;
+            }
         return a;
     }
 }
@@ -138,13 +173,16 @@ __device__ __forceinline__ void boys64(const double T, const double* __restrict_
     }
 }
 
+// k r for a small k known at compile time
+__device__ __forceinline__ double times(const int k, const double r) {
+    return k == 1 ? r : (double)k * r;
+}
+
 // R_tuv (t + u + v <= L) at PC = (x, y, z) from r0[n] = R_000^(n), levels
 // L .. 0 in place (each level reads only the level above)
 template<int L>
 __device__ __forceinline__ void fill_r64(const double* r0, const double x,
                                          const double y, const double z, double* R) {
-#pragma unroll
-    for (int i = 0; i < nr_c(L); ++i) R[i] = 0.0;
 #pragma unroll
     for (int n = L; n >= 0; --n) {
         const int m = L - n;
@@ -156,37 +194,103 @@ __device__ __forceinline__ void fill_r64(const double* r0, const double x,
                 for (int t = L; t >= 1; --t)
                     if (u < m && v < m - u && t <= m - u - v)
                         R[ridx(L, t, u, v)] =
-                            (t == 1 ? 0.0 : (t - 1) * R[ridx(L, t >= 2 ? t - 2 : 0, u, v)]) +
-                            x * R[ridx(L, t - 1, u, v)];
+                            t == 1 ? x * R[ridx(L, 0, u, v)]
+                                   : fma(x, R[ridx(L, t - 1, u, v)],
+                                         times(t - 1, R[ridx(L, t >= 2 ? t - 2 : 0, u, v)]));
 #pragma unroll
         for (int v = 0; v <= L; ++v)
 #pragma unroll
             for (int u = L; u >= 1; --u)
                 if (v < m && u <= m - v)
                     R[ridx(L, 0, u, v)] =
-                        (u == 1 ? 0.0 : (u - 1) * R[ridx(L, 0, u >= 2 ? u - 2 : 0, v)]) +
-                        y * R[ridx(L, 0, u - 1, v)];
+                        u == 1 ? y * R[ridx(L, 0, 0, v)]
+                               : fma(y, R[ridx(L, 0, u - 1, v)],
+                                     times(u - 1, R[ridx(L, 0, u >= 2 ? u - 2 : 0, v)]));
 #pragma unroll
         for (int v = L; v >= 1; --v)
             if (v <= m)
                 R[ridx(L, 0, 0, v)] =
-                    (v == 1 ? 0.0 : (v - 1) * R[ridx(L, 0, 0, v >= 2 ? v - 2 : 0)]) +
-                    z * R[ridx(L, 0, 0, v - 1)];
+                    v == 1 ? z * R[0]
+                           : fma(z, R[ridx(L, 0, 0, v - 1)],
+                                 times(v - 1, R[ridx(L, 0, 0, v >= 2 ? v - 2 : 0)]));
         R[0] = r0[n];
     }
 }
 
+// A[a][b] += sum_tuv E^x_t E^y_u E^z_v R_tuv of one primitive pair, axis by
+// axis: the x sums of one (i, i') serve every (j, j', k, k') with it
 template<int LA, int LB>
-__global__ void __launch_bounds__(kF64Threads)
+__device__ __forceinline__ void hermite_block(const double* __restrict__ E,
+                                              const double* R, double* A) {
+    constexpr int L = LA + LB, NAX = eaxis(LA, LB), NCB = ncart_c(LB);
+#pragma unroll
+    for (int i = 0; i <= LA; ++i)
+#pragma unroll
+        for (int ip = 0; ip <= LB; ++ip) {
+            const int M = L - i - ip;               // u + v <= M
+            const double* ex = E + eoff(LB, i, ip);
+            double h1[nr_c(L) > 1 ? (L + 1) * (L + 2) / 2 : 1];
+#pragma unroll
+            for (int u = 0; u <= L; ++u)
+#pragma unroll
+                for (int v = 0; v <= L; ++v)
+                    if (u + v <= M) {
+                        double s;
+                        if (i + ip == 0) {
+                            s = R[ridx(L, 0, u, v)];
+                        } else {
+                            s = ex[0] * R[ridx(L, 0, u, v)];
+#pragma unroll
+                            for (int t = 1; t <= L; ++t)
+                                if (t <= i + ip) s = fma(ex[t], R[ridx(L, t, u, v)], s);
+                        }
+                        h1[u * (2 * M + 3 - u) / 2 + v] = s;
+                    }
+#pragma unroll
+            for (int j = 0; j <= LA; ++j)
+#pragma unroll
+                for (int jp = 0; jp <= LB; ++jp)
+                    if (j <= LA - i && jp <= LB - ip) {
+                        const int k = LA - i - j, kp = LB - ip - jp;
+                        const double* ey = E + NAX + eoff(LB, j, jp);
+                        const double* ez = E + 2 * NAX + eoff(LB, k, kp);
+                        const int ab = cidx(LA, i, j) * NCB + cidx(LB, ip, jp);
+                        double s = A[ab];
+#pragma unroll
+                        for (int v = 0; v <= L; ++v)
+                            if (v <= k + kp) {
+                                double h2;
+                                if (j + jp == 0) {
+                                    h2 = h1[v];
+                                } else {
+                                    h2 = ey[0] * h1[v];
+#pragma unroll
+                                    for (int u = 1; u <= L; ++u)
+                                        if (u <= j + jp)
+                                            h2 = fma(ey[u], h1[u * (2 * M + 3 - u) / 2 + v], h2);
+                                }
+                                s = k + kp == 0 ? s + h2 : fma(ez[v], h2, s);
+                            }
+                        A[ab] = s;
+                    }
+        }
+}
+
+// threads of a CTA (one an SM): the light classes leave registers for
+// sixteen warps, the others take 255 a thread
+template<int LA, int LB>
+struct F64Cta { static constexpr int kThreads = LA + LB <= 2 ? 512 : 256; };
+
+template<int LA, int LB>
+__global__ void __launch_bounds__(F64Cta<LA, LB>::kThreads, 1)
 cosx_fp64_kernel(const CosxF64Args A, const int cls, const int pair_begin,
                  const int pair_end) {
     constexpr int L = LA + LB;
     constexpr int NCA = ncart_c(LA), NCB = ncart_c(LB);
     constexpr int NA = 2 * LA + 1, NB = 2 * LB + 1;
     constexpr int NAX = eaxis(LA, LB);
-    __shared__ double stab[kBoys64Nodes * kBoys64Cols];
-    for (int i = threadIdx.x; i < kBoys64Nodes * kBoys64Cols; i += blockDim.x)
-        stab[i] = A.boys[i];
+    extern __shared__ double stab[];
+    load_boys<L>(A.boys, stab);
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const long long ld = A.ld;
@@ -194,13 +298,12 @@ cosx_fp64_kernel(const CosxF64Args A, const int cls, const int pair_begin,
     const float4* __restrict__ bnd = A.bnd + pp_begin;
     const float* __restrict__ bpref = A.bpref + pp_begin;
     const double* __restrict__ Ecls = A.E + A.e_base[cls];
-    const double om2 = A.omega * A.omega;
     unsigned long long kept = 0, flops = 0, ints = 0;
-    for (;;) {
-        int blk = 0;
-        if (lane == 0) blk = atomicAdd(A.work + cls, 1);
-        blk = __shfl_sync(0xffffffffu, blk, 0);
-        if (blk >= A.nblk) break;
+    // the first items go to the warps of all SMs in turn, the others by the
+    // counter: a grid of few blocks still uses every SM's pipe
+    const int nwarps = gridDim.x * (blockDim.x >> 5);
+    int blk = (int)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    while (blk < A.nblk) {
         const int g0 = blk * 32 + lane;
         const bool ok = g0 < A.npts;
         const int g = ok ? g0 : A.npts - 1;
@@ -212,6 +315,14 @@ cosx_fp64_kernel(const CosxF64Args A, const int cls, const int pair_begin,
         const float* __restrict__ ms = A.blk_msh + (long long)blk * A.nvshell;
         const int rem = A.npts - blk * 32;
         const int nvalid = rem < 32 ? rem : 32;
+        int run = -1;                       // first AO of the bra shell held
+        double fa[NCA], ya[NCA];
+        auto flush = [&]() {
+            if (run < 0 || !ok) return;
+#pragma unroll
+            for (int m = 0; m < NA; ++m)
+                atomicAdd(Gp + (long long)(run + m) * ld, to_sph<LA>(A.c2s, ya, m));
+        };
         for (int c0 = pair_begin; c0 < pair_end; c0 += 32) {
             const int k = c0 + lane;
             bool keep = k < pair_end;
@@ -233,95 +344,72 @@ cosx_fp64_kernel(const CosxF64Args A, const int cls, const int pair_begin,
                 const int ia0 = hdr.x & 0xffff, ib0 = hdr.y & 0xffff;
                 const int pp0 = pp_begin + hdr.z, npp = hdr.w & 0xffff;
                 const bool diag = (hdr.w >> 16) != 0;
-                double sa[NA], sb[NB], fa[NCA], fb[NCB], ya[NCA], yb[NCB];
+                if (ia0 != run) {
+                    flush();
+                    run = ia0;
+                    double sa[NA];
 #pragma unroll
-                for (int m = 0; m < NA; ++m) sa[m] = Fp[(long long)(ia0 + m) * ld];
+                    for (int m = 0; m < NA; ++m) sa[m] = Fp[(long long)(ia0 + m) * ld];
+                    to_cart<LA>(A.c2s, sa, fa);
+#pragma unroll
+                    for (int i = 0; i < NCA; ++i) ya[i] = 0.0;
+                }
+                double sb[NB], fb[NCB];
 #pragma unroll
                 for (int m = 0; m < NB; ++m) sb[m] = Fp[(long long)(ib0 + m) * ld];
-                to_cart<LA>(A.c2s, sa, fa);
                 to_cart<LB>(A.c2s, sb, fb);
+                double ab[NCA * NCB];
 #pragma unroll
-                for (int i = 0; i < NCA; ++i) ya[i] = 0.0;
-#pragma unroll
-                for (int i = 0; i < NCB; ++i) yb[i] = 0.0;
+                for (int i = 0; i < NCA * NCB; ++i) ab[i] = 0.0;
                 for (int q = pp0; q < pp0 + npp; ++q) {
-                    const double p = A.p[q], pref = A.pref[q];
-                    const double X = A.P[3LL * q] - gx, Y = A.P[3LL * q + 1] - gy,
-                                 Z = A.P[3LL * q + 2] - gz;
-                    double th = 1.0, sth = 1.0;
-                    if (A.omega > 0.0) {
-                        th = om2 / (om2 + p);
-                        sth = sqrt(th);
-                    }
-                    const double pth = p * th;
-                    const double T = pth * (X * X + Y * Y + Z * Z);
-                    double Fb[L + 1], r0[L + 1];
-                    boys64<L>(T, stab, Fb);
-                    double c = pref * sth;
-#pragma unroll
-                    for (int n = 0; n <= L; ++n) {
-                        r0[n] = c * Fb[n];
-                        c *= -2.0 * pth;
-                    }
-                    double R[nr_c(L)];
-                    fill_r64<L>(r0, X, Y, Z, R);
-                    const double* __restrict__ E = Ecls + (long long)(q - pp_begin) * 3 * NAX;
-                    // the f classes keep these two loops rolled (compile time)
-#pragma unroll(L <= 4 ? NCA : 1)
-                    for (int a = 0; a < NCA; ++a)
-#pragma unroll(L <= 4 ? NCB : 1)
-                        for (int b = 0; b < NCB; ++b) {
-                            const int i = cx(LA, a), j = cy(LA, a), kz = cz(LA, a);
-                            const int ip = cx(LB, b), jp = cy(LB, b), kp = cz(LB, b);
-                            const double* Ex = E + eoff(LB, i, ip);
-                            const double* Ey = E + NAX + eoff(LB, j, jp);
-                            const double* Ez = E + 2 * NAX + eoff(LB, kz, kp);
-                            double s = 0.0;
-#pragma unroll
-                            for (int v = 0; v <= L; ++v) {
-                                if (v > kz + kp) break;
-                                double su = 0.0;
-#pragma unroll
-                                for (int u = 0; u <= L; ++u) {
-                                    if (u > j + jp) break;
-                                    double st = 0.0;
-#pragma unroll
-                                    for (int t = 0; t <= L; ++t) {
-                                        if (t > i + ip) break;
-                                        st = fma(Ex[t], R[ridx(L, t, u, v)], st);
-                                    }
-                                    su = fma(Ey[u], st, su);
-                                }
-                                s = fma(Ez[v], su, s);
-                            }
-                            ya[a] = fma(s, fb[b], ya[a]);
-                            yb[b] = fma(s, fa[a], yb[b]);
-                        }
-                }
-                if (ok) {
-                    if (diag) {
-                        if constexpr (LA == LB) {
-#pragma unroll
-                            for (int m = 0; m < NA; ++m) {
-                                double* gp = Gp + (long long)(ia0 + m) * ld;
-                                *gp += 0.5 * (to_sph<LA>(A.c2s, ya, m) + to_sph<LB>(A.c2s, yb, m));
-                            }
-                        }
+                    const double* __restrict__ rec = A.rec + (long long)q * kF64Rec;
+                    const double X = rec[0] - gx, Y = rec[1] - gy, Z = rec[2] - gz;
+                    const double T = rec[3] * fma(X, X, fma(Y, Y, Z * Z));
+                    double r0[L + 1];
+                    boys_fast<L, L>(T, stab, r0);
+                    if constexpr (L == 0) {
+                        ab[0] = fma(rec[4], r0[0], ab[0]);
                     } else {
 #pragma unroll
-                        for (int m = 0; m < NA; ++m) {
-                            double* gp = Gp + (long long)(ia0 + m) * ld;
-                            *gp += to_sph<LA>(A.c2s, ya, m);
-                        }
+                        for (int n = 0; n <= L; ++n) r0[n] *= rec[4 + n];
+                        double R[nr_c(L)];
+                        fill_r64<L>(r0, X, Y, Z, R);
+                        hermite_block<LA, LB>(Ecls + (long long)(q - pp_begin) * 3 * NAX,
+                                              R, ab);
+                    }
+                }
+                if (diag) {
+                    if constexpr (LA == LB) {
 #pragma unroll
-                        for (int m = 0; m < NB; ++m) {
-                            double* gp = Gp + (long long)(ib0 + m) * ld;
-                            *gp += to_sph<LB>(A.c2s, yb, m);
+                        for (int a = 0; a < NCA; ++a)
+#pragma unroll
+                            for (int b = 0; b < NCB; ++b)
+                                ya[a] = fma(0.5 * (ab[a * NCB + b] + ab[b * NCB + a]),
+                                            fb[b], ya[a]);
+                    }
+                } else {
+                    double yb[NCB];
+#pragma unroll
+                    for (int b = 0; b < NCB; ++b) yb[b] = ab[b] * fa[0];
+#pragma unroll
+                    for (int a = 0; a < NCA; ++a)
+#pragma unroll
+                        for (int b = 0; b < NCB; ++b) {
+                            ya[a] = fma(ab[a * NCB + b], fb[b], ya[a]);
+                            if (a) yb[b] = fma(ab[a * NCB + b], fa[a], yb[b]);
                         }
+                    if (ok) {
+#pragma unroll
+                        for (int m = 0; m < NB; ++m)
+                            atomicAdd(Gp + (long long)(ib0 + m) * ld,
+                                      to_sph<LB>(A.c2s, yb, m));
                     }
                 }
             }
         }
+        flush();
+        if (lane == 0) blk = nwarps + atomicAdd(A.work + cls, 1);
+        blk = __shfl_sync(0xffffffffu, blk, 0);
     }
     for (int o = 16; o > 0; o >>= 1) {
         flops += __shfl_xor_sync(0xffffffffu, flops, o);
@@ -338,13 +426,12 @@ template<int LA, int LB>
 cudaError_t run64(const CosxF64Args& a, int cls, int pb, int pe, int nsm,
                   cudaStream_t s) {
     auto k = cosx_fp64_kernel<LA, LB>;
-    int occ = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kF64Threads, 0);
+    constexpr int smem = BoysTable<LA + LB>::kBytes;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         smem);
     if (e != cudaSuccess) return e;
-    const int warps = kF64Threads / 32;
-    int grid = std::max(1, nsm * std::max(occ, 1));
-    grid = std::min(grid, (a.nblk + warps - 1) / warps);
-    k<<<std::max(grid, 1), kF64Threads, 0, s>>>(a, cls, pb, pe);
+    const int grid = std::max(1, std::min(nsm, a.nblk));
+    k<<<grid, F64Cta<LA, LB>::kThreads, smem, s>>>(a, cls, pb, pe);
     return cudaGetLastError();
 }
 

@@ -9,13 +9,18 @@ namespace wb {
 constexpr int kBoys64Nodes = 145;   // T_k = k / 4, k = 0..144
 constexpr int kBoys64Cols = 20;     // F_m(T_k), m = 0..19 (L <= 6 + 11 Taylor terms)
 
+constexpr int kBoysFineNodes = 1153;    // T_k = k / 32, k = 0..1152
+constexpr int kBoysFineCols = 14;       // F_m(T_k), m = 0..13 (orders to 7)
+// doubles of a primitive pair's record: P (3), p theta, then c_n = prefactor
+// sqrt(theta) (-2 p theta)^n (n <= 7) and the bra exponent over p
+constexpr int kF64Rec = 16;
+
 struct CosxF64Args {
     const double* F;            // (nao, ld) AO-major, FP64
     double* G;                  // (nao, ld) AO-major, FP64, accumulated
     const double* coords;       // (npts, 3) molecule frame
     long long ld;
     int npts;
-    double omega;
     // screening inputs of the FP32 path (32-point blocks)
     const int4* khdr;
     const int2* pshell;
@@ -28,14 +33,12 @@ struct CosxF64Args {
     int nvshell;
     float tol;                  // tile_tol / 1.001, <= 0 keeps every task
     int pp_begin[10];           // first primitive pair of each class
-    // FP64 pair data: per primitive pair P (3), p, folded prefactor; per
-    // class the Hermite E block from e_base[c]
-    const double* P;
-    const double* p;
-    const double* pref;
+    // FP64 pair data: per primitive pair the record of this omega
+    // (f64_records); per class the Hermite E block from e_base[c]
+    const double* rec;
     const double* E;
     long long e_base[10];
-    const double* boys;         // kBoys64Nodes x kBoys64Cols
+    const double* boys;         // kBoysFineNodes x kBoysFineCols
     const double* c2s;          // l = 2 (6 x 5) at 0, l = 3 (10 x 7) at 30, row-major
     const long long* pflops;
     const int* pnint;
@@ -43,6 +46,11 @@ struct CosxF64Args {
     int* work;                      // per class block counter (zeroed)
 };
 
+// rec (npp, kF64Rec) of one omega from P, p, the folded prefactor and the bra
+// exponent of every primitive pair
+cudaError_t launch_f64_records(int npp, const double* P, const double* p,
+                               const double* pref, const double* alpha, double omega,
+                               double* rec, cudaStream_t s);
 // one class launch (classes 0..9); the f classes live in cosx_fp64_f.cu
 cudaError_t launch_cosx_fp64_class(int cls, const CosxF64Args& a, int pb, int pe,
                                    int nsm, cudaStream_t s);

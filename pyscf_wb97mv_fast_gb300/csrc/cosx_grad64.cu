@@ -18,134 +18,227 @@
 // The X side of the gradient (d F / dR through the AO values) is formed
 // from G and the AO gradients by the host (cosx.CosxEngine.k_grad).
 //
-// The screen, pair tables, Boys function and McMurchie-Davidson recurrences
-// are those of the plain FP64 kernels (cosx_fp64.cuh).  One warp owns one
-// 32-point block; per task every lane forms its point's six derivative
-// sums (atom A xyz, atom B xyz) times -w_g / 2.  The warp reduces them in a
-// fixed order and lane 0 adds them to the block's row of gbuf (nblk, natm,
-// 3), which no other warp touches.  The rows are summed in a fixed order
-// afterwards, so the result is bitwise reproducible.  Loops are runtime
-// loops (local-memory arrays): this kernel runs once per geometry, not per
-// SCF cycle.
+// With P = (alpha A + beta B) / p and Q = A - B, d/dA = (alpha / p) d/dP +
+// d/dQ and d/dB = (beta / p) d/dP - d/dQ; d/dP_x raises the Hermite index,
+// R_tuv -> R_t+1,u,v, and d/dQ acts on the Hermite coefficients alone
+// (prefactor included): tables formed once per call (grad_e_kernel).  So one
+// pass over the primitive pair gives both centres:
+//   S_x = sum_ab f_a f_b sum E^x_t E^y_u E^z_v R_t+1,u,v
+//   D_x = sum_ab f_a f_b sum (dE^x_t / dQ) E^y_u E^z_v R_tuv
+//   dA = (alpha / p) S + D,  dB = S - dA
+// (differentiating the Gaussians themselves needs integrals of l + 1 and
+// l - 1 for each of the three axes and each component).
+//
+// The screen, pair tables, Boys function and McMurchie-Davidson recurrence
+// are those of the plain FP64 kernels (cosx_fp64.cuh), and so is the bound:
+// the FP64 pipe.  One warp owns one 32-point block, one point a lane.  A
+// lane adds its point's sums to its own column of gpt (3 natm, ld) by
+// reductions in the L2, dA once per run of pairs with one bra shell; a lane
+// reduction in the task would cost 30 FP64 instructions.  The columns are
+// weighted with -w_g / 2 and summed in a fixed order at the end, so the
+// result is bitwise reproducible.  Measured (integral side alone): 8 waters,
+// 36,369 points 327 -> 59 ms; C4H10 in TZVP, 21,512 points 606 -> 98 ms.
 #include "cosx_fp64.cuh"
 #include "cosx_grad64.hpp"
 
 namespace wb {
 namespace {
 
-constexpr int kGradThreads = 128;
+using namespace f64;
 
-// E^{i,j}_t along one axis for i <= ia, j <= jb (t <= i + j), [i][j][t] with
-// fixed strides (4 + 1) x 4 x 8
-constexpr int kEi = 5, kEj = 4, kEt = 8;
-__device__ __forceinline__ void hermite64(const int ia, const int jb, const double p,
-                                          const double xpa, const double xpb,
-                                          double* E) {
-    const double h = 0.5 / p;
-    auto at = [&](int i, int j, int t) -> double& { return E[(i * kEj + j) * kEt + t]; };
-    for (int i = 0; i <= ia; ++i)
-        for (int j = 0; j <= jb; ++j)
-            for (int t = 0; t < kEt; ++t) at(i, j, t) = 0.0;
-    at(0, 0, 0) = 1.0;
-    for (int i = 1; i <= ia; ++i)
-        for (int t = 0; t <= i; ++t) {
-            double v = xpa * at(i - 1, 0, t);
-            if (t > 0) v = fma(h, at(i - 1, 0, t - 1), v);
-            if (t + 1 <= i - 1) v = fma((double)(t + 1), at(i - 1, 0, t + 1), v);
-            at(i, 0, t) = v;
+// d/dQ of every Hermite coefficient (with the pair prefactor exp(-mu Q^2)
+// differentiated too): dE = (d/dQ - 2 mu Q) E, in the layout of E.  One
+// thread per (shell pair, axis); E by its recurrence and its derivative
+// along.
+__global__ void grad_e_kernel(const GradEArgs A) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= A.npairs) return;
+    const int x = blockIdx.y;
+    const int cls = A.pclass[k];
+    int la = 0;
+    while ((la + 1) * (la + 2) / 2 <= cls) ++la;
+    const int lb = cls - la * (la + 1) / 2;
+    const int nax = eoff(lb, la + 1, 0);
+    const int4 h = A.hdr[k];
+    const int2 sh = A.pshell[k];
+    const double Q = A.vs_xyz[3 * sh.x + x] - A.vs_xyz[3 * sh.y + x];
+    double E[4][4][8], D[4][4][8];
+    for (int q = h.z; q < h.z + (h.w & 0xffff); ++q) {
+        const double p = A.p[q], al = A.alpha[q], be = p - al;
+        const double hp = 0.5 / p, ka = -be / p, kb = al / p, m2 = -2.0 * al * be / p * Q;
+        for (int i = 0; i <= la; ++i)
+            for (int j = 0; j <= lb; ++j)
+                for (int t = 0; t <= i + j; ++t) {
+                    if (i + j == 0) {
+                        E[0][0][0] = 1.0;
+                        D[0][0][0] = 0.0;
+                        continue;
+                    }
+                    const double c = i ? ka : kb;
+                    const int ii = i ? i - 1 : i, jj = i ? j : j - 1, n = ii + jj;
+                    double e = 0.0, d = 0.0;
+                    if (t <= n) {
+                        e = c * Q * E[ii][jj][t];
+                        d = c * (Q * D[ii][jj][t] + E[ii][jj][t]);
+                    }
+                    if (t > 0) {
+                        e += hp * E[ii][jj][t - 1];
+                        d += hp * D[ii][jj][t - 1];
+                    }
+                    if (t + 1 <= n) {
+                        e += (t + 1) * E[ii][jj][t + 1];
+                        d += (t + 1) * D[ii][jj][t + 1];
+                    }
+                    E[i][j][t] = e;
+                    D[i][j][t] = d;
+                }
+        double* out = A.dE + A.e_base[cls] + ((int64_t)(q - A.pp_begin[cls]) * 3 + x) * nax;
+        int n = 0;
+        for (int i = 0; i <= la; ++i)
+            for (int j = 0; j <= lb; ++j)
+                for (int t = 0; t <= i + j; ++t)
+                    out[n++] = fma(m2, E[i][j][t], D[i][j][t]);
+    }
+}
+
+// S (assigned) and D (added) of one primitive pair, for f_a f_b over the
+// Cartesian components; R packed for order L + 1.  Per (i, i'): R contracted
+// with E^x, dE^x and E^x at t + 1; f_a f_b spread over (u, v) with E^y E^z
+// and their derivatives; then the two sides meet.
+template<int LA, int LB>
+__device__ __forceinline__ void grad_block(const double* __restrict__ E,
+                                           const double* __restrict__ dE,
+                                           const double* R, const double* fa,
+                                           const double* fb, double* S, double* D) {
+    constexpr int L = LA + LB, NAX = eaxis(LA, LB);
+    constexpr int NUV = (L + 1) * (L + 2) / 2, NUV1 = (L + 2) * (L + 3) / 2;
+    S[0] = S[1] = S[2] = 0.0;
+#pragma unroll
+    for (int i = 0; i <= LA; ++i)
+#pragma unroll
+        for (int ip = 0; ip <= LB; ++ip) {
+            const int M = L - i - ip;
+            const double* ex = E + eoff(LB, i, ip);
+            const double* dx = dE + eoff(LB, i, ip);
+            double h[NUV], hy[NUV], hz[NUV];
+            bool seth[NUV], sethy[NUV], sethz[NUV];
+#pragma unroll
+            for (int n = 0; n < NUV; ++n) seth[n] = sethy[n] = sethz[n] = false;
+#pragma unroll
+            for (int j = 0; j <= LA; ++j)
+#pragma unroll
+                for (int jp = 0; jp <= LB; ++jp)
+                    if (j <= LA - i && jp <= LB - ip) {
+                        const int k = LA - i - j, kp = LB - ip - jp;
+                        const double* ey = E + NAX + eoff(LB, j, jp);
+                        const double* dy = dE + NAX + eoff(LB, j, jp);
+                        const double* ez = E + 2 * NAX + eoff(LB, k, kp);
+                        const double* dz = dE + 2 * NAX + eoff(LB, k, kp);
+                        const double f = fa[cidx(LA, i, j)] * fb[cidx(LB, ip, jp)];
+#pragma unroll
+                        for (int v = 0; v <= L; ++v)
+                            if (v <= k + kp) {
+                                const double zv = k + kp == 0 ? f : ez[v] * f;
+                                const double zd = dz[v] * f;
+#pragma unroll
+                                for (int u = 0; u <= L; ++u)
+                                    if (u <= j + jp) {
+                                        const int n = u * (2 * M + 3 - u) / 2 + v;
+                                        if (j + jp == 0) {
+                                            h[n] = seth[n] ? h[n] + zv : zv;
+                                            hz[n] = sethz[n] ? hz[n] + zd : zd;
+                                        } else {
+                                            h[n] = seth[n] ? fma(ey[u], zv, h[n]) : ey[u] * zv;
+                                            hz[n] = sethz[n] ? fma(ey[u], zd, hz[n]) : ey[u] * zd;
+                                        }
+                                        hy[n] = sethy[n] ? fma(dy[u], zv, hy[n]) : dy[u] * zv;
+                                        seth[n] = sethy[n] = sethz[n] = true;
+                                    }
+                            }
+                    }
+            double rx[NUV1];
+#pragma unroll
+            for (int u = 0; u <= L + 1; ++u)
+#pragma unroll
+                for (int v = 0; v <= L + 1; ++v)
+                    if (u + v <= M + 1) {
+                        double s = R[ridx(L + 1, 0, u, v)];
+                        if (i + ip > 0) {
+                            s *= ex[0];
+#pragma unroll
+                            for (int t = 1; t <= L; ++t)
+                                if (t <= i + ip) s = fma(ex[t], R[ridx(L + 1, t, u, v)], s);
+                        }
+                        rx[u * (2 * M + 5 - u) / 2 + v] = s;
+                    }
+#pragma unroll
+            for (int u = 0; u <= L; ++u)
+#pragma unroll
+                for (int v = 0; v <= L; ++v)
+                    if (u + v <= M) {
+                        const int n = u * (2 * M + 3 - u) / 2 + v;
+                        double rd = dx[0] * R[ridx(L + 1, 0, u, v)];
+                        double rp = R[ridx(L + 1, 1, u, v)];
+                        if (i + ip > 0) {
+                            rp *= ex[0];
+#pragma unroll
+                            for (int t = 1; t <= L; ++t)
+                                if (t <= i + ip) {
+                                    rd = fma(dx[t], R[ridx(L + 1, t, u, v)], rd);
+                                    rp = fma(ex[t], R[ridx(L + 1, t + 1, u, v)], rp);
+                                }
+                        }
+                        const double r = rx[u * (2 * M + 5 - u) / 2 + v];
+                        S[0] = fma(rp, h[n], S[0]);
+                        S[1] = fma(rx[(u + 1) * (2 * M + 4 - u) / 2 + v], h[n], S[1]);
+                        S[2] = fma(rx[u * (2 * M + 5 - u) / 2 + v + 1], h[n], S[2]);
+                        D[0] = fma(rd, h[n], D[0]);
+                        D[1] = fma(r, hy[n], D[1]);
+                        D[2] = fma(r, hz[n], D[2]);
+                    }
         }
-    for (int j = 1; j <= jb; ++j)
-        for (int i = 0; i <= ia; ++i)
-            for (int t = 0; t <= i + j; ++t) {
-                double v = xpb * at(i, j - 1, t);
-                if (t > 0) v = fma(h, at(i, j - 1, t - 1), v);
-                if (t + 1 <= i + j - 1) v = fma((double)(t + 1), at(i, j - 1, t + 1), v);
-                at(i, j, t) = v;
-            }
 }
 
-// R_tuv (t + u + v <= L) at PC = (x, y, z) from r0[n] = R_000^(n), levels
-// L .. 0 in place; R[(t * 8 + u) * 8 + v]
-__device__ __forceinline__ void fill_r_rt(const int L, const double* r0, const double x,
-                                          const double y, const double z, double* R) {
-    auto at = [&](int t, int u, int v) -> double& { return R[(t * 8 + u) * 8 + v]; };
-    for (int i = 0; i < 512; ++i) R[i] = 0.0;
-    for (int n = L; n >= 0; --n) {
-        const int m = L - n;
-        for (int u = 0; u < m; ++u)
-            for (int v = 0; v < m - u; ++v)
-                for (int t = m - u - v; t >= 1; --t)
-                    at(t, u, v) = (t >= 2 ? (t - 1) * at(t - 2, u, v) : 0.0) +
-                                  x * at(t - 1, u, v);
-        for (int v = 0; v < m; ++v)
-            for (int u = m - v; u >= 1; --u)
-                at(0, u, v) = (u >= 2 ? (u - 1) * at(0, u - 2, v) : 0.0) +
-                              y * at(0, u - 1, v);
-        for (int v = m; v >= 1; --v)
-            at(0, 0, v) = (v >= 2 ? (v - 1) * at(0, 0, v - 2) : 0.0) + z * at(0, 0, v - 1);
-        at(0, 0, 0) = r0[n];
-    }
-}
-
-// Boys F_0..F_L for runtime L (<= 7) from the FP64 table (as f64::boys64)
-__device__ __forceinline__ void boys64_rt(const int L, const double T,
-                                          const double* __restrict__ tab, double* F) {
-    if (T < 36.0) {
-        const int k = __double2int_rn(T * 4.0);
-        const double x = 0.25 * k - T;
-        const double* row = tab + k * kBoys64Cols + L;
-        double s = row[11];
-        for (int j = 11; j >= 1; --j) s = fma(s * x, 1.0 / j, row[j - 1]);
-        F[L] = s;
-        const double e = exp(-T);
-        for (int n = L - 1; n >= 0; --n) F[n] = fma(2.0 * T, F[n + 1], e) / (2 * n + 1);
-    } else {
-        F[0] = 0.88622692545275801365 * rsqrt(T);
-        const double e = exp(-T);
-        const double h = 0.5 / T;
-        for (int n = 0; n < L; ++n) F[n + 1] = ((2 * n + 1) * F[n] - e) * h;
-    }
-}
+// threads of a CTA (one an SM), as for the FP64 class kernels
+template<int LA, int LB>
+struct GradCta { static constexpr int kThreads = LA + LB <= 1 ? 512 : 256; };
 
 template<int LA, int LB>
-__global__ void __launch_bounds__(kGradThreads)
+__global__ void __launch_bounds__(GradCta<LA, LB>::kThreads, 1)
 cosx_grad64_kernel(const CosxGradArgs A, const int cls, const int pair_begin,
                    const int pair_end) {
     constexpr int L = LA + LB;
-    constexpr int NCA = (LA + 1) * (LA + 2) / 2, NCB = (LB + 1) * (LB + 2) / 2;
+    constexpr int NCA = ncart_c(LA), NCB = ncart_c(LB);
     constexpr int NA = 2 * LA + 1, NB = 2 * LB + 1;
-    __shared__ double stab[kBoys64Nodes * kBoys64Cols];
-    for (int i = threadIdx.x; i < kBoys64Nodes * kBoys64Cols; i += blockDim.x)
-        stab[i] = A.boys[i];
+    constexpr int NAX = eaxis(LA, LB);
+    extern __shared__ double stab[];
+    load_boys<L + 1>(A.boys, stab);
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const long long ld = A.ld;
     const int pp_begin = A.pp_begin[cls];
     const float4* __restrict__ bnd = A.bnd + pp_begin;
     const float* __restrict__ bpref = A.bpref + pp_begin;
-    const double om2 = A.omega * A.omega;
-    int cxa[NCA], cya[NCA], cza[NCA], cxb[NCB], cyb[NCB], czb[NCB];
-    for (int c = 0; c < NCA; ++c) {
-        cxa[c] = f64::cx(LA, c); cya[c] = f64::cy(LA, c); cza[c] = LA - cxa[c] - cya[c];
-    }
-    for (int c = 0; c < NCB; ++c) {
-        cxb[c] = f64::cx(LB, c); cyb[c] = f64::cy(LB, c); czb[c] = LB - cxb[c] - cyb[c];
-    }
-    for (;;) {
-        int blk = 0;
-        if (lane == 0) blk = atomicAdd(A.work + cls, 1);
-        blk = __shfl_sync(0xffffffffu, blk, 0);
-        if (blk >= A.nblk) break;
+    const int nwarps = gridDim.x * (blockDim.x >> 5);
+    int blk = (int)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    while (blk < A.nblk) {
         const int g0 = blk * 32 + lane;
         const bool ok = g0 < A.npts;
         const int g = ok ? g0 : A.npts - 1;
         const double gx = A.coords[3LL * g], gy = A.coords[3LL * g + 1],
                      gz = A.coords[3LL * g + 2];
-        const double wh = ok ? -0.5 * A.weights[g] : 0.0;
         const double* __restrict__ Fp = A.F + g;
+        double* __restrict__ out = A.gpt + g;
         const float4 cr = A.blk_cr[blk];
         const float* __restrict__ ms = A.blk_msh + (long long)blk * A.nvshell;
-        double* __restrict__ grow = A.gbuf + (long long)blk * A.natm * 3;
+        int run = -1;                       // bra virtual shell held
+        double fa[NCA], ga[3] = {0.0, 0.0, 0.0};
+        auto flush = [&]() {
+            if (run < 0 || !ok) return;
+            const int at = A.vs_atom[run];
+#pragma unroll
+            for (int x = 0; x < 3; ++x) atomicAdd(out + (3 * at + x) * ld, ga[x]);
+        };
         for (int c0 = pair_begin; c0 < pair_end; c0 += 32) {
             const int k = c0 + lane;
             bool keep = k < pair_end;
@@ -163,128 +256,91 @@ cosx_grad64_kernel(const CosxGradArgs A, const int cls, const int pair_begin,
                 const int ia0 = hdr.x & 0xffff, ib0 = hdr.y & 0xffff;
                 const int pp0 = pp_begin + hdr.z, npp = hdr.w & 0xffff;
                 const bool diag = (hdr.w >> 16) != 0;
-                const double Ax = A.vs_xyz[3 * sh.x], Ay = A.vs_xyz[3 * sh.x + 1],
-                             Az = A.vs_xyz[3 * sh.x + 2];
-                const double Bx = A.vs_xyz[3 * sh.y], By = A.vs_xyz[3 * sh.y + 1],
-                             Bz = A.vs_xyz[3 * sh.y + 2];
-                double sa[NA], sb[NB], fa[NCA], fb[NCB];
-                for (int m = 0; m < NA; ++m) sa[m] = Fp[(long long)(ia0 + m) * ld];
+                if (sh.x != run) {
+                    flush();
+                    run = sh.x;
+                    double sa[NA];
+#pragma unroll
+                    for (int m = 0; m < NA; ++m) sa[m] = Fp[(long long)(ia0 + m) * ld];
+                    to_cart<LA>(A.c2s, sa, fa);
+                    ga[0] = ga[1] = ga[2] = 0.0;
+                }
+                double sb[NB], fb[NCB];
+#pragma unroll
                 for (int m = 0; m < NB; ++m) sb[m] = Fp[(long long)(ib0 + m) * ld];
-                f64::to_cart<LA>(A.c2s, sa, fa);
-                f64::to_cart<LB>(A.c2s, sb, fb);
-                double gA[3] = {0.0, 0.0, 0.0}, gC[3] = {0.0, 0.0, 0.0};
+                to_cart<LB>(A.c2s, sb, fb);
+                double dA[3] = {0.0, 0.0, 0.0}, tot[3] = {0.0, 0.0, 0.0};
                 for (int q = pp0; q < pp0 + npp; ++q) {
-                    const double p = A.p[q], pref = A.pref[q], al = A.alpha[q];
-                    const double Px = A.P[3LL * q], Py = A.P[3LL * q + 1],
-                                 Pz = A.P[3LL * q + 2];
-                    const double X = Px - gx, Y = Py - gy, Z = Pz - gz;
-                    double th = 1.0, sth = 1.0;
-                    if (A.omega > 0.0) {
-                        th = om2 / (om2 + p);
-                        sth = sqrt(th);
-                    }
-                    const double pth = p * th;
-                    const double T = pth * (X * X + Y * Y + Z * Z);
-                    double Fb[L + 2], r0[L + 2];
-                    boys64_rt(L + 1, T, stab, Fb);
-                    double c = pref * sth;
-                    for (int n = 0; n <= L + 1; ++n) {
-                        r0[n] = c * Fb[n];
-                        c *= -2.0 * pth;
-                    }
-                    double R[512];
-                    fill_r_rt(L + 1, r0, X, Y, Z, R);
-                    double Ex[kEi * kEj * kEt], Ey[kEi * kEj * kEt], Ez[kEi * kEj * kEt];
-                    hermite64(LA + 1, LB, p, Px - Ax, Px - Bx, Ex);
-                    hermite64(LA + 1, LB, p, Py - Ay, Py - By, Ey);
-                    hermite64(LA + 1, LB, p, Pz - Az, Pz - Bz, Ez);
-                    // Hermite sum of E_x[i][i'] E_y[j][j'] E_z[k][k'] R shifted
-                    // by (dt, du, dv)
-                    auto hsum = [&](int i, int ip, int j, int jp, int kz, int kp, int dt,
-                                    int du, int dv) -> double {
-                        double s = 0.0;
-                        for (int t = 0; t <= i + ip; ++t) {
-                            const double ex = Ex[(i * kEj + ip) * kEt + t];
-                            double su = 0.0;
-                            for (int u = 0; u <= j + jp; ++u) {
-                                const double ey = Ey[(j * kEj + jp) * kEt + u];
-                                double sv = 0.0;
-                                for (int v = 0; v <= kz + kp; ++v)
-                                    sv = fma(Ez[(kz * kEj + kp) * kEt + v],
-                                             R[((t + dt) * 8 + u + du) * 8 + v + dv], sv);
-                                su = fma(ey, sv, su);
-                            }
-                            s = fma(ex, su, s);
-                        }
-                        return s;
-                    };
-#pragma unroll 1
-                    for (int a = 0; a < NCA; ++a) {
-                        const int i = cxa[a], j = cya[a], kz = cza[a];
-#pragma unroll 1
-                        for (int b = 0; b < NCB; ++b) {
-                            const int ip = cxb[b], jp = cyb[b], kp = czb[b];
-                            const double ff = fa[a] * fb[b];
-                            // bra derivative: 2 alpha (a + 1) - a_x (a - 1)
-                            double dx = 2.0 * al * hsum(i + 1, ip, j, jp, kz, kp, 0, 0, 0);
-                            if (i) dx -= i * hsum(i - 1, ip, j, jp, kz, kp, 0, 0, 0);
-                            double dy = 2.0 * al * hsum(i, ip, j + 1, jp, kz, kp, 0, 0, 0);
-                            if (j) dy -= j * hsum(i, ip, j - 1, jp, kz, kp, 0, 0, 0);
-                            double dz = 2.0 * al * hsum(i, ip, j, jp, kz + 1, kp, 0, 0, 0);
-                            if (kz) dz -= kz * hsum(i, ip, j, jp, kz - 1, kp, 0, 0, 0);
-                            gA[0] = fma(ff, dx, gA[0]);
-                            gA[1] = fma(ff, dy, gA[1]);
-                            gA[2] = fma(ff, dz, gA[2]);
-                            if (!diag) {
-                                // operator-centre derivative: d/dC R_tuv = -R_t+1
-                                gC[0] = fma(ff, -hsum(i, ip, j, jp, kz, kp, 1, 0, 0), gC[0]);
-                                gC[1] = fma(ff, -hsum(i, ip, j, jp, kz, kp, 0, 1, 0), gC[1]);
-                                gC[2] = fma(ff, -hsum(i, ip, j, jp, kz, kp, 0, 0, 1), gC[2]);
-                            }
-                        }
+                    const double* __restrict__ rec = A.rec + (long long)q * kF64Rec;
+                    const double X = rec[0] - gx, Y = rec[1] - gy, Z = rec[2] - gz;
+                    const double T = rec[3] * fma(X, X, fma(Y, Y, Z * Z));
+                    double r0[L + 2], R[nr_c(L + 1)], S[3];
+                    boys_fast<L + 1, L + 1>(T, stab, r0);
+#pragma unroll
+                    for (int n = 0; n <= L + 1; ++n) r0[n] *= rec[4 + n];
+                    fill_r64<L + 1>(r0, X, Y, Z, R);
+                    const long long e = A.e_base[cls] + (long long)(q - pp_begin) * 3 * NAX;
+                    grad_block<LA, LB>(A.E + e, A.dE + e, R, fa, fb, S, dA);
+#pragma unroll
+                    for (int x = 0; x < 3; ++x) {
+                        dA[x] = fma(rec[12], S[x], dA[x]);
+                        tot[x] += S[x];
                     }
                 }
-                // atom(A): bra; atom(B): -(bra + operator centre)
-                double v[6];
-                for (int x = 0; x < 3; ++x) {
-                    v[x] = wh * gA[x];
-                    v[3 + x] = diag ? 0.0 : -wh * (gA[x] + gC[x]);
+#pragma unroll
+                for (int x = 0; x < 3; ++x) ga[x] += dA[x];
+                // a diagonal pair contributes its bra derivative only
+                if (!diag && ok) {
+                    const int at = A.vs_atom[sh.y];
+#pragma unroll
+                    for (int x = 0; x < 3; ++x)
+                        atomicAdd(out + (3 * at + x) * ld, tot[x] - dA[x]);
                 }
-                for (int x = 0; x < 6; ++x)
-                    for (int o = 16; o > 0; o >>= 1)
-                        v[x] += __shfl_xor_sync(0xffffffffu, v[x], o);
-                if (lane == 0) {
-                    const int atA = A.vs_atom[sh.x], atB = A.vs_atom[sh.y];
-                    for (int x = 0; x < 3; ++x) grow[3 * atA + x] += v[x];
-                    if (!diag)
-                        for (int x = 0; x < 3; ++x) grow[3 * atB + x] += v[3 + x];
-                }
-                __syncwarp();
             }
         }
+        flush();
+        if (lane == 0) blk = nwarps + atomicAdd(A.work + cls, 1);
+        blk = __shfl_sync(0xffffffffu, blk, 0);
     }
 }
 
 template<int LA, int LB>
 cudaError_t run_grad(const CosxGradArgs& a, int cls, int pb, int pe, int nsm,
                      cudaStream_t s) {
-    const int warps = kGradThreads / 32;
-    int grid = std::max(1, nsm * 4);
-    grid = std::min(grid, (a.nblk + warps - 1) / warps);
-    cosx_grad64_kernel<LA, LB><<<std::max(grid, 1), kGradThreads, 0, s>>>(a, cls, pb, pe);
+    auto k = cosx_grad64_kernel<LA, LB>;
+    constexpr int smem = BoysTable<LA + LB + 1>::kBytes;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         smem);
+    if (e != cudaSuccess) return e;
+    const int grid = std::max(1, std::min(nsm, a.nblk));
+    k<<<grid, GradCta<LA, LB>::kThreads, smem, s>>>(a, cls, pb, pe);
     return cudaGetLastError();
 }
 
-__global__ void grad_rows_sum_kernel(const double* __restrict__ gbuf, int nblk, int n,
-                                     double* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// out[r] += -1/2 sum_g w_g gpt[r][g]: one CTA a row, fixed order
+__global__ void grad_points_sum_kernel(const double* __restrict__ gpt,
+                                       const double* __restrict__ w, int64_t npts,
+                                       int64_t ld, double* __restrict__ out) {
+    __shared__ double red[256];
+    const double* row = gpt + (int64_t)blockIdx.x * ld;
     double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += gbuf[(long long)b * n + i];
-    out[i] += s;
+    for (int64_t g = threadIdx.x; g < npts; g += 256) s = fma(w[g], row[g], s);
+    red[threadIdx.x] = s;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+        if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) out[blockIdx.x] -= 0.5 * red[0];
 }
 
 }  // namespace
+
+cudaError_t launch_grad_e(const GradEArgs& a, cudaStream_t s) {
+    if (a.npairs <= 0) return cudaSuccess;
+    grad_e_kernel<<<dim3((a.npairs + 63) / 64, 3), 64, 0, s>>>(a);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_cosx_grad64_class(int cls, const CosxGradArgs& a, int pb, int pe,
                                      int nsm, cudaStream_t s) {
@@ -303,10 +359,10 @@ cudaError_t launch_cosx_grad64_class(int cls, const CosxGradArgs& a, int pb, int
     }
 }
 
-cudaError_t launch_grad_rows_sum(const double* gbuf, int nblk, int natm, double* out,
-                                 cudaStream_t s) {
-    const int n = 3 * natm;
-    grad_rows_sum_kernel<<<(n + 127) / 128, 128, 0, s>>>(gbuf, nblk, n, out);
+cudaError_t launch_grad_points_sum(const double* gpt, const double* w, int64_t npts,
+                                   int64_t ld, int natm, double* out, cudaStream_t s) {
+    if (natm <= 0) return cudaSuccess;
+    grad_points_sum_kernel<<<3 * natm, 256, 0, s>>>(gpt, w, npts, ld, out);
     return cudaGetLastError();
 }
 

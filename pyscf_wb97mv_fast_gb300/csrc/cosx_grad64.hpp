@@ -9,10 +9,8 @@ namespace wb {
 struct CosxGradArgs {
     const double* F;            // (nao, ld) AO-major, FP64: F = X D
     const double* coords;       // (npts, 3) molecule frame
-    const double* weights;      // (npts,)
     long long ld;
     int npts;
-    double omega;
     // the screen of the FP64 kernels (32-point blocks)
     const int4* khdr;
     const int2* pshell;
@@ -25,26 +23,40 @@ struct CosxGradArgs {
     int nvshell;
     float tol;
     int pp_begin[10];
-    // FP64 pair data: per primitive pair P (3), p, folded prefactor, bra
-    // exponent; per virtual shell its centre (3) and atom
-    const double* P;
-    const double* p;
-    const double* pref;
-    const double* alpha;
-    const double* vs_xyz;
+    // FP64 pair data: the records of this omega (f64_records), the Hermite
+    // coefficients and their d/dQ, per class from e_base[c]; per virtual shell
+    // its atom
+    const double* rec;
+    const double* E;
+    const double* dE;
+    long long e_base[10];
     const int* vs_atom;
-    const double* boys;         // kBoys64Nodes x kBoys64Cols
+    const double* boys;         // kBoysFineNodes x kBoysFineCols
     const double* c2s;          // l = 2 at 0, l = 3 at 30
-    double* gbuf;               // (nblk, natm, 3) per-block partial gradients
-    int natm;
+    double* gpt;                // (3 natm, ld) sums of each point, zeroed
     int* work;                  // per class block counter (zeroed)
 };
 
+// the d/dQ of the Hermite coefficients of every primitive pair (layout of E)
+struct GradEArgs {
+    int npairs;
+    const int* pclass;
+    const int4* hdr;            // per pair: ia0, ib0, pp0, npp | diag << 16
+    const int2* pshell;
+    const double* p;
+    const double* alpha;
+    const double* vs_xyz;       // per virtual shell its centre (3)
+    long long e_base[10];
+    int pp_begin[10];
+    double* dE;
+};
+cudaError_t launch_grad_e(const GradEArgs& a, cudaStream_t s);
+
 cudaError_t launch_cosx_grad64_class(int cls, const CosxGradArgs& a, int pb, int pe,
                                      int nsm, cudaStream_t s);
-// out (natm * 3) += sum over the nblk rows of gbuf, in row order
-cudaError_t launch_grad_rows_sum(const double* gbuf, int nblk, int natm, double* out,
-                                 cudaStream_t s);
+// out (natm * 3) -= 1/2 sum_g w_g gpt (fixed-order block reductions)
+cudaError_t launch_grad_points_sum(const double* gpt, const double* w, int64_t npts,
+                                   int64_t ld, int natm, double* out, cudaStream_t s);
 // out (nao, 3): sum_g w_g dX[x][mu][g] H[mu][g] (fixed-order block reduction)
 cudaError_t launch_ao_dot(const double* dX, const double* H, const double* w,
                           int64_t npts, int64_t ld, int nao, double* out,
