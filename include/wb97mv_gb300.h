@@ -340,6 +340,34 @@ int wb_cosx_ozaki_k64(wb_cosx* h, const double* x, const double* g,
                       double* k_out, void* workspace, size_t workspace_bytes,
                       void* stream);
 
+/* The same two products with no less accuracy than an FP64 GEMM (63-bit
+ * digits on the bf16 tensor cores; any nao), the GEMMs of the FP64 form and
+ * of the FP64 numint flows (gpu/vv10.py:288-297, :315-322):
+ *   wb_cosx_gemm64_f: f_out (nao, ld) FP64 = X QD;
+ *   wb_cosx_gemm64_k: k_out (+)= X^T (w o G), g (nao, ld) FP64, ld = npts
+ *     rounded up to 32.
+ * A point or column holding an infinity or NaN gives NaN.  Workspace:
+ * wb_gemm64_workspace_bytes(nao, ld) bytes. */
+size_t wb_gemm64_workspace_bytes(int nao, int64_t ld);
+int wb_cosx_gemm64_f(wb_cosx* h, const double* x, const double* qd,
+                     int64_t ld, double* f_out, void* workspace,
+                     size_t workspace_bytes, void* stream);
+int wb_cosx_gemm64_k(wb_cosx* h, const double* x, const double* g,
+                     const double* weights, int64_t npts, int accumulate,
+                     double* k_out, void* workspace, size_t workspace_bytes,
+                     void* stream);
+
+/* GGA density and Fock-side plane in FP64 (gpu/vv10.py:286-291, :315-321):
+ *   wb_gga_rho: rho_out (4, ld) FP64 = sum_mu T X_0, 2 sum_mu T X_d, with
+ *     x (4, nao, ld) the AO values and gradients and t (nao, ld) = D X_0,
+ *     FP64, or FP32 when t32 != 0; zero at or past npts;
+ *   wb_gga_aow: g_out (nao, ld) = sum_d v_d X_d, v (4, ld) FP64, stored as
+ *     FP64, or FP32 when g32 != 0; zero at or past npts. */
+int wb_gga_rho(wb_cosx* h, const double* x, const void* t, int t32, int64_t npts,
+               int64_t ld, double* rho_out, void* stream);
+int wb_gga_aow(wb_cosx* h, const double* x, const double* v, int64_t npts,
+               int64_t ld, int g32, void* g_out, void* stream);
+
 /* Engine of the F product (process-wide, every F of the K builds and of
  * wb_cosx_ozaki_f / _f64): WB_OZAKI_ENGINE_LIBRARY (the default) runs one
  * cuBLAS bf16 GEMM per level; WB_OZAKI_ENGINE_TC is this library's

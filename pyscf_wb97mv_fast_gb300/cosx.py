@@ -475,6 +475,84 @@ class CosxEngine:
             self._stream()), fn)
         return out
 
+    def gemm64_f(self, X, qd):
+        """QD^T X (nao, ld) FP64 with no less accuracy than an FP64 GEMM
+        (wb_cosx_gemm64_f); X (nao, ld) FP64, ld a multiple of 32."""
+        torch = _torch()
+        X = device_arg(X, 'X', torch.float64, self.device, (self.nao, None))
+        qd = self._dm_arg(qd)
+        ld = int(X.shape[1])
+        out = torch.empty((self.nao, ld), dtype=torch.float64, device=self.device)
+        if ld == 0:
+            return out
+        nbytes = int(_native.lib().wb_gemm64_workspace_bytes(self.nao, ld))
+        ws = self.workspace(nbytes)
+        _native.check(_native.lib().wb_cosx_gemm64_f(
+            self._h, _native.ptr(X), _native.ptr(qd), ld, _native.ptr(out),
+            _native.ptr(ws), nbytes, self._stream()), 'wb_cosx_gemm64_f')
+        return out
+
+    def gemm64_k(self, X, G, weights):
+        """X^T (w o G) (nao, nao) FP64 with no less accuracy than an FP64
+        GEMM (wb_cosx_gemm64_k); X, G (nao, ld) FP64, ld the number of
+        weights rounded up to 32."""
+        torch = _torch()
+        weights = device_arg(weights, 'weights', torch.float64, self.device, (None,))
+        npts = int(weights.shape[0])
+        ld = round32(npts)
+        X = device_arg(X, 'X', torch.float64, self.device, (self.nao, ld))
+        G = device_arg(G, 'G', torch.float64, self.device, (self.nao, ld))
+        out = torch.zeros((self.nao, self.nao), dtype=torch.float64, device=self.device)
+        if npts == 0:
+            return out
+        nbytes = int(_native.lib().wb_gemm64_workspace_bytes(self.nao, ld))
+        ws = self.workspace(nbytes)
+        _native.check(_native.lib().wb_cosx_gemm64_k(
+            self._h, _native.ptr(X), _native.ptr(G), _native.ptr(weights), npts, 0,
+            _native.ptr(out), _native.ptr(ws), nbytes, self._stream()),
+            'wb_cosx_gemm64_k')
+        return out
+
+    def gga_rho(self, X, T, npts):
+        """(rho, d rho / dx, dy, dz) (4, ld) FP64 from X (4, nao, ld) FP64 and
+        T = D X_0 (nao, ld), FP64 or FP32 (wb_gga_rho)."""
+        torch = _torch()
+        X = device_arg(X, 'X', torch.float64, self.device, (4, self.nao, None))
+        ld = int(X.shape[2])
+        t32 = getattr(T, 'dtype', None) == torch.float32
+        T = device_arg(T, 'T', torch.float32 if t32 else torch.float64, self.device,
+                       (self.nao, ld))
+        if not 0 <= int(npts) <= ld:
+            raise ValueError('npts must be in [0, %d]' % ld)
+        out = torch.empty((4, ld), dtype=torch.float64, device=self.device)
+        if ld == 0:
+            return out
+        _native.check(_native.lib().wb_gga_rho(
+            self._h, _native.ptr(X), _native.ptr(T), 1 if t32 else 0, int(npts), ld,
+            _native.ptr(out), self._stream()), 'wb_gga_rho')
+        return out
+
+    def gga_aow(self, X, v, npts, dtype=None):
+        """sum_d v_d X_d (nao, ld) of X (4, nao, ld) and v (4, ld) FP64, as
+        FP64 (default) or FP32 (wb_gga_aow)."""
+        torch = _torch()
+        X = device_arg(X, 'X', torch.float64, self.device, (4, self.nao, None))
+        ld = int(X.shape[2])
+        v = device_arg(v, 'v', torch.float64, self.device, (4, ld))
+        if not 0 <= int(npts) <= ld:
+            raise ValueError('npts must be in [0, %d]' % ld)
+        dtype = dtype or torch.float64
+        if dtype not in (torch.float32, torch.float64):
+            raise TypeError('dtype must be float32 or float64')
+        out = torch.empty((self.nao, ld), dtype=dtype, device=self.device)
+        if ld == 0:
+            return out
+        _native.check(_native.lib().wb_gga_aow(
+            self._h, _native.ptr(X), _native.ptr(v), int(npts), ld,
+            1 if dtype == torch.float32 else 0, _native.ptr(out), self._stream()),
+            'wb_gga_aow')
+        return out
+
     def ao_eval(self, coords_rel, out=None):
         """X (nao, ld) FP64 AO-major."""
         torch = _torch()

@@ -501,6 +501,82 @@ cudaError_t launch_xc_aow(const double* X, const double* v, int nao, int64_t ld,
     return cudaGetLastError();
 }
 
+// GGA density in FP64 (the VV10 flow, gpu/vv10.py:286-291): rho = sum_mu T X_0,
+// grad_d = 2 sum_mu T X_d.  A block takes 32 points; its eight warps take the
+// rows in turn (256-byte rows, four planes read once beside T) and their sums
+// are added in warp order.  Bound by HBM: 40 bytes per (point, AO) against 4
+// FP64 FMAs.
+template<typename T>
+__global__ void __launch_bounds__(256)
+gga_rho_kernel(const double* __restrict__ X, const T* __restrict__ t, int nao, int64_t ld,
+               int64_t npts, double* __restrict__ rho) {
+    __shared__ double part[8][4][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t g = (int64_t)blockIdx.x * 32 + lane;      // ld is a multiple of 32
+    const int64_t pl = (int64_t)nao * ld;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int mu = warp; mu < nao; mu += 8) {
+        const int64_t o = (int64_t)mu * ld + g;
+        const double tv = (double)t[o];
+#pragma unroll
+        for (int d = 0; d < 4; ++d) acc[d] = fma(tv, X[d * pl + o], acc[d]);
+    }
+#pragma unroll
+    for (int d = 0; d < 4; ++d) part[warp][d][lane] = acc[d];
+    __syncthreads();
+    if (warp < 4) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) s += part[w][warp][lane];
+        rho[warp * ld + g] = g < npts ? (warp ? 2.0 * s : s) : 0.0;
+    }
+}
+
+cudaError_t launch_gga_rho(const double* X, const void* t, bool t32, int nao, int64_t ld,
+                           int64_t npts, double* rho, cudaStream_t s) {
+    if (ld <= 0) return cudaSuccess;
+    const unsigned grid = (unsigned)(ld / 32);
+    if (t32)
+        gga_rho_kernel<<<grid, 256, 0, s>>>(X, static_cast<const float*>(t), nao, ld, npts,
+                                            rho);
+    else
+        gga_rho_kernel<<<grid, 256, 0, s>>>(X, static_cast<const double*>(t), nao, ld, npts,
+                                            rho);
+    return cudaGetLastError();
+}
+
+// The Fock-side plane of a GGA potential in FP64: sum_d v_d X_d, one thread
+// per AO and two points (HBM-bound: 32 bytes read and 8 written per element).
+template<typename T>
+__global__ void gga_aow_kernel(const double* __restrict__ X, const double* __restrict__ v,
+                               int nao, int64_t ld, int64_t npts, T* __restrict__ G) {
+    const int64_t g = 2 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    if (g >= ld) return;
+    const int64_t pl = (int64_t)nao * ld, o = (int64_t)blockIdx.y * ld + g;
+    double a = 0.0, b = 0.0;
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+        const double2 x = *reinterpret_cast<const double2*>(X + d * pl + o);
+        const double2 u = *reinterpret_cast<const double2*>(v + d * ld + g);
+        a = fma(u.x, x.x, a);
+        b = fma(u.y, x.y, b);
+    }
+    G[o] = (T)(g < npts ? a : 0.0);
+    G[o + 1] = (T)(g + 1 < npts ? b : 0.0);
+}
+
+cudaError_t launch_gga_aow(const double* X, const double* v, int nao, int64_t ld,
+                           int64_t npts, bool g32, void* G, cudaStream_t s) {
+    if (ld <= 0 || nao <= 0) return cudaSuccess;
+    const dim3 grid((unsigned)((ld / 2 + 255) / 256), (unsigned)nao);
+    if (g32)
+        gga_aow_kernel<<<grid, 256, 0, s>>>(X, v, nao, ld, npts, static_cast<float*>(G));
+    else
+        gga_aow_kernel<<<grid, 256, 0, s>>>(X, v, nao, ld, npts, static_cast<double*>(G));
+    return cudaGetLastError();
+}
+
 cudaError_t launch_gsum(const float* gc, const int4* src, int nao, int64_t ld,
                         float* G, cudaStream_t s) {
     if (nao <= 0 || ld <= 0) return cudaSuccess;

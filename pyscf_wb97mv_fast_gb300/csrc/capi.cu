@@ -21,6 +21,7 @@
 #include "generated/cosx_layout.h"
 #include "scf.hpp"
 #include "launch.hpp"
+#include "gemm64.hpp"
 #include "ozaki.hpp"
 #include "wb97mv_gb300.h"
 
@@ -632,6 +633,27 @@ int read_stats(wb_cosx* h, void* ws, const WsLayout& L, int64_t ntasks_total,
     return WB_OK;
 }
 
+// the products of the FP64 flows (gemm64.cu) on the handle's cuBLAS
+int gemm64_f(wb_cosx* h, const double* X, const double* qd, int64_t ld, double* F,
+             void* ws, cudaStream_t s) {
+    WB_CUBLAS(cublasSetStream(h->cublas, s));
+    WB_CUBLAS(cublasSetMathMode(h->cublas, CUBLAS_DEFAULT_MATH));
+    const int r = wb::gemm64_f(h->cublas, X, qd, h->hp.nao, ld, F, ws, s);
+    if (r) return fail(r >= 1000 ? WB_ERR_CUBLAS : WB_ERR_CUDA,
+                       "FP64 F GEMM failed, code " + std::to_string(r));
+    return WB_OK;
+}
+int gemm64_k(wb_cosx* h, const double* X, const double* G, const double* w, int64_t ld,
+             int64_t npts, int accumulate, double* K, void* ws, cudaStream_t s) {
+    WB_CUBLAS(cublasSetStream(h->cublas, s));
+    WB_CUBLAS(cublasSetMathMode(h->cublas, CUBLAS_DEFAULT_MATH));
+    const int r = wb::gemm64_k(h->cublas, X, G, w, h->hp.nao, ld, npts, accumulate, K, ws,
+                               s);
+    if (r) return fail(r >= 1000 ? WB_ERR_CUBLAS : WB_ERR_CUDA,
+                       "FP64 K GEMM failed, code " + std::to_string(r));
+    return WB_OK;
+}
+
 // FP64 pair data, FP64 Boys table and the FP64 c2s constants of the plain
 // FP64 form, built and uploaded on its first call (synchronous copies)
 int ensure_fp64(wb_cosx* h) {
@@ -786,7 +808,7 @@ int64_t hartree_ndh(const wb::HostPairs& hp) {
 
 struct WsLayout64 {
     WsLayout base;                  // counters, work, block statistics
-    size_t X = 0, F64 = 0, F32 = 0, G64 = 0, WG = 0, rec = 0, total = 0;
+    size_t X = 0, F64 = 0, F32 = 0, G64 = 0, rec = 0, gemm = 0, total = 0;
 };
 
 WsLayout64 ws_layout_fp64(const wb_cosx* h, int64_t ld) {
@@ -805,12 +827,13 @@ WsLayout64 ws_layout_fp64(const wb_cosx* h, int64_t ld) {
         L.base.subcr[b] = take(sizeof(float4) * (size_t)nblk);
         L.base.msh[b] = take(sizeof(float) * (size_t)nblk * std::max(h->hp.nvshell, 1));
     }
-    const size_t n = (size_t)h->hp.nao * ld;
+    const int nao64 = h->hp.nao;
+    const size_t n = (size_t)nao64 * ld;
     L.X = take(sizeof(double) * n);
     L.F64 = take(sizeof(double) * n);
     L.F32 = take(sizeof(float) * n);
     L.G64 = take(sizeof(double) * n);
-    L.WG = take(sizeof(double) * n);
+    L.gemm = take(wb::gemm64_bytes(nao64, ld));
     L.rec = take(sizeof(double) * wb::kF64Rec * (size_t)std::max(h->hp.npp, 1));
     L.total = off;
     return L;
@@ -1450,14 +1473,11 @@ int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
     }
     int st = ensure_fp64(h);
     if (st != WB_OK) return st;
-    WB_CUBLAS(cublasSetStream(h->cublas, s));
-    WB_CUBLAS(cublasSetMathMode(h->cublas, CUBLAS_DEFAULT_MATH));
     double* X = at<double>(workspace, L.X);
     double* F64 = at<double>(workspace, L.F64);
     float* F32 = at<float>(workspace, L.F32);
     double* G64 = at<double>(workspace, L.G64);
-    double* WG = at<double>(workspace, L.WG);
-    const double one = 1.0, zero = 0.0;
+    void* gemm = at<void>(workspace, L.gemm);
     wb::AoArgs ao;
     ao.coords = coords; ao.npts = npts; ao.ld = ld; ao.nbas = h->nbas;
     ao.sh_l = h->sh_l; ao.sh_np = h->sh_np; ao.sh_nc = h->sh_nc;
@@ -1467,8 +1487,7 @@ int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
     WB_CUDA(wb::launch_ao_eval(ao, s));
     // F = X QD in FP64 (no rounding); its FP32 copy feeds only the block
     // statistics of the screen, as in the mixed-precision path
-    WB_CUBLAS(cublasDgemm(h->cublas, CUBLAS_OP_N, CUBLAS_OP_T, (int)ld, nao, nao,
-                          &one, X, (int)ld, qd, nao, &zero, F64, (int)ld));
+    if ((st = gemm64_f(h, X, qd, ld, F64, gemm, s)) != WB_OK) return st;
     WB_CUDA(wb::launch_f64_to_f32(F64, F32, (int64_t)nao * ld, s));
     wb::BlockStatsOut bo;
     for (int b = 0; b < 3; ++b) {
@@ -1477,7 +1496,7 @@ int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
     }
     WB_CUDA(wb::launch_sub_stats(coords, weights, F32, npts, ld, h->hp.nvshell,
                                  h->vs_ao0, h->vs_nf, bo, s));
-    launches += 4;
+    launches += 3 + wb::gemm64_f_launches(nao, ld);
     wb::CosxF64Args a;
     std::memset(&a, 0, sizeof(a));
     a.F = F64;
@@ -1523,11 +1542,10 @@ int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
             ++launches;
         }
         ntasks += (ld / 32) * (int64_t)h->hp.npairs;
-        WB_CUDA(wb::launch_weight_g64(G64, weights, npts, ld, nao, WG, s));
-        WB_CUBLAS(cublasDgemm(h->cublas, CUBLAS_OP_T, CUBLAS_OP_N, nao, nao, (int)ld,
-                              &one, WG, (int)ld, X, (int)ld, &zero, k_out + kk * j,
-                              nao));
-        launches += 2;
+        if ((st = gemm64_k(h, X, G64, weights, ld, npts, 0, k_out + kk * j, gemm, s)) !=
+            WB_OK)
+            return st;
+        launches += wb::gemm64_k_launches(npts);
     }
     return read_stats(h, workspace, L.base, ntasks, s, stats, launches);
 }
@@ -1985,10 +2003,8 @@ int wb_cosx_k_grad(wb_cosx* h, const double* coords, const double* weights,
     double* F64 = at<double>(workspace, L.F64);
     float* F32 = at<float>(workspace, L.F32);
     double* G64 = at<double>(workspace, L.G64);
-    double* H = at<double>(workspace, L.WG);
-    WB_CUBLAS(cublasSetStream(h->cublas, s));
-    WB_CUBLAS(cublasSetMathMode(h->cublas, CUBLAS_DEFAULT_MATH));
-    const double one = 1.0, zero = 0.0;
+    double* H = at<double>(workspace, L.X);     // free here: the AO values are Xd
+    void* gemm = at<void>(workspace, L.gemm);
     wb::AoArgs ao;
     ao.coords = coords; ao.npts = npts; ao.ld = ld; ao.nbas = h->nbas;
     ao.sh_l = h->sh_l; ao.sh_np = h->sh_np; ao.sh_nc = h->sh_nc;
@@ -1997,8 +2013,7 @@ int wb_cosx_k_grad(wb_cosx* h, const double* coords, const double* weights,
     ao.nao = nao;
     WB_CUDA(wb::launch_ao_eval_d1(ao, s));
     // F = X D (FP64); fl32(F) feeds the screen's block statistics only
-    WB_CUBLAS(cublasDgemm(h->cublas, CUBLAS_OP_N, CUBLAS_OP_T, (int)ld, nao, nao, &one,
-                          Xd, (int)ld, dm, nao, &zero, F64, (int)ld));
+    if ((st = gemm64_f(h, Xd, dm, ld, F64, gemm, s)) != WB_OK) return st;
     WB_CUDA(wb::launch_f64_to_f32(F64, F32, (int64_t)n, s));
     wb::BlockStatsOut bo;
     for (int b = 0; b < 3; ++b) {
@@ -2035,8 +2050,7 @@ int wb_cosx_k_grad(wb_cosx* h, const double* coords, const double* weights,
         if (pe > pb) WB_CUDA(wb::launch_cosx_fp64_class(c, a, pb, pe, h->nsm, s));
     }
     // X side: 1/2 sum_g w_g sum_{mu on C} grad X_g,mu (G D)_g,mu
-    WB_CUBLAS(cublasDgemm(h->cublas, CUBLAS_OP_N, CUBLAS_OP_T, (int)ld, nao, nao, &one,
-                          G64, (int)ld, dm, nao, &zero, H, (int)ld));
+    if ((st = gemm64_f(h, G64, dm, ld, H, gemm, s)) != WB_OK) return st;
     WB_CUDA(cudaMemsetAsync(grad_out, 0, sizeof(double) * 3 * (size_t)natm, s));
     WB_CUDA(wb::launch_ao_dot(Xd, H, weights, npts, ld, nao, aodot, s));
     WB_CUDA(wb::launch_atom_sum(aodot, h->vs_ao0, h->vs_nf, h->vs_atom, h->hp.nvshell,
@@ -2354,6 +2368,51 @@ int wb_cosx_ozaki_k64(wb_cosx* h, const double* x, const double* g,
                                      accumulate, k_out, workspace, s);
     if (r) return fail(r >= 1000 ? WB_ERR_CUBLAS : WB_ERR_CUDA,
                        "ozaki K64 GEMM failed, code " + std::to_string(r));
+    return WB_OK;
+}
+
+size_t wb_gemm64_workspace_bytes(int nao, int64_t ld) {
+    if (nao <= 0 || ld <= 0) return 0;
+    return wb::gemm64_bytes(nao, ld);
+}
+
+int wb_cosx_gemm64_f(wb_cosx* h, const double* x, const double* qd, int64_t ld,
+                     double* f_out, void* workspace, size_t workspace_bytes,
+                     void* stream) {
+    if (!h || !x || !qd || !f_out || ld <= 0 || ld % 32)
+        return fail(WB_ERR_INVALID_ARGUMENT, "wb_cosx_gemm64_f: bad arguments");
+    if (!workspace || workspace_bytes < wb::gemm64_bytes(h->hp.nao, ld))
+        return fail(WB_ERR_WORKSPACE, "wb_cosx_gemm64_f: workspace too small");
+    return gemm64_f(h, x, qd, ld, f_out, workspace, static_cast<cudaStream_t>(stream));
+}
+
+int wb_cosx_gemm64_k(wb_cosx* h, const double* x, const double* g, const double* weights,
+                     int64_t npts, int accumulate, double* k_out, void* workspace,
+                     size_t workspace_bytes, void* stream) {
+    if (!h || !x || !g || !weights || !k_out || npts <= 0)
+        return fail(WB_ERR_INVALID_ARGUMENT, "wb_cosx_gemm64_k: bad arguments");
+    const int64_t ld = round32(npts);
+    if (!workspace || workspace_bytes < wb::gemm64_bytes(h->hp.nao, ld))
+        return fail(WB_ERR_WORKSPACE, "wb_cosx_gemm64_k: workspace too small");
+    return gemm64_k(h, x, g, weights, ld, npts, accumulate, k_out, workspace,
+                    static_cast<cudaStream_t>(stream));
+}
+
+int wb_gga_rho(wb_cosx* h, const double* x, const void* t, int t32, int64_t npts,
+               int64_t ld, double* rho_out, void* stream) {
+    if (!h || !x || !t || !rho_out || ld <= 0 || ld % 32 || npts < 0 || npts > ld)
+        return fail(WB_ERR_INVALID_ARGUMENT, "wb_gga_rho: bad arguments");
+    WB_CUDA(wb::launch_gga_rho(x, t, t32 != 0, h->hp.nao, ld, npts, rho_out,
+                               static_cast<cudaStream_t>(stream)));
+    return WB_OK;
+}
+
+int wb_gga_aow(wb_cosx* h, const double* x, const double* v, int64_t npts, int64_t ld,
+               int g32, void* g_out, void* stream) {
+    if (!h || !x || !v || !g_out || ld <= 0 || ld % 32 || npts < 0 || npts > ld)
+        return fail(WB_ERR_INVALID_ARGUMENT, "wb_gga_aow: bad arguments");
+    WB_CUDA(wb::launch_gga_aow(x, v, h->hp.nao, ld, npts, g32 != 0, g_out,
+                               static_cast<cudaStream_t>(stream)));
     return WB_OK;
 }
 

@@ -1,5 +1,5 @@
 // Plain FP64 form of the fused screen + G kernels: the s/p/d classes, the
-// class dispatcher and the FP64 weight pass (the kernel itself is in
+// class dispatcher and the per-omega records (the kernel itself is in
 // cosx_fp64.cuh).
 #include "cosx_fp64.cuh"
 
@@ -19,16 +19,6 @@ cudaError_t launch_cosx_fp64_class(int cls, const CosxF64Args& a, int pb, int pe
 }
 
 namespace {
-__global__ void weight_g64_kernel(const double* __restrict__ G,
-                                  const double* __restrict__ w, int64_t npts,
-                                  int64_t ld, int nao, double* __restrict__ out) {
-    const int64_t n = (int64_t)nao * ld;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t g = i % ld;
-        out[i] = g < npts ? w[g] * G[i] : 0.0;
-    }
-}
 
 // the lane-independent factors of a primitive pair, once per omega: in the
 // class kernels the division and the square root would take 30 FP64
@@ -67,15 +57,6 @@ cudaError_t launch_f64_records(int npp, const double* P, const double* p,
     if (npp <= 0) return cudaSuccess;
     f64_records_kernel<<<(npp + 127) / 128, 128, 0, s>>>(npp, P, p, pref, alpha,
                                                          omega * omega, rec);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_weight_g64(const double* G, const double* w, int64_t npts,
-                              int64_t ld, int nao, double* out, cudaStream_t s) {
-    const int64_t n = (int64_t)nao * ld;
-    const int64_t blocks = grid_stride_blocks(n, 256, 32);
-    weight_g64_kernel<<<(int)std::max<int64_t>(blocks, 1), 256, 0, s>>>(G, w, npts, ld,
-                                                                      nao, out);
     return cudaGetLastError();
 }
 

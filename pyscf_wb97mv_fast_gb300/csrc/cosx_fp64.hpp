@@ -56,7 +56,5 @@ cudaError_t launch_cosx_fp64_class(int cls, const CosxF64Args& a, int pb, int pe
                                    int nsm, cudaStream_t s);
 cudaError_t launch_cosx_fp64_f(int cls, const CosxF64Args& a, int pb, int pe,
                                int nsm, cudaStream_t s);
-cudaError_t launch_weight_g64(const double* G, const double* w, int64_t npts,
-                              int64_t ld, int nao, double* out, cudaStream_t s);
 
 }  // namespace wb

@@ -1,0 +1,432 @@
+// FP64 GEMMs of the FP64 flows on the bf16 tensor cores.
+//
+// GB300's FP64 rate is 1.2 TFLOP/s, DGEMM included (0.95 measured), so in an
+// FP64 Fock build, in VV10 and in the gradient the products with D and X
+// outweighed the kernels between them.  They run here as an Ozaki split
+// (K. Ozaki et al., Numer. Algorithms 59 (2012) 95-118), as the 42-bit split
+// of ozaki.cu, but wide enough to lose nothing of FP64: S = 9 balanced digits
+// of B = 7 bits, W = 63 bits below the largest entry of the row (point) or
+// column (AO), against the 53 of a double.  An entry is cut only where it is
+// below 2^-10 of that largest one, and then by 2^-63 of it; the dropped
+// products (digit levels i + j >= 9) are as small.  Error against exact
+// arithmetic: below cuBLAS DGEMM's own rounding in the 2-norm and in the
+// largest entry, on the densities and orbitals of the test (waters and
+// alkanes, FP64 AO values), whose rows span 10 orders of magnitude.
+//
+// Exactness: digits are at most 64 in magnitude (exact in bf16), products
+// 2^12, so a bf16 GEMM of at most kPiece = 4096 terms has only integers up to
+// 2^24 as partial sums: FP32 accumulation is exact in any order.  Level l =
+// i + j is the product of the first (l + 1) slices of A with the last (l + 1)
+// slices of B, cut every 4096 terms into pieces; pieces and levels are added
+// as integers and rounded once.  45 slice products, so 45/2 x the flops of a
+// DGEMM at some 1500 times its rate.
+//
+// Measured against cuBLAS DGEMM: F of 442 AOs x 157,256 points 64 -> 4.5 ms,
+// 192 x 70,478 4.8 -> 0.66 ms, K of the latter 5.0 -> 0.80 ms; below some 64
+// AOs and 10,000 points the fixed 0.11 ms of launches is about the DGEMM's
+// time, so there is no other path.
+//
+// Point tiles (F) and groups of chunks (K) bound the workspace to some GB.
+// A row or column with an infinity or a NaN gives NaN, as FP64 arithmetic
+// mostly would; magnitudes from subnormal to the largest double are taken.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+
+#include "gemm64.hpp"
+#include "launch.hpp"
+
+namespace wb {
+namespace {
+
+constexpr int kS = 9, kBits = 7, kW = kS * kBits;
+constexpr int kPiece = 4096;             // terms of an exact FP32 sum
+constexpr int kKc = 512;                 // points per chunk of the K product
+constexpr int kGroup = 128;              // chunks in flight
+constexpr int64_t kTile = 65536;         // points per tile of the F product
+constexpr int kNonfinite = 1 << 20;      // exponent of a row that holds one
+
+size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
+// slices are padded to 8 entries: cuBLAS needs 16-byte rows for its
+// tensor-memory kernels (unaligned ones ran on mma.sync kernels at a third of
+// the rate)
+int pad8(int n) { return (n + 7) & ~7; }
+int pieces(int terms) { return (terms + kPiece - 1) / kPiece; }
+int planes(int inner) {
+    int n = 0;
+    for (int l = 0; l < kS; ++l) n += pieces((l + 1) * inner);
+    return n;
+}
+
+// e with |x| < 2^e for the bits of the largest |x|
+__device__ __forceinline__ int exponent_of(const unsigned long long bits) {
+    const int E = (int)(bits >> 52);
+    if (E == 0x7ff) return kNonfinite;
+    return E ? E - 1022 : -1022;
+}
+
+// the nine digits of q = rint(x 2^(62 - e)), |x| < 2^e, most significant first
+__device__ __forceinline__ void digits9(const double x, const int e, int* d) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int E = (int)((b >> 52) & 0x7ff);
+    unsigned long long m = b & 0xfffffffffffffull;
+    if (E) m |= 1ull << 52;
+    const int sh = (E ? E - 1075 : -1074) + (kW - 1) - e;      // <= 9
+    unsigned long long q = 0;
+    if (sh >= 0) {
+        q = m << min(sh, 9);
+    } else if (sh > -64) {
+        const int r = -sh;
+        q = m >> r;
+        const unsigned long long rem = m & ((1ull << r) - 1), half = 1ull << (r - 1);
+        if (rem > half || (rem == half && (q & 1ull))) ++q;
+    }
+    if (e == kNonfinite) q = 0;
+    // q in base 2^7, balanced: 28 bits, 28 bits and the rest, 32-bit steps
+    long long v = (b >> 63) ? -(long long)q : (long long)q;
+    int part[3];
+    part[2] = (int)(v & 0xfffffff);
+    v >>= 28;
+    part[1] = (int)(v & 0xfffffff);
+    part[0] = (int)(v >> 28);
+    int carry = 0;
+#pragma unroll
+    for (int i = kS - 1; i >= 1; --i) {
+        int& p = part[(i + 3) / 4];
+        if (i == kS - 1 || i == kS - 5) p += carry;
+        const int di = ((p + 64) & 127) - 64;
+        d[i] = di;
+        p = (p - di) >> 7;
+        if (i == kS - 4 || i == kS - 8) carry = p;
+    }
+    d[0] = part[0] + carry;
+}
+
+// RN(v 2^sc), v = hi 2^28 + lo, with integer arithmetic (the conversions
+// would be FP64-pipe instructions)
+__device__ __forceinline__ double round_sum(const long long hi, const long long lo,
+                                            const int sc) {
+    const __int128 v = ((__int128)hi << 28) + lo;
+    if (v == 0) return 0.0;
+    const unsigned __int128 a = v < 0 ? (unsigned __int128)0 - (unsigned __int128)v
+                                      : (unsigned __int128)v;
+    const unsigned long long ah = (unsigned long long)(a >> 64), alo = (unsigned long long)a;
+    const int nb = ah ? 128 - __clzll((long long)ah) : 64 - __clzll((long long)alo);
+    const int r = nb - 53;
+    unsigned long long q;
+    if (r > 0) {
+        q = (unsigned long long)(a >> r);
+        const unsigned __int128 rem = a & (((unsigned __int128)1 << r) - 1);
+        const unsigned __int128 half = (unsigned __int128)1 << (r - 1);
+        if (rem > half || (rem == half && (q & 1ull))) ++q;
+    } else {
+        q = alo << -r;
+    }
+    const int E = r + sc + 52 + 1023;           // exponent field of q = 2^52
+    double out;
+    if (E >= 1 && E <= 2045)
+        out = __longlong_as_double((long long)(((unsigned long long)E << 52) +
+                                               (q - (1ull << 52))));
+    else
+        out = scalbn((double)q, max(-4000, min(4000, r + sc)));
+    return v < 0 ? -out : out;
+}
+
+// integer sums of the levels: hi = levels 0 .. 4, lo = 5 .. 8, so that the
+// value is (hi 2^28 + lo) 2^(sc)
+struct LevelSum {
+    long long hi = 0, lo = 0;
+    __device__ __forceinline__ void add(const int l, const float c) {
+        const long long t = (long long)__float2int_rn(c);
+        if (l <= 4) hi += t << (kBits * (4 - l));
+        else lo += t << (kBits * (8 - l));
+    }
+};
+// exponent of the last digit level kept: x y = 2^(ex + ey - 2 (W - 1) +
+// B (S - 1)) sum_l C_l 2^(B (S - 1 - l))
+__device__ __forceinline__ int level_scale(const int ex, const int ey) {
+    return ex + ey - 2 * (kW - 1) + kBits * (kS - 1);
+}
+__device__ __forceinline__ double finish(const LevelSum& v, const int ex, const int ey) {
+    if (ex == kNonfinite || ey == kNonfinite) return __longlong_as_double(0x7ff8000000000000ll);
+    return round_sum(v.hi, v.lo, level_scale(ex, ey));
+}
+
+__device__ __forceinline__ unsigned long long abs_bits(const double x) {
+    return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+}
+
+// exponent of each point's largest |X(l, g)|, g0 <= g < g0 + n
+__global__ void point_exponents_kernel(const double* __restrict__ X, const int nao,
+                                       const int64_t ld, const int n, int* __restrict__ e) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= n) return;
+    unsigned long long m = 0;
+    int l = 0;
+    for (; l + 8 <= nao; l += 8) {
+        unsigned long long b[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) b[u] = abs_bits(__ldg(X + (int64_t)(l + u) * ld + g));
+#pragma unroll
+        for (int u = 0; u < 8; ++u) m = b[u] > m ? b[u] : m;
+    }
+    for (; l < nao; ++l) {
+        const unsigned long long b = abs_bits(__ldg(X + (int64_t)l * ld + g));
+        m = b > m ? b : m;
+    }
+    e[g] = exponent_of(m);
+}
+
+// A (n x S np, column-major): column i np + l = digit i of X(l, :), zero for
+// l >= nao; one thread per (l, two points)
+__global__ void slice_points_kernel(const double* __restrict__ X, const int nao, const int np,
+                                    const int64_t ld, const int n, const int* __restrict__ e,
+                                    __nv_bfloat16* __restrict__ A) {
+    const int l = blockIdx.y;
+    const int g = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (g >= n) return;                         // n is even
+    int d0[kS], d1[kS];
+    if (l < nao) {
+        const double2 x = *reinterpret_cast<const double2*>(X + (int64_t)l * ld + g);
+        digits9(x.x, e[g], d0);
+        digits9(x.y, e[g + 1], d1);
+    } else {
+#pragma unroll
+        for (int i = 0; i < kS; ++i) d0[i] = d1[i] = 0;
+    }
+#pragma unroll
+    for (int i = 0; i < kS; ++i)
+        *reinterpret_cast<__nv_bfloat162*>(A + ((int64_t)i * np + l) * n + g) =
+            __floats2bfloat162_rn((float)d0[i], (float)d1[i]);
+}
+
+// largest |bits| of a block of 256 threads
+__device__ __forceinline__ unsigned long long block_max(unsigned long long m) {
+    __shared__ unsigned long long red[8];
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long t = __shfl_xor_sync(0xffffffffu, m, o);
+        m = t > m ? t : m;
+    }
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m = red[j] > m ? red[j] : m;
+    __syncthreads();
+    return m;
+}
+
+// B (S np x nao, column-major): row (S - 1 - i) np + l of column mu = digit i
+// of QD(l, mu); one block of 256 threads per column
+__global__ void __launch_bounds__(256)
+slice_matrix_kernel(const double* __restrict__ QD, const int nao, const int np,
+                    int* __restrict__ e, __nv_bfloat16* __restrict__ B) {
+    const int mu = blockIdx.x;
+    unsigned long long m = 0;
+    for (int l = threadIdx.x; l < nao; l += 256) {
+        const unsigned long long b = abs_bits(QD[(int64_t)l * nao + mu]);
+        m = b > m ? b : m;
+    }
+    const int ec = exponent_of(block_max(m));
+    if (threadIdx.x == 0) e[mu] = ec;
+    for (int l = threadIdx.x; l < np; l += 256) {
+        int d[kS];
+        digits9(l < nao ? QD[(int64_t)l * nao + mu] : 0.0, ec, d);
+#pragma unroll
+        for (int i = 0; i < kS; ++i)
+            B[((int64_t)mu * kS + (kS - 1 - i)) * np + l] = __float2bfloat16_rn((float)d[i]);
+    }
+}
+
+// F[mu][g] from the level planes C (plane, mu, n)
+__global__ void combine_points_kernel(const float* __restrict__ C, const int nao, const int np,
+                                      const int64_t ld, const int n,
+                                      const int* __restrict__ ep, const int* __restrict__ ec,
+                                      double* __restrict__ F) {
+    const int mu = blockIdx.y;
+    const int g = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (g >= n) return;
+    const int64_t plane = (int64_t)nao * n;
+    const float* c = C + (int64_t)mu * n + g;
+    LevelSum v0, v1;
+#pragma unroll
+    for (int l = 0; l < kS; ++l)
+        for (int left = (l + 1) * np; left > 0; left -= kPiece, c += plane) {
+            const float2 t = __ldg(reinterpret_cast<const float2*>(c));
+            v0.add(l, t.x);
+            v1.add(l, t.y);
+        }
+    const int e = ec[mu];
+    *reinterpret_cast<double2*>(F + (int64_t)mu * ld + g) =
+        make_double2(finish(v0, ep[g], e), finish(v1, ep[g + 1], e));
+}
+
+// Digits of one chunk's column of X (ascending slices) or of w o G
+// (descending): out (chunk, column, S, kKc), columns past nao zero.  One block
+// of 256 threads, two points a thread, per (chunk, column).
+template<bool WG>
+__global__ void __launch_bounds__(256)
+slice_chunk_kernel(const double* __restrict__ X, const double* __restrict__ w, const int nao,
+                   const int64_t ld, const int64_t npts, const int64_t g_base,
+                   int* __restrict__ e, __nv_bfloat16* __restrict__ out) {
+    const int np = gridDim.y, col = blockIdx.y;
+    const int64_t slot = (int64_t)blockIdx.x * np + col;
+    const int k = 2 * threadIdx.x;
+    const int64_t g = g_base + (int64_t)blockIdx.x * kKc + k;
+    double x0 = 0.0, x1 = 0.0;
+    if (col < nao) {
+        const double* x = X + (int64_t)col * ld;
+        if (g < npts) x0 = WG ? w[g] * x[g] : x[g];
+        if (g + 1 < npts) x1 = WG ? w[g + 1] * x[g + 1] : x[g + 1];
+    }
+    const unsigned long long a = abs_bits(x0), b = abs_bits(x1);
+    const int ee = exponent_of(block_max(a > b ? a : b));
+    if (threadIdx.x == 0) e[slot] = ee;
+    int d0[kS], d1[kS];
+    digits9(x0, ee, d0);
+    digits9(x1, ee, d1);
+    __nv_bfloat16* o = out + slot * kS * kKc + k;
+#pragma unroll
+    for (int i = 0; i < kS; ++i)
+        *reinterpret_cast<__nv_bfloat162*>(o + (WG ? kS - 1 - i : i) * kKc) =
+            __floats2bfloat162_rn((float)d0[i], (float)d1[i]);
+}
+
+// K (+)= the chunks of one group, in chunk order: C (plane, chunk, np x np)
+__global__ void combine_chunks_kernel(const float* __restrict__ C, const int nao, const int np,
+                                      const int nchunk, const int* __restrict__ ex,
+                                      const int* __restrict__ eg, const int add,
+                                      double* __restrict__ K) {
+    const int64_t nn = (int64_t)np * np;
+    const int64_t plane = nn * nchunk;
+    const int mu = blockIdx.x * blockDim.x + threadIdx.x, nu = blockIdx.y;
+    if (mu >= nao) return;
+    double acc = 0.0;
+#pragma unroll 2
+    for (int c = 0; c < nchunk; ++c) {
+        const float* p = C + (int64_t)c * nn + (int64_t)nu * np + mu;
+        LevelSum v;
+#pragma unroll
+        for (int l = 0; l < kS; ++l)
+#pragma unroll
+            for (int left = (l + 1) * kKc; left > 0; left -= kPiece, p += plane)
+                v.add(l, __ldg(p));
+        acc += finish(v, ex[c * np + mu], eg[c * np + nu]);
+    }
+    const int64_t o = (int64_t)mu * nao + nu;
+    K[o] = add ? K[o] + acc : acc;
+}
+
+size_t f_bytes(int nao, int64_t ld) {
+    const size_t np = pad8(nao), n = (size_t)std::min(ld, kTile);
+    return al(sizeof(int) * n) + al(sizeof(int) * nao) + al(2 * kS * np * n) +
+           al(2 * kS * np * nao) + al(sizeof(float) * planes((int)np) * nao * n);
+}
+
+size_t k_bytes(int nao, int64_t ld) {
+    const size_t np = pad8(nao);
+    const size_t nc = (size_t)std::min<int64_t>((ld + kKc - 1) / kKc, kGroup);
+    return 2 * (al(sizeof(int) * nc * np) + al(2 * kS * kKc * nc * np)) +
+           al(sizeof(float) * planes(kKc) * nc * np * np);
+}
+
+}  // namespace
+
+size_t gemm64_bytes(int nao, int64_t ld) { return std::max(f_bytes(nao, ld), k_bytes(nao, ld)); }
+
+int gemm64_f_launches(int nao, int64_t ld) {
+    return 1 + (int)((ld + kTile - 1) / kTile) * (3 + planes(pad8(nao)));
+}
+int gemm64_k_launches(int64_t npts) {
+    return (int)((npts + (int64_t)kKc * kGroup - 1) / ((int64_t)kKc * kGroup)) *
+           (3 + planes(kKc));
+}
+
+#define G64_CUBLAS(call)                                          \
+    do {                                                          \
+        cublasStatus_t st_ = (call);                              \
+        if (st_ != CUBLAS_STATUS_SUCCESS) return (int)st_ + 1000; \
+    } while (0)
+#define G64_CUDA(call)                       \
+    do {                                     \
+        cudaError_t e_ = (call);             \
+        if (e_ != cudaSuccess) return (int)e_; \
+    } while (0)
+
+int gemm64_f(cublasHandle_t hb, const double* X, const double* QD, int nao, int64_t ld,
+             double* F, void* ws, cudaStream_t s) {
+    const int np = pad8(nao);
+    const int64_t nmax = std::min(ld, kTile);
+    char* p = static_cast<char*>(ws);
+    int* ep = reinterpret_cast<int*>(p); p += al(sizeof(int) * nmax);
+    int* ec = reinterpret_cast<int*>(p); p += al(sizeof(int) * nao);
+    __nv_bfloat16* A = reinterpret_cast<__nv_bfloat16*>(p);
+    p += al((size_t)2 * kS * np * nmax);
+    __nv_bfloat16* B = reinterpret_cast<__nv_bfloat16*>(p);
+    p += al((size_t)2 * kS * np * nao);
+    float* C = reinterpret_cast<float*>(p);
+    slice_matrix_kernel<<<nao, 256, 0, s>>>(QD, nao, np, ec, B);
+    G64_CUDA(cudaGetLastError());
+    const float one = 1.0f, zero = 0.0f;
+    for (int64_t g = 0; g < ld; g += kTile) {
+        const int n = (int)std::min(kTile, ld - g);
+        const dim3 grid((n / 2 + 255) / 256, np);
+        point_exponents_kernel<<<(n + 255) / 256, 256, 0, s>>>(X + g, nao, ld, n, ep);
+        G64_CUDA(cudaGetLastError());
+        slice_points_kernel<<<grid, 256, 0, s>>>(X + g, nao, np, ld, n, ep, A);
+        G64_CUDA(cudaGetLastError());
+        float* c = C;
+        for (int l = 0; l < kS; ++l)
+            for (int k0 = 0; k0 < (l + 1) * np; k0 += kPiece, c += (size_t)nao * n)
+                G64_CUBLAS(cublasGemmEx(hb, CUBLAS_OP_N, CUBLAS_OP_N, n, nao,
+                                        std::min(kPiece, (l + 1) * np - k0), &one,
+                                        A + (size_t)k0 * n, CUDA_R_16BF, n,
+                                        B + (size_t)(kS - 1 - l) * np + k0, CUDA_R_16BF,
+                                        kS * np, &zero, c, CUDA_R_32F, n,
+                                        CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT));
+        combine_points_kernel<<<dim3((n / 2 + 255) / 256, nao), 256, 0, s>>>(
+            C, nao, np, ld, n, ep, ec, F + g);
+        G64_CUDA(cudaGetLastError());
+    }
+    return 0;
+}
+
+int gemm64_k(cublasHandle_t hb, const double* X, const double* G, const double* w, int nao,
+             int64_t ld, int64_t npts, int accumulate, double* K, void* ws, cudaStream_t s) {
+    const int np = pad8(nao);
+    const int nchunk = (int)((npts + kKc - 1) / kKc);
+    const int gmax = (int)std::min<int64_t>((ld + kKc - 1) / kKc, kGroup);
+    char* p = static_cast<char*>(ws);
+    int* ex = reinterpret_cast<int*>(p); p += al(sizeof(int) * (size_t)gmax * np);
+    int* eg = reinterpret_cast<int*>(p); p += al(sizeof(int) * (size_t)gmax * np);
+    __nv_bfloat16* A = reinterpret_cast<__nv_bfloat16*>(p);
+    p += al((size_t)2 * kS * kKc * gmax * np);
+    __nv_bfloat16* B = reinterpret_cast<__nv_bfloat16*>(p);
+    p += al((size_t)2 * kS * kKc * gmax * np);
+    float* C = reinterpret_cast<float*>(p);
+    const float one = 1.0f, zero = 0.0f;
+    const long long slab = (long long)kS * kKc * np, nn = (long long)np * np;
+    for (int c0 = 0; c0 < nchunk; c0 += kGroup) {
+        const int nc = std::min(kGroup, nchunk - c0);
+        const dim3 grid(nc, np);
+        slice_chunk_kernel<false><<<grid, 256, 0, s>>>(X, w, nao, ld, npts, (int64_t)c0 * kKc,
+                                                       ex, A);
+        G64_CUDA(cudaGetLastError());
+        slice_chunk_kernel<true><<<grid, 256, 0, s>>>(G, w, nao, ld, npts, (int64_t)c0 * kKc,
+                                                      eg, B);
+        G64_CUDA(cudaGetLastError());
+        float* c = C;
+        for (int l = 0; l < kS; ++l)
+            for (int k0 = 0; k0 < (l + 1) * kKc; k0 += kPiece, c += (size_t)nc * nn)
+                G64_CUBLAS(cublasGemmStridedBatchedEx(
+                    hb, CUBLAS_OP_T, CUBLAS_OP_N, np, np, std::min(kPiece, (l + 1) * kKc - k0),
+                    &one, A + k0, CUDA_R_16BF, kS * kKc, slab,
+                    B + (size_t)(kS - 1 - l) * kKc + k0, CUDA_R_16BF, kS * kKc, slab, &zero, c,
+                    CUDA_R_32F, np, nn, nc, CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT));
+        combine_chunks_kernel<<<dim3((nao + 127) / 128, nao), 128, 0, s>>>(
+            C, nao, np, nc, ex, eg, accumulate || c0 > 0, K);
+        G64_CUDA(cudaGetLastError());
+    }
+    return 0;
+}
+
+}  // namespace wb

@@ -177,20 +177,18 @@ def vv10_prepare(eng, g, D, nlc_pars, gemm='fp64'):
     if gemm not in ('fp64', 'split64', 'fp32'):
         raise ValueError("gemm must be 'fp64', 'split64' or 'fp32'")
     n = g.n
-    ao = g.X[:, :, :n]
     w = g.weights
     if gemm == 'fp32':
-        T = eng.ozaki_f(g.X[0], D)[:, :n].to(torch.float64)
+        T = eng.ozaki_f(g.X[0], D)
     elif gemm == 'split64':
-        T = eng.ozaki_f(g.X[0], D, fp64=True)[:, :n]
+        T = eng.ozaki_f(g.X[0], D, fp64=True)
     else:
-        T = D @ ao[0]
-    rho0 = (T * ao[0]).sum(dim=0)
-    grad = 2.0 * torch.einsum('mp,dmp->dp', T, ao[1:4])
-    ind = rho0 >= THRESH
+        T = eng.gemm64_f(g.X[0], D.T)
+    rho = eng.gga_rho(g.X, T, n)                          # (4, ld)
+    ind = torch.nonzero(rho[0, :n] >= THRESH).squeeze(1)
     q, W0, kappa, dW0dR, dW0dG, dKdR, Beta = vv10_pointwise(
-        rho0[ind], grad[:, ind], w[ind], nlc_pars)
-    return dict(eng=eng, g=g, gemm=gemm, n=n, rho0=rho0, grad=grad, ind=ind,
+        rho[0, ind], rho[1:4, ind], w[ind], nlc_pars)
+    return dict(eng=eng, g=g, gemm=gemm, n=n, rho=rho, ind=ind,
                 xyz=g.coords[ind].to(torch.float32), q=q, W0=W0, kappa=kappa,
                 dW0dR=dW0dR, dW0dG=dW0dG, dKdR=dKdR, Beta=Beta)
 
@@ -199,34 +197,22 @@ def vv10_finish(st, F, U, W):
     """E_nl and V_nl from a vv10_prepare state and the double sums F, U, W
     of its points."""
     torch = _torch()
-    g, n, ind, w = st['g'], st['n'], st['ind'], st['g'].weights
-    ao = g.X[:, :, :n]
+    eng, g, n, ind, rho = (st[k] for k in ('eng', 'g', 'n', 'ind', 'rho'))
+    w = g.weights
     Beta = st['Beta']
-    dev = st['rho0'].device
-    exc = torch.zeros(n, dtype=torch.float64, device=dev)
-    v0 = torch.zeros_like(exc)
-    v1 = torch.zeros_like(exc)
+    exc = torch.zeros(n, dtype=torch.float64, device=rho.device)
     exc[ind] = Beta + 0.5 * F
-    v0[ind] = Beta + F + 1.5 * (U * st['dKdR'] + W * st['dW0dR'])
-    v1[ind] = 1.5 * W * st['dW0dG']
-    e_nl = (st['rho0'] * w * exc).sum()
-    grad = st['grad']
-    if st['gemm'] != 'fp64':
-        # G = 1/2 v0 X0 + sum_d 2 v1 grad_d X_d, then X0^T (w o G), G FP64
-        # or rounded once to FP32
-        vv = torch.empty((4, n), dtype=torch.float64, device=dev)
-        vv[0] = 0.5 * v0
-        vv[1:4] = 2.0 * v1[None, :] * grad
-        dt = torch.float32 if st['gemm'] == 'fp32' else torch.float64
-        G = torch.zeros_like(g.X[0], dtype=dt)
-        G[:, :n] = torch.einsum('dmp,dp->mp', ao, vv).to(dt)
-        vmat = st['eng'].ozaki_k(g.X[0], G, w)
-        return e_nl, vmat + vmat.T
-    wv = torch.empty((4, n), dtype=torch.float64, device=dev)
-    wv[0] = 0.5 * v0 * w
-    wv[1:4] = 2.0 * v1[None, :] * grad * w[None, :]
-    aow = torch.einsum('dmp,dp->mp', ao, wv)
-    vmat = ao[0] @ aow.T
+    e_nl = (rho[0, :n] * w * exc).sum()
+    # G = 1/2 v0 X0 + sum_d 2 v1 grad_d X_d, then X0^T (w o G); G FP64, or
+    # rounded once to FP32 (gemm 'fp32')
+    vv = torch.zeros_like(rho)
+    vv[0, ind] = 0.5 * (Beta + F + 1.5 * (U * st['dKdR'] + W * st['dW0dR']))
+    vv[1:4, ind] = (3.0 * W * st['dW0dG'])[None, :] * rho[1:4, ind]
+    G = eng.gga_aow(g.X, vv, n, torch.float32 if st['gemm'] == 'fp32' else None)
+    if st['gemm'] == 'fp64':
+        vmat = eng.gemm64_k(g.X[0], G, w)
+    else:
+        vmat = eng.ozaki_k(g.X[0], G, w)
     return e_nl, vmat + vmat.T
 
 
@@ -239,7 +225,7 @@ def vv10_energy_fock(eng, g, D, nlc_pars, kernel=None, fp32=False, gemm='fp64'):
     GGA potential and vmat = X^T (w v) X + transpose.  Returns (E_nl
     device scalar, V_nl (nao, nao)).  The two GEMMs (D X and the Fock
     side) run as gemm:
-      'fp64'    plain FP64 GEMMs;
+      'fp64'    FP64 GEMMs (CosxEngine.gemm64_f / gemm64_k);
       'split64' the bf16 Ozaki split with FP64 operands and results (42
                 bits of the per-row / per-column maxima), the SCF's FP64
                 tail;
@@ -270,29 +256,24 @@ def gpu_nr_nlc_vxc(ctx, ni, mol, grids, xc_code, dm, relativity=0, hermi=1,
     coords = eng.relative(np.asarray(grids.coords, dtype=np.float64))
     w = torch.as_tensor(np.asarray(grids.weights, dtype=np.float64), device=dev)
     n = int(coords.shape[0])
-    ao = eng.ao_eval_deriv1(coords)[:, :, :n]             # (4, nao, n)
+    X = eng.ao_eval_deriv1(coords)                        # (4, nao, ld)
     D = torch.as_tensor(dm, device=dev)
-    T = D @ ao[0]                                         # (nao, n)
-    rho0 = (T * ao[0]).sum(dim=0)
-    grad = 2.0 * torch.einsum('mp,dmp->dp', T, ao[1:4])
-    nelec = float((rho0 * w).sum())
+    rho = eng.gga_rho(X, eng.gemm64_f(X[0], D.T), n)      # (4, ld)
+    rho0 = rho[0, :n]
     exc = torch.zeros(n, dtype=torch.float64, device=dev)
-    v0 = torch.zeros_like(exc)
-    v1 = torch.zeros_like(exc)
+    vv = torch.zeros_like(rho)          # d/d rho (half of it) and d/d grad
     c32 = coords.to(torch.float32)
+    ind = torch.nonzero(rho0 >= THRESH).squeeze(1)
     for nlc_pars, fac in nlc_coefs:
-        ind = rho0 >= THRESH
         q, W0, kappa, dW0dR, dW0dG, dKdR, Beta = vv10_pointwise(
-            rho0[ind], grad[:, ind], w[ind], nlc_pars)
+            rho0[ind], rho[1:4, ind], w[ind], nlc_pars)
         F, U, W = ctx.kernel.kernel_sum(c32[ind], q, W0, kappa)
         exc[ind] += fac * (Beta + 0.5 * F)
-        v0[ind] += fac * (Beta + F + 1.5 * (U * dKdR + W * dW0dR))
-        v1[ind] += fac * (1.5 * W * dW0dG)
-    excsum = float((rho0 * w * exc).sum())
-    wv = torch.empty((4, n), dtype=torch.float64, device=dev)
-    wv[0] = 0.5 * v0 * w                                  # *.5 for vmat + vmat^T
-    wv[1:4] = 2.0 * v1[None, :] * grad * w[None, :]
-    aow = torch.einsum('dmp,dp->mp', ao, wv)
-    vmat = ao[0] @ aow.T
+        vv[0, ind] += (0.5 * fac) * (Beta + F + 1.5 * (U * dKdR + W * dW0dR))
+        vv[1:4, ind] += (3.0 * fac * W * dW0dG)[None, :] * rho[1:4, ind]
+    # vmat = X0^T (w o G) + its transpose, G = 1/2 v0 X0 + sum_d v_d X_d
+    vmat = eng.gemm64_k(X[0], eng.gga_aow(X, vv, n), w)
     vmat = vmat + vmat.T
+    nelec = float((rho0 * w).sum())
+    excsum = float((rho0 * w * exc).sum())
     return nelec, excsum, vmat.cpu().numpy()

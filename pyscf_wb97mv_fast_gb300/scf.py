@@ -265,16 +265,14 @@ class DeviceRKS:
 
     def _vmat(self, g, v, gemm):
         """X^T diag(w v) X over grid g (deriv-0 AO values), symmetric.
-        gemm: 'fp64' (plain FP64 GEMM), 'split64' (the bf16 Ozaki split
+        gemm: 'fp64' (FP64 GEMM, gemm64_k), 'split64' (the bf16 Ozaki split
         with the FP64 G = X v) or 'fp32' (the split with G rounded to
         FP32); True / False stand for 'fp64' / 'fp32'."""
         torch = _torch()
         gemm = _gemm_mode(gemm)
         X = g.X if g.deriv == 0 else g.X[0]
         if gemm == 'fp64':
-            wv = torch.zeros(g.ld, dtype=torch.float64, device=self.device)
-            wv[:g.n] = g.weights * v[:g.n]
-            M = (X * wv[None, :]) @ X.T
+            M = self.eng.gemm64_k(X, X, g.weights * v[:g.n])
         else:
             dt = torch.float32 if gemm == 'fp32' else torch.float64
             G = torch.zeros_like(X, dtype=dt)
@@ -287,7 +285,7 @@ class DeviceRKS:
         gemm = _gemm_mode(gemm)
         X = g.X if g.deriv == 0 else g.X[0]
         if gemm == 'fp64':
-            T = D @ X
+            T = self.eng.gemm64_f(X, D.T)
         elif gemm == 'split64':
             T = self.eng.ozaki_f(X, D, fp64=True)
         else:
