@@ -47,8 +47,11 @@ namespace wb {
 // F = X QD.  X (nao, ld) AO-major = column-major A (ld x nao) scaled per row
 // g; QD row-major = column-major Q (nao x nao) with Q(mu, l) = QD(l, mu);
 // B = Q^T scaled per column mu (= per row mu of Q).
-// A_all (ld x S*nao, col-major): column block i = slice i.
-// B_all (S*nao x nao, col-major): row block r = slice S-1-r.
+// A_all (ld x S*np, col-major): column block i = slice i.
+// B_all (S*np x nao, col-major): row block r = slice S-1-r.
+// np = nao rounded up to 8, the slices zero past nao: cuBLAS takes its
+// tensor-memory kernels only for operands with 16-byte rows (356 AOs x
+// 75,265 points: the seven level GEMMs 2.1 -> 0.6 ms).
 // ---------------------------------------------------------------------------
 // exponent of max_l |X(l, g)| per point g: eight rows in flight per thread
 __global__ void f_rowmax_kernel(const double* __restrict__ X, int nao,
@@ -77,25 +80,26 @@ __global__ void f_rowmax_kernel(const double* __restrict__ X, int nao,
 
 // slices of X: one thread per (row l, two points); bf16 pairs per store
 template<int S>
-__global__ void f_slice_x_kernel(const double* __restrict__ X, int nao,
+__global__ void f_slice_x_kernel(const double* __restrict__ X, int nao, int np,
                                  int64_t ld, const int* __restrict__ erow,
                                  __nv_bfloat16* __restrict__ A) {
     const int l = blockIdx.y;
     const int64_t g = 2 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
     if (g >= ld) return;                    // ld is even (a multiple of 32)
-    const double2 x = *reinterpret_cast<const double2*>(X + (int64_t)l * ld + g);
+    double2 x = make_double2(0.0, 0.0);
+    if (l < nao) x = *reinterpret_cast<const double2*>(X + (int64_t)l * ld + g);
     const int2 e = *reinterpret_cast<const int2*>(erow + g);
     float d0[S], d1[S];
     digits<S>(x.x, e.x, d0);
     digits<S>(x.y, e.y, d1);
 #pragma unroll
     for (int i = 0; i < S; ++i)
-        *reinterpret_cast<__nv_bfloat162*>(A + ((int64_t)i * nao + l) * ld + g) =
+        *reinterpret_cast<__nv_bfloat162*>(A + ((int64_t)i * np + l) * ld + g) =
             __floats2bfloat162_rn(d0[i], d1[i]);
 }
 
 template<int S>
-__global__ void f_slice_qd_kernel(const double* __restrict__ QD, int nao,
+__global__ void f_slice_qd_kernel(const double* __restrict__ QD, int nao, int np,
                                   int* __restrict__ ecol,
                                   __nv_bfloat16* __restrict__ B) {
     // one block per column mu of B = Q^T, i.e. QD(:, mu)
@@ -117,13 +121,13 @@ __global__ void f_slice_qd_kernel(const double* __restrict__ QD, int nao,
     }
     const int e = exp_of_bits(red[0]);
     if (threadIdx.x == 0) ecol[mu] = e;
-    const int64_t ldb = (int64_t)S * nao;
-    for (int l = threadIdx.x; l < nao; l += blockDim.x) {
+    const int64_t ldb = (int64_t)S * np;
+    for (int l = threadIdx.x; l < np; l += blockDim.x) {
         float d[S];
-        digits<S>(QD[(int64_t)l * nao + mu], e, d);
+        digits<S>(l < nao ? QD[(int64_t)l * nao + mu] : 0.0, e, d);
 #pragma unroll
         for (int i = 0; i < S; ++i)
-            B[(int64_t)mu * ldb + (int64_t)(S - 1 - i) * nao + l] =
+            B[(int64_t)mu * ldb + (int64_t)(S - 1 - i) * np + l] =
                 __float2bfloat16_rn(d[i]);
     }
 }
@@ -169,12 +173,14 @@ __global__ void f_combine_kernel(const float* __restrict__ C, int nao,
 // B_c(k, nu) = w_k G[nu, c KC + k]; layouts (col-major, ld = S KC):
 //   A: column mu = [slice 0 (KC) | slice 1 | ... ]     (ascending)
 //   B: column nu = [slice S-1 | ... | slice 0]          (descending)
-// chunk stride S KC nao.  One CTA of 256 threads per (chunk, column).
+// chunk stride S KC np (np = nao rounded up to 8, the columns past nao zero:
+// 16-byte rows and outputs, as for F).  One CTA of KC / 8 threads per (chunk,
+// column).
 // ---------------------------------------------------------------------------
 // DOX = false: the X slices and exponents of this tile are already in A /
 // ex (an earlier omega of the same tile); only w o G is sliced.  B holds nb
 // columns per chunk (several right-hand sides side by side); this launch
-// fills columns boff .. boff + nao - 1.
+// fills columns boff .. boff + np - 1 (np = gridDim.y).
 template<int S, int KC, bool DOX, typename GT>
 __global__ void __launch_bounds__(KC / 8, 4)
 k_slice_kernel(const double* __restrict__ X, const GT* __restrict__ G,
@@ -183,13 +189,14 @@ k_slice_kernel(const double* __restrict__ X, const GT* __restrict__ G,
                __nv_bfloat16* __restrict__ A, __nv_bfloat16* __restrict__ B,
                int nb, int boff) {
     constexpr int T = KC / 8;               // threads: eight points each
-    const int c = blockIdx.x, col = blockIdx.y;
+    const int c = blockIdx.x, col = blockIdx.y, np = gridDim.y;
+    const int64_t nlive = col < nao ? npts : 0;     // a column past nao is zero
     __shared__ unsigned long long rx[T / 32], rw[T / 32];
     const int k0 = 8 * threadIdx.x;
     const int64_t g0 = (int64_t)c * KC + k0;
     double xv[8], wv[8];
     unsigned long long mx = 0, mw = 0;
-    if (g0 + 8 <= npts) {
+    if (g0 + 8 <= nlive) {
         const double2* xp = reinterpret_cast<const double2*>(X + (int64_t)col * ld + g0);
         const double2* wp = reinterpret_cast<const double2*>(w + g0);
         double gv[8];
@@ -225,7 +232,7 @@ k_slice_kernel(const double* __restrict__ X, const GT* __restrict__ G,
             const int64_t g = g0 + u;
             xv[u] = 0.0;
             wv[u] = 0.0;
-            if (g < npts) {
+            if (g < nlive) {
                 if (DOX) xv[u] = X[(int64_t)col * ld + g];
                 wv[u] = w[g] * (double)G[(int64_t)col * ld + g];
             }
@@ -258,10 +265,10 @@ k_slice_kernel(const double* __restrict__ X, const GT* __restrict__ G,
     }
     const int e1 = exp_of_bits(mx), e2 = exp_of_bits(mw);
     if (threadIdx.x == 0) {
-        if (DOX) ex[(int64_t)c * nao + col] = e1;
+        if (DOX) ex[(int64_t)c * np + col] = e1;
         ew[(int64_t)c * nb + boff + col] = e2;
     }
-    const int64_t colbase = (int64_t)c * S * KC * nao + (int64_t)col * S * KC;
+    const int64_t colbase = (int64_t)c * S * KC * np + (int64_t)col * S * KC;
     const int64_t colbase_b = (int64_t)c * S * KC * nb + (int64_t)(boff + col) * S * KC;
     // one operand's digits at a time: the X slices, then the w o G ones
     // (half the live registers of both at once)
@@ -284,20 +291,21 @@ k_slice_kernel(const double* __restrict__ X, const GT* __restrict__ G,
 }
 
 // K_r[mu, nu] (+)= sum_c 2^(ex+ew-2W+2+B(S-1)) [sum_l C[l][c] 2^(B (S-1-l))]
-// for the nb / nao right-hand sides r (column r nao + nu of C)
+// for the nb / np right-hand sides r (column r np + nu of C)
 struct KOut {
     double* k[8];
 };
 
 template<int S>
-__global__ void k_combine_kernel(const float* __restrict__ C, int nao, int nb,
+__global__ void k_combine_kernel(const float* __restrict__ C, int nao, int np, int nb,
                                  int nchunk, const int* __restrict__ ex,
                                  const int* __restrict__ ew, int accumulate,
                                  const KOut Ks) {
-    const int64_t nc = (int64_t)nao * nb;
+    const int64_t nc = (int64_t)np * nb;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nc;
          i += (int64_t)gridDim.x * blockDim.x) {
-        const int mu = (int)(i % nao), col = (int)(i / nao);   // C col-major
+        const int mu = (int)(i % np), col = (int)(i / np);     // C col-major
+        if (mu >= nao || col % np >= nao) continue;
         double acc = 0.0;
         // four chunks' loads in flight at once; the sum stays in chunk order
         constexpr int U = 4;
@@ -310,7 +318,7 @@ __global__ void k_combine_kernel(const float* __restrict__ C, int nao, int nb,
 #pragma unroll
                 for (int l = 0; l < S; ++l)
                     v[u][l] = __ldg(C + ((int64_t)l * nchunk + c + u) * nc + i);
-                sc[u] = ex[(int64_t)(c + u) * nao + mu] + ew[(int64_t)(c + u) * nb + col] -
+                sc[u] = ex[(int64_t)(c + u) * np + mu] + ew[(int64_t)(c + u) * nb + col] -
                         2 * kW + 2 + kB * (S - 1);
             }
 #pragma unroll
@@ -321,12 +329,12 @@ __global__ void k_combine_kernel(const float* __restrict__ C, int nao, int nb,
 #pragma unroll
             for (int l = 0; l < S; ++l) v[l] = C[((int64_t)l * nchunk + c) * nc + i];
             const long long lv = combine_levels<S>(v);
-            const int sc = ex[(int64_t)c * nao + mu] + ew[(int64_t)c * nb + col] -
+            const int sc = ex[(int64_t)c * np + mu] + ew[(int64_t)c * nb + col] -
                            2 * kW + 2 + kB * (S - 1);
             acc += (double)lv * pow2(sc);
         }
-        double* K = Ks.k[col / nao];
-        const int64_t o = (int64_t)mu * nao + col % nao;       // K row-major
+        double* K = Ks.k[col / np];
+        const int64_t o = (int64_t)mu * nao + col % np;        // K row-major
         K[o] = accumulate ? K[o] + acc : acc;
     }
 }
@@ -334,22 +342,41 @@ __global__ void k_combine_kernel(const float* __restrict__ C, int nao, int nb,
 // ---------------------------------------------------------------------------
 static inline size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
 
+static inline int pad8(int n) { return (n + 7) & ~7; }
+
+// Points per chunk of the K product.  2048 is the largest with exact level
+// sums and moves the least level output per point; where it would leave SMs
+// idle (fewer than one 128 x 128 tile per SM over the chunks of a level GEMM),
+// 512 gives four times the tiles, each a quarter as long (48 AOs x 9,931
+// points: the seven GEMMs 89 -> 42 us).
+static inline int k_chunk(int np, int64_t ld) {
+    const int64_t t = (np + 127) / 128;
+    return t * t * ((ld + kOzKc - 1) / kOzKc) < sm_count() ? kOzKcSmall : kOzKc;
+}
+
 size_t ozaki_f_bytes(int nao, int64_t ld) {
-    const size_t S = kOzSlices;
+    const size_t S = kOzSlices, np = pad8(nao);
     const size_t lib = al(sizeof(int) * ld) + al(sizeof(int) * nao) +
-                       al(sizeof(__nv_bfloat16) * S * nao * ld) +
-                       al(sizeof(__nv_bfloat16) * S * nao * nao) +
+                       al(sizeof(__nv_bfloat16) * S * np * ld) +
+                       al(sizeof(__nv_bfloat16) * S * np * nao) +
                        al(sizeof(float) * S * nao * ld);
     return std::max(lib, ozaki_f_tc_bytes(nao, ld));
 }
 
 size_t ozaki_k_bytes(int nao, int64_t ld, int nrhs) {
-    const size_t S = kOzSlices;
-    const int64_t nchunk = (ld + kOzKc - 1) / kOzKc;
-    return al(sizeof(int) * nchunk * nao) + al(sizeof(int) * nchunk * nao * nrhs) +
-           al(sizeof(__nv_bfloat16) * S * kOzKc * nchunk * nao) +
-           al(sizeof(__nv_bfloat16) * S * kOzKc * nchunk * nao * nrhs) +
-           al(sizeof(float) * S * nchunk * (size_t)nao * nao * nrhs);
+    const size_t S = kOzSlices, np = pad8(nao);
+    auto bytes = [&](size_t kc, int64_t n) {
+        const size_t nchunk = (n + kc - 1) / kc;
+        return al(sizeof(int) * nchunk * np) + al(sizeof(int) * nchunk * np * nrhs) +
+               al(sizeof(__nv_bfloat16) * S * kc * nchunk * np) +
+               al(sizeof(__nv_bfloat16) * S * kc * nchunk * np * nrhs) +
+               al(sizeof(float) * S * nchunk * np * np * nrhs);
+    };
+    // enough for every grid of up to ld points (a ragged last tile may take
+    // the small chunks where the full one does not)
+    const int64_t t = ((int64_t)np + 127) / 128;
+    const int64_t small = std::min(ld, (sm_count() - 1) / (t * t) * (int64_t)kOzKc);
+    return std::max(bytes(kOzKc, ld), bytes(kOzKcSmall, small));
 }
 
 #define OZ_CUBLAS(call)                                        \
@@ -394,30 +421,31 @@ template<typename T>
 static int f_gemm_cublas_t(cublasHandle_t hb, const double* X, const double* QD,
                            int nao, int64_t ld, T* F, void* ws, cudaStream_t s) {
     constexpr int S = kOzSlices;
+    const int np = pad8(nao);
     char* p = static_cast<char*>(ws);
     int* erow = reinterpret_cast<int*>(p); p += al(sizeof(int) * ld);
     int* ecol = reinterpret_cast<int*>(p); p += al(sizeof(int) * nao);
     __nv_bfloat16* A = reinterpret_cast<__nv_bfloat16*>(p);
-    p += al(sizeof(__nv_bfloat16) * (size_t)S * nao * ld);
+    p += al(sizeof(__nv_bfloat16) * (size_t)S * np * ld);
     __nv_bfloat16* B = reinterpret_cast<__nv_bfloat16*>(p);
-    p += al(sizeof(__nv_bfloat16) * (size_t)S * nao * nao);
+    p += al(sizeof(__nv_bfloat16) * (size_t)S * np * nao);
     float* C = reinterpret_cast<float*>(p);
     f_rowmax_kernel<<<(unsigned)((ld + 255) / 256), 256, 0, s>>>(X, nao, ld, erow);
     OZ_CUDA(cudaGetLastError());
     {
-        dim3 grid((unsigned)((ld / 2 + 255) / 256), (unsigned)nao);
-        f_slice_x_kernel<S><<<grid, 256, 0, s>>>(X, nao, ld, erow, A);
+        dim3 grid((unsigned)((ld / 2 + 255) / 256), (unsigned)np);
+        f_slice_x_kernel<S><<<grid, 256, 0, s>>>(X, nao, np, ld, erow, A);
         OZ_CUDA(cudaGetLastError());
     }
-    f_slice_qd_kernel<S><<<nao, 256, 0, s>>>(QD, nao, ecol, B);
+    f_slice_qd_kernel<S><<<nao, 256, 0, s>>>(QD, nao, np, ecol, B);
     OZ_CUDA(cudaGetLastError());
     const float one = 1.0f, zero = 0.0f;
     for (int l = 0; l < S; ++l) {
-        // C_l (ld x nao) = A[:, 0:(l+1) nao] * B[(S-1-l) nao : S nao, :]
+        // C_l (ld x nao) = A[:, 0:(l+1) np] * B[(S-1-l) np : S np, :]
         OZ_CUBLAS(cublasGemmEx(hb, CUBLAS_OP_N, CUBLAS_OP_N, (int)ld, nao,
-                               (l + 1) * nao, &one, A, CUDA_R_16BF, (int)ld,
-                               B + (size_t)(S - 1 - l) * nao, CUDA_R_16BF,
-                               S * nao, &zero, C + (size_t)l * nao * ld,
+                               (l + 1) * np, &one, A, CUDA_R_16BF, (int)ld,
+                               B + (size_t)(S - 1 - l) * np, CUDA_R_16BF,
+                               S * np, &zero, C + (size_t)l * nao * ld,
                                CUDA_R_32F, (int)ld, CUBLAS_COMPUTE_32F,
                                CUBLAS_GEMM_DEFAULT));
     }
@@ -439,20 +467,20 @@ int ozaki_f_gemm_cublas64(cublasHandle_t hb, const double* X, const double* QD,
     return f_gemm_cublas_t<double>(hb, X, QD, nao, ld, F, ws, s);
 }
 
-template<typename GT>
+template<int KC, typename GT>
 static int k_gemm_multi_t(cublasHandle_t hb, const double* X, const GT* const* G,
                           int nrhs, const double* w, int nao, int64_t ld,
                           int64_t npts, int accumulate, double* const* K, void* ws,
                           cudaStream_t s, bool x_sliced) {
-    constexpr int S = kOzSlices, KC = kOzKc;
+    constexpr int S = kOzSlices;
     if (nrhs < 1 || nrhs > 8) return (int)cudaErrorInvalidValue;
     const int nchunk = (int)((ld + KC - 1) / KC);
-    const int nb = nrhs * nao;
+    const int np = pad8(nao), nb = nrhs * np;
     // the X side (ex, A) first, at offsets independent of nrhs, so that a
     // later call with x_sliced finds them whatever its nrhs
     char* p = static_cast<char*>(ws);
-    int* ex = reinterpret_cast<int*>(p); p += al(sizeof(int) * (size_t)nchunk * nao);
-    const size_t slab = (size_t)S * KC * nchunk * nao;
+    int* ex = reinterpret_cast<int*>(p); p += al(sizeof(int) * (size_t)nchunk * np);
+    const size_t slab = (size_t)S * KC * nchunk * np;
     __nv_bfloat16* A = reinterpret_cast<__nv_bfloat16*>(p);
     p += al(sizeof(__nv_bfloat16) * slab);
     int* ew = reinterpret_cast<int*>(p); p += al(sizeof(int) * (size_t)nchunk * nb);
@@ -461,48 +489,58 @@ static int k_gemm_multi_t(cublasHandle_t hb, const double* X, const GT* const* G
     float* C = reinterpret_cast<float*>(p);
     KOut Kd = {};
     for (int r = 0; r < nrhs; ++r) Kd.k[r] = K[r];
-    dim3 grid(nchunk, nao);
+    dim3 grid(nchunk, np);
     for (int r = 0; r < nrhs; ++r) {
         if (x_sliced || r > 0)
             k_slice_kernel<S, KC, false, GT><<<grid, KC / 8, 0, s>>>(
-                X, G[r], w, nao, ld, npts, ex, ew, A, B, nb, r * nao);
+                X, G[r], w, nao, ld, npts, ex, ew, A, B, nb, r * np);
         else
             k_slice_kernel<S, KC, true, GT><<<grid, KC / 8, 0, s>>>(
-                X, G[r], w, nao, ld, npts, ex, ew, A, B, nb, r * nao);
+                X, G[r], w, nao, ld, npts, ex, ew, A, B, nb, r * np);
         OZ_CUDA(cudaGetLastError());
     }
     const float one = 1.0f, zero = 0.0f;
-    const long long stride_a = (long long)S * KC * nao;
+    const long long stride_a = (long long)S * KC * np;
     const long long stride_b = (long long)S * KC * nb;
-    const long long nc = (long long)nao * nb;
+    const long long nc = (long long)np * nb;
     for (int l = 0; l < S; ++l) {
         OZ_CUBLAS(cublasGemmStridedBatchedEx(
-            hb, CUBLAS_OP_T, CUBLAS_OP_N, nao, nb, (l + 1) * KC, &one, A,
+            hb, CUBLAS_OP_T, CUBLAS_OP_N, np, nb, (l + 1) * KC, &one, A,
             CUDA_R_16BF, S * KC, stride_a, B + (size_t)(S - 1 - l) * KC,
             CUDA_R_16BF, S * KC, stride_b, &zero, C + (size_t)l * nchunk * nc,
-            CUDA_R_32F, nao, nc, nchunk, CUBLAS_COMPUTE_32F,
+            CUDA_R_32F, np, nc, nchunk, CUBLAS_COMPUTE_32F,
             CUBLAS_GEMM_DEFAULT));
     }
     const int64_t blocks = grid_stride_blocks(nc, 256, 32);
-    k_combine_kernel<S><<<(unsigned)blocks, 256, 0, s>>>(C, nao, nb, nchunk, ex, ew,
+    k_combine_kernel<S><<<(unsigned)blocks, 256, 0, s>>>(C, nao, np, nb, nchunk, ex, ew,
                                                         accumulate, Kd);
     OZ_CUDA(cudaGetLastError());
     return 0;
+}
+
+template<typename GT>
+static int k_gemm_any(cublasHandle_t hb, const double* X, const GT* const* G, int nrhs,
+                      const double* w, int nao, int64_t ld, int64_t npts, int accumulate,
+                      double* const* K, void* ws, cudaStream_t s, bool x_sliced) {
+    return k_chunk(pad8(nao), ld) == kOzKc
+               ? k_gemm_multi_t<kOzKc, GT>(hb, X, G, nrhs, w, nao, ld, npts, accumulate, K,
+                                           ws, s, x_sliced)
+               : k_gemm_multi_t<kOzKcSmall, GT>(hb, X, G, nrhs, w, nao, ld, npts, accumulate,
+                                                K, ws, s, x_sliced);
 }
 
 int ozaki_k_gemm_multi(cublasHandle_t hb, const double* X, const float* const* G,
                        int nrhs, const double* w, int nao, int64_t ld,
                        int64_t npts, int accumulate, double* const* K, void* ws,
                        cudaStream_t s, bool x_sliced) {
-    return k_gemm_multi_t<float>(hb, X, G, nrhs, w, nao, ld, npts, accumulate, K, ws, s,
-                                 x_sliced);
+    return k_gemm_any<float>(hb, X, G, nrhs, w, nao, ld, npts, accumulate, K, ws, s,
+                             x_sliced);
 }
 
 int ozaki_k_gemm64(cublasHandle_t hb, const double* X, const double* G,
                    const double* w, int nao, int64_t ld, int64_t npts,
                    int accumulate, double* K, void* ws, cudaStream_t s) {
-    return k_gemm_multi_t<double>(hb, X, &G, 1, w, nao, ld, npts, accumulate, &K, ws, s,
-                                  false);
+    return k_gemm_any<double>(hb, X, &G, 1, w, nao, ld, npts, accumulate, &K, ws, s, false);
 }
 
 int ozaki_k_gemm(cublasHandle_t hb, const double* X, const float* G,

@@ -11,6 +11,7 @@ namespace wb {
 constexpr int kOzBits = 6;     // balanced digits, |d| <= 32
 constexpr int kOzSlices = 7;   // 42 bits per operand
 constexpr int kOzKc = 2048;    // K-GEMM chunk: (l + 1) * Kc < 2^14 for l < 7
+constexpr int kOzKcSmall = 512;     // where 2048-point chunks would leave SMs idle
 
 // exact FP32 level sums need kOzSlices * K < 2^14 along the inner dimension
 inline bool ozaki_f_supported(int nao) { return kOzSlices * nao < (1 << 14); }
