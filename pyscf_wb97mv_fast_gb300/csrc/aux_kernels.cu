@@ -2,6 +2,7 @@
 // grid coordinate split, sub-block statistics for the screen, FP64 AO
 // evaluation, precision casts, the dense validation kernel and the Boys
 // batch kernel.
+#include <algorithm>
 #include <cmath>
 
 #include "boys.cuh"
@@ -180,6 +181,11 @@ __device__ __forceinline__ float4 centroid_radius(const double* sum, int n,
                        (float)(sum[2] / n), r);
 }
 
+// The shells are shared out over gridDim.y: one warp walking all of them is a
+// serial chain of loads (70 us for the 24 shells and 9,931 points of two
+// waters, a third of the HBM rate on large grids).
+constexpr int kStatsShells = 6;
+
 __global__ void sub_stats_kernel(const BlockStatsOut O,
                                  const double* __restrict__ coords,
                                  const double* __restrict__ w,
@@ -191,6 +197,9 @@ __global__ void sub_stats_kernel(const BlockStatsOut O,
     const int lane = threadIdx.x & 31;
     const int nblk128 = (int)((ld + 127) / 128);
     if (blk >= nblk128) return;
+    // this CTA's share of the shells; the first share also writes the centroids
+    const int sh0 = blockIdx.y * kStatsShells;
+    const int sh1 = min(nvshell, sh0 + kStatsShells);
     // blocks of each level that exist: 32 * 2^k points starting inside ld
     int64_t g[4];
     bool valid[4];
@@ -201,49 +210,51 @@ __global__ void sub_stats_kernel(const BlockStatsOut O,
         valid[q] = g[q] < npts;
         for (int x = 0; x < 3; ++x) c[q][x] = valid[q] ? coords[g[q] * 3 + x] : 0.0;
     }
-    int nv[4];
+    if (blockIdx.y == 0) {
+        int nv[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int64_t rem = npts - ((int64_t)blk * 128 + 32 * q);
-        nv[q] = rem >= 32 ? 32 : (rem > 0 ? (int)rem : 0);
-    }
-    double s[4][3];
+        for (int q = 0; q < 4; ++q) {
+            const int64_t rem = npts - ((int64_t)blk * 128 + 32 * q);
+            nv[q] = rem >= 32 ? 32 : (rem > 0 ? (int)rem : 0);
+        }
+        double s[4][3];
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-        for (int x = 0; x < 3; ++x) s[q][x] = warp_sum_d(c[q][x]);
-    // level k = 0, 1, 2: block j of the level covers quarters [j 2^k, (j+1) 2^k)
+        for (int q = 0; q < 4; ++q)
+            for (int x = 0; x < 3; ++x) s[q][x] = warp_sum_d(c[q][x]);
+        // level k = 0, 1, 2: block j of the level covers quarters [j 2^k, (j+1) 2^k)
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int span = 1 << k;
+        for (int k = 0; k < 3; ++k) {
+            const int span = 1 << k;
 #pragma unroll
-        for (int j = 0; j < 4 / span; ++j) {
-            double sum[3] = {0.0, 0.0, 0.0};
-            int n = 0;
-            for (int q = j * span; q < (j + 1) * span; ++q) {
-                for (int x = 0; x < 3; ++x) sum[x] += s[q][x];
-                n += nv[q];
-            }
-            double m[3];
-            for (int x = 0; x < 3; ++x) m[x] = n ? sum[x] / n : 0.0;
-            double d = 0.0;
-            for (int q = j * span; q < (j + 1) * span; ++q) {
-                if (!valid[q]) continue;
-                double e2 = 0.0;
-                for (int x = 0; x < 3; ++x) {
-                    const double e = c[q][x] - m[x];
-                    e2 += e * e;
+            for (int j = 0; j < 4 / span; ++j) {
+                double sum[3] = {0.0, 0.0, 0.0};
+                int n = 0;
+                for (int q = j * span; q < (j + 1) * span; ++q) {
+                    for (int x = 0; x < 3; ++x) sum[x] += s[q][x];
+                    n += nv[q];
                 }
-                d = fmax(d, sqrt(e2));
+                double m[3];
+                for (int x = 0; x < 3; ++x) m[x] = n ? sum[x] / n : 0.0;
+                double d = 0.0;
+                for (int q = j * span; q < (j + 1) * span; ++q) {
+                    if (!valid[q]) continue;
+                    double e2 = 0.0;
+                    for (int x = 0; x < 3; ++x) {
+                        const double e = c[q][x] - m[x];
+                        e2 += e * e;
+                    }
+                    d = fmax(d, sqrt(e2));
+                }
+                d = warp_max_d(d);
+                const int64_t b = (int64_t)blk * (4 / span) + j;
+                if (lane == 0 && b * 32 * span < ld) O.cr[k][b] = centroid_radius(sum, n, d);
             }
-            d = warp_max_d(d);
-            const int64_t b = (int64_t)blk * (4 / span) + j;
-            if (lane == 0 && b * 32 * span < ld) O.cr[k][b] = centroid_radius(sum, n, d);
         }
     }
     float wq[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) wq[q] = valid[q] ? (float)w[g[q]] : 0.0f;
-    for (int sh = 0; sh < nvshell; ++sh) {
+    for (int sh = sh0; sh < sh1; ++sh) {
         const int a0 = vs_ao0[sh], nf = vs_nf[sh];
         float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         for (int t = 0; t < nf; ++t) {
@@ -281,7 +292,9 @@ cudaError_t launch_sub_stats(const double* coords, const double* weights,
     const int64_t nblk = (ld + 127) / 128;
     if (nblk <= 0) return cudaSuccess;
     const int warps = 4;
-    sub_stats_kernel<<<(unsigned)((nblk + warps - 1) / warps), 32 * warps, 0, s>>>(
+    const dim3 grid((unsigned)((nblk + warps - 1) / warps),
+                    (unsigned)std::max(1, (nvshell + kStatsShells - 1) / kStatsShells));
+    sub_stats_kernel<<<grid, 32 * warps, 0, s>>>(
         out, coords, weights, F, npts, ld, nvshell, vs_ao0, vs_nf);
     return cudaGetLastError();
 }
