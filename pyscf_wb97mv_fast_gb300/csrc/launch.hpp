@@ -56,7 +56,8 @@ int cosx_class_blocks_per_sm(int cls, bool far, size_t stage_smem,
 struct AoArgs {
     const double* coords;       // (npts, 3) molecule frame
     int64_t npts, ld;
-    int nbas;
+    int ncentre;                // runs of shells with one centre and
+    const int* centre;          // consecutive AOs: first shells (ncentre + 1)
     const int* sh_l;
     const int* sh_np;
     const int* sh_nc;
@@ -76,7 +77,7 @@ cudaError_t upload_c2s_tables(const double* t0, const double* t1,
                               const double* t2, const double* t3);
 cudaError_t upload_c2s_f(const float* all /* 4 x 70 */);
 // 2^(-j/64), j = 0..63, for the AO kernels' exp
-cudaError_t upload_exp_table(const double* t64);
+cudaError_t upload_exp_table(const unsigned long long* t64);
 
 // class ranges and record layout for launch_pack_records (classes with no
 // primitive pairs have pp_begin == pp_end)
