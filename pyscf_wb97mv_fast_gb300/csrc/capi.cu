@@ -210,7 +210,7 @@ struct wb_cosx {
     double* f64_P = nullptr;
     double* f64_E = nullptr;
     double* f64_boys = nullptr;
-    double* f64_fine = nullptr;      // the fine-node Boys table (fp64_boys.cuh)
+    double* f64_fine = nullptr;      // the fine-node Boys and exp tables (fp64_boys.cuh)
     long long f64_ebase[wb::NCLASS] = {0};
     double* f64_alpha = nullptr;     // bra exponent per primitive pair
     double* f64_vsxyz = nullptr;     // virtual shell centres (3 each)
@@ -709,6 +709,12 @@ int ensure_fp64(wb_cosx* h) {
         for (int k = 0; k < wb::kBoysFineNodes; ++k)
             wb::boys_f64(wb::kBoysFineCols - 1, k / 32.0,
                          t.data() + (size_t)k * wb::kBoysFineCols);
+        const std::vector<unsigned long long> e = exp2m_table();
+        for (unsigned long long v : e) {
+            double d;
+            std::memcpy(&d, &v, sizeof(d));
+            t.push_back(d);
+        }
         return t;
     }();
     std::vector<double> vxyz;
@@ -827,6 +833,7 @@ int64_t hartree_ndh(const wb::HostPairs& hp) {
 struct WsLayout64 {
     WsLayout base;                  // counters, work, block statistics
     size_t X = 0, F64 = 0, F32 = 0, G64 = 0, rec = 0, gemm = 0, total = 0;
+    int nseg = 1;                   // copies of G (f64_segments)
 };
 
 WsLayout64 ws_layout_fp64(const wb_cosx* h, int64_t ld) {
@@ -850,7 +857,8 @@ WsLayout64 ws_layout_fp64(const wb_cosx* h, int64_t ld) {
     L.X = take(sizeof(double) * n);
     L.F64 = take(sizeof(double) * n);
     L.F32 = take(sizeof(float) * n);
-    L.G64 = take(sizeof(double) * n);
+    L.nseg = wb::f64_segments(ld / 32, h->nsm);
+    L.G64 = take(sizeof(double) * n * L.nseg);
     L.gemm = take(wb::gemm64_bytes(nao64, ld));
     L.rec = take(sizeof(double) * wb::kF64Rec * (size_t)std::max(h->hp.npp, 1));
     L.total = off;
@@ -1516,6 +1524,8 @@ int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
     std::memset(&a, 0, sizeof(a));
     a.F = F64;
     a.G = G64;
+    a.gstride = (long long)nao * ld;
+    a.nseg = L.nseg;
     a.coords = coords;
     a.ld = ld;
     a.npts = (int)npts;
@@ -1547,7 +1557,7 @@ int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
     for (int j = 0; j < nomega; ++j) {
         WB_CUDA(wb::launch_f64_records(h->hp.npp, h->f64_P, h->p, h->pref, h->f64_alpha,
                                        omegas[j], rec, s));
-        WB_CUDA(cudaMemsetAsync(G64, 0, sizeof(double) * (size_t)nao * ld, s));
+        WB_CUDA(cudaMemsetAsync(G64, 0, sizeof(double) * (size_t)nao * ld * L.nseg, s));
         WB_CUDA(cudaMemsetAsync(a.work, 0, sizeof(int) * wb::NCLASS, s));
         launches += 3;
         for (int c = 0; c < wb::NCLASS; ++c) {
@@ -1557,6 +1567,8 @@ int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
             ++launches;
         }
         ntasks += (ld / 32) * (int64_t)h->hp.npairs;
+        WB_CUDA(wb::launch_f64_segment_sum(G64, (int64_t)nao * ld, L.nseg, s));
+        launches += L.nseg > 1;
         if ((st = gemm64_k(h, X, G64, weights, ld, npts, 0, k_out + kk * j, gemm, s)) !=
             WB_OK)
             return st;
@@ -1962,7 +1974,7 @@ GradLayout grad_layout(const wb_cosx* h, int64_t ld, int natm) {
             const wb::ClassRange& r = h->hp.cls[wb::class_of(la, lb)];
             ne += (int64_t)(r.pp_end - r.pp_begin) * 3 * wb::e64_axis(la, lb);
         }
-    const size_t sizes[4] = {4 * (size_t)h->hp.nao * ld, 3 * (size_t)natm * ld, (size_t)ne,
+    const size_t sizes[4] = {4 * (size_t)h->hp.nao * ld, 3 * (size_t)natm * ld * L.f64.nseg, (size_t)ne,
                              3 * (size_t)h->hp.nao};
     size_t* offs[4] = {&L.X, &L.gpt, &L.dE, &L.aodot};
     size_t off = L.f64.total;
@@ -2032,7 +2044,7 @@ int wb_cosx_k_grad(wb_cosx* h, const double* coords, const double* weights,
     // G = A F by the FP64 class kernels
     wb::CosxF64Args a;
     std::memset(&a, 0, sizeof(a));
-    a.F = F64; a.G = G64; a.coords = coords; a.ld = ld; a.npts = (int)npts;
+    a.F = F64; a.G = G64; a.gstride = (long long)n; a.nseg = L.nseg; a.coords = coords; a.ld = ld; a.npts = (int)npts;
     a.khdr = h->khdr; a.pshell = h->pshell; a.ptau = h->ptau;
     a.bnd = h->bnd; a.bpref = h->bpref; a.blk_cr = bo.cr[0]; a.blk_msh = bo.msh[0];
     a.nblk = nblk; a.nvshell = h->hp.nvshell; a.tol = tol;
@@ -2048,13 +2060,14 @@ int wb_cosx_k_grad(wb_cosx* h, const double* coords, const double* weights,
     WB_CUDA(cudaMemsetAsync(a.counters, 0, sizeof(unsigned long long) * kCounterWords, s));
     WB_CUDA(wb::launch_f64_records(h->hp.npp, h->f64_P, h->p, h->pref, h->f64_alpha, omega,
                                    rec, s));
-    WB_CUDA(cudaMemsetAsync(G64, 0, sizeof(double) * n, s));
+    WB_CUDA(cudaMemsetAsync(G64, 0, sizeof(double) * n * L.nseg, s));
     WB_CUDA(cudaMemsetAsync(work, 0, sizeof(int) * wb::NCLASS, s));
     for (int c = 0; c < wb::NCLASS; ++c) {
         const int pb = h->hp.cls[c].pair_begin, pe = h->hp.cls[c].pair_end;
         if (pe > pb) WB_CUDA(wb::launch_cosx_fp64_class(c, a, pb, pe, h->nsm, s));
     }
     // X side: 1/2 sum_g w_g sum_{mu on C} grad X_g,mu (G D)_g,mu
+    WB_CUDA(wb::launch_f64_segment_sum(G64, (int64_t)n, L.nseg, s));
     if ((st = gemm64_f(h, G64, dm, ld, H, gemm, s)) != WB_OK) return st;
     WB_CUDA(cudaMemsetAsync(grad_out, 0, sizeof(double) * 3 * (size_t)natm, s));
     WB_CUDA(wb::launch_ao_dot(Xd, H, weights, npts, ld, nao, aodot, s));
@@ -2068,7 +2081,8 @@ int wb_cosx_k_grad(wb_cosx* h, const double* coords, const double* weights,
     g.bnd = h->bnd; g.bpref = h->bpref; g.blk_cr = bo.cr[0]; g.blk_msh = bo.msh[0];
     g.nblk = nblk; g.nvshell = h->hp.nvshell; g.tol = tol;
     g.rec = rec; g.E = h->f64_E; g.dE = dE; g.vs_atom = h->vs_atom; g.boys = h->f64_fine;
-    g.c2s = a.c2s; g.gpt = gpt; g.work = work;
+    g.c2s = a.c2s; g.gpt = gpt; g.gstride = 3 * (long long)natm * ld; g.nseg = L.nseg;
+    g.work = work;
     wb::GradEArgs ge;
     ge.npairs = h->hp.npairs; ge.pclass = h->pclass; ge.hdr = h->hdr; ge.pshell = h->pshell;
     ge.p = h->p; ge.alpha = h->f64_alpha; ge.vs_xyz = h->f64_vsxyz; ge.dE = dE;
@@ -2077,13 +2091,13 @@ int wb_cosx_k_grad(wb_cosx* h, const double* coords, const double* weights,
         g.e_base[c] = ge.e_base[c] = h->f64_ebase[c];
     }
     WB_CUDA(wb::launch_grad_e(ge, s));
-    WB_CUDA(cudaMemsetAsync(gpt, 0, sizeof(double) * 3 * (size_t)natm * ld, s));
+    WB_CUDA(cudaMemsetAsync(gpt, 0, sizeof(double) * 3 * (size_t)natm * ld * L.nseg, s));
     WB_CUDA(cudaMemsetAsync(work, 0, sizeof(int) * wb::NCLASS, s));
     for (int c = 0; c < wb::NCLASS; ++c) {
         const int pb = h->hp.cls[c].pair_begin, pe = h->hp.cls[c].pair_end;
         if (pe > pb) WB_CUDA(wb::launch_cosx_grad64_class(c, g, pb, pe, h->nsm, s));
     }
-    WB_CUDA(wb::launch_grad_points_sum(gpt, weights, npts, ld, natm, grad_out, s));
+    WB_CUDA(wb::launch_grad_points_sum(gpt, weights, npts, ld, natm, L.nseg, grad_out, s));
     return WB_OK;
 }
 

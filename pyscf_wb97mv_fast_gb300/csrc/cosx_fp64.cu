@@ -2,6 +2,7 @@
 // class dispatcher and the per-omega records (the kernel itself is in
 // cosx_fp64.cuh).
 #include "cosx_fp64.cuh"
+#include "launch.hpp"
 
 namespace wb {
 
@@ -49,7 +50,28 @@ __global__ void f64_records_kernel(const int npp, const double* __restrict__ P,
     }
     r[12] = alpha[q] / pq;
 }
+
+__global__ void f64_segment_sum_kernel(double* __restrict__ G, const int64_t n,
+                                       const int nseg) {
+    for (int64_t i = 2 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x); i < n;
+         i += 2 * (int64_t)gridDim.x * blockDim.x) {
+        double2 a = *reinterpret_cast<const double2*>(G + i);
+        for (int s = 1; s < nseg; ++s) {
+            const double2 b = *reinterpret_cast<const double2*>(G + s * n + i);
+            a.x += b.x;
+            a.y += b.y;
+        }
+        *reinterpret_cast<double2*>(G + i) = a;
+    }
+}
 }  // namespace
+
+cudaError_t launch_f64_segment_sum(double* G, int64_t n, int nseg, cudaStream_t s) {
+    if (nseg < 2 || n <= 0) return cudaSuccess;      // n is a multiple of 32
+    f64_segment_sum_kernel<<<(unsigned)grid_stride_blocks((n + 1) / 2, 256, 8), 256, 0, s>>>(
+        G, n, nseg);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_f64_records(int npp, const double* P, const double* p,
                                const double* pref, const double* alpha, double omega,

@@ -15,8 +15,9 @@
 // pairs; then G_A += c2s (A c2s^T F_B) and G_B += c2s (A^T c2s^T F_A)
 // (diagonal pairs: G_A += c2s (A + A^T) / 2 c2s^T F_A).  F_A and the sums of
 // G_A stay in registers over a run of pairs with one bra shell.  Each lane
-// owns its point's column of G and the classes run one after another on one
-// stream, so every element of G has one writer and a fixed summation order.
+// owns its point's column of its range's G and the classes run one after
+// another on one stream, so every element has one writer and a fixed summation
+// order; the ranges' G are added in order afterwards.
 //
 // What bounds it: the FP64 pipe, 2 lanes per clock and SM, 64 times below
 // FP32.  Everything is arranged to spend few FP64 instructions, the other
@@ -29,7 +30,7 @@
 // Eight to sixteen warps an SM fill the pipe, so one CTA an SM with the
 // whole register file and the Boys table in shared memory is enough.
 // Measured on 8 waters (192 AOs, 70,478 points, both omegas): class kernels
-// 165 -> 63 ms, at 82-88 % of the FP64 pipe's issue rate.
+// 165 -> 55 ms, at 82-88 % of the FP64 pipe's issue rate.
 #pragma once
 #include <algorithm>
 #include <cuda_runtime.h>
@@ -221,6 +222,23 @@ __device__ __forceinline__ void hermite_block(const double* __restrict__ E,
                         const double* ez = E + 2 * NAX + eoff(LB, k, kp);
                         const int ab = cidx(LA, i, j) * NCB + cidx(LB, ip, jp);
                         double s = A[ab];
+                        if (k + kp == 0 && j + jp > 0) {
+                            // one v: the y sum continues A
+#pragma unroll
+                            for (int u = 0; u <= L; ++u)
+                                if (u <= j + jp)
+                                    s = fma(ey[u], h1[u * (2 * M + 3 - u) / 2], s);
+                            A[ab] = s;
+                            continue;
+                        }
+                        if (j + jp + k + kp == 0 && i + ip > 0) {
+                            // only this component uses the x sum
+#pragma unroll
+                            for (int t = 0; t <= L; ++t)
+                                if (t <= i + ip) s = fma(ex[t], R[ridx(L, t, 0, 0)], s);
+                            A[ab] = s;
+                            continue;
+                        }
 #pragma unroll
                         for (int v = 0; v <= L; ++v)
                             if (v <= k + kp) {
@@ -239,6 +257,11 @@ __device__ __forceinline__ void hermite_block(const double* __restrict__ E,
                         A[ab] = s;
                     }
         }
+}
+
+// pairs of one of nseg ranges (whole screening chunks)
+__host__ __device__ constexpr int segment_pairs(int npairs, int nseg) {
+    return ((npairs + nseg - 1) / nseg + 31) / 32 * 32;
 }
 
 // threads of a CTA (one an SM): the light classes leave registers for
@@ -264,18 +287,25 @@ cosx_fp64_kernel(const CosxF64Args A, const int cls, const int pair_begin,
     const float* __restrict__ bpref = A.bpref + pp_begin;
     const double* __restrict__ Ecls = A.E + A.e_base[cls];
     unsigned long long kept = 0, flops = 0, ints = 0;
-    // the first items go to the warps of all SMs in turn, the others by the
-    // counter: a grid of few blocks still uses every SM's pipe
+    // An item is a block and one of nseg ranges of the pairs; each range adds
+    // to a G of its own.  The first items go to the warps of all SMs in turn,
+    // the others by the counter: a grid of few blocks still uses every SM's
+    // pipe.
     const int nwarps = gridDim.x * (blockDim.x >> 5);
-    int blk = (int)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    while (blk < A.nblk) {
+    const int nitem = A.nblk * A.nseg;
+    const int seg_pairs = segment_pairs(pair_end - pair_begin, A.nseg);
+    int item = (int)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    while (item < nitem) {
+        const int seg = item / A.nblk, blk = item - seg * A.nblk;
+        const int k0 = pair_begin + seg * seg_pairs;
+        const int k1 = min(pair_end, k0 + seg_pairs);
         const int g0 = blk * 32 + lane;
         const bool ok = g0 < A.npts;
         const int g = ok ? g0 : A.npts - 1;
         const double gx = A.coords[3LL * g], gy = A.coords[3LL * g + 1],
                      gz = A.coords[3LL * g + 2];
         const double* __restrict__ Fp = A.F + g;
-        double* __restrict__ Gp = A.G + g;
+        double* __restrict__ Gp = A.G + seg * A.gstride + g;
         const float4 cr = A.blk_cr[blk];
         const float* __restrict__ ms = A.blk_msh + (long long)blk * A.nvshell;
         const int rem = A.npts - blk * 32;
@@ -288,9 +318,9 @@ cosx_fp64_kernel(const CosxF64Args A, const int cls, const int pair_begin,
             for (int m = 0; m < NA; ++m)
                 atomicAdd(Gp + (long long)(run + m) * ld, to_sph<LA>(A.c2s, ya, m));
         };
-        for (int c0 = pair_begin; c0 < pair_end; c0 += 32) {
+        for (int c0 = k0; c0 < k1; c0 += 32) {
             const int k = c0 + lane;
-            bool keep = k < pair_end;
+            bool keep = k < k1;
             if (keep && A.tol > 0.0f) {
                 const int2 sh = A.pshell[k];
                 keep = screen_pair(A.tol, bnd, bpref, cr, A.khdr[k], A.ptau[k],
@@ -331,7 +361,7 @@ cosx_fp64_kernel(const CosxF64Args A, const int cls, const int pair_begin,
                     const double X = rec[0] - gx, Y = rec[1] - gy, Z = rec[2] - gz;
                     const double T = rec[3] * fma(X, X, fma(Y, Y, Z * Z));
                     double r0[L + 1];
-                    boys_fast<L, L>(T, stab, r0);
+                    boys_fast<L>(T, stab, r0);
                     if constexpr (L == 0) {
                         ab[0] = fma(rec[4], r0[0], ab[0]);
                     } else {
@@ -373,8 +403,8 @@ cosx_fp64_kernel(const CosxF64Args A, const int cls, const int pair_begin,
             }
         }
         flush();
-        if (lane == 0) blk = nwarps + atomicAdd(A.work + cls, 1);
-        blk = __shfl_sync(0xffffffffu, blk, 0);
+        if (lane == 0) item = nwarps + atomicAdd(A.work + cls, 1);
+        item = __shfl_sync(0xffffffffu, item, 0);
     }
     for (int o = 16; o > 0; o >>= 1) {
         flops += __shfl_xor_sync(0xffffffffu, flops, o);
@@ -395,7 +425,7 @@ cudaError_t run64(const CosxF64Args& a, int cls, int pb, int pe, int nsm,
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          smem);
     if (e != cudaSuccess) return e;
-    const int grid = std::max(1, std::min(nsm, a.nblk));
+    const int grid = std::max(1, std::min(nsm, a.nblk * a.nseg));
     k<<<grid, F64Cta<LA, LB>::kThreads, smem, s>>>(a, cls, pb, pe);
     return cudaGetLastError();
 }

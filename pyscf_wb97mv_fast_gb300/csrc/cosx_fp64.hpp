@@ -17,7 +17,9 @@ constexpr int kF64Rec = 16;
 
 struct CosxF64Args {
     const double* F;            // (nao, ld) AO-major, FP64
-    double* G;                  // (nao, ld) AO-major, FP64, accumulated
+    double* G;                  // nseg x (nao, ld) AO-major, FP64, accumulated
+    long long gstride;          // nao ld
+    int nseg;                   // ranges of a class's pairs (f64_segments)
     const double* coords;       // (npts, 3) molecule frame
     long long ld;
     int npts;
@@ -38,7 +40,7 @@ struct CosxF64Args {
     const double* rec;
     const double* E;
     long long e_base[10];
-    const double* boys;         // kBoysFineNodes x kBoysFineCols
+    const double* boys;         // the tables of fp64_boys.cuh
     const double* c2s;          // l = 2 (6 x 5) at 0, l = 3 (10 x 7) at 30, row-major
     const long long* pflops;
     const int* pnint;
@@ -51,6 +53,16 @@ struct CosxF64Args {
 cudaError_t launch_f64_records(int npp, const double* P, const double* p,
                                const double* pref, const double* alpha, double omega,
                                double* rec, cudaStream_t s);
+// Ranges that the pairs of a block are split into.  One warp a block leaves
+// the FP64 pipe idle on grids of fewer than some 16 blocks an SM and in the
+// last blocks of larger ones (an FP64 Fock build of 4 waters, 591 blocks: 21.2
+// -> 18.0 ms with the leaner Boys function).  Ranges beyond 8 cost more screening than they gain.
+inline int f64_segments(int64_t nblk, int nsm) {
+    const int64_t n = (24 * (int64_t)nsm + nblk - 1) / (nblk > 0 ? nblk : 1);
+    return (int)(n < 1 ? 1 : n > 8 ? 8 : n);
+}
+// G[0] += the other nseg - 1 ranges, in order; n elements each
+cudaError_t launch_f64_segment_sum(double* G, int64_t n, int nseg, cudaStream_t s);
 // one class launch (classes 0..9); the f classes live in cosx_fp64_f.cu
 cudaError_t launch_cosx_fp64_class(int cls, const CosxF64Args& a, int pb, int pe,
                                    int nsm, cudaStream_t s);

@@ -32,12 +32,12 @@
 // The screen, pair tables, Boys function and McMurchie-Davidson recurrence
 // are those of the plain FP64 kernels (cosx_fp64.cuh), and so is the bound:
 // the FP64 pipe.  One warp owns one 32-point block, one point a lane.  A
-// lane adds its point's sums to its own column of gpt (3 natm, ld) by
+// lane adds its point's sums to its own column of its range's gpt (3 natm, ld) by
 // reductions in the L2, dA once per run of pairs with one bra shell; a lane
 // reduction in the task would cost 30 FP64 instructions.  The columns are
 // weighted with -w_g / 2 and summed in a fixed order at the end, so the
 // result is bitwise reproducible.  Measured (integral side alone): 8 waters,
-// 36,369 points 327 -> 59 ms; C4H10 in TZVP, 21,512 points 606 -> 98 ms.
+// 36,369 points 327 -> 47 ms; C4H10 in TZVP, 21,512 points 606 -> 69 ms.
 #include "cosx_fp64.cuh"
 #include "cosx_grad64.hpp"
 
@@ -220,15 +220,20 @@ cosx_grad64_kernel(const CosxGradArgs A, const int cls, const int pair_begin,
     const float4* __restrict__ bnd = A.bnd + pp_begin;
     const float* __restrict__ bpref = A.bpref + pp_begin;
     const int nwarps = gridDim.x * (blockDim.x >> 5);
-    int blk = (int)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    while (blk < A.nblk) {
+    const int nitem = A.nblk * A.nseg;
+    const int seg_pairs = segment_pairs(pair_end - pair_begin, A.nseg);
+    int item = (int)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    while (item < nitem) {
+        const int seg = item / A.nblk, blk = item - seg * A.nblk;
+        const int k0 = pair_begin + seg * seg_pairs;
+        const int k1 = min(pair_end, k0 + seg_pairs);
         const int g0 = blk * 32 + lane;
         const bool ok = g0 < A.npts;
         const int g = ok ? g0 : A.npts - 1;
         const double gx = A.coords[3LL * g], gy = A.coords[3LL * g + 1],
                      gz = A.coords[3LL * g + 2];
         const double* __restrict__ Fp = A.F + g;
-        double* __restrict__ out = A.gpt + g;
+        double* __restrict__ out = A.gpt + seg * A.gstride + g;
         const float4 cr = A.blk_cr[blk];
         const float* __restrict__ ms = A.blk_msh + (long long)blk * A.nvshell;
         int run = -1;                       // bra virtual shell held
@@ -239,9 +244,9 @@ cosx_grad64_kernel(const CosxGradArgs A, const int cls, const int pair_begin,
 #pragma unroll
             for (int x = 0; x < 3; ++x) atomicAdd(out + (3 * at + x) * ld, ga[x]);
         };
-        for (int c0 = pair_begin; c0 < pair_end; c0 += 32) {
+        for (int c0 = k0; c0 < k1; c0 += 32) {
             const int k = c0 + lane;
-            bool keep = k < pair_end;
+            bool keep = k < k1;
             if (keep && A.tol > 0.0f) {
                 const int2 sh = A.pshell[k];
                 keep = screen_pair(A.tol, bnd, bpref, cr, A.khdr[k], A.ptau[k],
@@ -275,7 +280,7 @@ cosx_grad64_kernel(const CosxGradArgs A, const int cls, const int pair_begin,
                     const double X = rec[0] - gx, Y = rec[1] - gy, Z = rec[2] - gz;
                     const double T = rec[3] * fma(X, X, fma(Y, Y, Z * Z));
                     double r0[L + 2], R[nr_c(L + 1)], S[3];
-                    boys_fast<L + 1, L + 1>(T, stab, r0);
+                    boys_fast<L + 1>(T, stab, r0);
 #pragma unroll
                     for (int n = 0; n <= L + 1; ++n) r0[n] *= rec[4 + n];
                     fill_r64<L + 1>(r0, X, Y, Z, R);
@@ -299,8 +304,8 @@ cosx_grad64_kernel(const CosxGradArgs A, const int cls, const int pair_begin,
             }
         }
         flush();
-        if (lane == 0) blk = nwarps + atomicAdd(A.work + cls, 1);
-        blk = __shfl_sync(0xffffffffu, blk, 0);
+        if (lane == 0) item = nwarps + atomicAdd(A.work + cls, 1);
+        item = __shfl_sync(0xffffffffu, item, 0);
     }
 }
 
@@ -312,19 +317,21 @@ cudaError_t run_grad(const CosxGradArgs& a, int cls, int pb, int pe, int nsm,
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          smem);
     if (e != cudaSuccess) return e;
-    const int grid = std::max(1, std::min(nsm, a.nblk));
+    const int grid = std::max(1, std::min(nsm, a.nblk * a.nseg));
     k<<<grid, GradCta<LA, LB>::kThreads, smem, s>>>(a, cls, pb, pe);
     return cudaGetLastError();
 }
 
-// out[r] += -1/2 sum_g w_g gpt[r][g]: one CTA a row, fixed order
+// out[r] += -1/2 sum_g w_g gpt[r][g] over the ranges: one CTA a row, fixed order
 __global__ void grad_points_sum_kernel(const double* __restrict__ gpt,
                                        const double* __restrict__ w, int64_t npts,
-                                       int64_t ld, double* __restrict__ out) {
+                                       int64_t ld, int nseg, int64_t gstride,
+                                       double* __restrict__ out) {
     __shared__ double red[256];
     const double* row = gpt + (int64_t)blockIdx.x * ld;
     double s = 0.0;
-    for (int64_t g = threadIdx.x; g < npts; g += 256) s = fma(w[g], row[g], s);
+    for (int q = 0; q < nseg; ++q, row += gstride)
+        for (int64_t g = threadIdx.x; g < npts; g += 256) s = fma(w[g], row[g], s);
     red[threadIdx.x] = s;
     __syncthreads();
     for (int o = 128; o > 0; o >>= 1) {
@@ -360,9 +367,11 @@ cudaError_t launch_cosx_grad64_class(int cls, const CosxGradArgs& a, int pb, int
 }
 
 cudaError_t launch_grad_points_sum(const double* gpt, const double* w, int64_t npts,
-                                   int64_t ld, int natm, double* out, cudaStream_t s) {
+                                   int64_t ld, int natm, int nseg, double* out,
+                                   cudaStream_t s) {
     if (natm <= 0) return cudaSuccess;
-    grad_points_sum_kernel<<<3 * natm, 256, 0, s>>>(gpt, w, npts, ld, out);
+    grad_points_sum_kernel<<<3 * natm, 256, 0, s>>>(gpt, w, npts, ld, nseg,
+                                                    3 * (int64_t)natm * ld, out);
     return cudaGetLastError();
 }
 

@@ -31,9 +31,11 @@ struct CosxGradArgs {
     const double* dE;
     long long e_base[10];
     const int* vs_atom;
-    const double* boys;         // kBoysFineNodes x kBoysFineCols
+    const double* boys;         // the tables of fp64_boys.cuh
     const double* c2s;          // l = 2 at 0, l = 3 at 30
-    double* gpt;                // (3 natm, ld) sums of each point, zeroed
+    double* gpt;                // nseg x (3 natm, ld) sums of each point, zeroed
+    long long gstride;          // 3 natm ld
+    int nseg;                   // ranges of a class's pairs (f64_segments)
     int* work;                  // per class block counter (zeroed)
 };
 
@@ -56,7 +58,8 @@ cudaError_t launch_cosx_grad64_class(int cls, const CosxGradArgs& a, int pb, int
                                      int nsm, cudaStream_t s);
 // out (natm * 3) -= 1/2 sum_g w_g gpt (fixed-order block reductions)
 cudaError_t launch_grad_points_sum(const double* gpt, const double* w, int64_t npts,
-                                   int64_t ld, int natm, double* out, cudaStream_t s);
+                                   int64_t ld, int natm, int nseg, double* out,
+                                   cudaStream_t s);
 // out (nao, 3): sum_g w_g dX[x][mu][g] H[mu][g] (fixed-order block reduction)
 cudaError_t launch_ao_dot(const double* dX, const double* H, const double* w,
                           int64_t npts, int64_t ld, int nao, double* out,
