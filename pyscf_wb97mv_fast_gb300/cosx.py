@@ -431,7 +431,7 @@ class CosxEngine:
             self.last_stats = st.as_dict()
         return out
 
-    def ozaki_f(self, X, qd, fp64=False):
+    def ozaki_f(self, X, qd, fp64=False, out=None):
         """F (nao, ld) = X^T-side product QD^T X through the bf16 Ozaki split:
         FP32 (fl32 of the product) or, with fp64, FP64 (the 42-bit level
         sums rounded once)."""
@@ -442,7 +442,9 @@ class CosxEngine:
         nbytes = int(_native.lib().wb_ozaki_workspace_bytes(self.nao, ld))
         ws = self.workspace(nbytes)
         dt = torch.float64 if fp64 else torch.float32
-        out = torch.empty((self.nao, ld), dtype=dt, device=self.device)
+        if out is None:
+            out = torch.empty((self.nao, ld), dtype=dt, device=self.device)
+        device_out(out, 'out', dt, self.device, (self.nao, ld))
         fn = 'wb_cosx_ozaki_f64' if fp64 else 'wb_cosx_ozaki_f'
         _native.check(getattr(_native.lib(), fn)(
             self._h, _native.ptr(X), _native.ptr(qd), ld,

@@ -36,6 +36,11 @@ SUPPORTED_XCTYPE = ('LDA', 'GGA', 'MGGA')
 Unsupported = _native.Unsupported
 # points per tile: X, T and G take (32 + 16 + 16) bytes per point and AO
 DEFAULT_TILE_PTS = 1 << 20
+# A grid of at least two tiles of this size is cut into (up to) four, so that
+# the functional of one tile runs on the host while the GPU works on the next:
+# in one piece the GPU waited for it (8 of 32 ms, 16 waters, 233,999 points).
+# Below this size a tile's kernels no longer fill the GPU.
+OVERLAP_TILE_PTS = 1 << 15
 
 
 def _torch():
@@ -118,10 +123,21 @@ def _t_planes(eng, X, D, planes):
     exact = 7 * nao < (1 << 14)
     for d in range(planes):
         if exact:
-            T[d] = eng.ozaki_f(X[d], D)
+            eng.ozaki_f(X[d], D, out=T[d])
         else:
             T[d] = (D.T @ X[d]).to(torch.float32)
     return T
+
+
+def _tiles(n, tile_pts):
+    """[(i0, i1)] of at most tile_pts points (at least 32): one tile, or up to
+    four of at least OVERLAP_TILE_PTS (whole 2048-point chunks of the K
+    split), or what tile_pts asks for."""
+    tile = max(32, int(tile_pts))
+    parts = min(4, n // OVERLAP_TILE_PTS)
+    if parts > 1:
+        tile = min(tile, -(-n // (parts * 2048)) * 2048)
+    return [(i, min(n, i + tile)) for i in range(0, n, tile)]
 
 
 def gpu_nr_rks(ctx, ni, mol, grids, xc_code, dms, relativity=0, hermi=1,
@@ -153,29 +169,45 @@ def gpu_nr_rks(ctx, ni, mol, grids, xc_code, dms, relativity=0, hermi=1,
     vtau = torch.zeros_like(vmat) if mgga else None
     nelec = 0.0
     excsum = 0.0
-    tile = max(32, ctx.tile_pts)
-    for i0 in range(0, n, tile):
-        i1 = min(n, i0 + tile)
+
+    def density(i0, i1):
+        """AO values and density parameters of one tile, the latter on their
+        way to the host."""
         nt = i1 - i0
         c = eng.relative(coords[i0:i1])
         w = torch.as_tensor(weights[i0:i1], device=dev)
         X = eng.ao_eval_deriv1(c)                       # (4, nao, ld)
         T = _t_planes(eng, X, D, planes)
         rho_d = eng.xc_rho(X, T, nt, mgga)              # (5, ld)
-        del T
-        rho = rho_d[:, :nt].cpu().numpy()
+        rho_h = torch.empty((5, nt), dtype=torch.float64, pin_memory=True)
+        rho_h.copy_(rho_d[:, :nt], non_blocking=True)
+        arrived = torch.cuda.Event()
+        arrived.record()
+        return i0, i1, w, X, int(rho_d.shape[1]), rho_h, arrived
+
+    tiles = _tiles(n, ctx.tile_pts)
+    ahead = density(*tiles[0]) if tiles else None
+    for k in range(len(tiles)):
+        i0, i1, w, X, ld, rho_h, arrived = ahead
+        nt = i1 - i0
+        # the next tile's kernels are queued before the host waits
+        ahead = density(*tiles[k + 1]) if k + 1 < len(tiles) else None
+        arrived.synchronize()
+        rho = rho_h.numpy()
         exc, vrho, vsigma, vt = functional.eval(rho)
         exc, v = chain_rule(rho, exc, vrho, vsigma, vt)
-        w_h = weights[i0:i1]
-        nelec += float((rho[0] * w_h).sum())
-        excsum += float((rho[0] * w_h * exc).sum())
-        v_d = torch.zeros_like(rho_d)
-        v_d[:, :nt] = torch.from_numpy(v).to(dev)
+        v_h = torch.empty((5, nt), dtype=torch.float64, pin_memory=True)
+        v_h.numpy()[:] = v
+        v_d = torch.zeros((5, ld), dtype=torch.float64, device=dev)
+        v_d[:, :nt].copy_(v_h, non_blocking=True)
         G = eng.xc_aow(X, v_d, nt, mgga)                # (planes, nao, ld)
         eng.ozaki_k(X[0], G[0], w, out=vmat, accumulate=True)
         for d in range(1, planes):
             eng.ozaki_k(X[d], G[d], w, out=vtau, accumulate=True)
         del X, G
+        w_h = weights[i0:i1]
+        nelec += float((rho[0] * w_h).sum())
+        excsum += float((rho[0] * w_h * exc).sum())
     vmat = vmat + vmat.T
     if mgga:
         # sum_d X_d^T (w o fl32(1/2 vtau X_d)) is symmetric up to the FP32
