@@ -216,12 +216,10 @@ struct wb_cosx {
     double* f64_vsxyz = nullptr;     // virtual shell centres (3 each)
     int* vs_atom = nullptr;          // virtual shell atoms
     double origin[3] = {0.0, 0.0, 0.0};   // frame of the device coordinates
-    // SCF helpers (wb_scf_int1e, wb_hartree), set up on first use: per pair
-    // L = la + lb; per primitive pair the offset of its Hermite density and
-    // p in FP32; nuclei (x, y, z, Z) in the handle frame
-    int* pair_L = nullptr;
+    // SCF helpers (wb_scf_int1e, wb_hartree), set up on first use: per
+    // primitive pair the offset of its Hermite density; nuclei (x, y, z, Z) in
+    // the handle frame
     long long* dh_off = nullptr;
-    float* p32 = nullptr;
     int64_t ndh = 0;
     double* nuc = nullptr;
     int nuc_cap = 0;
@@ -756,51 +754,38 @@ inline int64_t hartree_nr_padded(int l) {
     return ((int64_t)(l + 1) * (l + 2) * (l + 3) / 6 + 3) & ~(int64_t)3;
 }
 
-// per-pair L, per-primitive-pair Hermite-density offsets and FP32 p of
-// the Hartree potential (first wb_hartree call on the handle)
+// the Hermite-density offset of each primitive pair (first wb_hartree call on
+// the handle)
 int ensure_hartree(wb_cosx* h) {
-    if (h->pair_L) return WB_OK;
+    if (h->dh_off) return WB_OK;
     const wb::HostPairs& hp = h->hp;
-    std::vector<int> L((size_t)std::max(hp.npairs, 1), 0);
     std::vector<long long> off((size_t)std::max(hp.npp, 1), 0);
-    std::vector<float> p32((size_t)std::max(hp.npp, 1), 0.0f);
     long long tot = 0;
     for (int k = 0; k < hp.npairs; ++k) {
         const int l = hp.vsh[hp.pshell[2 * k]].l + hp.vsh[hp.pshell[2 * k + 1]].l;
-        L[k] = l;
         const int pp0 = hp.hdr[4 * k + 2], npp = hp.hdr[4 * k + 3] & 0xffff;
         for (int m = pp0; m < pp0 + npp; ++m) {
             off[m] = tot;
             tot += hartree_nr_padded(l);
         }
     }
-    for (int m = 0; m < hp.npp; ++m) p32[m] = (float)hp.p[m];
-    int* dL = nullptr;
     long long* dO = nullptr;
-    float* dP = nullptr;
-    cudaError_t e = cudaMalloc(&dL, sizeof(int) * L.size());
-    if (e == cudaSuccess) e = cudaMalloc(&dO, sizeof(long long) * off.size());
-    if (e == cudaSuccess) e = cudaMalloc(&dP, sizeof(float) * p32.size());
-    if (e == cudaSuccess)
-        e = cudaMemcpy(dL, L.data(), sizeof(int) * L.size(), cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMalloc(&dO, sizeof(long long) * off.size());
     if (e == cudaSuccess)
         e = cudaMemcpy(dO, off.data(), sizeof(long long) * off.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(dP, p32.data(), sizeof(float) * p32.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
-        for (void* q : {(void*)dL, (void*)dO, (void*)dP})
-            if (q) cudaFree(q);
+        if (dO) cudaFree(dO);
         return cuda_fail(e, "Hartree pair tables");
     }
-    h->pair_L = dL;
     h->dh_off = dO;
-    h->p32 = dP;
     h->ndh = std::max<long long>(tot, 1);
     return WB_OK;
 }
 
 struct HartreeLayout {
-    size_t counters = 0, cr = 0, dabs = 0, dh64 = 0, dh32 = 0, total = 0;
+    size_t counters = 0, cr = 0, dabs = 0, dh64 = 0, dh32 = 0, rec = 0, p32 = 0, vpart = 0;
+    size_t total = 0;
+    int nseg = 1;
 };
 
 HartreeLayout hartree_layout(const wb_cosx* h, int64_t npts, int64_t ndh) {
@@ -817,6 +802,12 @@ HartreeLayout hartree_layout(const wb_cosx* h, int64_t npts, int64_t ndh) {
     L.dabs = take(sizeof(float) * (size_t)std::max(h->hp.npairs, 1));
     L.dh64 = take(sizeof(double) * (size_t)ndh);
     L.dh32 = take(sizeof(float) * (size_t)ndh);
+    L.rec = take(sizeof(double) * wb::kF64Rec * (size_t)std::max(h->hp.npp, 1));
+    L.p32 = take(sizeof(float) * (size_t)std::max(h->hp.npp, 1));
+    L.nseg = wb::f64_segments(nblk, h->nsm);
+    // (and one row for each mixed chunk: at most one a class boundary, and the last)
+    L.vpart = take(sizeof(double) * 32 * (size_t)std::max<int64_t>(nblk, 1) *
+                   (L.nseg + wb::NCLASS + 1));
     L.total = off;
     return L;
 }
@@ -1192,7 +1183,7 @@ int wb_cosx_destroy(wb_cosx* h) {
     if (h->f64_alpha) cudaFree(h->f64_alpha);
     if (h->f64_vsxyz) cudaFree(h->f64_vsxyz);
     if (h->vs_atom) cudaFree(h->vs_atom);
-    for (void* q : {(void*)h->pair_L, (void*)h->dh_off, (void*)h->p32, (void*)h->nuc})
+    for (void* q : {(void*)h->dh_off, (void*)h->nuc})
         if (q) cudaFree(q);
     delete h;
     return WB_OK;
@@ -2219,26 +2210,52 @@ int wb_hartree(wb_cosx* h, const double* coords, int64_t npts, const double* dm,
     a.nblk = nblk;
     a.npairs = h->hp.npairs;
     a.hdr = h->hdr;
-    a.pair_L = h->pair_L;
+    a.nseg = L.nseg;
     a.ptau = h->ptau;
     a.bnd = h->bnd;
     a.bpref = h->bpref;
     a.pair_dabs = d.pair_dabs;
-    a.P = h->f64_P;
-    a.p = h->p;
+    a.rec = at<double>(workspace, L.rec);
     a.geo = h->geo;
-    a.p32 = h->p32;
+    a.p32 = at<float>(workspace, L.p32);
     a.dh_off = h->dh_off;
     a.dh64 = d.dh64;
     a.dh32 = d.dh32;
     a.boys32 = h->boys;
-    a.boys64 = h->f64_boys;
+    a.boys64 = h->f64_fine;
     a.tol = tol > 0.0 ? (float)(tol / 1.001) : 0.0f;
     if (tol > 0.0 && a.tol <= 0.0f) a.tol = 1e-38f;
-    a.v = v_out;
+    a.vpart = at<double>(workspace, L.vpart);
     a.work = at<int>(workspace, L.counters);
     a.kept = at<unsigned long long>(workspace, L.counters + 64);
-    WB_CUDA(wb::scf::launch_hartree(a, fp64 != 0, s));
+    if (fp64)
+        WB_CUDA(wb::launch_f64_records(h->hp.npp, h->f64_P, h->p, h->pref, h->f64_alpha, 0.0,
+                                       at<double>(workspace, L.rec), s));
+    else
+        WB_CUDA(wb::launch_f64_to_f32(h->p, at<float>(workspace, L.p32), h->hp.npp, s));
+    WB_CUDA(cudaMemsetAsync(a.vpart, 0, sizeof(double) * 32 * (size_t)nblk * L.nseg, s));
+    a.vmixed = a.vpart + (size_t)32 * nblk * L.nseg;
+    for (int la = 0; la <= wb::LMAX; ++la)
+        for (int lb = 0; lb <= la; ++lb) {
+            const int c = wb::class_of(la, lb);
+            int pb = h->hp.cls[c].pair_begin, pe = h->hp.cls[c].pair_end;
+            a.cls_end[c] = pe;
+            a.cls_l[c] = la + lb;
+            if (!fp64 && pe > pb) {
+                // whole chunks of 32 pairs of the list; the others are mixed
+                const int first = (pb + 31) / 32 * 32, last = pe / 32 * 32;
+                const int edge[2] = {pb / 32 * 32, last};
+                for (int e = 0; e < 2; ++e)
+                    if ((e ? pe != last : pb != first) &&
+                        (a.nmixed == 0 || a.mixed[a.nmixed - 1] != edge[e]))
+                        a.mixed[a.nmixed++] = edge[e];
+                pb = first;
+                pe = std::max(first, last);
+            }
+            WB_CUDA(wb::scf::launch_hartree_class(a, fp64 != 0, c, la + lb, pb, pe, s));
+        }
+    WB_CUDA(wb::scf::launch_hartree_mixed(a, s));
+    WB_CUDA(wb::scf::launch_hartree_sum(a, v_out, s));
     if (tasks_kept) {
         unsigned long long kept = 0;
         WB_CUDA(cudaMemcpyAsync(&kept, a.kept, sizeof(kept), cudaMemcpyDeviceToHost, s));

@@ -43,8 +43,6 @@
 namespace wb {
 namespace f64 {
 
-constexpr int kTaylor = 12;              // terms of the 1/4-node Boys series
-
 constexpr __host__ __device__ int nr_c(int L) { return (L + 1) * (L + 2) * (L + 3) / 6; }
 // packed index of R_tuv (t + u + v <= L): v-major, then u, then t
 constexpr __host__ __device__ int ridx(int L, int t, int u, int v) {
@@ -103,39 +101,6 @@ __device__ __forceinline__ double to_sph(const double* __restrict__ c2s,
                 first = false;
             }
         return a;
-    }
-}
-
-// F_0 .. F_L at T in FP64.  T < 36: Taylor series of F_L about the nearest
-// node k/4 (|dT| <= 1/8, kTaylor terms: truncation below 1e-20 relative)
-// from the table tab[k][m] = F_m(k/4), then the downward recursion
-// F_n = (2T F_{n+1} + e^-T) / (2n + 1).  T >= 36: erf(sqrt T) = 1 in FP64,
-// F_0 = sqrt(pi / T) / 2 and the upward recursion F_{n+1} = ((2n+1) F_n -
-// e^-T) / (2T), stable for T > n.
-template<int L>
-__device__ __forceinline__ void boys64(const double T, const double* __restrict__ tab,
-                                       double* F) {
-    if (T < 36.0) {
-        const int k = __double2int_rn(T * 4.0);
-        const double x = 0.25 * k - T;
-        const double* row = tab + k * kBoys64Cols + L;
-        double s = row[kTaylor - 1];
-#pragma unroll
-        for (int j = kTaylor - 1; j >= 1; --j) s = fma(s * x, 1.0 / j, row[j - 1]);
-        F[L] = s;
-        if constexpr (L > 0) {
-            const double e = exp(-T);
-#pragma unroll
-            for (int n = L - 1; n >= 0; --n) F[n] = fma(2.0 * T, F[n + 1], e) * (1.0 / (2 * n + 1));
-        }
-    } else {
-        F[0] = 0.88622692545275801365 * rsqrt(T);
-        if constexpr (L > 0) {
-            const double e = exp(-T);
-            const double h = 0.5 / T;
-#pragma unroll
-            for (int n = 0; n < L; ++n) F[n + 1] = ((2 * n + 1) * F[n] - e) * h;
-        }
     }
 }
 

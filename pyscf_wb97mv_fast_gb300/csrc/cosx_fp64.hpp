@@ -8,6 +8,7 @@ namespace wb {
 
 constexpr int kBoys64Nodes = 145;   // T_k = k / 4, k = 0..144
 constexpr int kBoys64Cols = 20;     // F_m(T_k), m = 0..19 (L <= 6 + 11 Taylor terms)
+constexpr int kBoysTaylor = 12;     // terms of the 1/4-node series
 
 constexpr int kBoysFineNodes = 1153;    // T_k = k / 32, k = 0..1152
 constexpr int kBoysFineCols = 14;       // F_m(T_k), m = 0..13 (orders to 7)

@@ -51,23 +51,26 @@ struct HartreeArgs {
     int nblk;
     int npairs;
     const int4* hdr;
-    const int* pair_L;
+    int nseg;                   // ranges of a class's pairs (f64_segments)
     const float2* ptau;
     const float4* bnd;          // per primitive pair (global index)
     const float* bpref;
     const float* pair_dabs;
-    const double* P;            // per primitive pair, FP64
-    const double* p;
-    const float4* geo;          // per primitive pair: P hi, P lo (FP32)
-    const float* p32;
+    const double* rec;          // FP64: the records of omega = 0 (f64_records)
+    const float4* geo;          // FP32, per primitive pair: P hi, P lo
+    const float* p32;           // FP32: p
     const long long* dh_off;
     const double* dh64;
     const float* dh32;
     const float4* boys32;
     const double* boys64;
     float tol;                  // screening tolerance / 1.001 (0 keeps all)
-    double* v;                  // (npts,) output
-    int* work;                  // zeroed block counter
+    double* vpart;              // nseg x (32 nblk) partial potentials, zeroed,
+    double* vmixed;             // then nmixed rows of the mixed chunks
+    int nmixed;                 // FP32: chunks of several classes (launch_hartree_mixed)
+    int mixed[12];              // their first pairs
+    int cls_end[10], cls_l[10]; // class ends in the pair list and their la + lb
+    int* work;                  // zeroed item counter of each class
     unsigned long long* kept;   // kept (block, pair) tasks, or null
 };
 
@@ -76,7 +79,13 @@ cudaError_t launch_int1e(const Int1eArgs& a, cudaStream_t s);
 cudaError_t launch_dh(const DhArgs& a, cudaStream_t s);
 cudaError_t launch_block_geom(const double* xyz, int64_t npts, int nblk, float4* cr,
                               cudaStream_t s);
-cudaError_t launch_hartree(const HartreeArgs& a, bool fp64, cudaStream_t s);
+// the pairs of one class, total angular momentum L
+cudaError_t launch_hartree_class(const HartreeArgs& a, bool fp64, int cls, int L, int pb,
+                                 int pe, cudaStream_t s);
+// FP32: the mixed chunks
+cudaError_t launch_hartree_mixed(const HartreeArgs& a, cudaStream_t s);
+// v (npts,) = the sum of the ranges and mixed chunks
+cudaError_t launch_hartree_sum(const HartreeArgs& a, double* v, cudaStream_t s);
 
 }  // namespace scf
 }  // namespace wb

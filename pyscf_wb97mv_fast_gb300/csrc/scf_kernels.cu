@@ -23,7 +23,6 @@
 namespace wb {
 namespace scf {
 
-using f64::boys64;
 using f64::cx;
 using f64::cy;
 using f64::cz;
@@ -143,9 +142,9 @@ __device__ void boys_rt(const int L, const double T, const double* tab, double* 
         const int k = __double2int_rn(T * 4.0);
         const double x = 0.25 * k - T;
         const double* row = tab + k * kBoys64Cols + L;
-        double s = row[f64::kTaylor - 1];
+        double s = row[kBoysTaylor - 1];
 #pragma unroll 1
-        for (int j = f64::kTaylor - 1; j >= 1; --j) s = fma(s * x, 1.0 / j, row[j - 1]);
+        for (int j = kBoysTaylor - 1; j >= 1; --j) s = fma(s * x, 1.0 / j, row[j - 1]);
         F[L] = s;
         const double e = exp(-T);
 #pragma unroll 1
@@ -321,8 +320,9 @@ cudaError_t launch_int1e(const Int1eArgs& a, cudaStream_t s) {
 // One thread per shell pair (la >= lb): Dc = c2s'_A^T D_AB c2s'_B in the
 // Cartesian components (c2s' = the d/f transforms; identity for s and p,
 // whose angular factors are folded into pref), then for each of its
-// primitive pairs dh[tuv] = w pref sum_{ab} Dc_ab E^x E^y E^z, w = 2 for
-// A != B (the D_BA half) and 1 for a diagonal pair.  Also the pair's
+// primitive pairs dh[tuv] = w sum_{ab} Dc_ab E^x E^y E^z, w = 2 for
+// A != B (the D_BA half) and 1 for a diagonal pair; the FP32 copy carries the
+// prefactor too, the FP64 kernels have it in the records.  Also the pair's
 // screening factor w sum |D_AB| (FP32, rounded up).
 __global__ void __launch_bounds__(64) dh_kernel(const DhArgs A) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -399,13 +399,12 @@ __global__ void __launch_bounds__(64) dh_kernel(const DhArgs A) {
                     }
             }
         }
-        const double pre = w * A.pref[m];
         const int64_t off = A.dh_off[m];
 #pragma unroll 1
         for (int q = 0; q < nr; ++q) {
-            const double val = pre * dh[q];
+            const double val = w * dh[q];
             A.dh64[off + q] = val;
-            A.dh32[off + q] = (float)val;
+            A.dh32[off + q] = (float)(w * A.pref[m] * dh[q]);
         }
     }
 }
@@ -447,51 +446,52 @@ __global__ void block_geom_kernel(const double* __restrict__ xyz, int64_t npts,
 
 // -- Hartree potential ---------------------------------------------------------
 
-// Precision traits: FP64 (FP64 Boys table, coordinates and Hermite
-// densities) or FP32 (FP32 Boys, coordinates as hi + lo, FP32 Hermite
-// densities and R; each 32-pair chunk summed in FP32, then in FP64).
+// Precision traits: FP64 (FP64 coordinates, records and Hermite densities,
+// fp64_boys.cuh) or FP32 (coordinates as hi + lo, FP32 Boys, Hermite densities
+// and R; each 32-pair chunk summed in FP32, then in FP64).
 template<bool F64> struct HartreeTraits;
 template<> struct HartreeTraits<true> {
     typedef double Real;
-    static constexpr int kTabBytes = kBoys64Nodes * kBoys64Cols * 8;
+    static constexpr int kThreads = 512, kCtas = 1;
+    template<int L> static constexpr int table_bytes() { return f64::BoysTable<L>::kBytes; }
 };
 template<> struct HartreeTraits<false> {
     typedef float Real;
-    static constexpr int kTabBytes = 145 * 5 * 16;
+    static constexpr int kThreads = 256, kCtas = 3;
+    template<int L> static constexpr int table_bytes() { return 145 * 5 * 16; }
 };
 
+// one primitive pair at one point, for total angular momentum L
 template<bool F64, int L>
-__device__ __forceinline__ typename HartreeTraits<F64>::Real hartree_pp(const HartreeArgs& A, const int m,
-                                             const double gx, const double gy,
-                                             const double gz, const float3 gh,
-                                             const float3 gl, const void* stab) {
+__device__ __forceinline__ typename HartreeTraits<F64>::Real hartree_pp(
+    const HartreeArgs& A, const int m, const long long off, const double gx, const double gy,
+    const double gz, const float3 gh, const float3 gl, const void* stab) {
     typedef typename HartreeTraits<F64>::Real Real;
-    Real px, py, pz, p;
+    Real px, py, pz, r0[L + 1];
+    const Real* dh;
     if constexpr (F64) {
-        px = A.P[3 * m] - gx; py = A.P[3 * m + 1] - gy; pz = A.P[3 * m + 2] - gz;
-        p = A.p[m];
+        const double* rec = A.rec + (int64_t)m * kF64Rec;
+        px = rec[0] - gx; py = rec[1] - gy; pz = rec[2] - gz;
+        f64::boys_fast<L>(rec[3] * fma(px, px, fma(py, py, pz * pz)),
+                          static_cast<const double*>(stab), r0);
+#pragma unroll
+        for (int n = 0; n <= L; ++n) r0[n] *= rec[4 + n];
+        dh = A.dh64 + off;
     } else {
         const float4 hi = A.geo[2 * m], lo = A.geo[2 * m + 1];
+        const float p = A.p32[m];
         px = (hi.x - gh.x) + (lo.x - gl.x);
         py = (hi.y - gh.y) + (lo.y - gl.y);
         pz = (hi.z - gh.z) + (lo.z - gl.z);
-        p = A.p32[m];
-    }
-    const Real T = p * (px * px + py * py + pz * pz);
-    Real F[L + 1], r0[L + 1];
-    if constexpr (F64)
-        boys64<L>(T, static_cast<const double*>(stab), F);
-    else
-        boys_fp32<L>(T, F, static_cast<const float4*>(stab));
-    Real m2p = Real(1);
+        boys_fp32<L>(p * (px * px + py * py + pz * pz), r0, static_cast<const float4*>(stab));
+        float m2p = 1.0f;
 #pragma unroll
-    for (int n = 0; n <= L; ++n) {
-        r0[n] = m2p * F[n];
-        m2p *= Real(-2) * p;
+        for (int n = 0; n <= L; ++n) {
+            r0[n] *= m2p;
+            m2p *= -2.0f * p;
+        }
+        dh = A.dh32 + off;
     }
-    const int64_t off = A.dh_off[m];
-    const Real* dh;
-    if constexpr (F64) dh = A.dh64 + off; else dh = A.dh32 + off;
     if constexpr (L == 0) return hermite_dot_0<Real>(r0, px, py, pz, dh);
     else if constexpr (L == 1) return hermite_dot_1<Real>(r0, px, py, pz, dh);
     else if constexpr (L == 2) return hermite_dot_2<Real>(r0, px, py, pz, dh);
@@ -501,52 +501,42 @@ __device__ __forceinline__ typename HartreeTraits<F64>::Real hartree_pp(const Ha
     else return hermite_dot_6<Real>(r0, px, py, pz, dh);
 }
 
-template<bool F64>
-__device__ __forceinline__ typename HartreeTraits<F64>::Real hartree_pair(
-    const HartreeArgs& A, const int L, const int pp0, const int npp, const double gx,
-    const double gy, const double gz, const float3 gh, const float3 gl,
-    const void* stab) {
-    typename HartreeTraits<F64>::Real s = 0;
-    for (int m = pp0; m < pp0 + npp; ++m) {
-        switch (L) {
-        case 0: s += hartree_pp<F64, 0>(A, m, gx, gy, gz, gh, gl, stab); break;
-        case 1: s += hartree_pp<F64, 1>(A, m, gx, gy, gz, gh, gl, stab); break;
-        case 2: s += hartree_pp<F64, 2>(A, m, gx, gy, gz, gh, gl, stab); break;
-        case 3: s += hartree_pp<F64, 3>(A, m, gx, gy, gz, gh, gl, stab); break;
-        case 4: s += hartree_pp<F64, 4>(A, m, gx, gy, gz, gh, gl, stab); break;
-        case 5: s += hartree_pp<F64, 5>(A, m, gx, gy, gz, gh, gl, stab); break;
-        default: s += hartree_pp<F64, 6>(A, m, gx, gy, gz, gh, gl, stab); break;
-        }
-    }
-    return s;
-}
-
-// One warp per 32-point block (one point per lane), blocks taken from a
-// counter.  For 32 pairs at a time each lane screens one pair (the COSX
-// kernels' locked bound times w sum |D_AB|), a ballot keeps the warp on the
-// kept pairs, and every lane adds the pair's primitive pairs at its point.
-// The FP32 form sums each 32-pair chunk in FP32 and the chunks in FP64; the
-// FP64 form sums in FP64.  Fixed order: bitwise reproducible.
-template<bool F64>
-__global__ void __launch_bounds__(128) hartree_kernel(const HartreeArgs A) {
+// The pairs [pair_begin, pair_end) of one class (total angular momentum L).
+// One warp per item, a 32-point block (one point per lane) and one of nseg
+// ranges of the pairs, items taken from a counter.  For 32 pairs at a time
+// each lane screens one pair (the COSX kernels' locked bound times w sum
+// |D_AB|), a ballot keeps the warp on the kept pairs, and every lane adds the
+// pair's primitive pairs at its point.  The sum of a range goes to its own
+// row of vpart, the ranges and classes in a fixed order: bitwise reproducible.
+//
+// A launch per class keeps the angular momentum a compile-time constant (one
+// kernel for all of them held the registers of the largest and a switch in
+// its inner loop).  The FP64 form is bound by the FP64 pipe and arranged as
+// the FP64 class kernels (cosx_fp64.cuh); the FP32 form by the latency of its
+// loads and instruction issue.  8 waters, 70,479 points, FP32: 6.0 -> 4.3 ms; 4
+// waters, 18,912 points, FP64: 6.9 -> 3.4 ms.
+template<bool F64, int L>
+__global__ void __launch_bounds__(HartreeTraits<F64>::kThreads, HartreeTraits<F64>::kCtas)
+hartree_kernel(const HartreeArgs A, const int cls, const int pair_begin, const int pair_end) {
     extern __shared__ float4 smem[];
-    {
-        const int n = HartreeTraits<F64>::kTabBytes / 16;
-        const float4* src = F64 ? reinterpret_cast<const float4*>(A.boys64) : A.boys32;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) smem[i] = src[i];
+    if constexpr (F64) {
+        f64::load_boys<L>(A.boys64, reinterpret_cast<double*>(smem));
+    } else {
+        for (int i = threadIdx.x; i < 145 * 5; i += blockDim.x) smem[i] = A.boys32[i];
     }
     __syncthreads();
-    const void* stab = smem;
     const int lane = threadIdx.x & 31;
     unsigned long long kept = 0;
-    for (;;) {
-        int blk = 0;
-        if (lane == 0) blk = atomicAdd(A.work, 1);
-        blk = __shfl_sync(0xffffffffu, blk, 0);
-        if (blk >= A.nblk) break;
+    const int nwarps = gridDim.x * (blockDim.x >> 5);
+    const int nitem = A.nblk * A.nseg;
+    const int seg_pairs = f64::segment_pairs(pair_end - pair_begin, A.nseg);
+    int item = (int)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    while (item < nitem) {
+        const int seg = item / A.nblk, blk = item - seg * A.nblk;
+        const int k0 = pair_begin + seg * seg_pairs;
+        const int k1 = min(pair_end, k0 + seg_pairs);
         const int64_t g0 = (int64_t)blk * 32 + lane;
-        const bool ok = g0 < A.npts;
-        const int64_t g = ok ? g0 : A.npts - 1;
+        const int64_t g = g0 < A.npts ? g0 : A.npts - 1;
         const double gx = A.coords[3 * g], gy = A.coords[3 * g + 1], gz = A.coords[3 * g + 2];
         float3 gh = make_float3(0.f, 0.f, 0.f), gl = gh;
         if (!F64) {
@@ -556,9 +546,9 @@ __global__ void __launch_bounds__(128) hartree_kernel(const HartreeArgs A) {
         }
         const float4 cr = A.blk_cr[blk];
         double v = 0.0;
-        for (int c0 = 0; c0 < A.npairs; c0 += 32) {
+        for (int c0 = k0; c0 < k1; c0 += 32) {
             const int k = c0 + lane;
-            bool keep = k < A.npairs;
+            bool keep = k < k1;
             int4 h = make_int4(0, 0, 0, 0);
             if (keep) {
                 h = A.hdr[k];
@@ -572,17 +562,88 @@ __global__ void __launch_bounds__(128) hartree_kernel(const HartreeArgs A) {
             while (mask) {
                 const int src = __ffs(mask) - 1;
                 mask &= mask - 1;
-                const int kk = c0 + src;
                 const int pp0 = __shfl_sync(0xffffffffu, h.z, src);
                 const int npp = __shfl_sync(0xffffffffu, h.w, src) & 0xffff;
-                const int L = A.pair_L[kk];
-                chunk += hartree_pair<F64>(A, L, pp0, npp, gx, gy, gz, gh, gl, stab);
+                // the Hermite densities of a class are padded alike
+                constexpr int NR = ((L + 1) * (L + 2) * (L + 3) / 6 + 3) & ~3;
+                long long off = A.dh_off[pp0];
+                typename HartreeTraits<F64>::Real pair = 0;
+                for (int m = pp0; m < pp0 + npp; ++m, off += NR)
+                    pair += hartree_pp<F64, L>(A, m, off, gx, gy, gz, gh, gl, smem);
+                chunk += pair;
             }
             v += (double)chunk;
         }
-        if (ok) A.v[g0] = v;
+        A.vpart[((int64_t)seg * A.nblk + blk) * 32 + lane] += v;
+        if (lane == 0) item = nwarps + atomicAdd(A.work + cls, 1);
+        item = __shfl_sync(0xffffffffu, item, 0);
     }
-    if (lane == 0 && A.kept) atomicAdd(A.kept, kept);
+    if (lane == 0 && A.kept && kept) atomicAdd(A.kept, kept);
+}
+
+// FP32: the screening chunks of 32 pairs that hold pairs of more than one class
+// (starts in A.mixed) and the last, partial one.  A chunk is summed in FP32 as
+// a whole, so these few are not divided between the class launches.
+__global__ void __launch_bounds__(128) hartree_mixed_kernel(const HartreeArgs A) {
+    extern __shared__ float4 smem[];
+    for (int i = threadIdx.x; i < 145 * 5; i += blockDim.x) smem[i] = A.boys32[i];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int item = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (item >= A.nblk * A.nmixed) return;
+    const int blk = item / A.nmixed, q = item - blk * A.nmixed;
+    const int64_t g0 = (int64_t)blk * 32 + lane;
+    const int64_t g = g0 < A.npts ? g0 : A.npts - 1;
+    const double gx = A.coords[3 * g], gy = A.coords[3 * g + 1], gz = A.coords[3 * g + 2];
+    const float3 gh = make_float3((float)gx, (float)gy, (float)gz);
+    const float3 gl = make_float3((float)(gx - (double)gh.x), (float)(gy - (double)gh.y),
+                                  (float)(gz - (double)gh.z));
+    const float4 cr = A.blk_cr[blk];
+    const int k = A.mixed[q] + lane;
+    bool keep = k < A.npairs;
+    int4 h = make_int4(0, 0, 0, 0);
+    if (keep) {
+        h = A.hdr[k];
+        if (A.tol > 0.0f)
+            keep = screen_pair(A.tol, A.bnd, A.bpref, cr, h, A.ptau[k], A.pair_dabs[k]);
+    }
+    unsigned mask = __ballot_sync(0xffffffffu, keep);
+    if (lane == 0 && A.kept) atomicAdd(A.kept, (unsigned long long)__popc(mask));
+    float chunk = 0.0f;
+    while (mask) {
+        const int src = __ffs(mask) - 1;
+        mask &= mask - 1;
+        const int kk = A.mixed[q] + src;
+        const int pp0 = __shfl_sync(0xffffffffu, h.z, src);
+        const int npp = __shfl_sync(0xffffffffu, h.w, src) & 0xffff;
+        int c = 0;                  // the pair's class
+        while (c < 9 && kk >= A.cls_end[c]) ++c;
+        float pair = 0.0f;
+        for (int m = pp0; m < pp0 + npp; ++m) {
+            const long long off = A.dh_off[m];
+            switch (A.cls_l[c]) {
+            case 0: pair += hartree_pp<false, 0>(A, m, off, gx, gy, gz, gh, gl, smem); break;
+            case 1: pair += hartree_pp<false, 1>(A, m, off, gx, gy, gz, gh, gl, smem); break;
+            case 2: pair += hartree_pp<false, 2>(A, m, off, gx, gy, gz, gh, gl, smem); break;
+            case 3: pair += hartree_pp<false, 3>(A, m, off, gx, gy, gz, gh, gl, smem); break;
+            case 4: pair += hartree_pp<false, 4>(A, m, off, gx, gy, gz, gh, gl, smem); break;
+            case 5: pair += hartree_pp<false, 5>(A, m, off, gx, gy, gz, gh, gl, smem); break;
+            default: pair += hartree_pp<false, 6>(A, m, off, gx, gy, gz, gh, gl, smem); break;
+            }
+        }
+        chunk += pair;
+    }
+    A.vmixed[((int64_t)q * A.nblk + blk) * 32 + lane] = (double)chunk;
+}
+
+__global__ void hartree_sum_kernel(const double* __restrict__ vpart, const int64_t npts,
+                                   const int64_t stride, const int nrow,
+                                   double* __restrict__ v) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= npts) return;
+    double s = 0.0;
+    for (int q = 0; q < nrow; ++q) s += vpart[q * stride + g];
+    v[g] = s;
 }
 
 cudaError_t launch_block_geom(const double* xyz, int64_t npts, int nblk, float4* cr,
@@ -593,24 +654,44 @@ cudaError_t launch_block_geom(const double* xyz, int64_t npts, int nblk, float4*
     return cudaGetLastError();
 }
 
-// One point per lane.  A two-point form (the pair's data read once for
-// both points, each point keeping its own sub-block's screen: bitwise the
-// same values) measured slower in the device SCF (J 0.250 against
-// 0.234 s on 8 waters): its extra registers cost more occupancy than the
-// shared loads saved.
-cudaError_t launch_hartree(const HartreeArgs& a, bool fp64, cudaStream_t s) {
-    if (a.nblk <= 0) return cudaSuccess;
-    const int grid = std::max(1, std::min(a.nblk / 4 + 1, sm_count() * 8));
-    if (fp64) {
-        const size_t smem = HartreeTraits<true>::kTabBytes;
-        cudaError_t e = cudaFuncSetAttribute(hartree_kernel<true>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return e;
-        hartree_kernel<true><<<grid, 128, smem, s>>>(a);
-    } else {
-        hartree_kernel<false><<<grid, 128, HartreeTraits<false>::kTabBytes, s>>>(a);
+template<bool F64, int L>
+static cudaError_t run_hartree(const HartreeArgs& a, int cls, int pb, int pe, cudaStream_t s) {
+    typedef HartreeTraits<F64> Tr;
+    auto k = hartree_kernel<F64, L>;
+    constexpr int smem = Tr::template table_bytes<L>();
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const int grid = std::max(1, std::min(sm_count() * Tr::kCtas, a.nblk * a.nseg));
+    k<<<grid, Tr::kThreads, smem, s>>>(a, cls, pb, pe);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_hartree_class(const HartreeArgs& a, bool fp64, int cls, int L, int pb,
+                                 int pe, cudaStream_t s) {
+    if (a.nblk <= 0 || pe <= pb) return cudaSuccess;
+    switch (L) {
+    case 0: return fp64 ? run_hartree<true, 0>(a, cls, pb, pe, s) : run_hartree<false, 0>(a, cls, pb, pe, s);
+    case 1: return fp64 ? run_hartree<true, 1>(a, cls, pb, pe, s) : run_hartree<false, 1>(a, cls, pb, pe, s);
+    case 2: return fp64 ? run_hartree<true, 2>(a, cls, pb, pe, s) : run_hartree<false, 2>(a, cls, pb, pe, s);
+    case 3: return fp64 ? run_hartree<true, 3>(a, cls, pb, pe, s) : run_hartree<false, 3>(a, cls, pb, pe, s);
+    case 4: return fp64 ? run_hartree<true, 4>(a, cls, pb, pe, s) : run_hartree<false, 4>(a, cls, pb, pe, s);
+    case 5: return fp64 ? run_hartree<true, 5>(a, cls, pb, pe, s) : run_hartree<false, 5>(a, cls, pb, pe, s);
+    default: return fp64 ? run_hartree<true, 6>(a, cls, pb, pe, s) : run_hartree<false, 6>(a, cls, pb, pe, s);
     }
+}
+
+cudaError_t launch_hartree_mixed(const HartreeArgs& a, cudaStream_t s) {
+    const int64_t warps = (int64_t)a.nblk * a.nmixed;
+    if (warps <= 0) return cudaSuccess;
+    hartree_mixed_kernel<<<(unsigned)((warps + 3) / 4), 128,
+                           HartreeTraits<false>::table_bytes<0>(), s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_hartree_sum(const HartreeArgs& a, double* v, cudaStream_t s) {
+    if (a.npts <= 0) return cudaSuccess;
+    hartree_sum_kernel<<<(unsigned)((a.npts + 255) / 256), 256, 0, s>>>(
+        a.vpart, a.npts, 32 * (int64_t)a.nblk, a.nseg + a.nmixed, v);
     return cudaGetLastError();
 }
 
