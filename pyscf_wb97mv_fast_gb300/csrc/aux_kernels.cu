@@ -617,7 +617,7 @@ cudaError_t launch_gsum2(const float* gc0, const float* gc1, const int4* src, in
 // integer pipe, the angular factors skip the zeros of the transform, and the
 // gradient is rad1 S d + rad0 grad S from the solid harmonic S and its
 // derivatives rather than from every Cartesian component.  648 AOs x 384,998
-// points: 6.0 -> 3.0 ms; with gradients, 442 x 157,256: 3.5 -> 1.2 ms.
+// points: 6.0 -> 1.4 ms; with gradients, 442 x 157,256: 3.5 -> 1.1 ms.
 __constant__ double c_c2s0[1];
 __constant__ double c_c2s1[9];
 __constant__ double c_c2s2[30];
@@ -717,7 +717,8 @@ __device__ __forceinline__ constexpr bool solid_flat(const int m, const int a) {
 template<int L, bool D>
 __device__ __forceinline__ void ao_shell(const AoArgs& A, const int sh, const int64_t g,
                                          const double dx, const double dy, const double dz,
-                                         const double r2, const unsigned long long* etab) {
+                                         const double r2, const float r2f,
+                                         const unsigned long long* etab) {
     constexpr int NS = 2 * L + 1;
     const int np = A.sh_np[sh], nc = A.sh_nc[sh];
     const double* ex = A.exps + A.sh_eoff[sh];
@@ -732,11 +733,19 @@ __device__ __forceinline__ void ao_shell(const AoArgs& A, const int sh, const in
         double rad0 = 0.0, rad1 = 0.0;
         bool live = false;
         for (int k = 0; k < np; ++k) {
-            const double a = ex[k] * r2;
+            // far out: decided in FP32 (exp(-71) and below), no FP64 product
+            const double exk = ex[k];
+            if (f64::narrow(exk) * r2f > 71.0f) continue;
+            const double a = exk * r2;
             if (!below70(a)) continue;
-            const double e = co[k * nc + ci] * f64::exp_neg(a, etab);
-            rad0 += e;
-            if constexpr (D) rad1 = fma(-2.0 * ex[k], e, rad1);
+            const double e = f64::exp_neg(a, etab);
+            if constexpr (D) {
+                const double w = co[k * nc + ci] * e;
+                rad0 += w;
+                rad1 = fma(-f64::twice(exk), w, rad1);
+            } else {
+                rad0 = fma(co[k * nc + ci], e, rad0);
+            }
             live = true;
         }
         double* out = A.X + (int64_t)(ao0 + ci * NS) * A.ld + g;
@@ -745,6 +754,26 @@ __device__ __forceinline__ void ao_shell(const AoArgs& A, const int sh, const in
             for (int m = 0; m < NS; ++m)
 #pragma unroll
                 for (int p = 0; p < (D ? 4 : 1); ++p) out[p * plane + (int64_t)m * A.ld] = 0.0;
+            continue;
+        }
+        if constexpr (L == 1) {
+            // S_m = c d_m: fewer products than by S
+            const double c = c_c2s1[0], d[3] = {dx, dy, dz}, v0 = rad0 * c;
+#pragma unroll
+            for (int m = 0; m < 3; ++m) out[(int64_t)m * A.ld] = v0 * d[m];
+            if constexpr (D) {
+                const double t = rad1 * c;
+#pragma unroll
+                for (int m = 0; m < 3; ++m) {
+                    const double u = t * d[m];
+#pragma unroll
+                    for (int x = m; x < 3; ++x) {
+                        const double g2 = x == m ? fma(u, d[x], v0) : u * d[x];
+                        out[(x + 1) * plane + (int64_t)m * A.ld] = g2;
+                        if (x != m) out[(m + 1) * plane + (int64_t)x * A.ld] = g2;
+                    }
+                }
+            }
             continue;
         }
         if (!have) {
@@ -787,12 +816,13 @@ __global__ void __launch_bounds__(128) ao_eval_kernel(const AoArgs A) {
     const double dy = A.coords[g * 3 + 1] - A.sh_ctr[s0 * 3 + 1];
     const double dz = A.coords[g * 3 + 2] - A.sh_ctr[s0 * 3 + 2];
     const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    const float r2f = f64::narrow(r2);
     for (int sh = s0; sh < s1; ++sh)
         switch (A.sh_l[sh]) {
-        case 0: ao_shell<0, D>(A, sh, g, dx, dy, dz, r2, etab); break;
-        case 1: ao_shell<1, D>(A, sh, g, dx, dy, dz, r2, etab); break;
-        case 2: ao_shell<2, D>(A, sh, g, dx, dy, dz, r2, etab); break;
-        default: ao_shell<3, D>(A, sh, g, dx, dy, dz, r2, etab); break;
+        case 0: ao_shell<0, D>(A, sh, g, dx, dy, dz, r2, r2f, etab); break;
+        case 1: ao_shell<1, D>(A, sh, g, dx, dy, dz, r2, r2f, etab); break;
+        case 2: ao_shell<2, D>(A, sh, g, dx, dy, dz, r2, r2f, etab); break;
+        default: ao_shell<3, D>(A, sh, g, dx, dy, dz, r2, r2f, etab); break;
         }
 }
 
