@@ -1325,7 +1325,7 @@ int wb_cosx_get_k_multi(wb_cosx* h, const double* coords,
                 at<unsigned long long>(workspace, L.counters) + 3 * wb::NCLASS);
             if (r) return fail(r >= 1000 ? WB_ERR_CUBLAS : WB_ERR_CUDA,
                                "ozaki F GEMM failed, code " + std::to_string(r));
-            launches += wb::ozaki_f_launches();
+            launches += wb::ozaki_f_launches(nao);
         } else {
             // F(g, mu) = sum_l X(g, l) QD(l, mu); QD row-major = col-major QD^T
             WB_CUBLAS(cublasDgemm(h->cublas, CUBLAS_OP_N, CUBLAS_OP_T, (int)ldt,
@@ -1352,7 +1352,7 @@ int wb_cosx_get_k_multi(wb_cosx* h, const double* coords,
                 if (r) return fail(r >= 1000 ? WB_ERR_CUBLAS : WB_ERR_CUDA,
                                    "ozaki K GEMM failed, code " + std::to_string(r));
                 x_sliced = true;
-                launches += 2 + wb::kOzSlices;
+                launches += wb::ozaki_k_launches(nao, ldt);
             } else {
                 if ((rs = phase_to(4)) != WB_OK) return rs;
                 WB_CUDA(wb::launch_weight_g(Gsrc, w, nt, ldt, nao, F64, s));
@@ -1392,7 +1392,7 @@ int wb_cosx_get_k_multi(wb_cosx* h, const double* coords,
                     if (r) return fail(r >= 1000 ? WB_ERR_CUBLAS : WB_ERR_CUDA,
                                        "ozaki K GEMM failed, code " + std::to_string(r));
                     x_sliced = true;
-                    launches += 3 + wb::kOzSlices;
+                    launches += wb::ozaki_k_launches(nao, ldt);
                     if ((st = phase_to(3)) != WB_OK) return st;
                 } else {
                     if ((st = k_gemm(ja, G32)) != WB_OK) return st;
@@ -1819,7 +1819,7 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
                 at<unsigned long long>(ws, L.counters) + 3 * wb::NCLASS);
             if (r) return fail(r >= 1000 ? WB_ERR_CUBLAS : WB_ERR_CUDA,
                                "ozaki F GEMM failed, code " + std::to_string(r));
-            launches += wb::ozaki_f_launches();
+            launches += wb::ozaki_f_launches(nao);
         } else {
             double* F64 = static_cast<double*>(b->scratch);
             WB_CUBLAS(cublasDgemm(h->cublas, CUBLAS_OP_N, CUBLAS_OP_T, (int)ld, nao, nao,
@@ -1906,7 +1906,7 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
                                                  b->scratch, s, false);
             if (r) return fail(r >= 1000 ? WB_ERR_CUBLAS : WB_ERR_CUDA,
                                "ozaki K GEMM failed, code " + std::to_string(r));
-            launches += 3 + wb::kOzSlices;
+            launches += wb::ozaki_k_launches(nao, ld);
         } else {
             double* WG = static_cast<double*>(b->scratch);
             for (int w = 0; w < b->nom; ++w) {

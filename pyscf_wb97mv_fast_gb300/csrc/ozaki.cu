@@ -8,15 +8,20 @@
 //
 //   x = 2^(e-W+1) sum_i d_i 2^(B (S-1-i)),  |d_i| <= 2^(B-1)  (bf16-exact)
 //
-// with e per row / column (chunk), B = 6-bit balanced digits, S = 7 slices
-// (W = 42 bits), the digits cut from rint(x 2^(W-1-e)) with integer ops.
+// with e per row / column (chunk), W = B S = 42 bits, the balanced digits cut
+// from rint(x 2^(W-1-e)) with integer ops: S = 6 slices of B = 7 bits, 21
+// slice products, where the sums below stay exact, else 7 of 6 bits, 28.
 // A product level l = i + j collects sum_{i+j=l} A_i B_j in ONE bf16 GEMM
 // with FP32 accumulation: storing the A slices ascending and the B slices
 // descending along K makes every level a prefix of A times a suffix of B.
-// Every product is an integer of magnitude <= 2^(2B-2) = 1024 and a level
-// sums at most (l+1) * Kc of them, so with (l+1) Kc < 2^14 every partial
-// sum is an integer below 2^24: the FP32 accumulation is exact, whatever
-// order the tensor cores use.  Levels are combined exactly in int64 and
+// Every product is an integer of magnitude <= 2^(2B-2), so while a GEMM sums
+// at most 2^(26-2B) of them every partial sum is an integer up to 2^24: the
+// FP32 accumulation is exact, whatever order the tensor cores use.  F sums
+// (l+1) nao terms: 7-bit digits to nao = 680, 6-bit ones above.  The K product
+// always takes 7-bit digits, its longer levels cut into pieces of 4096 terms,
+// each a GEMM of its own (27 waters, 384,998 points: F 7.8 -> 6.4
+// ms, K product of one right-hand side 9.1 -> 7.5 ms against 6-bit digits
+// throughout).  Pieces and levels are combined exactly in int64 and
 // scaled once in FP64.  The result carries W = 42 bits relative to the
 // per-row / per-column maxima; the truncated products (i + j >= S) are
 // below 2^-W of them.
@@ -26,9 +31,9 @@
 // kernels.  ozaki_set_f_engine(kOzEngineTc) runs the F product on this
 // library's own tensor-core kernel instead (ozaki_tc.cu: TMA, tcgen05 MMAs
 // into TMEM, the level combination fused into its epilogue) -- bitwise the
-// same result; its seven exact level accumulators leave room for 64-wide
+// same result; its six or seven exact level accumulators leave room for 64-wide
 // N tiles only, and it measured 2.4x slower than the library form on the
-// bench step (18.4 vs 7.65 ms).  The K product's level GEMMs are cuBLAS.
+// bench step (18.4 vs 7.65 ms with 6-bit digits).  The K product's level GEMMs are cuBLAS.
 #include <cublas_v2.h>
 #include <cuda_bf16.h>
 
@@ -79,7 +84,7 @@ __global__ void f_rowmax_kernel(const double* __restrict__ X, int nao,
 }
 
 // slices of X: one thread per (row l, two points); bf16 pairs per store
-template<int S>
+template<int B_, int S>
 __global__ void f_slice_x_kernel(const double* __restrict__ X, int nao, int np,
                                  int64_t ld, const int* __restrict__ erow,
                                  __nv_bfloat16* __restrict__ A) {
@@ -90,15 +95,15 @@ __global__ void f_slice_x_kernel(const double* __restrict__ X, int nao, int np,
     if (l < nao) x = *reinterpret_cast<const double2*>(X + (int64_t)l * ld + g);
     const int2 e = *reinterpret_cast<const int2*>(erow + g);
     float d0[S], d1[S];
-    digits<S>(x.x, e.x, d0);
-    digits<S>(x.y, e.y, d1);
+    digits<B_, S>(x.x, e.x, d0);
+    digits<B_, S>(x.y, e.y, d1);
 #pragma unroll
     for (int i = 0; i < S; ++i)
         *reinterpret_cast<__nv_bfloat162*>(A + ((int64_t)i * np + l) * ld + g) =
             __floats2bfloat162_rn(d0[i], d1[i]);
 }
 
-template<int S>
+template<int B_, int S>
 __global__ void f_slice_qd_kernel(const double* __restrict__ QD, int nao, int np,
                                   int* __restrict__ ecol,
                                   __nv_bfloat16* __restrict__ B) {
@@ -124,7 +129,7 @@ __global__ void f_slice_qd_kernel(const double* __restrict__ QD, int nao, int np
     const int64_t ldb = (int64_t)S * np;
     for (int l = threadIdx.x; l < np; l += blockDim.x) {
         float d[S];
-        digits<S>(l < nao ? QD[(int64_t)l * nao + mu] : 0.0, e, d);
+        digits<B_, S>(l < nao ? QD[(int64_t)l * nao + mu] : 0.0, e, d);
 #pragma unroll
         for (int i = 0; i < S; ++i)
             B[(int64_t)mu * ldb + (int64_t)(S - 1 - i) * np + l] =
@@ -134,7 +139,7 @@ __global__ void f_slice_qd_kernel(const double* __restrict__ QD, int nao, int np
 
 // x y = 2^(e+f-2W+2) sum_l C_l 2^(B (2S-2-l))
 //     = 2^(e+f-2W+2+B(S-1)) * [sum_l C_l 2^(B (S-1-l))]
-template<int S, typename T>
+template<int B_, int S, typename T>
 __global__ void f_combine_kernel(const float* __restrict__ C, int nao,
                                  int64_t ld, const int* __restrict__ erow,
                                  const int* __restrict__ ecol,
@@ -149,16 +154,17 @@ __global__ void f_combine_kernel(const float* __restrict__ C, int nao,
     for (int l = 0; l < S; ++l)
         c[l] = __ldg(reinterpret_cast<const float4*>(C + (int64_t)l * plane + i));
     const int4 er = *reinterpret_cast<const int4*>(erow + g);
-    const int base = ecol[mu] - 2 * kW + 2 + kB * (S - 1);
-    float v[4][S];
+    const int base = ecol[mu] - 2 * kW + 2 + B_ * (S - 1);
+    long long v[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int l = 0; l < S; ++l) {
-        v[0][l] = c[l].x; v[1][l] = c[l].y; v[2][l] = c[l].z; v[3][l] = c[l].w;
+        v[0] += level_term<B_, S>(l, c[l].x); v[1] += level_term<B_, S>(l, c[l].y);
+        v[2] += level_term<B_, S>(l, c[l].z); v[3] += level_term<B_, S>(l, c[l].w);
     }
-    const T o0 = scaled_ll_to<T>(combine_levels<S>(v[0]), er.x + base);
-    const T o1 = scaled_ll_to<T>(combine_levels<S>(v[1]), er.y + base);
-    const T o2 = scaled_ll_to<T>(combine_levels<S>(v[2]), er.z + base);
-    const T o3 = scaled_ll_to<T>(combine_levels<S>(v[3]), er.w + base);
+    const T o0 = scaled_ll_to<T>(v[0], er.x + base);
+    const T o1 = scaled_ll_to<T>(v[1], er.y + base);
+    const T o2 = scaled_ll_to<T>(v[2], er.z + base);
+    const T o3 = scaled_ll_to<T>(v[3], er.w + base);
     if constexpr (sizeof(T) == 4) {
         *reinterpret_cast<float4*>(F + i) = make_float4(o0, o1, o2, o3);
     } else {
@@ -177,19 +183,26 @@ __global__ void f_combine_kernel(const float* __restrict__ C, int nao,
 // 16-byte rows and outputs, as for F).  One CTA of KC / 8 threads per (chunk,
 // column).
 // ---------------------------------------------------------------------------
-// DOX = false: the X slices and exponents of this tile are already in A /
-// ex (an earlier omega of the same tile); only w o G is sliced.  B holds nb
-// columns per chunk (several right-hand sides side by side); this launch
-// fills columns boff .. boff + np - 1 (np = gridDim.y).
-template<int S, int KC, bool DOX, typename GT>
+// gridDim.z right-hand sides: B holds nb columns per chunk, those of right-hand
+// side r at r np (np = gridDim.y).  The CTAs of the first one also slice X,
+// unless slice_x is 0: the X slices and exponents of this tile are then already
+// in A / ex (an earlier omega of the same tile).
+template<typename GT>
+struct KIn {
+    const GT* g[8];
+};
+template<int B_, int S, int KC, typename GT>
 __global__ void __launch_bounds__(KC / 8, 4)
-k_slice_kernel(const double* __restrict__ X, const GT* __restrict__ G,
+k_slice_kernel(const double* __restrict__ X, const __grid_constant__ KIn<GT> Gs, const int slice_x,
                const double* __restrict__ w, int nao, int64_t ld,
                int64_t npts, int* __restrict__ ex, int* __restrict__ ew,
                __nv_bfloat16* __restrict__ A, __nv_bfloat16* __restrict__ B,
-               int nb, int boff) {
+               int nb) {
     constexpr int T = KC / 8;               // threads: eight points each
     const int c = blockIdx.x, col = blockIdx.y, np = gridDim.y;
+    const int boff = blockIdx.z * np;
+    const bool dox = slice_x && blockIdx.z == 0;
+    const GT* __restrict__ G = Gs.g[blockIdx.z];
     const int64_t nlive = col < nao ? npts : 0;     // a column past nao is zero
     __shared__ unsigned long long rx[T / 32], rw[T / 32];
     const int k0 = 8 * threadIdx.x;
@@ -217,7 +230,7 @@ k_slice_kernel(const double* __restrict__ X, const GT* __restrict__ G,
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const double2 b = __ldg(wp + u);
-            if (DOX) {
+            if (dox) {
                 const double2 a = __ldg(xp + u);
                 xv[2 * u] = a.x; xv[2 * u + 1] = a.y;
             } else {
@@ -233,7 +246,7 @@ k_slice_kernel(const double* __restrict__ X, const GT* __restrict__ G,
             xv[u] = 0.0;
             wv[u] = 0.0;
             if (g < nlive) {
-                if (DOX) xv[u] = X[(int64_t)col * ld + g];
+                if (dox) xv[u] = X[(int64_t)col * ld + g];
                 wv[u] = w[g] * (double)G[(int64_t)col * ld + g];
             }
         }
@@ -265,7 +278,7 @@ k_slice_kernel(const double* __restrict__ X, const GT* __restrict__ G,
     }
     const int e1 = exp_of_bits(mx), e2 = exp_of_bits(mw);
     if (threadIdx.x == 0) {
-        if (DOX) ex[(int64_t)c * np + col] = e1;
+        if (dox) ex[(int64_t)c * np + col] = e1;
         ew[(int64_t)c * nb + boff + col] = e2;
     }
     const int64_t colbase = (int64_t)c * S * KC * np + (int64_t)col * S * KC;
@@ -275,7 +288,7 @@ k_slice_kernel(const double* __restrict__ X, const GT* __restrict__ G,
     auto store = [&](const double* v, const int e, __nv_bfloat16* dst, const bool desc) {
         float d[8][S];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) digits<S>(v[u], e, d[u]);
+        for (int u = 0; u < 8; ++u) digits<B_, S>(v[u], e, d[u]);
 #pragma unroll
         for (int i = 0; i < S; ++i) {
             __nv_bfloat162 p[4];
@@ -286,53 +299,62 @@ k_slice_kernel(const double* __restrict__ X, const GT* __restrict__ G,
                 *reinterpret_cast<const uint4*>(p);
         }
     };
-    if (DOX) store(xv, e1, A + colbase, false);
+    if (dox) store(xv, e1, A + colbase, false);
     store(wv, e2, B + colbase_b, true);
 }
 
 // K_r[mu, nu] (+)= sum_c 2^(ex+ew-2W+2+B(S-1)) [sum_l C[l][c] 2^(B (S-1-l))]
 // for the nb / np right-hand sides r (column r np + nu of C)
+constexpr int kKB = 7, kKS = 6;         // the K product's digits
+constexpr int kOzPiece = 4096;          // terms of an exact FP32 sum of 7-bit products
+
 struct KOut {
     double* k[8];
 };
 
-template<int S>
+// C holds the level planes in order, a level of more than kOzPiece terms as
+// several planes (pieces), each (chunk, np x nb)
+template<int B_, int S, int KC>
 __global__ void k_combine_kernel(const float* __restrict__ C, int nao, int np, int nb,
                                  int nchunk, const int* __restrict__ ex,
                                  const int* __restrict__ ew, int accumulate,
-                                 const KOut Ks) {
+                                 const __grid_constant__ KOut Ks) {
     const int64_t nc = (int64_t)np * nb;
+    const int64_t plane = nc * nchunk;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nc;
          i += (int64_t)gridDim.x * blockDim.x) {
         const int mu = (int)(i % np), col = (int)(i / np);     // C col-major
         if (mu >= nao || col % np >= nao) continue;
         double acc = 0.0;
-        // four chunks' loads in flight at once; the sum stays in chunk order
-        constexpr int U = 4;
+        // three chunks' loads in flight at once; the sum stays in chunk order
+        constexpr int U = 3;
+        auto value = [&](int c) -> long long {
+            const float* p = C + (int64_t)c * nc + i;
+            long long v = 0;
+#pragma unroll
+            for (int l = 0; l < S; ++l)
+#pragma unroll
+                for (int left = (l + 1) * KC; left > 0; left -= kOzPiece, p += plane)
+                    v += level_term<B_, S>(l, __ldg(p));
+            return v;
+        };
+        auto scale = [&](int c) -> int {
+            return ex[(int64_t)c * np + mu] + ew[(int64_t)c * nb + col] - 2 * kW + 2 +
+                   B_ * (S - 1);
+        };
         int c = 0;
         for (; c + U <= nchunk; c += U) {
-            float v[U][S];
+            long long v[U];
             int sc[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-#pragma unroll
-                for (int l = 0; l < S; ++l)
-                    v[u][l] = __ldg(C + ((int64_t)l * nchunk + c + u) * nc + i);
-                sc[u] = ex[(int64_t)(c + u) * np + mu] + ew[(int64_t)(c + u) * nb + col] -
-                        2 * kW + 2 + kB * (S - 1);
+                v[u] = value(c + u);
+                sc[u] = scale(c + u);
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) acc += (double)combine_levels<S>(v[u]) * pow2(sc[u]);
+            for (int u = 0; u < U; ++u) acc += (double)v[u] * pow2(sc[u]);
         }
-        for (; c < nchunk; ++c) {
-            float v[S];
-#pragma unroll
-            for (int l = 0; l < S; ++l) v[l] = C[((int64_t)l * nchunk + c) * nc + i];
-            const long long lv = combine_levels<S>(v);
-            const int sc = ex[(int64_t)c * np + mu] + ew[(int64_t)c * nb + col] -
-                           2 * kW + 2 + kB * (S - 1);
-            acc += (double)lv * pow2(sc);
-        }
+        for (; c < nchunk; ++c) acc += (double)value(c) * pow2(scale(c));
         double* K = Ks.k[col / np];
         const int64_t o = (int64_t)mu * nao + col % np;        // K row-major
         K[o] = accumulate ? K[o] + acc : acc;
@@ -343,6 +365,13 @@ __global__ void k_combine_kernel(const float* __restrict__ C, int nao, int np, i
 static inline size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
 
 static inline int pad8(int n) { return (n + 7) & ~7; }
+
+// level planes of the K product
+static inline int k_planes(int kc) {
+    int n = 0;
+    for (int l = 0; l < kKS; ++l) n += ((l + 1) * kc + kOzPiece - 1) / kOzPiece;
+    return n;
+}
 
 // Points per chunk of the K product.  2048 is the largest with exact level
 // sums and moves the least level output per point; where it would leave SMs
@@ -355,7 +384,7 @@ static inline int k_chunk(int np, int64_t ld) {
 }
 
 size_t ozaki_f_bytes(int nao, int64_t ld) {
-    const size_t S = kOzSlices, np = pad8(nao);
+    const size_t S = ozaki_f_seven_bit(nao) ? 6 : 7, np = pad8(nao);
     const size_t lib = al(sizeof(int) * ld) + al(sizeof(int) * nao) +
                        al(sizeof(__nv_bfloat16) * S * np * ld) +
                        al(sizeof(__nv_bfloat16) * S * np * nao) +
@@ -364,13 +393,13 @@ size_t ozaki_f_bytes(int nao, int64_t ld) {
 }
 
 size_t ozaki_k_bytes(int nao, int64_t ld, int nrhs) {
-    const size_t S = kOzSlices, np = pad8(nao);
+    const size_t S = kKS, np = pad8(nao);
     auto bytes = [&](size_t kc, int64_t n) {
         const size_t nchunk = (n + kc - 1) / kc;
         return al(sizeof(int) * nchunk * np) + al(sizeof(int) * nchunk * np * nrhs) +
                al(sizeof(__nv_bfloat16) * S * kc * nchunk * np) +
                al(sizeof(__nv_bfloat16) * S * kc * nchunk * np * nrhs) +
-               al(sizeof(float) * S * nchunk * np * np * nrhs);
+               al(sizeof(float) * k_planes((int)kc) * nchunk * np * np * nrhs);
     };
     // enough for every grid of up to ld points (a ragged last tile may take
     // the small chunks where the full one does not)
@@ -417,10 +446,9 @@ int ozaki_f_gemm64(cublasHandle_t hb, const double* X, const double* QD,
     return ozaki_f_gemm_cublas64(hb, X, QD, nao, ld, F, ws, s);
 }
 
-template<typename T>
+template<int B_, int S, typename T>
 static int f_gemm_cublas_t(cublasHandle_t hb, const double* X, const double* QD,
                            int nao, int64_t ld, T* F, void* ws, cudaStream_t s) {
-    constexpr int S = kOzSlices;
     const int np = pad8(nao);
     char* p = static_cast<char*>(ws);
     int* erow = reinterpret_cast<int*>(p); p += al(sizeof(int) * ld);
@@ -434,10 +462,10 @@ static int f_gemm_cublas_t(cublasHandle_t hb, const double* X, const double* QD,
     OZ_CUDA(cudaGetLastError());
     {
         dim3 grid((unsigned)((ld / 2 + 255) / 256), (unsigned)np);
-        f_slice_x_kernel<S><<<grid, 256, 0, s>>>(X, nao, np, ld, erow, A);
+        f_slice_x_kernel<B_, S><<<grid, 256, 0, s>>>(X, nao, np, ld, erow, A);
         OZ_CUDA(cudaGetLastError());
     }
-    f_slice_qd_kernel<S><<<nao, 256, 0, s>>>(QD, nao, np, ecol, B);
+    f_slice_qd_kernel<B_, S><<<nao, 256, 0, s>>>(QD, nao, np, ecol, B);
     OZ_CUDA(cudaGetLastError());
     const float one = 1.0f, zero = 0.0f;
     for (int l = 0; l < S; ++l) {
@@ -451,7 +479,7 @@ static int f_gemm_cublas_t(cublasHandle_t hb, const double* X, const double* QD,
     }
     {
         dim3 grid((unsigned)((ld / 4 + 255) / 256), (unsigned)nao);
-        f_combine_kernel<S, T><<<grid, 256, 0, s>>>(C, nao, ld, erow, ecol, F);
+        f_combine_kernel<B_, S, T><<<grid, 256, 0, s>>>(C, nao, ld, erow, ecol, F);
         OZ_CUDA(cudaGetLastError());
     }
     return 0;
@@ -459,12 +487,16 @@ static int f_gemm_cublas_t(cublasHandle_t hb, const double* X, const double* QD,
 
 int ozaki_f_gemm_cublas(cublasHandle_t hb, const double* X, const double* QD,
                         int nao, int64_t ld, float* F, void* ws, cudaStream_t s) {
-    return f_gemm_cublas_t<float>(hb, X, QD, nao, ld, F, ws, s);
+    return ozaki_f_seven_bit(nao)
+               ? f_gemm_cublas_t<7, 6, float>(hb, X, QD, nao, ld, F, ws, s)
+               : f_gemm_cublas_t<6, 7, float>(hb, X, QD, nao, ld, F, ws, s);
 }
 
 int ozaki_f_gemm_cublas64(cublasHandle_t hb, const double* X, const double* QD,
                           int nao, int64_t ld, double* F, void* ws, cudaStream_t s) {
-    return f_gemm_cublas_t<double>(hb, X, QD, nao, ld, F, ws, s);
+    return ozaki_f_seven_bit(nao)
+               ? f_gemm_cublas_t<7, 6, double>(hb, X, QD, nao, ld, F, ws, s)
+               : f_gemm_cublas_t<6, 7, double>(hb, X, QD, nao, ld, F, ws, s);
 }
 
 template<int KC, typename GT>
@@ -472,7 +504,7 @@ static int k_gemm_multi_t(cublasHandle_t hb, const double* X, const GT* const* G
                           int nrhs, const double* w, int nao, int64_t ld,
                           int64_t npts, int accumulate, double* const* K, void* ws,
                           cudaStream_t s, bool x_sliced) {
-    constexpr int S = kOzSlices;
+    constexpr int S = kKS;
     if (nrhs < 1 || nrhs > 8) return (int)cudaErrorInvalidValue;
     const int nchunk = (int)((ld + KC - 1) / KC);
     const int np = pad8(nao), nb = nrhs * np;
@@ -489,33 +521,32 @@ static int k_gemm_multi_t(cublasHandle_t hb, const double* X, const GT* const* G
     float* C = reinterpret_cast<float*>(p);
     KOut Kd = {};
     for (int r = 0; r < nrhs; ++r) Kd.k[r] = K[r];
-    dim3 grid(nchunk, np);
-    for (int r = 0; r < nrhs; ++r) {
-        if (x_sliced || r > 0)
-            k_slice_kernel<S, KC, false, GT><<<grid, KC / 8, 0, s>>>(
-                X, G[r], w, nao, ld, npts, ex, ew, A, B, nb, r * np);
-        else
-            k_slice_kernel<S, KC, true, GT><<<grid, KC / 8, 0, s>>>(
-                X, G[r], w, nao, ld, npts, ex, ew, A, B, nb, r * np);
-        OZ_CUDA(cudaGetLastError());
-    }
+    KIn<GT> in = {};
+    for (int r = 0; r < nrhs; ++r) in.g[r] = G[r];
+    k_slice_kernel<kKB, S, KC, GT><<<dim3(nchunk, np, nrhs), KC / 8, 0, s>>>(
+        X, in, x_sliced ? 0 : 1, w, nao, ld, npts, ex, ew, A, B, nb);
+    OZ_CUDA(cudaGetLastError());
     const float one = 1.0f, zero = 0.0f;
     const long long stride_a = (long long)S * KC * np;
     const long long stride_b = (long long)S * KC * nb;
     const long long nc = (long long)np * nb;
-    for (int l = 0; l < S; ++l) {
-        OZ_CUBLAS(cublasGemmStridedBatchedEx(
-            hb, CUBLAS_OP_T, CUBLAS_OP_N, np, nb, (l + 1) * KC, &one, A,
-            CUDA_R_16BF, S * KC, stride_a, B + (size_t)(S - 1 - l) * KC,
-            CUDA_R_16BF, S * KC, stride_b, &zero, C + (size_t)l * nchunk * nc,
-            CUDA_R_32F, np, nc, nchunk, CUBLAS_COMPUTE_32F,
-            CUBLAS_GEMM_DEFAULT));
-    }
+    float* c = C;
+    for (int l = 0; l < S; ++l)
+        for (int k0 = 0; k0 < (l + 1) * KC; k0 += kOzPiece, c += (size_t)nchunk * nc)
+            OZ_CUBLAS(cublasGemmStridedBatchedEx(
+                hb, CUBLAS_OP_T, CUBLAS_OP_N, np, nb, std::min(kOzPiece, (l + 1) * KC - k0),
+                &one, A + k0, CUDA_R_16BF, S * KC, stride_a,
+                B + (size_t)(S - 1 - l) * KC + k0, CUDA_R_16BF, S * KC, stride_b, &zero, c,
+                CUDA_R_32F, np, nc, nchunk, CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT));
     const int64_t blocks = grid_stride_blocks(nc, 256, 32);
-    k_combine_kernel<S><<<(unsigned)blocks, 256, 0, s>>>(C, nao, np, nb, nchunk, ex, ew,
+    k_combine_kernel<kKB, S, KC><<<(unsigned)blocks, 256, 0, s>>>(C, nao, np, nb, nchunk, ex, ew,
                                                         accumulate, Kd);
     OZ_CUDA(cudaGetLastError());
     return 0;
+}
+
+int ozaki_k_launches(int nao, int64_t ld) {
+    return 2 + k_planes(k_chunk(pad8(nao), ld));
 }
 
 template<typename GT>

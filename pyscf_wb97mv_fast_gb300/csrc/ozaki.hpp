@@ -8,13 +8,16 @@
 
 namespace wb {
 
-constexpr int kOzBits = 6;     // balanced digits, |d| <= 32
-constexpr int kOzSlices = 7;   // 42 bits per operand
-constexpr int kOzKc = 2048;    // K-GEMM chunk: (l + 1) * Kc < 2^14 for l < 7
+constexpr int kOzWidth = 42;        // bits per operand: 7 digits of 6 or 6 of 7
+constexpr int kOzKc = 2048;         // points of a K-GEMM chunk
 constexpr int kOzKcSmall = 512;     // where 2048-point chunks would leave SMs idle
 
-// exact FP32 level sums need kOzSlices * K < 2^14 along the inner dimension
-inline bool ozaki_f_supported(int nao) { return kOzSlices * nao < (1 << 14); }
+// The digits of the F product: 6 of 7 bits (21 slice products) where a level's
+// (l + 1) nao terms of up to 2^12 stay within 2^24, exact in FP32, else 7 of 6
+// bits (28), which holds to 7 nao < 2^14.  Both engines take the same, so their
+// F agree bitwise.
+inline bool ozaki_f_seven_bit(int nao) { return 6 * ((nao + 7) / 8 * 8) <= (1 << 12); }
+inline bool ozaki_f_supported(int nao) { return 7 * nao < (1 << 14); }
 
 size_t ozaki_f_bytes(int nao, int64_t ld);
 // workspace of the K split for nrhs right-hand sides (w o G of several
@@ -47,7 +50,11 @@ constexpr int kOzEngineTc = 1;
 void ozaki_set_f_engine(int engine);
 int ozaki_get_f_engine();
 // this library's kernel launches of one F product under the current engine
-inline int ozaki_f_launches() { return ozaki_get_f_engine() == kOzEngineTc ? 4 : 4 + kOzSlices; }
+inline int ozaki_f_launches(int nao) {
+    return ozaki_get_f_engine() == kOzEngineTc ? 4 : 4 + (ozaki_f_seven_bit(nao) ? 6 : 7);
+}
+// the same of one K product
+int ozaki_k_launches(int nao, int64_t ld);
 int ozaki_f_gemm_cublas(cublasHandle_t hb, const double* X, const double* QD,
                         int nao, int64_t ld, float* F, void* ws, cudaStream_t s);
 int ozaki_f_gemm_tc(const double* X, const double* QD, int nao, int64_t ld, float* F,

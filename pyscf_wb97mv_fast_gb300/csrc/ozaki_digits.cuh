@@ -12,12 +12,12 @@ namespace wb {
 
 // Fixed-point digits.  A value x with |x| < 2^e becomes the integer
 // q = rint(x 2^(W - 1 - e)), W = B S bits, |q| < 2^(W-1), written as
-// balanced base-2^B digits q = sum_i d_i 2^(B (S-1-i)), |d_i| <= 2^(B-1),
+// balanced base-2^B digits q = sum_i d_i 2^(B (S-1-i)), |d_i| <= 2^(B-1) (S =
+// 7 digits of B = 6 bits, or 6 of 7),
 // extracted from the least significant end with integer arithmetic only
 // (the one FP64 multiply by an exact power of two and one FP64 -> int64
 // conversion per element are the only FP64 operations).
-constexpr int kB = kOzBits;
-constexpr int kW = kOzBits * kOzSlices;
+constexpr int kW = kOzWidth;
 
 __device__ __forceinline__ double pow2(int k) {
     // exact 2^k for -1022 <= k <= 1023
@@ -62,27 +62,28 @@ __device__ __forceinline__ long long fixed_q(double x, int e) {
     return (b >> 63) ? -(long long)q : (long long)q;
 }
 
-template<int S>
+template<int B, int S>
 __device__ __forceinline__ void digits(double x, int e, float* d) {
-    // q (|q| < 2^(W-1) = 2^41) split as q = hi 2^24 + lo, lo in [0, 2^24):
-    // the four low digits come from lo, the carry goes into hi, the rest
-    // from hi -- 32-bit integer arithmetic throughout
-    static_assert(S == 7 && kB == 6, "digit split assumes 7 x 6 bits");
+    // q (|q| < 2^(W-1) = 2^41) split as q = hi 2^(B P) + lo, lo of P digits:
+    // the low digits come from lo, the carry goes into hi, the rest from hi --
+    // 32-bit integer arithmetic throughout
+    static_assert(S * B == kW && (B == 6 || B == 7), "42 bits in 6- or 7-bit digits");
+    constexpr int P = B == 6 ? 4 : 3, H = 1 << (B - 1), M = (1 << B) - 1;
     const long long q = fixed_q(x, e);
-    int lo = (int)(q & 0xFFFFFF);
-    int hi = (int)(q >> 24);
+    int lo = (int)(q & ((1 << (B * P)) - 1));
+    int hi = (int)(q >> (B * P));
 #pragma unroll
-    for (int i = S - 1; i >= S - 4; --i) {
-        const int di = ((lo + 32) & 63) - 32;
+    for (int i = S - 1; i >= S - P; --i) {
+        const int di = ((lo + H) & M) - H;
         d[i] = (float)di;
-        lo = (lo - di) >> 6;
+        lo = (lo - di) >> B;
     }
     hi += lo;
 #pragma unroll
-    for (int i = S - 5; i >= 1; --i) {
-        const int di = ((hi + 32) & 63) - 32;
+    for (int i = S - P - 1; i >= 1; --i) {
+        const int di = ((hi + H) & M) - H;
         d[i] = (float)di;
-        hi = (hi - di) >> 6;
+        hi = (hi - di) >> B;
     }
     d[0] = (float)hi;
 }
@@ -131,15 +132,12 @@ template<> __device__ __forceinline__ double scaled_ll_to<double>(long long v, i
     return scaled_ll_to_double(v, sc);
 }
 
-// value of the combined levels: sum_l C_l 2^(B (S-1-l)) as an exact int64
-// (every level is an integer below 2^24 in magnitude: 32-bit conversion)
-template<int S>
-__device__ __forceinline__ long long combine_levels(const float* c) {
-    long long acc = 0;
-#pragma unroll
-    for (int l = 0; l < S; ++l)
-        acc += ((long long)__float2int_rn(c[l])) << (kB * (S - 1 - l));
-    return acc;
+// a level's contribution to the combined value sum_l C_l 2^(B (S-1-l)), an
+// exact int64 (every level, or piece of one, is an integer up to 2^24 in
+// magnitude: 32-bit conversion)
+template<int B, int S>
+__device__ __forceinline__ long long level_term(const int l, const float c) {
+    return ((long long)__float2int_rn(c)) << (B * (S - 1 - l));
 }
 
 }  // namespace wb

@@ -2,9 +2,9 @@
 // hand-written: TMA tile loads, tcgen05 MMAs into TMEM, and the exact level
 // combination fused into the epilogue (no FP32 level array in HBM).
 //
-// The split is the one of ozaki.cu (S = 7 balanced 6-bit digits per
-// operand, per-point / per-column exponents): the product level l collects
-// sum_{i+j=l} A_i B_j over the AO index, every partial sum an integer below
+// The split is the one of ozaki.cu (S = 6 balanced digits of 7 bits, or 7 of
+// 6, per operand, per-point / per-column exponents): the product level l collects
+// sum_{i+j=l} A_i B_j over the AO index, every partial sum an integer up to
 // 2^24, so the FP32 accumulation is exact in any order and the result is
 // bitwise the one of the library-GEMM form.
 //
@@ -12,11 +12,11 @@
 // multiple of 8, and zero beyond nao):
 //   A (points x slices x kp):  A[g][i][l] = digit i of X(l, g)
 //   B (AOs x slices x kp):     B[mu][j][l] = digit j of QD(l, mu)
-// Output tile: 128 points x 64 AOs per CTA.  The seven level accumulators
-// live side by side in TMEM (7 x 64 of 512 columns).  For each 64-wide
-// block of the AO index the CTA loads the seven B slices (one buffer of
+// Output tile: 128 points x 64 AOs per CTA.  The S level accumulators
+// live side by side in TMEM (up to 7 x 64 of 512 columns).  For each 64-wide
+// block of the AO index the CTA loads the S B slices (one buffer of
 // two) and, one stage at a time, each A slice i; slice i meets B slices
-// j = 0 .. 6 - i, four K = 16 MMAs each.  Warp roles: lane 0 of warp 0
+// j = 0 .. S - 1 - i, four K = 16 MMAs each.  Warp roles: lane 0 of warp 0
 // issues the TMA loads, lane 0 of warp 1 the MMAs; all four warps then
 // read the accumulators (one TMEM lane per thread), combine the levels in
 // int64 and store F.
@@ -37,18 +37,20 @@ namespace wb {
 
 namespace {
 
-constexpr int S = kOzSlices;
 constexpr int kBM = 128;                 // points per tile
 constexpr int kBN = 64;                  // AOs per tile
 constexpr int kBK = 64;                  // AO index per block (128 B of bf16)
 constexpr int kAStages = 4;
 constexpr int kATile = kBM * kBK * 2;    // 16 KB
 constexpr int kBTile = kBN * kBK * 2;    // 8 KB
-constexpr int kBSet = S * kBTile;        // 56 KB: the seven B slices of a block
-constexpr int kSmemTiles = 2 * kBSet + kAStages * kATile;
-constexpr int kSmemBytes = kSmemTiles + 1024 /* align */ + 256 /* barriers */;
-constexpr uint32_t kTmemCols = 512;      // 7 levels x 64 columns
-static_assert(S * kBN <= (int)kTmemCols, "levels must fit in TMEM");
+// S slices: the B slices of a block (48 or 56 KB), the tiles, and the whole
+__host__ __device__ constexpr int b_set(int S) { return S * kBTile; }
+__host__ __device__ constexpr int smem_tiles(int S) { return 2 * b_set(S) + kAStages * kATile; }
+__host__ __device__ constexpr int smem_bytes(int S) {
+    return smem_tiles(S) + 1024 /* align */ + 256 /* barriers */;
+}
+constexpr uint32_t kTmemCols = 512;      // up to 7 levels x 64 columns
+static_assert(7 * kBN <= (int)kTmemCols, "levels must fit in TMEM");
 
 __host__ __device__ constexpr int pad8(int n) { return (n + 7) & ~7; }
 
@@ -56,6 +58,7 @@ __host__ __device__ constexpr int pad8(int n) { return (n + 7) & ~7; }
 
 // A: a block per (64 points, 64 AOs); X read along points, A written along
 // the AO index (bf16 pairs)
+template<int B_, int S>
 __global__ void __launch_bounds__(256)
 f_slice_x_km_kernel(const double* __restrict__ X, int nao, int64_t ld,
                     const int* __restrict__ erow, __nv_bfloat16* __restrict__ A) {
@@ -79,8 +82,8 @@ f_slice_x_km_kernel(const double* __restrict__ X, int nao, int64_t ld,
         if (g >= ld) break;
         const int e = erow[g];
         float d0[S], d1[S];
-        digits<S>(xs[2 * lp][gg], e, d0);
-        digits<S>(xs[2 * lp + 1][gg], e, d1);
+        digits<B_, S>(xs[2 * lp][gg], e, d0);
+        digits<B_, S>(xs[2 * lp + 1][gg], e, d1);
         __nv_bfloat16* row = A + g * (int64_t)S * kp;
 #pragma unroll
         for (int i = 0; i < S; ++i)
@@ -90,6 +93,7 @@ f_slice_x_km_kernel(const double* __restrict__ X, int nao, int64_t ld,
 }
 
 // B: a block per AO column mu of QD (its exponent from the column maximum)
+template<int B_, int S>
 __global__ void __launch_bounds__(256)
 f_slice_qd_km_kernel(const double* __restrict__ QD, int nao, int* __restrict__ ecol,
                      __nv_bfloat16* __restrict__ B) {
@@ -116,7 +120,7 @@ f_slice_qd_km_kernel(const double* __restrict__ QD, int nao, int* __restrict__ e
     for (int l = threadIdx.x; l < kp; l += blockDim.x) {
         float d[S];
         if (l < nao) {
-            digits<S>(QD[(int64_t)l * nao + mu], e, d);
+            digits<B_, S>(QD[(int64_t)l * nao + mu], e, d);
         } else {
 #pragma unroll
             for (int i = 0; i < S; ++i) d[i] = 0.0f;
@@ -139,14 +143,15 @@ struct FTcArgs {
     unsigned long long* status;   // bit 0: a wait gave up
 };
 
-template<typename T>
+template<int B_, int S, typename T>
 __global__ void __launch_bounds__(128, 1)
 ozaki_f_tc_kernel(const __grid_constant__ CUtensorMap mapA,
                   const __grid_constant__ CUtensorMap mapB, const FTcArgs<T> P) {
+    constexpr int kBSet = b_set(S), kSmemTiles = smem_tiles(S);
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = tc::smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
-    const uint32_t sB = base;                            // 2 x 7 B tiles
+    const uint32_t sB = base;                            // 2 x S B tiles
     const uint32_t sA = base + 2 * kBSet;                // 4 A stages
     uint8_t* bars_p = smem_raw + (base - raw) + kSmemTiles;
     uint64_t* bars = reinterpret_cast<uint64_t*>(bars_p);
@@ -185,7 +190,7 @@ ozaki_f_tc_kernel(const __grid_constant__ CUtensorMap mapA,
     // one's phase is what the clean-up waits for)
     int issuedA[kAStages] = {0, 0, 0, 0}, issuedB[2] = {0, 0};
     if (warp == 0 && lane == 0) {
-        // producer: per AO block the seven B slices, then A slice by slice
+        // producer: per AO block the S B slices, then A slice by slice
         int it = 0;
         for (int kb = 0; kb < nkb && !*abort_flag; ++kb) {
             const int bs = kb & 1;
@@ -262,14 +267,14 @@ ozaki_f_tc_kernel(const __grid_constant__ CUtensorMap mapA,
             tc::tmem_ld16(tl + (uint32_t)(l * kBN + 16 * c), v);
 #pragma unroll
             for (int q = 0; q < 16; ++q)
-                acc[q] += ((long long)__float2int_rn(v[q])) << (kB * (S - 1 - l));
+                acc[q] += level_term<B_, S>(l, v[q]);
         }
         if (g < P.ld) {
 #pragma unroll
             for (int q = 0; q < 16; ++q) {
                 const int mu = n0 + 16 * c + q;
                 if (mu < P.nao) {
-                    const int sc = er + P.ecol[mu] - 2 * kW + 2 + kB * (S - 1);
+                    const int sc = er + P.ecol[mu] - 2 * kW + 2 + B_ * (S - 1);
                     P.F[(int64_t)mu * P.ld + g] =
                         bad ? (T)__int_as_float(0x7fc00000) : scaled_ll_to<T>(acc[q], sc);
                 }
@@ -309,7 +314,8 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 // (rows x S slices x kp) bf16, K-major, box 64 (K) x 1 x box_rows, 128-byte
 // swizzle, zero fill beyond nao along K and beyond rows
-bool make_map(CUtensorMap* m, const void* base, int nao, int64_t rows, int box_rows) {
+bool make_map(CUtensorMap* m, const void* base, int S, int nao, int64_t rows,
+              int box_rows) {
     auto fn = encode_fn();
     if (!fn) return false;
     const int kp = pad8(nao);
@@ -328,14 +334,14 @@ inline size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
 }  // namespace
 
 size_t ozaki_f_tc_bytes(int nao, int64_t ld) {
-    const size_t kp = (size_t)pad8(nao);
+    const size_t kp = (size_t)pad8(nao), S = ozaki_f_seven_bit(nao) ? 6 : 7;
     return al(sizeof(int) * ld) + al(sizeof(int) * nao) +
            al(sizeof(__nv_bfloat16) * (size_t)ld * S * kp) +
            al(sizeof(__nv_bfloat16) * (size_t)nao * S * kp) +
            al(sizeof(unsigned long long));
 }
 
-template<typename T>
+template<int B_, int S, typename T>
 static int f_gemm_tc_t(const double* X, const double* QD, int nao, int64_t ld, T* F,
                        void* ws, cudaStream_t s, unsigned long long* status) {
     if (!ozaki_f_supported(nao) || ld % 2 != 0 || ld > (int64_t)kBM * 65535)
@@ -351,32 +357,38 @@ static int f_gemm_tc_t(const double* X, const double* QD, int nao, int64_t ld, T
     if (!status) status = reinterpret_cast<unsigned long long*>(p);
 
     CUtensorMap mapA, mapB;
-    if (!make_map(&mapA, A, nao, ld, kBM) || !make_map(&mapB, B, nao, nao, kBN))
+    if (!make_map(&mapA, A, S, nao, ld, kBM) || !make_map(&mapB, B, S, nao, nao, kBN))
         return (int)cudaErrorNotSupported;
-    cudaError_t e = cudaFuncSetAttribute(ozaki_f_tc_kernel<T>,
+    auto kernel = ozaki_f_tc_kernel<B_, S, T>;
+    constexpr int kSmemBytes = smem_bytes(S);
+    cudaError_t e = cudaFuncSetAttribute(kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     f_rowmax(X, nao, ld, erow, s);
     {
         dim3 grid((unsigned)((ld + 63) / 64), (unsigned)((kp + 63) / 64));
-        f_slice_x_km_kernel<<<grid, 256, 0, s>>>(X, nao, ld, erow, A);
+        f_slice_x_km_kernel<B_, S><<<grid, 256, 0, s>>>(X, nao, ld, erow, A);
     }
-    f_slice_qd_km_kernel<<<nao, 256, 0, s>>>(QD, nao, ecol, B);
+    f_slice_qd_km_kernel<B_, S><<<nao, 256, 0, s>>>(QD, nao, ecol, B);
     FTcArgs<T> a{erow, ecol, F, nao, ld, (nao + kBK - 1) / kBK, status};
     dim3 grid((unsigned)((nao + kBN - 1) / kBN), (unsigned)((ld + kBM - 1) / kBM));
-    ozaki_f_tc_kernel<T><<<grid, 128, kSmemBytes, s>>>(mapA, mapB, a);
+    kernel<<<grid, 128, kSmemBytes, s>>>(mapA, mapB, a);
     return (int)cudaGetLastError();
 }
 
 int ozaki_f_gemm_tc(const double* X, const double* QD, int nao, int64_t ld, float* F,
                     void* ws, cudaStream_t s, unsigned long long* status) {
-    return f_gemm_tc_t<float>(X, QD, nao, ld, F, ws, s, status);
+    return ozaki_f_seven_bit(nao)
+               ? f_gemm_tc_t<7, 6, float>(X, QD, nao, ld, F, ws, s, status)
+               : f_gemm_tc_t<6, 7, float>(X, QD, nao, ld, F, ws, s, status);
 }
 
 int ozaki_f_gemm_tc64(const double* X, const double* QD, int nao, int64_t ld, double* F,
                       void* ws, cudaStream_t s, unsigned long long* status) {
-    return f_gemm_tc_t<double>(X, QD, nao, ld, F, ws, s, status);
+    return ozaki_f_seven_bit(nao)
+               ? f_gemm_tc_t<7, 6, double>(X, QD, nao, ld, F, ws, s, status)
+               : f_gemm_tc_t<6, 7, double>(X, QD, nao, ld, F, ws, s, status);
 }
 
 }  // namespace wb
