@@ -360,12 +360,12 @@ __global__ void gsum_kernel(const float* __restrict__ gc,
 }
 
 // the same over two buffer sets (the two halves of split blocks): the
-// first set's rows, then the second's, in fixed order
-__global__ void gsum2_kernel(const float* __restrict__ gc0,
-                             const float* __restrict__ gc1,
-                             const int4* __restrict__ src, int64_t ld,
-                             float* __restrict__ G) {
+// first set's rows, then the second's, in fixed order; gridDim.z omegas
+__global__ void gsum2_kernel(const __grid_constant__ GSum2 S, const int4* __restrict__ src, int64_t ld) {
     const int mu = blockIdx.y;
+    const float* __restrict__ gc0 = S.gc0[blockIdx.z];
+    const float* __restrict__ gc1 = S.gc1[blockIdx.z];
+    float* __restrict__ G = S.G[blockIdx.z];
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i >= ld) return;
     const int4 sr = src[mu];
@@ -601,11 +601,12 @@ cudaError_t launch_gsum(const float* gc, const int4* src, int nao, int64_t ld,
     return cudaGetLastError();
 }
 
-cudaError_t launch_gsum2(const float* gc0, const float* gc1, const int4* src, int nao,
-                         int64_t ld, float* G, cudaStream_t s) {
+cudaError_t launch_gsum2(const GSum2& g, int nom, const int4* src, int nao, int64_t ld,
+                         cudaStream_t s) {
+    if (nao <= 0 || ld <= 0) return cudaSuccess;
     const int64_t quads = ld / 4;
-    dim3 grid((unsigned)((quads + 255) / 256), (unsigned)nao);
-    gsum2_kernel<<<grid, 256, 0, s>>>(gc0, gc1, src, ld, G);
+    dim3 grid((unsigned)((quads + 255) / 256), (unsigned)nao, (unsigned)nom);
+    gsum2_kernel<<<grid, 256, 0, s>>>(g, src, ld);
     return cudaGetLastError();
 }
 

@@ -542,8 +542,8 @@ int run_g_classes(wb_cosx* h, int64_t npts_t, int64_t ldt, const float* F,
         if (st != WB_OK) return st;
     }
 #if WB_COSX_SPLIT
-    WB_CUDA(wb::launch_gsum2(at<float>(ws, L.gcls), at<float>(ws, L.gclsH), h->gsrc,
-                             h->hp.nao, ldt, G, s));
+    const wb::GSum2 gs = {{at<float>(ws, L.gcls)}, {at<float>(ws, L.gclsH)}, {G}};
+    WB_CUDA(wb::launch_gsum2(gs, 1, h->gsrc, h->hp.nao, ldt, s));
 #else
     WB_CUDA(wb::launch_gsum(at<float>(ws, L.gcls), h->gsrc, h->hp.nao, ldt, G, s));
 #endif
@@ -614,15 +614,16 @@ int run_g_classes_dual(wb_cosx* h, int64_t npts_t, int64_t ldt, const float* F,
         if (st != WB_OK) return st;
     }
 #if WB_COSX_SPLIT
-    WB_CUDA(wb::launch_gsum2(at<float>(ws, L.gcls), at<float>(ws, L.gclsH), h->gsrc,
-                             h->hp.nao, ldt, Ga, s));
-    WB_CUDA(wb::launch_gsum2(at<float>(ws, L.gcls2), at<float>(ws, L.gcls2H), h->gsrc,
-                             h->hp.nao, ldt, Gb, s));
+    const wb::GSum2 gs = {{at<float>(ws, L.gcls), at<float>(ws, L.gcls2)},
+                          {at<float>(ws, L.gclsH), at<float>(ws, L.gcls2H)},
+                          {Ga, Gb}};
+    WB_CUDA(wb::launch_gsum2(gs, 2, h->gsrc, h->hp.nao, ldt, s));
+    *launches += 1;
 #else
     WB_CUDA(wb::launch_gsum(at<float>(ws, L.gcls), h->gsrc, h->hp.nao, ldt, Ga, s));
     WB_CUDA(wb::launch_gsum(at<float>(ws, L.gcls2), h->gsrc, h->hp.nao, ldt, Gb, s));
-#endif
     *launches += 2;
+#endif
     return WB_OK;
 }
 
@@ -1309,6 +1310,28 @@ int wb_cosx_get_k_multi(wb_cosx* h, const double* coords,
     };
     if (prof) WB_CUDA(cudaEventRecord(ev[0], s));
     int st = WB_OK;
+    // With one pair of omegas (or one omega) the per-omega records serve every
+    // tile.  They depend on nothing that comes before the class kernels, so
+    // they are formed on a class stream beside the AO values and F (five
+    // small kernels, 40 us of the 420 us build of two waters).
+    const bool ahead = nomega == 1 || (nomega == 2 && h->dual_ok);
+    if (ahead) {
+        const cudaStream_t side = h->cstream[0];
+        WB_CUDA(cudaEventRecord(h->fork, s));
+        WB_CUDA(cudaStreamWaitEvent(side, h->fork, 0));
+        if (nomega == 1)
+            st = prepare_omega(h, omegas[0], workspace, L, side);
+        else
+            st = prepare_omega_dual(h, std::min(omegas[0], omegas[1]),
+                                    std::max(omegas[0], omegas[1]), workspace, L, side);
+        // joined in any case: nothing may be left running on the workspace
+        WB_CUDA(cudaEventRecord(h->cdone[0], side));
+        if (st != WB_OK) {
+            WB_CUDA(cudaStreamWaitEvent(s, h->cdone[0], 0));
+            return st;
+        }
+        launches += nomega + 1;
+    }
     for (int64_t i0 = 0; i0 < npts; i0 += tile) {
         const int64_t nt = std::min(tile, npts - i0);
         const int64_t ldt = round32(nt);
@@ -1338,6 +1361,7 @@ int wb_cosx_get_k_multi(wb_cosx* h, const double* coords,
         if ((st = phase_to(3)) != WB_OK) return st;
         if ((st = tile_prep(h, c, w, nt, ldt, F32, workspace, L, s, &launches)) != WB_OK)
             return st;
+        if (ahead && i0 == 0) WB_CUDA(cudaStreamWaitEvent(s, h->cdone[0], 0));
         // K += X^T (w o G) of omega j from the G in Gsrc; the X slices of
         // this tile serve every omega after the first
         bool x_sliced = false;
@@ -1372,10 +1396,12 @@ int wb_cosx_get_k_multi(wb_cosx* h, const double* coords,
                 // all-far-first branch order) takes the smaller omega
                 int ja = j, jb = j + 1;
                 if (omegas[jb] < omegas[ja]) std::swap(ja, jb);
-                if ((st = prepare_omega_dual(h, omegas[ja], omegas[jb], workspace, L,
-                                             s)) != WB_OK)
-                    return st;
-                launches += 3;
+                if (!ahead) {
+                    if ((st = prepare_omega_dual(h, omegas[ja], omegas[jb], workspace, L,
+                                                 s)) != WB_OK)
+                        return st;
+                    launches += 3;
+                }
                 if ((st = run_g_classes_dual(h, nt, ldt, F32, G32, G32b, omegas[ja],
                                              omegas[jb], tile_tol, workspace, L, s,
                                              &launches)) != WB_OK)
@@ -1401,8 +1427,10 @@ int wb_cosx_get_k_multi(wb_cosx* h, const double* coords,
                 j += 2;
                 continue;
             }
-            if ((st = prepare_omega(h, omegas[j], workspace, L, s)) != WB_OK) return st;
-            launches += 2;
+            if (!ahead) {
+                if ((st = prepare_omega(h, omegas[j], workspace, L, s)) != WB_OK) return st;
+                launches += 2;
+            }
             if ((st = run_g_classes(h, nt, ldt, F32, G32, omegas[j], tile_tol,
                                     workspace, L, s, &launches)) != WB_OK)
                 return st;
@@ -1891,14 +1919,19 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
         double* Ks[2] = {k_out[m] + kk * b->kidx[0], k_out[m] + kk * b->kidx[1]};
 #if WB_COSX_SPLIT
         const size_t gclH[2] = {L.gclsH, L.gcls2H};
-        for (int w = 0; w < b->nom; ++w)
-            WB_CUDA(wb::launch_gsum2(at<float>(ws, gcl[w]), at<float>(ws, gclH[w]),
-                                     h->gsrc, nao, ld, Gs[w], s));
+        wb::GSum2 gs = {};
+        for (int w = 0; w < b->nom; ++w) {
+            gs.gc0[w] = at<float>(ws, gcl[w]);
+            gs.gc1[w] = at<float>(ws, gclH[w]);
+            gs.G[w] = Gs[w];
+        }
+        WB_CUDA(wb::launch_gsum2(gs, b->nom, h->gsrc, nao, ld, s));
+        launches += 1;
 #else
         for (int w = 0; w < b->nom; ++w)
             WB_CUDA(wb::launch_gsum(at<float>(ws, gcl[w]), h->gsrc, nao, ld, Gs[w], s));
-#endif
         launches += b->nom;
+#endif
         if (b->gemm == WB_K_GEMM_OZAKI_BF16) {
             const float* Gc[2] = {Gs[0], Gs[1]};
             const int r = wb::ozaki_k_gemm_multi(h->cublas, X, Gc, b->nom, b->weights[m],
