@@ -167,8 +167,8 @@ __device__ __forceinline__ void vv_block_count(unsigned long long v,
 
 // The pairs of one outer point with one staged inner tile (m points), the
 // one-reciprocal form: inv = 1/(g gp gt) from rcp.approx and one Newton
-// step, T = q inv and, with 1/g + 1/gt = (g + gt) gp inv, Tu = T (g + gt)
-// gp inv.  Plain FP32 sums over 16 pairs, merged into Kahan-compensated
+// step, T = q inv and, with 1/g + 1/gt = (g + gt) gp inv, Tu = T (g gp + gt
+// gp) inv.  Plain FP32 sums over 16 pairs, merged into Kahan-compensated
 // tile sums once per 16 pairs; the tile sums join the FP64 totals.  Shared
 // by the single-molecule and the batched kernels (same arithmetic, same
 // order).
@@ -184,12 +184,13 @@ __device__ __forceinline__ void vv10_tile_fast(const VvOuter& o, const float4* s
         const float g = fmaf(r2, o.w0, o.k);
         const float gp = fmaf(r2, kj.x, kj.y);
         const float gt = g + gp;
-        const float pr = g * gp * gt;
+        const float h = g * gp;
+        const float pr = h * gt;
         float inv;
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(pr));
         if (WB_VV10_NEWTON) inv = fmaf(inv, fmaf(-pr, inv, 1.0f), inv);
         const float T = pj.w * inv;
-        const float Tu = T * ((g + gt) * gp * inv);
+        const float Tu = T * (fmaf(gt, gp, h) * inv);
         pf += T;
         pu += Tu;
         pw = fmaf(Tu, r2, pw);
