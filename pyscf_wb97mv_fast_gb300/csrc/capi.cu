@@ -2110,6 +2110,7 @@ int wb_cosx_k_grad(wb_cosx* h, const double* coords, const double* weights,
     wb::GradEArgs ge;
     ge.npairs = h->hp.npairs; ge.pclass = h->pclass; ge.hdr = h->hdr; ge.pshell = h->pshell;
     ge.p = h->p; ge.alpha = h->f64_alpha; ge.vs_xyz = h->f64_vsxyz; ge.dE = dE;
+    ge.rec = rec;
     for (int c = 0; c < wb::NCLASS; ++c) {
         g.pp_begin[c] = ge.pp_begin[c] = h->hp.cls[c].pp_begin;
         g.e_base[c] = ge.e_base[c] = h->f64_ebase[c];

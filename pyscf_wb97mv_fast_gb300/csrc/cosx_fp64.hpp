@@ -13,7 +13,8 @@ constexpr int kBoysTaylor = 12;     // terms of the 1/4-node series
 constexpr int kBoysFineNodes = 1153;    // T_k = k / 32, k = 0..1152
 constexpr int kBoysFineCols = 14;       // F_m(T_k), m = 0..13 (orders to 7)
 // doubles of a primitive pair's record: P (3), p theta, then c_n = prefactor
-// sqrt(theta) (-2 p theta)^n (n <= 7) and the bra exponent over p
+// sqrt(theta) (-2 p theta)^n (n <= 7), the bra exponent over p and, in the
+// gradient, -2 mu Q (3)
 constexpr int kF64Rec = 16;
 
 struct CosxF64Args {

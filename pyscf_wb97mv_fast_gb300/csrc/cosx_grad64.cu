@@ -20,12 +20,14 @@
 //
 // With P = (alpha A + beta B) / p and Q = A - B, d/dA = (alpha / p) d/dP +
 // d/dQ and d/dB = (beta / p) d/dP - d/dQ; d/dP_x raises the Hermite index,
-// R_tuv -> R_t+1,u,v, and d/dQ acts on the Hermite coefficients alone
-// (prefactor included): tables formed once per call (grad_e_kernel).  So one
-// pass over the primitive pair gives both centres:
+// R_tuv -> R_t+1,u,v, and d/dQ acts on the Hermite coefficients (tables formed
+// once per call, grad_e_kernel) and on the prefactor exp(-mu Q^2).  So one pass
+// over the primitive pair gives both centres:
 //   S_x = sum_ab f_a f_b sum E^x_t E^y_u E^z_v R_t+1,u,v
-//   D_x = sum_ab f_a f_b sum (dE^x_t / dQ) E^y_u E^z_v R_tuv
+//   e   = sum_ab f_a f_b sum E^x_t E^y_u E^z_v R_tuv
+//   D_x = sum_ab f_a f_b sum (dE^x_t / dQ_x) E^y_u E^z_v R_tuv - 2 mu Q_x e
 //   dA = (alpha / p) S + D,  dB = S - dA
+// (dE^{ij}_t / dQ is zero for t >= i + j, so the three sums of D are short.)
 // (differentiating the Gaussians themselves needs integrals of l + 1 and
 // l - 1 for each of the three axes and each component).
 //
@@ -37,7 +39,7 @@
 // reduction in the task would cost 30 FP64 instructions.  The columns are
 // weighted with -w_g / 2 and summed in a fixed order at the end, so the
 // result is bitwise reproducible.  Measured (integral side alone): 8 waters,
-// 36,369 points 327 -> 47 ms; C4H10 in TZVP, 21,512 points 606 -> 69 ms.
+// 36,369 points 327 -> 40 ms; C4H10 in TZVP, 21,512 points 606 -> 60 ms.
 #include "cosx_fp64.cuh"
 #include "cosx_grad64.hpp"
 
@@ -46,10 +48,9 @@ namespace {
 
 using namespace f64;
 
-// d/dQ of every Hermite coefficient (with the pair prefactor exp(-mu Q^2)
-// differentiated too): dE = (d/dQ - 2 mu Q) E, in the layout of E.  One
-// thread per (shell pair, axis); E by its recurrence and its derivative
-// along.
+// d/dQ of every Hermite coefficient, in the layout of E, and -2 mu Q into the
+// records.  One thread per (shell pair, axis); E by its recurrence and its
+// derivative along.
 __global__ void grad_e_kernel(const GradEArgs A) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= A.npairs) return;
@@ -65,7 +66,8 @@ __global__ void grad_e_kernel(const GradEArgs A) {
     double E[4][4][8], D[4][4][8];
     for (int q = h.z; q < h.z + (h.w & 0xffff); ++q) {
         const double p = A.p[q], al = A.alpha[q], be = p - al;
-        const double hp = 0.5 / p, ka = -be / p, kb = al / p, m2 = -2.0 * al * be / p * Q;
+        const double hp = 0.5 / p, ka = -be / p, kb = al / p;
+        A.rec[(int64_t)q * kF64Rec + 13 + x] = -2.0 * al * be / p * Q;
         for (int i = 0; i <= la; ++i)
             for (int j = 0; j <= lb; ++j)
                 for (int t = 0; t <= i + j; ++t) {
@@ -97,21 +99,23 @@ __global__ void grad_e_kernel(const GradEArgs A) {
         for (int i = 0; i <= la; ++i)
             for (int j = 0; j <= lb; ++j)
                 for (int t = 0; t <= i + j; ++t)
-                    out[n++] = fma(m2, E[i][j][t], D[i][j][t]);
+                    out[n++] = D[i][j][t];
     }
 }
 
 // S (assigned) and D (added) of one primitive pair, for f_a f_b over the
-// Cartesian components; R packed for order L + 1.  Per (i, i'): R contracted
-// with E^x, dE^x and E^x at t + 1; f_a f_b spread over (u, v) with E^y E^z
-// and their derivatives; then the two sides meet.
+// Cartesian components; m2 = -2 mu Q; R packed for order L + 1.  Per (i, i'): R
+// contracted with E^x, dE^x and E^x at t + 1; f_a f_b spread over (u, v) with
+// E^y E^z and their derivatives; then the two sides meet.
 template<int LA, int LB>
 __device__ __forceinline__ void grad_block(const double* __restrict__ E,
                                            const double* __restrict__ dE,
+                                           const double* __restrict__ m2,
                                            const double* R, const double* fa,
                                            const double* fb, double* S, double* D) {
     constexpr int L = LA + LB, NAX = eaxis(LA, LB);
     constexpr int NUV = (L + 1) * (L + 2) / 2, NUV1 = (L + 2) * (L + 3) / 2;
+    double en = 0.0;
     S[0] = S[1] = S[2] = 0.0;
 #pragma unroll
     for (int i = 0; i <= LA; ++i)
@@ -139,20 +143,29 @@ __device__ __forceinline__ void grad_block(const double* __restrict__ E,
                         for (int v = 0; v <= L; ++v)
                             if (v <= k + kp) {
                                 const double zv = k + kp == 0 ? f : ez[v] * f;
-                                const double zd = dz[v] * f;
+                                const double zd = v < k + kp ? dz[v] * f : 0.0;
 #pragma unroll
                                 for (int u = 0; u <= L; ++u)
                                     if (u <= j + jp) {
                                         const int n = u * (2 * M + 3 - u) / 2 + v;
-                                        if (j + jp == 0) {
+                                        if (j + jp == 0)
                                             h[n] = seth[n] ? h[n] + zv : zv;
-                                            hz[n] = sethz[n] ? hz[n] + zd : zd;
-                                        } else {
+                                        else
                                             h[n] = seth[n] ? fma(ey[u], zv, h[n]) : ey[u] * zv;
-                                            hz[n] = sethz[n] ? fma(ey[u], zd, hz[n]) : ey[u] * zd;
+                                        seth[n] = true;
+                                        if (v < k + kp) {
+                                            if (j + jp == 0)
+                                                hz[n] = sethz[n] ? hz[n] + zd : zd;
+                                            else
+                                                hz[n] = sethz[n] ? fma(ey[u], zd, hz[n])
+                                                                 : ey[u] * zd;
+                                            sethz[n] = true;
                                         }
-                                        hy[n] = sethy[n] ? fma(dy[u], zv, hy[n]) : dy[u] * zv;
-                                        seth[n] = sethy[n] = sethz[n] = true;
+                                        if (u < j + jp) {
+                                            hy[n] = sethy[n] ? fma(dy[u], zv, hy[n])
+                                                             : dy[u] * zv;
+                                            sethy[n] = true;
+                                        }
                                     }
                             }
                     }
@@ -177,26 +190,29 @@ __device__ __forceinline__ void grad_block(const double* __restrict__ E,
                 for (int v = 0; v <= L; ++v)
                     if (u + v <= M) {
                         const int n = u * (2 * M + 3 - u) / 2 + v;
-                        double rd = dx[0] * R[ridx(L + 1, 0, u, v)];
                         double rp = R[ridx(L + 1, 1, u, v)];
                         if (i + ip > 0) {
+                            double rd = dx[0] * R[ridx(L + 1, 0, u, v)];
                             rp *= ex[0];
 #pragma unroll
                             for (int t = 1; t <= L; ++t)
                                 if (t <= i + ip) {
-                                    rd = fma(dx[t], R[ridx(L + 1, t, u, v)], rd);
+                                    if (t < i + ip) rd = fma(dx[t], R[ridx(L + 1, t, u, v)], rd);
                                     rp = fma(ex[t], R[ridx(L + 1, t + 1, u, v)], rp);
                                 }
+                            D[0] = fma(rd, h[n], D[0]);
                         }
                         const double r = rx[u * (2 * M + 5 - u) / 2 + v];
                         S[0] = fma(rp, h[n], S[0]);
                         S[1] = fma(rx[(u + 1) * (2 * M + 4 - u) / 2 + v], h[n], S[1]);
                         S[2] = fma(rx[u * (2 * M + 5 - u) / 2 + v + 1], h[n], S[2]);
-                        D[0] = fma(rd, h[n], D[0]);
-                        D[1] = fma(r, hy[n], D[1]);
-                        D[2] = fma(r, hz[n], D[2]);
+                        en = fma(r, h[n], en);
+                        if (sethy[n]) D[1] = fma(r, hy[n], D[1]);
+                        if (sethz[n]) D[2] = fma(r, hz[n], D[2]);
                     }
         }
+#pragma unroll
+    for (int x = 0; x < 3; ++x) D[x] = fma(m2[x], en, D[x]);
 }
 
 // threads of a CTA (one an SM), as for the FP64 class kernels
@@ -285,7 +301,7 @@ cosx_grad64_kernel(const CosxGradArgs A, const int cls, const int pair_begin,
                     for (int n = 0; n <= L + 1; ++n) r0[n] *= rec[4 + n];
                     fill_r64<L + 1>(r0, X, Y, Z, R);
                     const long long e = A.e_base[cls] + (long long)(q - pp_begin) * 3 * NAX;
-                    grad_block<LA, LB>(A.E + e, A.dE + e, R, fa, fb, S, dA);
+                    grad_block<LA, LB>(A.E + e, A.dE + e, rec + 13, R, fa, fb, S, dA);
 #pragma unroll
                     for (int x = 0; x < 3; ++x) {
                         dA[x] = fma(rec[12], S[x], dA[x]);

@@ -51,6 +51,7 @@ struct GradEArgs {
     long long e_base[10];
     int pp_begin[10];
     double* dE;
+    double* rec;                // the records: -2 mu Q is added to each
 };
 cudaError_t launch_grad_e(const GradEArgs& a, cudaStream_t s);
 
