@@ -224,9 +224,12 @@ __device__ __forceinline__ void hermite_block(const double* __restrict__ E,
         }
 }
 
-// pairs of one of nseg ranges (whole screening chunks)
-__host__ __device__ constexpr int segment_pairs(int npairs, int nseg) {
-    return ((npairs + nseg - 1) / nseg + 31) / 32 * 32;
+// pairs of one of nseg ranges, in whole units of align pairs.  The classes of
+// d and f shells have few pairs and long tasks, so a range may be shorter than
+// a screening chunk of 32 (C4H10 in TZVP has 10 pairs of f shells: its
+// gradient 81.3 -> 74.4 ms against ranges of whole chunks).
+__host__ __device__ constexpr int segment_pairs(int npairs, int nseg, int align = 1) {
+    return ((npairs + nseg - 1) / nseg + align - 1) / align * align;
 }
 
 // threads of a CTA (one an SM): the light classes leave registers for

@@ -38,8 +38,8 @@
 // reductions in the L2, dA once per run of pairs with one bra shell; a lane
 // reduction in the task would cost 30 FP64 instructions.  The columns are
 // weighted with -w_g / 2 and summed in a fixed order at the end, so the
-// result is bitwise reproducible.  Measured (integral side alone): 8 waters,
-// 36,369 points 327 -> 40 ms; C4H10 in TZVP, 21,512 points 606 -> 60 ms.
+// result is bitwise reproducible.  Measured (whole call): 8 waters, 36,369
+// points 370 -> 58 ms; C4H10 in TZVP, 21,512 points 692 -> 74 ms.
 #include "cosx_fp64.cuh"
 #include "cosx_grad64.hpp"
 

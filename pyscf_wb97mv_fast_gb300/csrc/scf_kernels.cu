@@ -529,7 +529,8 @@ hartree_kernel(const HartreeArgs A, const int cls, const int pair_begin, const i
     unsigned long long kept = 0;
     const int nwarps = gridDim.x * (blockDim.x >> 5);
     const int nitem = A.nblk * A.nseg;
-    const int seg_pairs = f64::segment_pairs(pair_end - pair_begin, A.nseg);
+    // FP32 chunks of 32 pairs are summed as a whole
+    const int seg_pairs = f64::segment_pairs(pair_end - pair_begin, A.nseg, F64 ? 1 : 32);
     int item = (int)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
     while (item < nitem) {
         const int seg = item / A.nblk, blk = item - seg * A.nblk;
