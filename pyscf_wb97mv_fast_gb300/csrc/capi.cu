@@ -825,10 +825,18 @@ int64_t hartree_ndh(const wb::HostPairs& hp) {
 struct WsLayout64 {
     WsLayout base;                  // counters, work, block statistics
     size_t X = 0, F64 = 0, F32 = 0, G64 = 0, rec = 0, gemm = 0, total = 0;
+    size_t G64b = 0, rec2 = 0;      // of a second omega
     int nseg = 1;                   // copies of G (f64_segments)
 };
 
-WsLayout64 ws_layout_fp64(const wb_cosx* h, int64_t ld) {
+// Two omegas at a time need a second G.  A grid whose G is above 24 GiB keeps
+// one (four and a half arrays of that size and the GEMMs' scratch would no
+// longer leave room for a caller's own on a 280 GB device).
+bool fp64_two(const wb_cosx* h, int64_t ld) {
+    return (double)h->hp.nao * (double)ld * sizeof(double) <= 24.0 * 1073741824.0;
+}
+
+WsLayout64 ws_layout_fp64(const wb_cosx* h, int64_t ld, bool two) {
     WsLayout64 L;
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -851,8 +859,10 @@ WsLayout64 ws_layout_fp64(const wb_cosx* h, int64_t ld) {
     L.F32 = take(sizeof(float) * n);
     L.nseg = wb::f64_segments(ld / 32, h->nsm);
     L.G64 = take(sizeof(double) * n * L.nseg);
+    if (two) L.G64b = take(sizeof(double) * n * L.nseg);
     L.gemm = take(wb::gemm64_bytes(nao64, ld));
     L.rec = take(sizeof(double) * wb::kF64Rec * (size_t)std::max(h->hp.npp, 1));
+    if (two) L.rec2 = take(sizeof(double) * wb::kF64Rec * (size_t)std::max(h->hp.npp, 1));
     L.total = off;
     return L;
 }
@@ -1485,7 +1495,8 @@ int wb_cosx_get_class_variant(const wb_cosx* h, int cls, int* dual, int* staged)
 
 size_t wb_cosx_fp64_workspace_bytes(const wb_cosx* h, int64_t npts) {
     if (!h || npts < 0) return 0;
-    return ws_layout_fp64(h, round32(std::max<int64_t>(npts, 1))).total;
+    const int64_t ld = round32(std::max<int64_t>(npts, 1));
+    return ws_layout_fp64(h, ld, fp64_two(h, ld)).total;
 }
 
 int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
@@ -1504,7 +1515,8 @@ int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
     const int64_t ld = round32(std::max<int64_t>(npts, 1));
     if (ld > INT32_MAX - 64)
         return fail(WB_ERR_UNSUPPORTED, "wb_cosx_get_k_fp64: above 2^31 points");
-    const WsLayout64 L = ws_layout_fp64(h, ld);
+    const bool two = fp64_two(h, ld);
+    const WsLayout64 L = ws_layout_fp64(h, ld, two);
     if (!workspace || workspace_bytes < L.total)
         return fail(WB_ERR_WORKSPACE, "wb_cosx_get_k_fp64: workspace needs " +
                                           std::to_string(L.total) + " bytes");
@@ -1572,26 +1584,44 @@ int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
     a.pnint = h->pnint;
     a.counters = at<unsigned long long>(workspace, L.base.counters);
     a.work = at<int>(workspace, L.base.work);
+    double* G64s[2] = {G64, at<double>(workspace, L.G64b)};
+    double* recs[2] = {rec, at<double>(workspace, L.rec2)};
     int64_t ntasks = 0;
-    for (int j = 0; j < nomega; ++j) {
-        WB_CUDA(wb::launch_f64_records(h->hp.npp, h->f64_P, h->p, h->pref, h->f64_alpha,
-                                       omegas[j], rec, s));
-        WB_CUDA(cudaMemsetAsync(G64, 0, sizeof(double) * (size_t)nao * ld * L.nseg, s));
-        WB_CUDA(cudaMemsetAsync(a.work, 0, sizeof(int) * wb::NCLASS, s));
-        launches += 3;
-        for (int c = 0; c < wb::NCLASS; ++c) {
-            const int pb = h->hp.cls[c].pair_begin, pe = h->hp.cls[c].pair_end;
-            if (pe <= pb) continue;
-            WB_CUDA(wb::launch_cosx_fp64_class(c, a, pb, pe, h->nsm, s));
-            ++launches;
+    for (int j = 0; j < nomega; j += two ? 2 : 1) {
+        // two omegas at a time: the light classes in one pass, the others one
+        // omega after the other
+        const int nw = two ? std::min(2, nomega - j) : 1;
+        for (int w = 0; w < nw; ++w) {
+            WB_CUDA(wb::launch_f64_records(h->hp.npp, h->f64_P, h->p, h->pref, h->f64_alpha,
+                                           omegas[j + w], recs[w], s));
+            WB_CUDA(cudaMemsetAsync(G64s[w], 0, sizeof(double) * (size_t)nao * ld * L.nseg, s));
+            launches += 2;
         }
-        ntasks += (ld / 32) * (int64_t)h->hp.npairs;
-        WB_CUDA(wb::launch_f64_segment_sum(G64, (int64_t)nao * ld, L.nseg, s));
-        launches += L.nseg > 1;
-        if ((st = gemm64_k(h, X, G64, weights, ld, npts, 0, k_out + kk * j, gemm, s)) !=
-            WB_OK)
-            return st;
-        launches += wb::gemm64_k_launches(npts);
+        a.rec2 = recs[1];
+        a.G2 = G64s[1];
+        for (int w = 0; w < nw; ++w) {
+            a.rec = recs[w];
+            a.G = G64s[w];
+            WB_CUDA(cudaMemsetAsync(a.work, 0, sizeof(int) * wb::NCLASS, s));
+            ++launches;
+            for (int c = 0; c < wb::NCLASS; ++c) {
+                const int pb = h->hp.cls[c].pair_begin, pe = h->hp.cls[c].pair_end;
+                const bool dual = nw == 2 && wb::fp64_dual(c);
+                if (pe <= pb || (dual && w == 1)) continue;
+                WB_CUDA(dual ? wb::launch_cosx_fp64_dual(c, a, pb, pe, h->nsm, s)
+                             : wb::launch_cosx_fp64_class(c, a, pb, pe, h->nsm, s));
+                ++launches;
+            }
+            ntasks += (ld / 32) * (int64_t)h->hp.npairs;
+        }
+        for (int w = 0; w < nw; ++w) {
+            WB_CUDA(wb::launch_f64_segment_sum(G64s[w], (int64_t)nao * ld, L.nseg, s));
+            launches += L.nseg > 1;
+            if ((st = gemm64_k(h, X, G64s[w], weights, ld, npts, 0, k_out + kk * (j + w), gemm,
+                               s)) != WB_OK)
+                return st;
+            launches += wb::gemm64_k_launches(npts);
+        }
     }
     return read_stats(h, workspace, L.base, ntasks, s, stats, launches);
 }
@@ -1991,7 +2021,7 @@ struct GradLayout {
 
 GradLayout grad_layout(const wb_cosx* h, int64_t ld, int natm) {
     GradLayout L;
-    L.f64 = ws_layout_fp64(h, ld);
+    L.f64 = ws_layout_fp64(h, ld, false);
     int64_t ne = 0;
     for (int la = 0; la <= wb::LMAX; ++la)
         for (int lb = 0; lb <= la; ++lb) {

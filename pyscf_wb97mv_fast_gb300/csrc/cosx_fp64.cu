@@ -19,6 +19,17 @@ cudaError_t launch_cosx_fp64_class(int cls, const CosxF64Args& a, int pb, int pe
     }
 }
 
+cudaError_t launch_cosx_fp64_dual(int cls, const CosxF64Args& a, int pb, int pe, int nsm,
+                                  cudaStream_t s) {
+    switch (cls) {
+    case 0: return f64::run64<0, 0, 2>(a, cls, pb, pe, nsm, s);
+    case 1: return f64::run64<1, 0, 2>(a, cls, pb, pe, nsm, s);
+    case 2: return f64::run64<1, 1, 2>(a, cls, pb, pe, nsm, s);
+    case 3: return f64::run64<2, 0, 2>(a, cls, pb, pe, nsm, s);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
 namespace {
 
 // the lane-independent factors of a primitive pair, once per omega: in the

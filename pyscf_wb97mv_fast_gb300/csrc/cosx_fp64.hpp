@@ -20,6 +20,7 @@ constexpr int kF64Rec = 16;
 struct CosxF64Args {
     const double* F;            // (nao, ld) AO-major, FP64
     double* G;                  // nseg x (nao, ld) AO-major, FP64, accumulated
+    double* G2;                 // the second omega's, with two (launch_cosx_fp64_dual)
     long long gstride;          // nao ld
     int nseg;                   // ranges of a class's pairs (f64_segments)
     const double* coords;       // (npts, 3) molecule frame
@@ -40,6 +41,7 @@ struct CosxF64Args {
     // FP64 pair data: per primitive pair the record of this omega
     // (f64_records); per class the Hermite E block from e_base[c]
     const double* rec;
+    const double* rec2;         // the second omega's
     const double* E;
     long long e_base[10];
     const double* boys;         // the tables of fp64_boys.cuh
@@ -65,6 +67,10 @@ inline int f64_segments(int64_t nblk, int nsm) {
 }
 // G[0] += the other nseg - 1 ranges, in order; n elements each
 cudaError_t launch_f64_segment_sum(double* G, int64_t n, int nseg, cudaStream_t s);
+// one class launch for two omegas (classes with fp64_dual)
+inline bool fp64_dual(int cls) { return cls <= 3; }        // la + lb <= 2
+cudaError_t launch_cosx_fp64_dual(int cls, const CosxF64Args& a, int pb, int pe, int nsm,
+                                  cudaStream_t s);
 // one class launch (classes 0..9); the f classes live in cosx_fp64_f.cu
 cudaError_t launch_cosx_fp64_class(int cls, const CosxF64Args& a, int pb, int pe,
                                    int nsm, cudaStream_t s);
