@@ -368,6 +368,24 @@ int wb_gga_rho(wb_cosx* h, const double* x, const void* t, int t32, int64_t npts
 int wb_gga_aow(wb_cosx* h, const double* x, const double* v, int64_t npts,
                int64_t ld, int g32, void* g_out, void* stream);
 
+/* The pointwise parts of VV10 (gpu/vv10.py:243-265, :300-314) at the nk points
+ * idx (their indices, int64) of a grid with density rho (4, ld) FP64
+ * (wb_gga_rho); kvv = 3/2 pi b (9 pi)^(-1/6), beta = (3 / b^2)^(3/4) / 32 and c
+ * of the parameters b, C:
+ *   wb_vv10_points: the double sum's inputs, FP32: coordinates (nk, 3) from
+ *     coords (npts, 3) FP64, q = rho w, W0 and kappa;
+ *   wb_vv10_potential: from its sums F, U, W (nk,) FP64 and weight fac, adds
+ *     the energy density per electron to exc (npts,) and the derivatives to
+ *     v (4, ld): half of d/d rho, and d/d grad. */
+int wb_vv10_points(const double* rho, int64_t ld, const double* coords,
+                   const double* weights, const int64_t* idx, int64_t nk,
+                   double kvv, double c, float* xyz, float* q, float* w0,
+                   float* kappa, void* stream);
+int wb_vv10_potential(const double* rho, int64_t ld, const int64_t* idx, int64_t nk,
+                      double kvv, double c, double beta, double fac,
+                      const double* f, const double* u, const double* w,
+                      double* exc, double* v, void* stream);
+
 /* Engine of the F product (process-wide, every F of the K builds and of
  * wb_cosx_ozaki_f / _f64): WB_OZAKI_ENGINE_LIBRARY (the default) runs one
  * cuBLAS bf16 GEMM per level; WB_OZAKI_ENGINE_TC is this library's

@@ -2516,6 +2516,29 @@ int wb_gga_aow(wb_cosx* h, const double* x, const double* v, int64_t npts, int64
     return WB_OK;
 }
 
+int wb_vv10_points(const double* rho, int64_t ld, const double* coords,
+                   const double* weights, const int64_t* idx, int64_t nk, double kvv,
+                   double c, float* xyz, float* q, float* w0, float* kappa,
+                   void* stream) {
+    if (nk < 0 || ld < 0 || (nk && (!rho || !coords || !weights || !idx || !xyz || !q ||
+                                    !w0 || !kappa)))
+        return fail(WB_ERR_INVALID_ARGUMENT, "wb_vv10_points: bad arguments");
+    WB_CUDA(wb::launch_vv10_points(rho, ld, coords, weights, idx, nk, kvv, c, xyz, q, w0,
+                                   kappa, static_cast<cudaStream_t>(stream)));
+    return WB_OK;
+}
+
+int wb_vv10_potential(const double* rho, int64_t ld, const int64_t* idx, int64_t nk,
+                      double kvv, double c, double beta, double fac, const double* f,
+                      const double* u, const double* w, double* exc, double* v,
+                      void* stream) {
+    if (nk < 0 || ld < 0 || (nk && (!rho || !idx || !f || !u || !w || !exc || !v)))
+        return fail(WB_ERR_INVALID_ARGUMENT, "wb_vv10_potential: bad arguments");
+    WB_CUDA(wb::launch_vv10_potential(rho, ld, idx, nk, kvv, c, beta, fac, f, u, w, exc, v,
+                                      static_cast<cudaStream_t>(stream)));
+    return WB_OK;
+}
+
 int wb_ozaki_set_f_engine(int engine) {
     if (engine != WB_OZAKI_ENGINE_LIBRARY && engine != WB_OZAKI_ENGINE_TC)
         return fail(WB_ERR_INVALID_ARGUMENT, "wb_ozaki_set_f_engine: unknown engine");

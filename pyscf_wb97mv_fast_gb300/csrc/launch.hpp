@@ -126,6 +126,14 @@ cudaError_t launch_block_order(const BlockOrderArgs& P, cudaStream_t s);
 // semilocal XC: density parameters (5, ld) FP64 and the Fock-side planes
 cudaError_t launch_xc_rho(const double* X, const float* T, int nao, int64_t ld,
                           int64_t npts, int mgga, double* rho, cudaStream_t s);
+cudaError_t launch_vv10_points(const double* rho, int64_t ld, const double* coords,
+                               const double* weights, const int64_t* idx, int64_t nk,
+                               double kvv, double c, float* xyz, float* q, float* w0,
+                               float* kap, cudaStream_t s);
+cudaError_t launch_vv10_potential(const double* rho, int64_t ld, const int64_t* idx,
+                                  int64_t nk, double kvv, double c, double beta, double fac,
+                                  const double* F, const double* U, const double* W,
+                                  double* exc, double* v, cudaStream_t s);
 cudaError_t launch_gga_rho(const double* X, const void* t, bool t32, int nao, int64_t ld,
                            int64_t npts, double* rho, cudaStream_t s);
 cudaError_t launch_gga_aow(const double* X, const double* v, int nao, int64_t ld,

@@ -530,6 +530,84 @@ size_t vv10_tile_stats_bytes(int64_t ntiles) {
     return (size_t)ntiles * sizeof(VvTileStats);
 }
 
+// -- pointwise parts (gpu/vv10.py:243-265, :300-314) -------------------------
+// One thread per point of the thresholded set, FP64.  As one kernel before and
+// one after the double sum: as elementwise array operations they were some
+// fifty launches of a few us each: the whole flow on 8 waters (70,478 points)
+// 7.17 -> 6.64 ms.
+struct VvTerms { double R, G, w2, W0, kappa; };
+
+__device__ __forceinline__ VvTerms vv_terms(const double* __restrict__ rho, const int64_t ld,
+                                            const int64_t i, const double kvv, const double c) {
+    VvTerms t;
+    t.R = rho[i];
+    const double gx = rho[ld + i], gy = rho[2 * ld + i], gz = rho[3 * ld + i];
+    t.G = gx * gx + gy * gy + gz * gz;
+    const double s = t.G / (t.R * t.R);
+    t.w2 = c * (s * s);
+    t.W0 = sqrt(t.w2 + (4.0 * M_PI / 3.0) * t.R);
+    t.kappa = kvv * pow(t.R, 1.0 / 6.0);
+    return t;
+}
+
+__global__ void vv10_points_kernel(const double* __restrict__ rho, int64_t ld,
+                                   const double* __restrict__ coords,
+                                   const double* __restrict__ weights,
+                                   const int64_t* __restrict__ idx, int64_t nk, double kvv,
+                                   double c, float* __restrict__ xyz, float* __restrict__ q,
+                                   float* __restrict__ w0, float* __restrict__ kap) {
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nk) return;
+    const int64_t i = idx[k];
+    const VvTerms t = vv_terms(rho, ld, i, kvv, c);
+#pragma unroll
+    for (int x = 0; x < 3; ++x) xyz[3 * k + x] = __double2float_rn(coords[3 * i + x]);
+    q[k] = __double2float_rn(t.R * weights[i]);
+    w0[k] = __double2float_rn(t.W0);
+    kap[k] = __double2float_rn(t.kappa);
+}
+
+cudaError_t launch_vv10_points(const double* rho, int64_t ld, const double* coords,
+                               const double* weights, const int64_t* idx, int64_t nk,
+                               double kvv, double c, float* xyz, float* q, float* w0,
+                               float* kap, cudaStream_t s) {
+    if (nk <= 0) return cudaSuccess;
+    vv10_points_kernel<<<(unsigned)((nk + 127) / 128), 128, 0, s>>>(
+        rho, ld, coords, weights, idx, nk, kvv, c, xyz, q, w0, kap);
+    return cudaGetLastError();
+}
+
+__global__ void vv10_potential_kernel(const double* __restrict__ rho, int64_t ld,
+                                      const int64_t* __restrict__ idx, int64_t nk, double kvv,
+                                      double c, double beta, double fac, const double* __restrict__ F,
+                                      const double* __restrict__ U,
+                                      const double* __restrict__ W, double* __restrict__ exc,
+                                      double* __restrict__ v) {
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nk) return;
+    const int64_t i = idx[k];
+    const VvTerms t = vv_terms(rho, ld, i, kvv, c);
+    // R dW0/dR, R dW0/dG and R d kappa/dR
+    const double dwr = (2.0 * M_PI / 3.0 * t.R - 2.0 * t.w2) / t.W0;
+    const double dwg = t.w2 * t.R / (t.G * t.W0);
+    const double f = F[k], u = U[k], w = W[k];
+    exc[i] += fac * (beta + 0.5 * f);
+    v[i] += 0.5 * fac * (beta + f + 1.5 * (u * (t.kappa / 6.0) + w * dwr));
+    const double h = 3.0 * fac * w * dwg;
+#pragma unroll
+    for (int x = 1; x < 4; ++x) v[x * ld + i] += h * rho[x * ld + i];
+}
+
+cudaError_t launch_vv10_potential(const double* rho, int64_t ld, const int64_t* idx,
+                                  int64_t nk, double kvv, double c, double beta, double fac,
+                                  const double* F, const double* U, const double* W,
+                                  double* exc, double* v, cudaStream_t s) {
+    if (nk <= 0) return cudaSuccess;
+    vv10_potential_kernel<<<(unsigned)((nk + 127) / 128), 128, 0, s>>>(
+        rho, ld, idx, nk, kvv, c, beta, fac, F, U, W, exc, v);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_vv10(const float* xyz, const float* q, const float* w0,
                         const float* kap, int64_t n, double tile_tol,
                         double* F, double* U, double* W, void* ws,

@@ -7,7 +7,9 @@ pyscf_wb97mv_fast/gpu/vv10.py).
   pruning when tile_tol > 0).  F is returned as -1.5 x the raw sum, the
   libdft VXC_vv10nlc convention the reference follows (:216-221).
 * ``vv10_pointwise``: the per-point FP64 quantities of PySCF's _vv10nlc
-  (reference :243-265), in torch on the device.
+  (reference :243-265) in torch; the flows below run them as one kernel
+  before the double sum and one after it (wb_vv10_points,
+  wb_vv10_potential).
 * ``gpu_nr_nlc_vxc``: same signature and result as
   ``NumInt.nr_nlc_vxc`` -> (nelec, excsum, vmat) (reference :268-342): AO
   values and gradients (FP64, native), GGA density, threshold
@@ -20,7 +22,7 @@ import math
 import numpy as np
 
 from pyscf_wb97mv_fast_gb300 import _native
-from pyscf_wb97mv_fast_gb300.cosx import CosxEngine, as_molecule
+from pyscf_wb97mv_fast_gb300.cosx import CosxEngine, as_molecule, device_arg, device_out
 
 THRESH = 1e-8
 Unsupported = _native.Unsupported
@@ -118,14 +120,19 @@ def _per_point(a, n, dev, name):
     return t
 
 
+def _constants(nlc_pars):
+    """K, C and Beta of the parameters (b, C)."""
+    Bvv, Cvv = nlc_pars
+    pi = math.pi
+    return (Bvv * 1.5 * pi * (9.0 * pi) ** (-1.0 / 6.0), Cvv,
+            ((3.0 / (Bvv * Bvv)) ** 0.75) / 32.0)
+
+
 def vv10_pointwise(rho0, grad, weights, nlc_pars):
     """Per-point FP64 terms on the thresholded set: q, W0, kappa, dW0/dR,
     dW0/dG, dK/dR, Beta (torch tensors; Beta a float)."""
-    Bvv, Cvv = nlc_pars
-    pi = math.pi
-    pi43 = 4.0 * pi / 3.0
-    Kvv = Bvv * 1.5 * pi * (9.0 * pi) ** (-1.0 / 6.0)
-    Beta = ((3.0 / (Bvv * Bvv)) ** 0.75) / 32.0
+    Kvv, Cvv, Beta = _constants(nlc_pars)
+    pi43 = 4.0 * math.pi / 3.0
     R = rho0
     G = (grad ** 2).sum(dim=0)
     W0tmp = Cvv * (G / (R * R)) ** 2
@@ -136,6 +143,45 @@ def vv10_pointwise(rho0, grad, weights, nlc_pars):
     dKdR = kappa / 6.0
     q = R * weights
     return q, W0, kappa, dW0dR, dW0dG, dKdR, Beta
+
+
+def _points(rho, coords, weights, ind, nlc_pars):
+    """The double sum's inputs (xyz, q, W0, kappa) FP32 at the points ind
+    (int64) of a grid: vv10_pointwise's quantities as one kernel
+    (wb_vv10_points).  rho (4, ld), coords (n, 3), weights (n,) FP64."""
+    torch = _torch()
+    dev = rho.device
+    nk, n = int(ind.shape[0]), int(weights.shape[0])
+    kvv, cvv, _ = _constants(nlc_pars)
+    rho = device_arg(rho, 'rho', torch.float64, dev, (4, None))
+    coords = device_arg(coords, 'coords', torch.float64, dev, (n, 3))
+    weights = device_arg(weights, 'weights', torch.float64, dev, (n,))
+    ind = device_arg(ind, 'ind', torch.int64, dev, (nk,))
+    out = [torch.empty((nk, 3) if i == 0 else nk, dtype=torch.float32, device=dev)
+           for i in range(4)]
+    _native.check(_native.lib().wb_vv10_points(
+        _native.ptr(rho), int(rho.shape[1]), _native.ptr(coords), _native.ptr(weights),
+        _native.ptr(ind), nk, kvv, cvv, *[_native.ptr(o) for o in out], CosxEngine._stream()), 'wb_vv10_points')
+    return out
+
+
+def _add_potential(rho, ind, nlc_pars, fac, F, U, W, exc, vv):
+    """Adds fac times the energy density to exc (n,) and the derivatives to
+    vv (4, ld) (half of d/d rho, and d/d grad) from the double sums at the
+    points ind (wb_vv10_potential)."""
+    torch = _torch()
+    dev = rho.device
+    nk = int(ind.shape[0])
+    kvv, cvv, beta = _constants(nlc_pars)
+    F, U, W = (device_arg(x.to(torch.float64), 'sum', torch.float64, dev, (nk,))
+               for x in (F, U, W))
+    rho = device_arg(rho, 'rho', torch.float64, dev, (4, None))
+    device_out(vv, 'vv', torch.float64, dev, tuple(rho.shape))
+    device_out(exc, 'exc', torch.float64, dev, tuple(exc.shape))
+    _native.check(_native.lib().wb_vv10_potential(
+        _native.ptr(rho), int(rho.shape[1]), _native.ptr(ind), nk, kvv, cvv,
+        beta, float(fac), _native.ptr(F), _native.ptr(U), _native.ptr(W),
+        _native.ptr(exc), _native.ptr(vv), CosxEngine._stream()), 'wb_vv10_potential')
 
 
 class Vv10Context:
@@ -186,11 +232,9 @@ def vv10_prepare(eng, g, D, nlc_pars, gemm='fp64'):
         T = eng.gemm64_f(g.X[0], D.T)
     rho = eng.gga_rho(g.X, T, n)                          # (4, ld)
     ind = torch.nonzero(rho[0, :n] >= THRESH).squeeze(1)
-    q, W0, kappa, dW0dR, dW0dG, dKdR, Beta = vv10_pointwise(
-        rho[0, ind], rho[1:4, ind], w[ind], nlc_pars)
-    return dict(eng=eng, g=g, gemm=gemm, n=n, rho=rho, ind=ind,
-                xyz=g.coords[ind].to(torch.float32), q=q, W0=W0, kappa=kappa,
-                dW0dR=dW0dR, dW0dG=dW0dG, dKdR=dKdR, Beta=Beta)
+    xyz, q, W0, kappa = _points(rho, g.coords, w, ind, nlc_pars)
+    return dict(eng=eng, g=g, gemm=gemm, n=n, rho=rho, ind=ind, nlc_pars=nlc_pars,
+                xyz=xyz, q=q, W0=W0, kappa=kappa)
 
 
 def vv10_finish(st, F, U, W):
@@ -199,15 +243,12 @@ def vv10_finish(st, F, U, W):
     torch = _torch()
     eng, g, n, ind, rho = (st[k] for k in ('eng', 'g', 'n', 'ind', 'rho'))
     w = g.weights
-    Beta = st['Beta']
     exc = torch.zeros(n, dtype=torch.float64, device=rho.device)
-    exc[ind] = Beta + 0.5 * F
+    vv = torch.zeros_like(rho)
+    _add_potential(rho, ind, st['nlc_pars'], 1.0, F, U, W, exc, vv)
     e_nl = (rho[0, :n] * w * exc).sum()
     # G = 1/2 v0 X0 + sum_d 2 v1 grad_d X_d, then X0^T (w o G); G FP64, or
     # rounded once to FP32 (gemm 'fp32')
-    vv = torch.zeros_like(rho)
-    vv[0, ind] = 0.5 * (Beta + F + 1.5 * (U * st['dKdR'] + W * st['dW0dR']))
-    vv[1:4, ind] = (3.0 * W * st['dW0dG'])[None, :] * rho[1:4, ind]
     G = eng.gga_aow(g.X, vv, n, torch.float32 if st['gemm'] == 'fp32' else None)
     if st['gemm'] == 'fp64':
         vmat = eng.gemm64_k(g.X[0], G, w)
@@ -262,15 +303,10 @@ def gpu_nr_nlc_vxc(ctx, ni, mol, grids, xc_code, dm, relativity=0, hermi=1,
     rho0 = rho[0, :n]
     exc = torch.zeros(n, dtype=torch.float64, device=dev)
     vv = torch.zeros_like(rho)          # d/d rho (half of it) and d/d grad
-    c32 = coords.to(torch.float32)
     ind = torch.nonzero(rho0 >= THRESH).squeeze(1)
     for nlc_pars, fac in nlc_coefs:
-        q, W0, kappa, dW0dR, dW0dG, dKdR, Beta = vv10_pointwise(
-            rho0[ind], rho[1:4, ind], w[ind], nlc_pars)
-        F, U, W = ctx.kernel.kernel_sum(c32[ind], q, W0, kappa)
-        exc[ind] += fac * (Beta + 0.5 * F)
-        vv[0, ind] += (0.5 * fac) * (Beta + F + 1.5 * (U * dKdR + W * dW0dR))
-        vv[1:4, ind] += (3.0 * fac * W * dW0dG)[None, :] * rho[1:4, ind]
+        F, U, W = ctx.kernel.kernel_sum(*_points(rho, coords, w, ind, nlc_pars))
+        _add_potential(rho, ind, nlc_pars, fac, F, U, W, exc, vv)
     # vmat = X0^T (w o G) + its transpose, G = 1/2 v0 X0 + sum_d v_d X_d
     vmat = eng.gemm64_k(X[0], eng.gga_aow(X, vv, n), w)
     vmat = vmat + vmat.T
