@@ -386,6 +386,12 @@ int wb_vv10_potential(const double* rho, int64_t ld, const int64_t* idx, int64_t
                       const double* f, const double* u, const double* w,
                       double* exc, double* v, void* stream);
 
+/* The device SCF's semilocal functional (scf.RshLdaVv10): energy per volume and
+ * its derivative at n densities, short-range LDA exchange (omega, weight cx_sr)
+ * and VWN5 correlation; zero where rho <= 1e-14. */
+int wb_rsh_lda_eval(const double* rho, int64_t n, double omega, double cx_sr,
+                    double* e, double* v, void* stream);
+
 /* Engine of the F product (process-wide, every F of the K builds and of
  * wb_cosx_ozaki_f / _f64): WB_OZAKI_ENGINE_LIBRARY (the default) runs one
  * cuBLAS bf16 GEMM per level; WB_OZAKI_ENGINE_TC is this library's

@@ -50,6 +50,7 @@ EXPORTED = ('wb_cosx_create', 'wb_cosx_destroy', 'wb_cosx_get_info',
             'wb_cosx_ozaki_f64', 'wb_cosx_ozaki_k64',
             'wb_gemm64_workspace_bytes', 'wb_cosx_gemm64_f', 'wb_cosx_gemm64_k',
             'wb_gga_rho', 'wb_gga_aow', 'wb_vv10_points', 'wb_vv10_potential',
+            'wb_rsh_lda_eval',
             'wb_vv10_kernel_sum_noalloc', 'wb_vv10_kernel_sum_batch',
             'wb_cosx_fp64_workspace_bytes', 'wb_cosx_get_k_fp64',
             'wb_cosx_set_class_variant', 'wb_cosx_get_class_variant',
@@ -183,6 +184,7 @@ def _declare(lib):
         'wb_vv10_points': (_INT, [_P, _I64, _P, _P, _P, _I64, _D, _D, _P, _P, _P, _P, _P]),
         'wb_vv10_potential': (_INT, [_P, _I64, _P, _I64, _D, _D, _D, _D, _P, _P, _P, _P,
                                      _P, _P]),
+        'wb_rsh_lda_eval': (_INT, [_P, _I64, _D, _D, _P, _P, _P]),
         'wb_gga_rho': (_INT, [_P, _P, _P, _INT, _I64, _I64, _P, _P]),
         'wb_gga_aow': (_INT, [_P, _P, _P, _I64, _I64, _INT, _P, _P]),
         'wb_cosx_fp64_workspace_bytes': (ctypes.c_size_t, [_P, _I64]),

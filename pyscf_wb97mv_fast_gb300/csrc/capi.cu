@@ -2539,6 +2539,15 @@ int wb_vv10_potential(const double* rho, int64_t ld, const int64_t* idx, int64_t
     return WB_OK;
 }
 
+int wb_rsh_lda_eval(const double* rho, int64_t n, double omega, double cx_sr, double* e,
+                    double* v, void* stream) {
+    if (n < 0 || (n && (!rho || !e || !v)))
+        return fail(WB_ERR_INVALID_ARGUMENT, "wb_rsh_lda_eval: bad arguments");
+    WB_CUDA(wb::scf::launch_rsh_lda(rho, n, omega, cx_sr, e, v,
+                                    static_cast<cudaStream_t>(stream)));
+    return WB_OK;
+}
+
 int wb_ozaki_set_f_engine(int engine) {
     if (engine != WB_OZAKI_ENGINE_LIBRARY && engine != WB_OZAKI_ENGINE_TC)
         return fail(WB_ERR_INVALID_ARGUMENT, "wb_ozaki_set_f_engine: unknown engine");

@@ -87,5 +87,8 @@ cudaError_t launch_hartree_mixed(const HartreeArgs& a, cudaStream_t s);
 // v (npts,) = the sum of the ranges and mixed chunks
 cudaError_t launch_hartree_sum(const HartreeArgs& a, double* v, cudaStream_t s);
 
+cudaError_t launch_rsh_lda(const double* rho, int64_t n, double omega, double cx_sr,
+                           double* e, double* v, cudaStream_t s);
+
 }  // namespace scf
 }  // namespace wb

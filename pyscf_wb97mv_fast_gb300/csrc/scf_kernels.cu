@@ -696,5 +696,74 @@ cudaError_t launch_hartree_sum(const HartreeArgs& a, double* v, cudaStream_t s) 
     return cudaGetLastError();
 }
 
+// -- the semilocal functional ---------------------------------------------------
+
+// Range-separated LDA exchange and VWN5 correlation (scf.RshLdaVv10.eval has the
+// formulas), one thread per point.  One kernel instead of some sixty elementwise
+// array operations in FP64, with the VV10 point kernels: Fock build of 8 waters
+// 18.3 -> 16.8 ms, of 4 waters in FP64 13.5 -> 12.2 ms.
+__global__ void __launch_bounds__(128)
+rsh_lda_kernel(const double* __restrict__ rho, const int64_t n, const double omega,
+               const double cx_sr, double* __restrict__ e_out, double* __restrict__ v_out) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double rin = rho[i];
+    if (!(rin > 1e-14)) {
+        e_out[i] = 0.0;
+        v_out[i] = 0.0;
+        return;
+    }
+    const double r = rin, third = cbrt(r);
+    const double ex_lda = -0.75 * cbrt(3.0 / M_PI) * r * third;
+    const double kf = cbrt(3.0 * M_PI * M_PI) * third;
+    const double a = omega / (2.0 * kf);
+    double F, dF;
+    if (a >= 1.5) {
+        // c_k a^(-2k), k = 1 .. 8
+        constexpr double c[8] = {1.0 / 36.0, -1.0 / 960.0, 1.0 / 26880.0, -1.0 / 829440.0,
+                                 1.0 / 28385280.0, -1.0 / 1073479680.0, 1.0 / 44590694400.0,
+                                 -1.0 / 2021444812800.0};
+        const double y = 1.0 / (a * a);
+        double yk = 1.0;
+        F = dF = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            yk *= y;
+            F += c[k] * yk;
+            dF -= 2.0 * (k + 1) * c[k] * yk;
+        }
+        dF /= a;
+    } else {
+        const double a3 = a * a * a, eb = exp(-1.0 / (4.0 * a * a));
+        const double g = sqrt(M_PI) * erf(1.0 / (2.0 * a)) + (2.0 * a - 4.0 * a3) * eb -
+                         3.0 * a + 4.0 * a3;
+        const double dg = 12.0 * a * a * (1.0 - eb) - 3.0;
+        F = 1.0 - 8.0 / 3.0 * a * g;
+        dF = -8.0 / 3.0 * (g + a * dg);
+    }
+    const double ex = ex_lda * F;
+    const double vx = (ex_lda / r) * (4.0 / 3.0 * F - a / 3.0 * dF);
+    const double A = 0.0310907, x0 = -0.10498, b = 3.72744, c = 12.9352;
+    const double Q = sqrt(4.0 * c - b * b), X0 = x0 * x0 + b * x0 + c;
+    const double x = sqrt(cbrt(3.0 / (4.0 * M_PI)) / third);
+    const double X = x * x + b * x + c, t = 2.0 * x + b;
+    const double at = atan(Q / t), den = t * t + Q * Q;
+    const double ec = A * (log(x * x / X) + 2.0 * b / Q * at -
+                           b * x0 / X0 * (log((x - x0) * (x - x0) / X) +
+                                          2.0 * (b + 2.0 * x0) / Q * at));
+    const double dec = A * (2.0 / x - t / X - 4.0 * b / den -
+                            b * x0 / X0 * (2.0 / (x - x0) - t / X -
+                                           4.0 * (b + 2.0 * x0) / den));
+    e_out[i] = cx_sr * ex + r * ec;
+    v_out[i] = cx_sr * vx + (ec - x / 6.0 * dec);
+}
+
+cudaError_t launch_rsh_lda(const double* rho, int64_t n, double omega, double cx_sr,
+                           double* e, double* v, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    rsh_lda_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(rho, n, omega, cx_sr, e, v);
+    return cudaGetLastError();
+}
+
 }  // namespace scf
 }  // namespace wb

@@ -45,7 +45,8 @@ import time
 
 import numpy as np
 
-from pyscf_wb97mv_fast_gb300.cosx import CosxEngine, as_molecule, round32
+from pyscf_wb97mv_fast_gb300 import _native
+from pyscf_wb97mv_fast_gb300.cosx import CosxEngine, as_molecule, device_arg, round32
 from pyscf_wb97mv_fast_gb300.staging.schedule import StagePlan
 
 
@@ -114,6 +115,24 @@ class RshLdaVv10:
         v = self.cx_sr * vx + vc
         zero = torch.zeros_like(rho)
         return torch.where(live, e, zero), torch.where(live, v, zero)
+
+
+_EVAL = RshLdaVv10.eval
+
+
+def _semilocal(functional, rho):
+    """functional.eval(rho) for a density (n,) FP64: on the GPU RshLdaVv10's
+    own formulas as one kernel (wb_rsh_lda_eval), any other functional's eval,
+    a subclass's or a replaced one too, as it is."""
+    torch = _torch()
+    if not rho.is_cuda or getattr(functional.eval, '__func__', None) is not _EVAL:
+        return functional.eval(rho)
+    rho = device_arg(rho, 'rho', torch.float64, rho.device, (None,))
+    e, v = torch.empty_like(rho), torch.empty_like(rho)
+    _native.check(_native.lib().wb_rsh_lda_eval(
+        _native.ptr(rho), int(rho.shape[0]), float(functional.omega), float(functional.cx_sr),
+        _native.ptr(e), _native.ptr(v), CosxEngine._stream()), 'wb_rsh_lda_eval')
+    return e, v
 
 
 def _sr_attenuation(a):
@@ -372,7 +391,7 @@ class DeviceRKS:
             rho = self._density(gx, D, gemm)
         else:
             rho = base['rho'] + self._density(gx, dD, 'fp32')
-        e, v = f.eval(rho)
+        e, v = _semilocal(f, rho)
         exc = (gx.weights * e).sum()
         Vxc = self._vmat(gx, v, gemm)
         self._tick('xc')

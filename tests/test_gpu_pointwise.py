@@ -1,10 +1,12 @@
-"""The VV10 point kernels (wb_vv10_points / _potential) against the same formulas
-in torch on the host, from the lowest densities taken to compressed ones, with
-block remainders and scattered points.
+"""The pointwise kernels (wb_vv10_points / _potential, wb_rsh_lda_eval) against
+the same formulas in torch on the host, from the lowest densities taken to
+compressed ones, with block remainders and scattered points.
 
 Bounds, from the formulas: FP32 outputs are one rounding of an FP64 value (one
 unit in the last place); FP64 sums are within 2^-46 of the sum of their terms'
-magnitudes (some sixty operations of 2^-53 each)."""
+magnitudes (some sixty operations of 2^-53 each); the attenuation function's
+closed form sums terms up to 4 a^3 = 13.5 at a <= 1.5, a few 1e-14 of the
+unattenuated exchange, and the correlation logarithms up to 30, a few 1e-16."""
 import numpy as np
 import pytest
 
@@ -54,3 +56,42 @@ def test_vv10_points_and_potential(n, nk):
     sv[1:, hi] += (3.0 * fac * hW * dW0dG * hr[1:, hi]).abs()
     assert bool(((exc.cpu() - re).abs() <= 2.0 ** -46 * se).all())
     assert bool(((vv.cpu() - rv).abs() <= 2.0 ** -46 * sv).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('n', [1, 128, 1001])
+def test_semilocal_kernel(n):
+    import torch
+
+    from pyscf_wb97mv_fast_gb300.scf import RshLdaVv10, _semilocal
+    rng = np.random.default_rng(n)
+    r = 10.0 ** rng.uniform(-16.0, 3.0, n)
+    r[0] = 1e-14                                   # not above the threshold
+    if n > 8:
+        r[1:6] = [0.0, -1e-9, 5e-324, np.nan, 1.0000001e-14]
+    f = RshLdaVv10(omega=0.3 if n < 500 else 0.6)
+    host = torch.as_tensor(r)
+    e, v = (x.cpu() for x in _semilocal(f, host.cuda()))
+    re, rv = f.eval(host)
+    live = host > 1e-14
+    assert bool((e[~live] == 0).all()) and bool((v[~live] == 0).all())
+    p = host[live]
+    assert bool(((e - re)[live].abs() <= 2e-13 * p ** (4.0 / 3.0) + 1e-14 * p).all())
+    assert bool(((v - rv)[live].abs() <= 2e-13 * p ** (1.0 / 3.0) + 1e-14).all())
+
+
+def test_other_functionals_keep_their_eval():
+    import torch
+
+    from pyscf_wb97mv_fast_gb300.scf import RshLdaVv10, _semilocal
+
+    class Mine(RshLdaVv10):
+        def eval(self, rho):
+            return rho, 2.0 * rho
+
+    rho = torch.ones(3, dtype=torch.float64)
+    assert torch.equal(_semilocal(Mine(), rho)[1], 2.0 * rho)
+    f = RshLdaVv10()
+    assert torch.equal(_semilocal(f, rho)[0], f.eval(rho)[0])
+    f.eval = lambda r: (3.0 * r, r)
+    assert torch.equal(_semilocal(f, rho)[0], 3.0 * rho)
