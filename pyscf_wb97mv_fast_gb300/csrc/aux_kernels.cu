@@ -170,17 +170,12 @@ __device__ __forceinline__ double warp_sum_d(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ double warp_max_d(double v) {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ float4 centroid_radius(const double* sum, int n,
-                                                  double d) {
-    float r = (float)d;
-    if ((double)r < d) r = nextafterf(r, INFINITY);
-    if (n <= 0) return make_float4(0.0f, 0.0f, 0.0f, r);
-    return make_float4((float)(sum[0] / n), (float)(sum[1] / n),
-                       (float)(sum[2] / n), r);
+// the largest of 32 non-negative doubles, by their bits
+__device__ __forceinline__ double warp_max_bits(double v) {
+    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    return __hiloint2double((int)mh, (int)ml);
 }
 
 // The shells are shared out over gridDim.y: one warp walking all of them is a
@@ -213,44 +208,65 @@ __global__ void sub_stats_kernel(const BlockStatsOut O,
         for (int x = 0; x < 3; ++x) c[q][x] = valid[q] ? coords[g[q] * 3 + x] : 0.0;
     }
     if (blockIdx.y == 0) {
-        int nv[4];
+        // The seven blocks: 0-3 the quarters, 4 and 5 the halves, 6 the whole.
+        // A warp's FP64 instruction takes 16 cycles whatever its active lanes,
+        // so the divisions run once, lane 3 b + x on component x of block b,
+        // the square roots once, lane b on the largest distance of block b, and
+        // the maxima on the integer pipe.
+        double s[7][3];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int64_t rem = npts - ((int64_t)blk * 128 + 32 * q);
-            nv[q] = rem >= 32 ? 32 : (rem > 0 ? (int)rem : 0);
+        for (int x = 0; x < 3; ++x) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) s[q][x] = warp_sum_d(c[q][x]);
+            s[4][x] = s[0][x] + s[1][x];
+            s[5][x] = s[2][x] + s[3][x];
+            s[6][x] = s[4][x] + s[2][x] + s[3][x];
         }
-        double s[4][3];
+        auto level = [](int b) { return b < 4 ? 0 : (b < 6 ? 1 : 2); };
+        auto first = [](int b) { return b < 4 ? b : (b < 6 ? 2 * (b - 4) : 0); };
+        auto count = [&](int b) {
+            const int64_t rem = npts - ((int64_t)blk * 128 + 32 * first(b));
+            const int full = 32 << level(b);
+            return rem >= full ? full : (rem > 0 ? (int)rem : 0);
+        };
+        double own = 0.0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            for (int x = 0; x < 3; ++x) s[q][x] = warp_sum_d(c[q][x]);
-        // level k = 0, 1, 2: block j of the level covers quarters [j 2^k, (j+1) 2^k)
+        for (int i = 0; i < 21; ++i)
+            if (lane == i) own = s[i / 3][i % 3];
+        const int nown = count(lane < 21 ? lane / 3 : 6);
+        own = nown ? own / nown : 0.0;
+        double dmax = 0.0;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const int span = 1 << k;
+        for (int b = 0; b < 7; ++b) {
+            double m[3];
 #pragma unroll
-            for (int j = 0; j < 4 / span; ++j) {
-                double sum[3] = {0.0, 0.0, 0.0};
-                int n = 0;
-                for (int q = j * span; q < (j + 1) * span; ++q) {
-                    for (int x = 0; x < 3; ++x) sum[x] += s[q][x];
-                    n += nv[q];
+            for (int x = 0; x < 3; ++x) m[x] = __shfl_sync(0xffffffffu, own, 3 * b + x);
+            double d = 0.0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (q < first(b) || q >= first(b) + (1 << level(b)) || !valid[q]) continue;
+                double e2 = 0.0;
+#pragma unroll
+                for (int x = 0; x < 3; ++x) {
+                    const double e = c[q][x] - m[x];
+                    e2 += e * e;
                 }
-                double m[3];
-                for (int x = 0; x < 3; ++x) m[x] = n ? sum[x] / n : 0.0;
-                double d = 0.0;
-                for (int q = j * span; q < (j + 1) * span; ++q) {
-                    if (!valid[q]) continue;
-                    double e2 = 0.0;
-                    for (int x = 0; x < 3; ++x) {
-                        const double e = c[q][x] - m[x];
-                        e2 += e * e;
-                    }
-                    d = fmax(d, sqrt(e2));
-                }
-                d = warp_max_d(d);
-                const int64_t b = (int64_t)blk * (4 / span) + j;
-                if (lane == 0 && b * 32 * span < ld) O.cr[k][b] = centroid_radius(sum, n, d);
+                d = fmax(d, e2);
             }
+            d = warp_max_bits(d);
+            if (lane == b) dmax = d;
+        }
+        const double d = sqrt(dmax);
+        float cen[3];
+#pragma unroll
+        for (int x = 0; x < 3; ++x)
+            cen[x] = (float)__shfl_sync(0xffffffffu, own, lane < 7 ? 3 * lane + x : 0);
+        float r = (float)d;
+        if ((double)r < d) r = nextafterf(r, INFINITY);
+        if (lane < 7) {
+            const int k = level(lane);
+            const int64_t b = ((int64_t)blk * 4 + first(lane)) >> k;
+            if (b * (32 << k) < ld) O.cr[k][b] = make_float4(cen[0], cen[1], cen[2], r);
         }
     }
     float wq[4];
@@ -293,7 +309,8 @@ cudaError_t launch_sub_stats(const double* coords, const double* weights,
                              const BlockStatsOut& out, cudaStream_t s) {
     const int64_t nblk = (ld + 127) / 128;
     if (nblk <= 0) return cudaSuccess;
-    const int warps = 4;
+    // one warp a CTA while the blocks are fewer than four an SM
+    const int warps = nblk < 4 * 152 ? 1 : 4;
     const dim3 grid((unsigned)((nblk + warps - 1) / warps),
                     (unsigned)std::max(1, (nvshell + kStatsShells - 1) / kStatsShells));
     sub_stats_kernel<<<grid, 32 * warps, 0, s>>>(
