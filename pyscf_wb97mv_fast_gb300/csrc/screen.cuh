@@ -28,8 +28,12 @@ __device__ __forceinline__ bool screen_pair(const float tol,
         float d = dist - cr.w - 1e-5f * (dist + cr.w) - 1e-6f;
         d = fmaxf(d, 0.0f);
         const float T = bp.w * d * d;
-        const float f0 = (T > 1e-12f)
-            ? 0.88622692545f * erff(sqrtf(T)) * rsqrtf(T) : 1.0f;
+        // erff is exactly 1 from 5 on
+        float f0 = 1.0f;
+        if (T > 25.0f)
+            f0 = 0.88622692545f * rsqrtf(T);
+        else if (T > 1e-12f)
+            f0 = 0.88622692545f * erff(sqrtf(T)) * rsqrtf(T);
         b += bpref[m] * f0;
     }
     return tp.x * b * f >= tol;
