@@ -7,6 +7,7 @@
 
 #include "boys.cuh"
 #include "cart.cuh"
+#include "cvt64.cuh"
 #include "fp64_boys.cuh"
 #include "launch.hpp"
 #include "screen.cuh"
@@ -448,47 +449,103 @@ cudaError_t launch_block_order(const BlockOrderArgs& P, cudaStream_t s) {
 // the FP64 AO values and gradients and T (1 or 4, nao, ld) = fl32(D^T X_d)
 // from the FP64-accurate F GEMM.  Products in FP32 (the reference's flow is
 // FP32 throughout), summed in FP32 over 8 AOs and in FP64 across groups.
-// One thread per point, rows read coalesced.  Points at or past npts: 0.
-__global__ void xc_rho_kernel(const double* __restrict__ X,
-                              const float* __restrict__ T, int nao, int64_t ld,
-                              int64_t npts, int mgga, double* __restrict__ rho) {
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= ld) return;
-    double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    if (g < npts) {
-        const int64_t pl = (int64_t)nao * ld;
-        for (int m0 = 0; m0 < nao; m0 += 8) {
-            float part[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+// Points at or past npts: 0.
+//
+// Bound by HBM (48 bytes per point and AO for MGGA).  A block takes 64 points,
+// two a lane, and its eight warps the groups of 8 AOs in turn, so that a tile
+// of the flow (57,000 points) has 7,000 warps in flight; one thread per point
+// left 1.5 CTAs an SM waiting on their loads.  X is rounded on the integer
+// pipe: a conversion instruction per element takes as long as its 8 bytes.
+template<bool V>
+__device__ __forceinline__ double2 load2(const double* p) {
+    if constexpr (V) return *reinterpret_cast<const double2*>(p);
+    else return make_double2(p[0], p[1]);
+}
+template<bool V>
+__device__ __forceinline__ float2 load2(const float* p) {
+    if constexpr (V) return *reinterpret_cast<const float2*>(p);
+    else return make_float2(p[0], p[1]);
+}
+// both elements of a pair load at every even offset from these
+inline bool pair_aligned(const void* f64_a, const void* f64_b, const void* f32) {
+    return (((uintptr_t)f64_a | (uintptr_t)f64_b) & 15) == 0 && ((uintptr_t)f32 & 7) == 0;
+}
+
+template<bool MGGA, bool V>
+__global__ void __launch_bounds__(256)
+xc_rho_kernel(const double* __restrict__ X, const float* __restrict__ T, int nao, int64_t ld,
+              int64_t npts, double* __restrict__ rho) {
+    constexpr int NK = MGGA ? 5 : 4;
+    __shared__ double2 sum[8][NK][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t g = (int64_t)blockIdx.x * 64 + 2 * lane;
+    const int64_t pl = (int64_t)nao * ld;
+    double2 acc[NK];
+#pragma unroll
+    for (int k = 0; k < NK; ++k) acc[k] = make_double2(0.0, 0.0);
+    if (g < ld) {
+        for (int m0 = 8 * warp; m0 < nao; m0 += 64) {
+            float2 part[NK];
+#pragma unroll
+            for (int k = 0; k < NK; ++k) part[k] = make_float2(0.0f, 0.0f);
             const int m1 = min(nao, m0 + 8);
+#pragma unroll 4
             for (int mu = m0; mu < m1; ++mu) {
                 const int64_t o = (int64_t)mu * ld + g;
-                const float t0 = T[o];
-                part[0] = fmaf(t0, (float)X[o], part[0]);
-                part[1] = fmaf(t0, (float)X[pl + o], part[1]);
-                part[2] = fmaf(t0, (float)X[2 * pl + o], part[2]);
-                part[3] = fmaf(t0, (float)X[3 * pl + o], part[3]);
-                if (mgga) {
-                    part[4] = fmaf(T[pl + o], (float)X[pl + o], part[4]);
-                    part[4] = fmaf(T[2 * pl + o], (float)X[2 * pl + o], part[4]);
-                    part[4] = fmaf(T[3 * pl + o], (float)X[3 * pl + o], part[4]);
+                const float2 t0 = load2<V>(T + o);
+                float2 x[4];
+#pragma unroll
+                for (int d = 0; d < 4; ++d) {
+                    const double2 xd = load2<V>(X + d * pl + o);
+                    x[d] = make_float2(to_f32(xd.x), to_f32(xd.y));
+                    part[d].x = fmaf(t0.x, x[d].x, part[d].x);
+                    part[d].y = fmaf(t0.y, x[d].y, part[d].y);
+                }
+                if constexpr (MGGA) {
+#pragma unroll
+                    for (int d = 1; d < 4; ++d) {
+                        const float2 t = load2<V>(T + d * pl + o);
+                        part[4].x = fmaf(t.x, x[d].x, part[4].x);
+                        part[4].y = fmaf(t.y, x[d].y, part[4].y);
+                    }
                 }
             }
 #pragma unroll
-            for (int k = 0; k < 5; ++k) acc[k] += (double)part[k];
+            for (int k = 0; k < NK; ++k) {
+                acc[k].x += to_f64(part[k].x);
+                acc[k].y += to_f64(part[k].y);
+            }
         }
     }
-    rho[g] = acc[0];
-    rho[ld + g] = 2.0 * acc[1];
-    rho[2 * ld + g] = 2.0 * acc[2];
-    rho[3 * ld + g] = 2.0 * acc[3];
-    rho[4 * ld + g] = 0.5 * acc[4];
+#pragma unroll
+    for (int k = 0; k < NK; ++k) sum[warp][k][lane] = acc[k];
+    __syncthreads();
+    // warp k adds quantity k of the block's 64 points in warp order
+    if (warp < 5 && g < ld) {
+        double2 r = make_double2(0.0, 0.0);
+        if (warp < NK) {
+#pragma unroll
+            for (int w = 0; w < 8; ++w) {
+                r.x += sum[w][warp][lane].x;
+                r.y += sum[w][warp][lane].y;
+            }
+        }
+        const double f = warp == 0 ? 1.0 : (warp == 4 ? 0.5 : 2.0);
+        rho[warp * ld + g] = g < npts ? f * r.x : 0.0;
+        rho[warp * ld + g + 1] = g + 1 < npts ? f * r.y : 0.0;
+    }
 }
 
 cudaError_t launch_xc_rho(const double* X, const float* T, int nao, int64_t ld,
                           int64_t npts, int mgga, double* rho, cudaStream_t s) {
     if (ld <= 0) return cudaSuccess;
-    xc_rho_kernel<<<(unsigned)((ld + 255) / 256), 256, 0, s>>>(X, T, nao, ld, npts,
-                                                              mgga, rho);
+    const unsigned grid = (unsigned)((ld + 63) / 64);
+    if (!pair_aligned(X, X, T))
+        (mgga ? xc_rho_kernel<true, false> : xc_rho_kernel<false, false>)
+            <<<grid, 256, 0, s>>>(X, T, nao, ld, npts, rho);
+    else
+        (mgga ? xc_rho_kernel<true, true> : xc_rho_kernel<false, true>)
+            <<<grid, 256, 0, s>>>(X, T, nao, ld, npts, rho);
     return cudaGetLastError();
 }
 
@@ -496,40 +553,72 @@ cudaError_t launch_xc_rho(const double* X, const float* T, int nao, int64_t ld,
 // (the reference's aow without the weights, which the K GEMM applies) and,
 // for MGGA, G_d = 1/2 vtau X_d (d = x, y, z); v (5, ld) FP64 are the
 // density-parameter derivatives (chain rule applied).  Points at or past
-// npts: 0.
-__global__ void xc_aow_kernel(const double* __restrict__ X,
-                              const double* __restrict__ v, int nao, int64_t ld,
-                              int64_t npts, int mgga, float* __restrict__ G) {
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int mu = blockIdx.y;
+// npts: 0.  Bound by HBM (48 bytes per point and AO for MGGA): a thread keeps
+// v of two points for eight rows and rounds X on the integer pipe.
+constexpr int kAowRows = 8;
+
+template<bool MGGA, bool V>
+__global__ void __launch_bounds__(128)
+xc_aow_kernel(const double* __restrict__ X, const double* __restrict__ v, int nao, int64_t ld,
+              int64_t npts, float* __restrict__ G) {
+    const int64_t g = 2 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
     if (g >= ld) return;
+    const int m0 = blockIdx.y * kAowRows, m1 = min(nao, m0 + kAowRows);
     const int64_t pl = (int64_t)nao * ld;
-    const int64_t o = (int64_t)mu * ld + g;
-    float g0 = 0.0f, gt[3] = {0.0f, 0.0f, 0.0f};
-    if (g < npts) {
-        const float u0 = (float)(0.5 * v[g]);
-        g0 = u0 * (float)X[o];
+    const bool in[2] = {g < npts, g + 1 < npts};
+    constexpr int NK = MGGA ? 5 : 4;
+    float2 u[NK];
 #pragma unroll
-        for (int d = 1; d < 4; ++d)
-            g0 = fmaf((float)v[d * ld + g], (float)X[d * pl + o], g0);
-        if (mgga) {
-            const float ut = (float)(0.5 * v[4 * ld + g]);
-#pragma unroll
-            for (int d = 1; d < 4; ++d) gt[d - 1] = ut * (float)X[d * pl + o];
-        }
+    for (int k = 0; k < NK; ++k) {
+        const double2 t = load2<V>(v + k * ld + g);
+        const bool half = k == 0 || k == 4;
+        u[k].x = in[0] ? (float)(half ? 0.5 * t.x : t.x) : 0.0f;
+        u[k].y = in[1] ? (float)(half ? 0.5 * t.y : t.y) : 0.0f;
     }
-    G[o] = g0;
-    if (mgga) {
+    auto store = [&](float* p, float a, float b) {
+        a = in[0] ? a : 0.0f;
+        b = in[1] ? b : 0.0f;
+        if constexpr (V) {
+            *reinterpret_cast<float2*>(p) = make_float2(a, b);
+        } else {
+            p[0] = a;
+            p[1] = b;
+        }
+    };
+#pragma unroll 2
+    for (int mu = m0; mu < m1; ++mu) {
+        const int64_t o = (int64_t)mu * ld + g;
+        float2 x[4];
 #pragma unroll
-        for (int d = 1; d < 4; ++d) G[d * pl + o] = gt[d - 1];
+        for (int d = 0; d < 4; ++d) {
+            const double2 xd = load2<V>(X + d * pl + o);
+            x[d] = make_float2(to_f32(xd.x), to_f32(xd.y));
+        }
+        float2 a = make_float2(u[0].x * x[0].x, u[0].y * x[0].y);
+#pragma unroll
+        for (int d = 1; d < 4; ++d) {
+            a.x = fmaf(u[d].x, x[d].x, a.x);
+            a.y = fmaf(u[d].y, x[d].y, a.y);
+        }
+        store(G + o, a.x, a.y);
+        if constexpr (MGGA) {
+#pragma unroll
+            for (int d = 1; d < 4; ++d)
+                store(G + d * pl + o, u[4].x * x[d].x, u[4].y * x[d].y);
+        }
     }
 }
 
 cudaError_t launch_xc_aow(const double* X, const double* v, int nao, int64_t ld,
                           int64_t npts, int mgga, float* G, cudaStream_t s) {
     if (ld <= 0 || nao <= 0) return cudaSuccess;
-    dim3 grid((unsigned)((ld + 255) / 256), (unsigned)nao);
-    xc_aow_kernel<<<grid, 256, 0, s>>>(X, v, nao, ld, npts, mgga, G);
+    const dim3 grid((unsigned)((ld + 255) / 256), (unsigned)((nao + kAowRows - 1) / kAowRows));
+    if (!pair_aligned(X, v, G))
+        (mgga ? xc_aow_kernel<true, false> : xc_aow_kernel<false, false>)
+            <<<grid, 128, 0, s>>>(X, v, nao, ld, npts, G);
+    else
+        (mgga ? xc_aow_kernel<true, true> : xc_aow_kernel<false, true>)
+            <<<grid, 128, 0, s>>>(X, v, nao, ld, npts, G);
     return cudaGetLastError();
 }
 
@@ -580,7 +669,7 @@ cudaError_t launch_gga_rho(const double* X, const void* t, bool t32, int nao, in
 
 // The Fock-side plane of a GGA potential in FP64: sum_d v_d X_d, one thread
 // per AO and two points (HBM-bound: 32 bytes read and 8 written per element).
-template<typename T>
+template<typename T, bool V>
 __global__ void gga_aow_kernel(const double* __restrict__ X, const double* __restrict__ v,
                                int nao, int64_t ld, int64_t npts, T* __restrict__ G) {
     const int64_t g = 2 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
@@ -589,8 +678,8 @@ __global__ void gga_aow_kernel(const double* __restrict__ X, const double* __res
     double a = 0.0, b = 0.0;
 #pragma unroll
     for (int d = 0; d < 4; ++d) {
-        const double2 x = *reinterpret_cast<const double2*>(X + d * pl + o);
-        const double2 u = *reinterpret_cast<const double2*>(v + d * ld + g);
+        const double2 x = load2<V>(X + d * pl + o);
+        const double2 u = load2<V>(v + d * ld + g);
         a = fma(u.x, x.x, a);
         b = fma(u.y, x.y, b);
     }
@@ -602,10 +691,13 @@ cudaError_t launch_gga_aow(const double* X, const double* v, int nao, int64_t ld
                            int64_t npts, bool g32, void* G, cudaStream_t s) {
     if (ld <= 0 || nao <= 0) return cudaSuccess;
     const dim3 grid((unsigned)((ld / 2 + 255) / 256), (unsigned)nao);
+    const bool al = pair_aligned(X, v, nullptr);
     if (g32)
-        gga_aow_kernel<<<grid, 256, 0, s>>>(X, v, nao, ld, npts, static_cast<float*>(G));
+        (al ? gga_aow_kernel<float, true> : gga_aow_kernel<float, false>)
+            <<<grid, 256, 0, s>>>(X, v, nao, ld, npts, static_cast<float*>(G));
     else
-        gga_aow_kernel<<<grid, 256, 0, s>>>(X, v, nao, ld, npts, static_cast<double*>(G));
+        (al ? gga_aow_kernel<double, true> : gga_aow_kernel<double, false>)
+            <<<grid, 256, 0, s>>>(X, v, nao, ld, npts, static_cast<double*>(G));
     return cudaGetLastError();
 }
 
