@@ -2481,6 +2481,8 @@ int wb_cosx_gemm64_f(wb_cosx* h, const double* x, const double* qd, int64_t ld,
                      void* stream) {
     if (!h || !x || !qd || !f_out || ld <= 0 || ld % 32)
         return fail(WB_ERR_INVALID_ARGUMENT, "wb_cosx_gemm64_f: bad arguments");
+    if (((uintptr_t)x | (uintptr_t)f_out) & 15)
+        return fail(WB_ERR_INVALID_ARGUMENT, "wb_cosx_gemm64_f: X and F on 16 bytes");
     if (!workspace || workspace_bytes < wb::gemm64_bytes(h->hp.nao, ld))
         return fail(WB_ERR_WORKSPACE, "wb_cosx_gemm64_f: workspace too small");
     return gemm64_f(h, x, qd, ld, f_out, workspace, static_cast<cudaStream_t>(stream));

@@ -35,11 +35,12 @@
 
 #include "gemm64.hpp"
 #include "launch.hpp"
+#include "ozaki_digits.cuh"
 
 namespace wb {
 namespace {
 
-constexpr int kS = 9, kBits = 7, kW = kS * kBits;
+constexpr int kS = 9, kBits = 7;
 constexpr int kPiece = 4096;             // terms of an exact FP32 sum
 constexpr int kKc = 512;                 // points per chunk of the K product
 constexpr int kGroup = 128;              // chunks in flight
@@ -58,48 +59,37 @@ int planes(int inner) {
     return n;
 }
 
-// e with |x| < 2^e for the bits of the largest |x|
-__device__ __forceinline__ int exponent_of(const unsigned long long bits) {
-    const int E = (int)(bits >> 52);
+// e with |x| < 2^e from the high word of the largest |x|
+__device__ __forceinline__ int exponent_of(const unsigned hi) {
+    const int E = (int)(hi >> 20);
     if (E == 0x7ff) return kNonfinite;
     return E ? E - 1022 : -1022;
 }
 
-// the nine digits of q = rint(x 2^(62 - e)), |x| < 2^e, most significant first
-__device__ __forceinline__ void digits9(const double x, const int e, int* d) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    const int E = (int)((b >> 52) & 0x7ff);
-    unsigned long long m = b & 0xfffffffffffffull;
-    if (E) m |= 1ull << 52;
-    const int sh = (E ? E - 1075 : -1074) + (kW - 1) - e;      // <= 9
-    unsigned long long q = 0;
-    if (sh >= 0) {
-        q = m << min(sh, 9);
-    } else if (sh > -64) {
-        const int r = -sh;
-        q = m >> r;
-        const unsigned long long rem = m & ((1ull << r) - 1), half = 1ull << (r - 1);
-        if (rem > half || (rem == half && (q & 1ull))) ++q;
-    }
-    if (e == kNonfinite) q = 0;
-    // q in base 2^7, balanced: 28 bits, 28 bits and the rest, 32-bit steps
-    long long v = (b >> 63) ? -(long long)q : (long long)q;
-    int part[3];
-    part[2] = (int)(v & 0xfffffff);
-    v >>= 28;
-    part[1] = (int)(v & 0xfffffff);
-    part[0] = (int)(v >> 28);
-    int carry = 0;
+// q = rint(x 2^(62 - e)), |x| < 2^e, with 64 added to each of its nine digits
+// (digit_pair then reads them as bit fields)
+__device__ __forceinline__ unsigned long long biased9(const double x, const int e) {
+    unsigned long long bias = 0;
 #pragma unroll
-    for (int i = kS - 1; i >= 1; --i) {
-        int& p = part[(i + 3) / 4];
-        if (i == kS - 1 || i == kS - 5) p += carry;
-        const int di = ((p + 64) & 127) - 64;
-        d[i] = di;
-        p = (p - di) >> 7;
-        if (i == kS - 4 || i == kS - 8) carry = p;
+    for (int i = 0; i < kS; ++i) bias |= 64ull << (kBits * i);
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int E = (int)((hi >> 20) & 0x7ffu);
+    if (e == kNonfinite) return bias;
+    // |x| = m 2^-10 2^(E - 1075), m the significand 10 bits up, so q = m >> k
+    // with 1 <= k; a subnormal x has no leading one
+    const unsigned top = E ? (hi & 0xfffffu) | 0x100000u : hi & 0xfffffu;
+    const int k = max(1023 + e - max(E, 1), 1);
+    unsigned long long q = 0;
+    if (k < 64) {
+        const unsigned long long m = ((unsigned long long)(top << 10 | lo >> 22) << 32) |
+                                     (unsigned long long)(lo << 10);
+        q = m >> k;
+        const unsigned long long rem = m << (64 - k);
+        const unsigned rh = (unsigned)(rem >> 32);
+        const unsigned sticky = (rh << 1) | (unsigned)rem | ((unsigned)q & 1u);
+        if ((int)rh < 0 && sticky) ++q;
     }
-    d[0] = part[0] + carry;
+    return (int)hi < 0 ? bias - q : bias + q;
 }
 
 // RN(v 2^sc), v = hi 2^28 + lo, with integer arithmetic (the conversions
@@ -145,15 +135,11 @@ struct LevelSum {
 // exponent of the last digit level kept: x y = 2^(ex + ey - 2 (W - 1) +
 // B (S - 1)) sum_l C_l 2^(B (S - 1 - l))
 __device__ __forceinline__ int level_scale(const int ex, const int ey) {
-    return ex + ey - 2 * (kW - 1) + kBits * (kS - 1);
+    return ex + ey - 2 * (kBits * kS - 1) + kBits * (kS - 1);
 }
 __device__ __forceinline__ double finish(const LevelSum& v, const int ex, const int ey) {
     if (ex == kNonfinite || ey == kNonfinite) return __longlong_as_double(0x7ff8000000000000ll);
     return round_sum(v.hi, v.lo, level_scale(ex, ey));
-}
-
-__device__ __forceinline__ unsigned long long abs_bits(const double x) {
-    return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
 }
 
 // exponent of each point's largest |X(l, g)|, g0 <= g < g0 + n
@@ -161,19 +147,16 @@ __global__ void point_exponents_kernel(const double* __restrict__ X, const int n
                                        const int64_t ld, const int n, int* __restrict__ e) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
-    unsigned long long m = 0;
+    unsigned m = 0;
     int l = 0;
     for (; l + 8 <= nao; l += 8) {
-        unsigned long long b[8];
+        double b[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) b[u] = abs_bits(__ldg(X + (int64_t)(l + u) * ld + g));
+        for (int u = 0; u < 8; ++u) b[u] = __ldg(X + (int64_t)(l + u) * ld + g);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) m = b[u] > m ? b[u] : m;
+        for (int u = 0; u < 8; ++u) m = max(m, abs_hi(b[u]));
     }
-    for (; l < nao; ++l) {
-        const unsigned long long b = abs_bits(__ldg(X + (int64_t)l * ld + g));
-        m = b > m ? b : m;
-    }
+    for (; l < nao; ++l) m = max(m, abs_hi(__ldg(X + (int64_t)l * ld + g)));
     e[g] = exponent_of(m);
 }
 
@@ -185,32 +168,23 @@ __global__ void slice_points_kernel(const double* __restrict__ X, const int nao,
     const int l = blockIdx.y;
     const int g = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (g >= n) return;                         // n is even
-    int d0[kS], d1[kS];
-    if (l < nao) {
-        const double2 x = *reinterpret_cast<const double2*>(X + (int64_t)l * ld + g);
-        digits9(x.x, e[g], d0);
-        digits9(x.y, e[g + 1], d1);
-    } else {
-#pragma unroll
-        for (int i = 0; i < kS; ++i) d0[i] = d1[i] = 0;
-    }
+    double2 x = make_double2(0.0, 0.0);
+    if (l < nao) x = *reinterpret_cast<const double2*>(X + (int64_t)l * ld + g);
+    const unsigned long long q0 = biased9(x.x, e[g]), q1 = biased9(x.y, e[g + 1]);
 #pragma unroll
     for (int i = 0; i < kS; ++i)
-        *reinterpret_cast<__nv_bfloat162*>(A + ((int64_t)i * np + l) * n + g) =
-            __floats2bfloat162_rn((float)d0[i], (float)d1[i]);
+        *reinterpret_cast<unsigned*>(A + ((int64_t)i * np + l) * n + g) =
+            digit_pair<kBits, kS>(q0, q1, i);
 }
 
-// largest |bits| of a block of 256 threads
-__device__ __forceinline__ unsigned long long block_max(unsigned long long m) {
-    __shared__ unsigned long long red[8];
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long t = __shfl_xor_sync(0xffffffffu, m, o);
-        m = t > m ? t : m;
-    }
+// the largest of a block of 256 threads
+__device__ __forceinline__ unsigned block_max(unsigned m) {
+    __shared__ unsigned red[8];
+    m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < 8; ++j) m = red[j] > m ? red[j] : m;
+    for (int j = 0; j < 8; ++j) m = max(m, red[j]);
     __syncthreads();
     return m;
 }
@@ -221,19 +195,16 @@ __global__ void __launch_bounds__(256)
 slice_matrix_kernel(const double* __restrict__ QD, const int nao, const int np,
                     int* __restrict__ e, __nv_bfloat16* __restrict__ B) {
     const int mu = blockIdx.x;
-    unsigned long long m = 0;
-    for (int l = threadIdx.x; l < nao; l += 256) {
-        const unsigned long long b = abs_bits(QD[(int64_t)l * nao + mu]);
-        m = b > m ? b : m;
-    }
+    unsigned m = 0;
+    for (int l = threadIdx.x; l < nao; l += 256) m = max(m, abs_hi(QD[(int64_t)l * nao + mu]));
     const int ec = exponent_of(block_max(m));
     if (threadIdx.x == 0) e[mu] = ec;
     for (int l = threadIdx.x; l < np; l += 256) {
-        int d[kS];
-        digits9(l < nao ? QD[(int64_t)l * nao + mu] : 0.0, ec, d);
+        const unsigned long long q = biased9(l < nao ? QD[(int64_t)l * nao + mu] : 0.0, ec);
 #pragma unroll
         for (int i = 0; i < kS; ++i)
-            B[((int64_t)mu * kS + (kS - 1 - i)) * np + l] = __float2bfloat16_rn((float)d[i]);
+            B[((int64_t)mu * kS + (kS - 1 - i)) * np + l] =
+                __ushort_as_bfloat16((unsigned short)digit_pair<kBits, kS>(q, q, i));
     }
 }
 
@@ -278,17 +249,14 @@ slice_chunk_kernel(const double* __restrict__ X, const double* __restrict__ w, c
         if (g < npts) x0 = WG ? w[g] * x[g] : x[g];
         if (g + 1 < npts) x1 = WG ? w[g + 1] * x[g + 1] : x[g + 1];
     }
-    const unsigned long long a = abs_bits(x0), b = abs_bits(x1);
-    const int ee = exponent_of(block_max(a > b ? a : b));
+    const int ee = exponent_of(block_max(max(abs_hi(x0), abs_hi(x1))));
     if (threadIdx.x == 0) e[slot] = ee;
-    int d0[kS], d1[kS];
-    digits9(x0, ee, d0);
-    digits9(x1, ee, d1);
+    const unsigned long long q0 = biased9(x0, ee), q1 = biased9(x1, ee);
     __nv_bfloat16* o = out + slot * kS * kKc + k;
 #pragma unroll
     for (int i = 0; i < kS; ++i)
-        *reinterpret_cast<__nv_bfloat162*>(o + (WG ? kS - 1 - i : i) * kKc) =
-            __floats2bfloat162_rn((float)d0[i], (float)d1[i]);
+        *reinterpret_cast<unsigned*>(o + (WG ? kS - 1 - i : i) * kKc) =
+            digit_pair<kBits, kS>(q0, q1, i);
 }
 
 // K (+)= the chunks of one group, in chunk order: C (plane, chunk, np x np)

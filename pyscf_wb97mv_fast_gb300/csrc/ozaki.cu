@@ -42,6 +42,7 @@
 #include <cmath>
 #include <cstdint>
 
+#include "cvt64.cuh"
 #include "launch.hpp"
 #include "ozaki.hpp"
 #include "ozaki_digits.cuh"
@@ -63,24 +64,17 @@ __global__ void f_rowmax_kernel(const double* __restrict__ X, int nao,
                                 int64_t ld, int* __restrict__ erow) {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ld) return;
-    const unsigned long long* Xb = reinterpret_cast<const unsigned long long*>(X);
-    unsigned long long m = 0;
+    unsigned m = 0;
     int l = 0;
     for (; l + 8 <= nao; l += 8) {
-        unsigned long long b[8];
+        double b[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) b[u] = __ldg(Xb + (int64_t)(l + u) * ld + g);
+        for (int u = 0; u < 8; ++u) b[u] = __ldg(X + (int64_t)(l + u) * ld + g);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const unsigned long long a = b[u] & 0x7fffffffffffffffull;
-            m = a > m ? a : m;
-        }
+        for (int u = 0; u < 8; ++u) m = max(m, abs_hi(b[u]));
     }
-    for (; l < nao; ++l) {
-        const unsigned long long a = __ldg(Xb + (int64_t)l * ld + g) & 0x7fffffffffffffffull;
-        m = a > m ? a : m;
-    }
-    erow[g] = exp_of_bits(m);
+    for (; l < nao; ++l) m = max(m, abs_hi(__ldg(X + (int64_t)l * ld + g)));
+    erow[g] = exp_of_hi(m);
 }
 
 // slices of X: one thread per (row l, two points); bf16 pairs per store
@@ -94,13 +88,11 @@ __global__ void f_slice_x_kernel(const double* __restrict__ X, int nao, int np,
     double2 x = make_double2(0.0, 0.0);
     if (l < nao) x = *reinterpret_cast<const double2*>(X + (int64_t)l * ld + g);
     const int2 e = *reinterpret_cast<const int2*>(erow + g);
-    float d0[S], d1[S];
-    digits<B_, S>(x.x, e.x, d0);
-    digits<B_, S>(x.y, e.y, d1);
+    const unsigned long long q0 = biased_q<B_, S>(x.x, e.x), q1 = biased_q<B_, S>(x.y, e.y);
 #pragma unroll
     for (int i = 0; i < S; ++i)
-        *reinterpret_cast<__nv_bfloat162*>(A + ((int64_t)i * np + l) * ld + g) =
-            __floats2bfloat162_rn(d0[i], d1[i]);
+        *reinterpret_cast<unsigned*>(A + ((int64_t)i * np + l) * ld + g) =
+            digit_pair<B_, S>(q0, q1, i);
 }
 
 template<int B_, int S>
@@ -109,14 +101,10 @@ __global__ void f_slice_qd_kernel(const double* __restrict__ QD, int nao, int np
                                   __nv_bfloat16* __restrict__ B) {
     // one block per column mu of B = Q^T, i.e. QD(:, mu)
     const int mu = blockIdx.x;
-    __shared__ unsigned long long red[256];
-    unsigned long long m = 0;
-    for (int l = threadIdx.x; l < nao; l += blockDim.x) {
-        const unsigned long long b =
-            (unsigned long long)__double_as_longlong(QD[(int64_t)l * nao + mu]) &
-            0x7fffffffffffffffull;
-        m = b > m ? b : m;
-    }
+    __shared__ unsigned red[256];
+    unsigned m = 0;
+    for (int l = threadIdx.x; l < nao; l += blockDim.x)
+        m = max(m, abs_hi(QD[(int64_t)l * nao + mu]));
     red[threadIdx.x] = m;
     __syncthreads();
     for (int s = blockDim.x / 2; s > 0; s >>= 1) {
@@ -124,16 +112,16 @@ __global__ void f_slice_qd_kernel(const double* __restrict__ QD, int nao, int np
             red[threadIdx.x] = red[threadIdx.x + s];
         __syncthreads();
     }
-    const int e = exp_of_bits(red[0]);
+    const int e = exp_of_hi(red[0]);
     if (threadIdx.x == 0) ecol[mu] = e;
     const int64_t ldb = (int64_t)S * np;
     for (int l = threadIdx.x; l < np; l += blockDim.x) {
-        float d[S];
-        digits<B_, S>(l < nao ? QD[(int64_t)l * nao + mu] : 0.0, e, d);
+        const unsigned long long q =
+            biased_q<B_, S>(l < nao ? QD[(int64_t)l * nao + mu] : 0.0, e);
 #pragma unroll
         for (int i = 0; i < S; ++i)
             B[(int64_t)mu * ldb + (int64_t)(S - 1 - i) * np + l] =
-                __float2bfloat16_rn(d[i]);
+                __ushort_as_bfloat16((unsigned short)digit_pair<B_, S>(q, q, i));
     }
 }
 
@@ -181,7 +169,10 @@ __global__ void f_combine_kernel(const float* __restrict__ C, int nao,
 //   B: column nu = [slice S-1 | ... | slice 0]          (descending)
 // chunk stride S KC np (np = nao rounded up to 8, the columns past nao zero:
 // 16-byte rows and outputs, as for F).  One CTA of KC / 8 threads per (chunk,
-// column).
+// column).  Bound by HBM (X, G and the slices once each, 36 bytes per entry of
+// both operands): on the FP64 pipe only the product with the weight.  27 waters
+// (648 AOs, 384,998 points, two G): 3.8 -> 2.4 ms; 1.2 of them had been spent on
+// |x| and G -> FP64 as FP64 instructions.
 // ---------------------------------------------------------------------------
 // gridDim.z right-hand sides: B holds nb columns per chunk, those of right-hand
 // side r at r np (np = gridDim.y).  The CTAs of the first one also slice X,
@@ -204,11 +195,11 @@ k_slice_kernel(const double* __restrict__ X, const __grid_constant__ KIn<GT> Gs,
     const bool dox = slice_x && blockIdx.z == 0;
     const GT* __restrict__ G = Gs.g[blockIdx.z];
     const int64_t nlive = col < nao ? npts : 0;     // a column past nao is zero
-    __shared__ unsigned long long rx[T / 32], rw[T / 32];
+    __shared__ unsigned rx[T / 32], rw[T / 32];
     const int k0 = 8 * threadIdx.x;
     const int64_t g0 = (int64_t)c * KC + k0;
     double xv[8], wv[8];
-    unsigned long long mx = 0, mw = 0;
+    unsigned mx = 0, mw = 0;
     if (g0 + 8 <= nlive) {
         const double2* xp = reinterpret_cast<const double2*>(X + (int64_t)col * ld + g0);
         const double2* wp = reinterpret_cast<const double2*>(w + g0);
@@ -216,8 +207,10 @@ k_slice_kernel(const double* __restrict__ X, const __grid_constant__ KIn<GT> Gs,
         if constexpr (sizeof(GT) == 4) {
             const float4* gp = reinterpret_cast<const float4*>(G + (int64_t)col * ld + g0);
             const float4 ga = __ldg(gp), gb = __ldg(gp + 1);
-            gv[0] = ga.x; gv[1] = ga.y; gv[2] = ga.z; gv[3] = ga.w;
-            gv[4] = gb.x; gv[5] = gb.y; gv[6] = gb.z; gv[7] = gb.w;
+            gv[0] = to_f64(ga.x); gv[1] = to_f64(ga.y);
+            gv[2] = to_f64(ga.z); gv[3] = to_f64(ga.w);
+            gv[4] = to_f64(gb.x); gv[5] = to_f64(gb.y);
+            gv[6] = to_f64(gb.z); gv[7] = to_f64(gb.w);
         } else {
             const double2* gp = reinterpret_cast<const double2*>(G + (int64_t)col * ld + g0);
 #pragma unroll
@@ -253,19 +246,11 @@ k_slice_kernel(const double* __restrict__ X, const __grid_constant__ KIn<GT> Gs,
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-        const unsigned long long bx =
-            (unsigned long long)__double_as_longlong(xv[u]) & 0x7fffffffffffffffull;
-        const unsigned long long bw =
-            (unsigned long long)__double_as_longlong(wv[u]) & 0x7fffffffffffffffull;
-        mx = bx > mx ? bx : mx;
-        mw = bw > mw ? bw : mw;
+        mx = max(mx, abs_hi(xv[u]));
+        mw = max(mw, abs_hi(wv[u]));
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long ox = __shfl_xor_sync(0xffffffffu, mx, o);
-        const unsigned long long ow = __shfl_xor_sync(0xffffffffu, mw, o);
-        mx = ox > mx ? ox : mx;
-        mw = ow > mw ? ow : mw;
-    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    mw = __reduce_max_sync(0xffffffffu, mw);
     const int warp = threadIdx.x >> 5;
     if ((threadIdx.x & 31) == 0) { rx[warp] = mx; rw[warp] = mw; }
     __syncthreads();
@@ -273,10 +258,10 @@ k_slice_kernel(const double* __restrict__ X, const __grid_constant__ KIn<GT> Gs,
     mw = 0;
 #pragma unroll
     for (int j = 0; j < T / 32; ++j) {
-        mx = rx[j] > mx ? rx[j] : mx;
-        mw = rw[j] > mw ? rw[j] : mw;
+        mx = max(mx, rx[j]);
+        mw = max(mw, rw[j]);
     }
-    const int e1 = exp_of_bits(mx), e2 = exp_of_bits(mw);
+    const int e1 = exp_of_hi(mx), e2 = exp_of_hi(mw);
     if (threadIdx.x == 0) {
         if (dox) ex[(int64_t)c * np + col] = e1;
         ew[(int64_t)c * nb + boff + col] = e2;
@@ -286,18 +271,14 @@ k_slice_kernel(const double* __restrict__ X, const __grid_constant__ KIn<GT> Gs,
     // one operand's digits at a time: the X slices, then the w o G ones
     // (half the live registers of both at once)
     auto store = [&](const double* v, const int e, __nv_bfloat16* dst, const bool desc) {
-        float d[8][S];
+        unsigned long long q[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) digits<B_, S>(v[u], e, d[u]);
+        for (int u = 0; u < 8; ++u) q[u] = biased_q<B_, S>(v[u], e);
 #pragma unroll
-        for (int i = 0; i < S; ++i) {
-            __nv_bfloat162 p[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                p[u] = __floats2bfloat162_rn(d[2 * u][i], d[2 * u + 1][i]);
+        for (int i = 0; i < S; ++i)
             *reinterpret_cast<uint4*>(dst + (int64_t)(desc ? S - 1 - i : i) * KC + k0) =
-                *reinterpret_cast<const uint4*>(p);
-        }
+                make_uint4(digit_pair<B_, S>(q[0], q[1], i), digit_pair<B_, S>(q[2], q[3], i),
+                           digit_pair<B_, S>(q[4], q[5], i), digit_pair<B_, S>(q[6], q[7], i));
     };
     if (dox) store(xv, e1, A + colbase, false);
     store(wv, e2, B + colbase_b, true);

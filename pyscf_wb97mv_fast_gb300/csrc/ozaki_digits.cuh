@@ -2,6 +2,7 @@
 // fixed-point conversion of FP64 values to balanced base-2^B digits, and
 // the exact int64 combination of FP32 level sums back to FP32 / FP64.
 #pragma once
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -13,10 +14,7 @@ namespace wb {
 // Fixed-point digits.  A value x with |x| < 2^e becomes the integer
 // q = rint(x 2^(W - 1 - e)), W = B S bits, |q| < 2^(W-1), written as
 // balanced base-2^B digits q = sum_i d_i 2^(B (S-1-i)), |d_i| <= 2^(B-1) (S =
-// 7 digits of B = 6 bits, or 6 of 7),
-// extracted from the least significant end with integer arithmetic only
-// (the one FP64 multiply by an exact power of two and one FP64 -> int64
-// conversion per element are the only FP64 operations).
+// 7 digits of B = 6 bits, or 6 of 7), with integer arithmetic only.
 constexpr int kW = kOzWidth;
 
 __device__ __forceinline__ double pow2(int k) {
@@ -24,15 +22,20 @@ __device__ __forceinline__ double pow2(int k) {
     return __longlong_as_double((long long)(1023 + k) << 52);
 }
 
-__device__ __forceinline__ int exp_of_bits(unsigned long long absbits) {
-    // smallest e with |x| < 2^e from the bit pattern of |x|, clamped to
+// the high word of |x|: it orders magnitudes as far as their exponents go.
+// (The compiler takes a mask of the whole bit pattern for a floating-point
+// absolute value and issues it to the FP64 pipe.)
+__device__ __forceinline__ unsigned abs_hi(const double x) {
+    return (unsigned)__double2hiint(x) & 0x7fffffffu;
+}
+
+__device__ __forceinline__ int exp_of_hi(const unsigned hi) {
+    // smallest e with |x| < 2^e from the high word of |x|, clamped to
     // [-400, 500]: rows whose largest entry is below 2^-400 are zero at this
     // precision, and the clamp keeps every scale factor 2^k of the kernels
     // (|k| <= 2 * 500 + 84) inside the normal FP64 range of pow2()
-    const int ebits = (int)(absbits >> 52);
-    int e = ebits - 1022;                           // |x| < 2^(ebits-1023+1)
-    if (absbits == 0ull || e < -400) e = -400;
-    return e > 500 ? 500 : e;
+    const int e = (int)(hi >> 20) - 1022;           // |x| < 2^(ebits-1023+1)
+    return e < -400 ? -400 : (e > 500 ? 500 : e);
 }
 
 // q = rint(x 2^(W-1-e)) from the bit pattern of x with integer arithmetic:
@@ -62,30 +65,49 @@ __device__ __forceinline__ long long fixed_q(double x, int e) {
     return (b >> 63) ? -(long long)q : (long long)q;
 }
 
+// fixed_q(x, e) + H sum_i 2^(B i), H = 2^(B-1): with every digit biased by H,
+// digit i is the bit field i of the sum, no carries to follow.  The same
+// integer as fixed_q with fewer instructions: |x| < 2^e leaves at least 12 bits
+// to drop, so the shift goes one way and what it drops decides the rounding.
 template<int B, int S>
-__device__ __forceinline__ void digits(double x, int e, float* d) {
-    // q (|q| < 2^(W-1) = 2^41) split as q = hi 2^(B P) + lo, lo of P digits:
-    // the low digits come from lo, the carry goes into hi, the rest from hi --
-    // 32-bit integer arithmetic throughout
+__device__ __forceinline__ unsigned long long biased_q(const double x, const int e) {
     static_assert(S * B == kW && (B == 6 || B == 7), "42 bits in 6- or 7-bit digits");
-    constexpr int P = B == 6 ? 4 : 3, H = 1 << (B - 1), M = (1 << B) - 1;
-    const long long q = fixed_q(x, e);
-    int lo = (int)(q & ((1 << (B * P)) - 1));
-    int hi = (int)(q >> (B * P));
+    unsigned long long bias = 0;
 #pragma unroll
-    for (int i = S - 1; i >= S - P; --i) {
-        const int di = ((lo + H) & M) - H;
-        d[i] = (float)di;
-        lo = (lo - di) >> B;
+    for (int i = 0; i < S; ++i) bias |= 1ull << (B * i + B - 1);
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    // x = +-m 2^-10 2^(E - 1075), m the significand 10 bits up; q = m >> k
+    const int k = 1086 - kW + e - (int)((hi >> 20) & 0x7ffu);
+    unsigned long long q = 0;
+    if (k < 22) {                           // beyond the clamp of exp_of_hi
+        return bias + (unsigned long long)fixed_q(x, e);
+    } else if (k < 64) {
+        const unsigned long long m =
+            ((unsigned long long)(((hi & 0xfffffu) | 0x100000u) << 10 | lo >> 22) << 32) |
+            (unsigned long long)(lo << 10);
+        q = m >> k;
+        const unsigned long long rem = m << (64 - k);
+        const unsigned rh = (unsigned)(rem >> 32);
+        const unsigned sticky = (rh << 1) | (unsigned)rem | ((unsigned)q & 1u);
+        if ((int)rh < 0 && sticky) ++q;
     }
-    hi += lo;
-#pragma unroll
-    for (int i = S - P - 1; i >= 1; --i) {
-        const int di = ((hi + H) & M) - H;
-        d[i] = (float)di;
-        hi = (hi - di) >> B;
-    }
-    d[0] = (float)hi;
+    return (int)hi < 0 ? bias - q : bias + q;
+}
+
+// digit i (0 the most significant) of two biased integers, as a pair of bf16:
+// 128 + field is the bit pattern 0x4300 + field, and subtracting 128 + H from
+// it is exact
+template<int B, int S>
+__device__ __forceinline__ unsigned digit_pair(const unsigned long long a,
+                                               const unsigned long long b, const int i) {
+    constexpr unsigned H = 1u << (B - 1), M = ((1u << B) - 1u) * 0x10001u;
+    const int sh = B * (S - 1 - i);
+    unsigned t = __byte_perm((unsigned)(a >> sh), (unsigned)(b >> sh), 0x5410);
+    t = i ? (t & M) | 0x43004300u : t + 0x43004300u;    // the first goes up to 2^B
+    const unsigned h = (0x4300u + H) * 0x10001u;
+    const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&t),
+                                     *reinterpret_cast<const __nv_bfloat162*>(&h));
+    return *reinterpret_cast<const unsigned*>(&d);
 }
 
 // RN(v 2^sc) as FP32 from the int64 v with integer arithmetic (one

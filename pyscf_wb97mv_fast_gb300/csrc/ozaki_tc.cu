@@ -81,14 +81,13 @@ f_slice_x_km_kernel(const double* __restrict__ X, int nao, int64_t ld,
         const int64_t g = g0 + gg;
         if (g >= ld) break;
         const int e = erow[g];
-        float d0[S], d1[S];
-        digits<B_, S>(xs[2 * lp][gg], e, d0);
-        digits<B_, S>(xs[2 * lp + 1][gg], e, d1);
+        const unsigned long long q0 = biased_q<B_, S>(xs[2 * lp][gg], e);
+        const unsigned long long q1 = biased_q<B_, S>(xs[2 * lp + 1][gg], e);
         __nv_bfloat16* row = A + g * (int64_t)S * kp;
 #pragma unroll
         for (int i = 0; i < S; ++i)
-            *reinterpret_cast<__nv_bfloat162*>(row + (int64_t)i * kp + l) =
-                __floats2bfloat162_rn(d0[i], d1[i]);
+            *reinterpret_cast<unsigned*>(row + (int64_t)i * kp + l) =
+                digit_pair<B_, S>(q0, q1, i);
     }
 }
 
@@ -99,14 +98,10 @@ f_slice_qd_km_kernel(const double* __restrict__ QD, int nao, int* __restrict__ e
                      __nv_bfloat16* __restrict__ B) {
     const int mu = blockIdx.x;
     const int kp = pad8(nao);
-    __shared__ unsigned long long red[256];
-    unsigned long long m = 0;
-    for (int l = threadIdx.x; l < nao; l += blockDim.x) {
-        const unsigned long long b =
-            (unsigned long long)__double_as_longlong(QD[(int64_t)l * nao + mu]) &
-            0x7fffffffffffffffull;
-        m = b > m ? b : m;
-    }
+    __shared__ unsigned red[256];
+    unsigned m = 0;
+    for (int l = threadIdx.x; l < nao; l += blockDim.x)
+        m = max(m, abs_hi(QD[(int64_t)l * nao + mu]));
     red[threadIdx.x] = m;
     __syncthreads();
     for (int s = blockDim.x / 2; s > 0; s >>= 1) {
@@ -114,19 +109,16 @@ f_slice_qd_km_kernel(const double* __restrict__ QD, int nao, int* __restrict__ e
             red[threadIdx.x] = red[threadIdx.x + s];
         __syncthreads();
     }
-    const int e = exp_of_bits(red[0]);
+    const int e = exp_of_hi(red[0]);
     if (threadIdx.x == 0) ecol[mu] = e;
     __nv_bfloat16* row = B + (int64_t)mu * S * kp;
     for (int l = threadIdx.x; l < kp; l += blockDim.x) {
-        float d[S];
-        if (l < nao) {
-            digits<B_, S>(QD[(int64_t)l * nao + mu], e, d);
-        } else {
+        const unsigned long long q =
+            biased_q<B_, S>(l < nao ? QD[(int64_t)l * nao + mu] : 0.0, e);
 #pragma unroll
-            for (int i = 0; i < S; ++i) d[i] = 0.0f;
-        }
-#pragma unroll
-        for (int i = 0; i < S; ++i) row[(int64_t)i * kp + l] = __float2bfloat16_rn(d[i]);
+        for (int i = 0; i < S; ++i)
+            row[(int64_t)i * kp + l] =
+                __ushort_as_bfloat16((unsigned short)digit_pair<B_, S>(q, q, i));
     }
 }
 
