@@ -501,6 +501,24 @@ int block_order_update(wb_cosx* h, const wb::CosxArgs& a, const bool* ran,
     return WB_OK;
 }
 
+// One class launch of want CTAs (four items each), at most cap at a time.  A
+// block's two items are serial chains over half the pairs of the class: where
+// all of them as half blocks fit the device at once (16 warps an SM), the light
+// classes run two warps a block.  Twice the warps hide more latency there;
+// beyond, the overhead that two points a lane share counts for more.  K of 4
+// waters (19,325 points, 1.0 CTA an SM) 928 -> 676 us, 8 (36,479) 2.98 -> 2.56
+// ms, C6H14 in TZVP (30,268) 6.37 -> 5.74; past the line 14 waters (61,580)
+// 7.8 -> 8.2 ms, 17 (74,184) 11.1 -> 12.2.
+cudaError_t launch_class(const wb_cosx* h, int c, const wb::CosxArgs& a,
+                         const wb::ClassRange& r, int want, int cap, cudaStream_t s, bool far,
+                         size_t smem, bool dual) {
+    if (2 * want <= 4 * h->nsm && wb::cosx_class_halves(c, smem, dual))
+        return wb::launch_cosx_class_half(c, a, r.pair_begin, r.pair_end, 2 * want, s, far,
+                                          smem, dual);
+    return wb::launch_cosx_class_range(c, a, r.pair_begin, r.pair_end,
+                                       std::max(1, std::min(want, cap)), s, far, smem, dual);
+}
+
 // the class launches of one tile (after tile_prep and prepare_omega); F and
 // G are (nao, ldt) AO-major.  The classes fill their own partial-G buffers
 // concurrently; G is their fixed-order sum.
@@ -527,11 +545,9 @@ int run_g_classes(wb_cosx* h, int64_t npts_t, int64_t ldt, const float* F,
         const int lvl = h->pts[c] == 4 ? 2 : h->pts[c] - 1;
         const int want = ((WB_COSX_SPLIT ? 2 : 1) * a.nblk[lvl] + 3) / 4;
         const int cap = std::max(1, h->blocks_per_sm[c][far ? 1 : 0]) * h->nsm;
-        const int grid = std::max(1, std::min(want, cap));
         WB_CUDA(cudaStreamWaitEvent(h->cstream[c], h->fork, 0));
-        WB_CUDA(wb::launch_cosx_class_range(c, a, r.pair_begin, r.pair_end,
-                                            grid, h->cstream[c], far,
-                                            h->stage_smem[c]));
+        WB_CUDA(launch_class(h, c, a, r, want, cap, h->cstream[c], far, h->stage_smem[c],
+                             false));
         WB_CUDA(cudaEventRecord(h->cdone[c], h->cstream[c]));
         WB_CUDA(cudaStreamWaitEvent(s, h->cdone[c], 0));
         ran[c] = true;
@@ -587,21 +603,16 @@ int run_g_classes_dual(wb_cosx* h, int64_t npts_t, int64_t ldt, const float* F,
         WB_CUDA(cudaStreamWaitEvent(h->cstream[c], h->fork, 0));
         if (h->dual_cls[c]) {
             const int cap = std::max(1, h->blocks_per_sm2[c]) * h->nsm;
-            WB_CUDA(wb::launch_cosx_class_range(c, a, r.pair_begin, r.pair_end,
-                                                std::max(1, std::min(want, cap)),
-                                                h->cstream[c], false,
-                                                h->stage_smem2[c], true));
+            WB_CUDA(launch_class(h, c, a, r, want, cap, h->cstream[c], false,
+                                 h->stage_smem2[c], true));
             *launches += 1;
         } else {
             const double om[2] = {omega_a, omega_b};
             for (int w = 0; w < 2; ++w) {
                 const bool far = om[w] == 0.0;
                 const int cap = std::max(1, h->blocks_per_sm[c][far ? 1 : 0]) * h->nsm;
-                WB_CUDA(wb::launch_cosx_class_range(c, w ? b : a, r.pair_begin,
-                                                    r.pair_end,
-                                                    std::max(1, std::min(want, cap)),
-                                                    h->cstream[c], far,
-                                                    h->stage_smem[c]));
+                WB_CUDA(launch_class(h, c, w ? b : a, r, want, cap, h->cstream[c], far,
+                                     h->stage_smem[c], false));
                 *launches += 1;
             }
         }

@@ -215,15 +215,21 @@ template<int LA, int LB, int NW = 1> struct ClassPts {
                                          : class_pts(LA * (LA + 1) / 2 + LB);
 };
 
+// Half blocks (HALF, the light classes on small grids): a block of two points
+// per lane is worked on by two warps of one point per lane each.  The screen
+// keeps the whole block's centroid and maxima, so each point sees the same
+// tasks in the same order and G is bitwise the same.
+//
 // One block (32 * PTS points) of one class kernel: every pair of the class
-// (screen, tasks, G) for the points of block blk.  A is the argument block
+// (screen, tasks, G) for the points of block blk (with HALF, those of its half
+// sub).  A is the argument block
 // of the block's molecule; wstage / rmax the warp's record buffers (two of
 // rmax float4) and sbuf the one in use; kept / flops / ints accumulate the
 // counters of the warp (with the TMA form, stg holds the buffers' copy
 // state).
-template<int LA, int LB, bool FAR, bool STAGE, int NW>
+template<int LA, int LB, bool FAR, bool STAGE, int NW, bool HALF = false>
 __device__ __forceinline__ void cosx_class_block(
-    const CosxArgs& A, const int pair_begin, const int pair_end, const int blk,
+    const CosxArgs& A, const int pair_begin, const int pair_end, const int blk, const int sub,
     const float4* __restrict__ stab, float4* wstage, const int rmax, int& sbuf,
     unsigned long long& kept, unsigned long long& flops,
     unsigned long long& ints WB_STAGER_PARAM WB_SPLIT_PARAM) {
@@ -231,7 +237,10 @@ __device__ __forceinline__ void cosx_class_block(
     constexpr int NCA = (LA + 1) * (LA + 2) / 2;
     constexpr int NA = 2 * LA + 1;
     constexpr int NB = 2 * LB + 1;
-    constexpr int PTS = ClassPts<LA, LB, NW>::value;
+    constexpr int BP = ClassPts<LA, LB, NW>::value;     // the block's points / 32
+    constexpr int PTS = HALF ? 1 : BP;
+    static_assert(!HALF || BP == 2, "half blocks are of two points per lane");
+    const int p0 = 32 * (blk * BP + (HALF ? sub : 0));  // the warp's first point
     const int lane = threadIdx.x & 31;
     constexpr int RS = NW == 2 ? kRecStride2[CLS] : kRecStride[CLS];
     const float4* __restrict__ recc = NW == 2 ? A.rec2[CLS] : A.rec[CLS];
@@ -246,11 +255,11 @@ __device__ __forceinline__ void cosx_class_block(
     const float tol = A.tol;
     const float4* __restrict__ bnd = A.bnd + A.pp_begin[CLS];
     const float* __restrict__ bpref = A.bpref + A.pp_begin[CLS];
-    constexpr int LVL = PTS == 4 ? 2 : PTS - 1;
+    constexpr int LVL = BP == 4 ? 2 : BP - 1;
     const float4* __restrict__ blk_cr = A.blk_cr[LVL];
     const float* __restrict__ blk_msh = A.blk_msh[LVL];
     unsigned long long bfl = 0;     // model flops kept in this block
-    // the lane's points: blk * 32 PTS + 32 p + lane (clamped to the
+    // the lane's points: p0 + 32 p + lane (clamped to the
     // arrays; ok marks the ones that exist)
     const float* __restrict__ Fp[PTS];
     float* Gp[NW * PTS];
@@ -258,7 +267,7 @@ __device__ __forceinline__ void cosx_class_block(
     float gxh[PTS], gyh[PTS], gzh[PTS], gxl[PTS], gyl[PTS], gzl[PTS];
 #pragma unroll
     for (int p = 0; p < PTS; ++p) {
-        const int g0 = blk * (32 * PTS) + 32 * p + lane;
+        const int g0 = p0 + 32 * p + lane;
         ok[p] = g0 < ld;
         const int g = ok[p] ? g0 : ld - 1;
         Fp[p] = A.F + g;
@@ -284,7 +293,7 @@ __device__ __forceinline__ void cosx_class_block(
         }
     }
     const float* __restrict__ ms = blk_msh + (long long)blk * A.nvshell;
-    const int rem = A.npts - blk * 32 * PTS;
+    const int rem = A.npts - p0;
     const int nvalid = rem < 32 * PTS ? (rem > 0 ? rem : 0) : 32 * PTS;
     const int nsb = (nvalid + 31) / 32;     // 32-point sub-blocks covered
     // run state: the current bra shell (packed header word), its class
@@ -486,19 +495,20 @@ __device__ __forceinline__ void cosx_class_block(
     }
     for (int o = 16; o > 0; o >>= 1) bfl += __shfl_xor_sync(0xffffffffu, bfl, o);
 #if WB_COSX_SPLIT
-    if (lane == 0 && A.bcost[CLS]) A.bcost[CLS][citem] = (float)bfl;
+    // (a half block's cost stands for both)
+    if (lane == 0 && A.bcost[CLS] && (!HALF || sub == 0)) A.bcost[CLS][citem] = (float)bfl;
 #else
-    if (lane == 0 && A.bcost[CLS]) A.bcost[CLS][blk] = (float)bfl;
+    if (lane == 0 && A.bcost[CLS] && (!HALF || sub == 0)) A.bcost[CLS][blk] = (float)bfl;
 #endif
 }
 
-template<int LA, int LB, bool FAR, bool STAGE, int NW>
+template<int LA, int LB, bool FAR, bool STAGE, int NW, bool HALF = false>
 __global__ void __launch_bounds__(kCtaThreads,
                                   min_blocks(LA * (LA + 1) / 2 + LB, NW))
 cosx_class_kernel(const CosxArgs A, const int pair_begin, const int pair_end) {
     static_assert(NW == 1 || (NW == 2 && STAGE), "dual-omega needs staging");
     constexpr int CLS = LA * (LA + 1) / 2 + LB;
-    constexpr int PTS = ClassPts<LA, LB, NW>::value;
+    constexpr int BP = ClassPts<LA, LB, NW>::value;
     __shared__ float4 stab[kBoysFloat4];
 #if WB_COSX_TMA
     RecStager stg = stager_init(threadIdx.x & 31);
@@ -512,18 +522,20 @@ cosx_class_kernel(const CosxArgs A, const int pair_begin, const int pair_end) {
     const int rmax = NW == 2 ? A.recmax2[CLS] : A.recmax[CLS];
     float4* wstage = s_stage + (threadIdx.x >> 5) * 2 * rmax;
     int sbuf = 0;
-    constexpr int LVL = PTS == 4 ? 2 : PTS - 1;
+    constexpr int LVL = BP == 4 ? 2 : BP - 1;
     const int nblk = A.nblk[LVL];
     unsigned long long kept = 0, flops = 0, ints = 0;
     const int* __restrict__ order = A.border[CLS];
 #if WB_COSX_SPLIT
-    // items 2 blk + h: half h of block blk
+    // items 2 blk + h: half h of block blk's pairs (with HALF, two warps each)
     const int nitem = 2 * nblk;
     const int split = A.cls_split[CLS];
     for (;;) {
         int item = 0;
         if (lane == 0) item = atomicAdd(A.work + CLS, 1);
         item = __shfl_sync(0xffffffffu, item, 0);
+        const int sub = HALF ? item & 1 : 0;
+        if constexpr (HALF) item >>= 1;
         if (item >= nitem) break;
         int it = item;
         if (order) {
@@ -531,16 +543,18 @@ cosx_class_kernel(const CosxArgs A, const int pair_begin, const int pair_end) {
             it = b >= 0 && b < nitem ? b : item;
         }
         const int blk = it >> 1, h = it & 1;
-        cosx_class_block<LA, LB, FAR, STAGE, NW>(A, h ? split : pair_begin,
-                                                 h ? pair_end : split, blk, stab,
-                                                 wstage, rmax, sbuf, kept, flops,
-                                                 ints WB_STAGER_ARG, h, it);
+        cosx_class_block<LA, LB, FAR, STAGE, NW, HALF>(A, h ? split : pair_begin,
+                                                       h ? pair_end : split, blk, sub, stab,
+                                                       wstage, rmax, sbuf, kept, flops,
+                                                       ints WB_STAGER_ARG, h, it);
     }
 #else
     for (;;) {
         int item = 0;
         if (lane == 0) item = atomicAdd(A.work + CLS, 1);
         item = __shfl_sync(0xffffffffu, item, 0);
+        const int sub = HALF ? item & 1 : 0;
+        if constexpr (HALF) item >>= 1;
         if (item >= nblk) break;
         // costliest blocks first (the order is a permutation of 0 .. nblk-1)
         int blk = item;
@@ -548,9 +562,9 @@ cosx_class_kernel(const CosxArgs A, const int pair_begin, const int pair_end) {
             const int b = order[item];
             blk = b >= 0 && b < nblk ? b : item;
         }
-        cosx_class_block<LA, LB, FAR, STAGE, NW>(A, pair_begin, pair_end, blk, stab,
-                                                 wstage, rmax, sbuf, kept, flops,
-                                                 ints WB_STAGER_ARG);
+        cosx_class_block<LA, LB, FAR, STAGE, NW, HALF>(A, pair_begin, pair_end, blk, sub,
+                                                       stab, wstage, rmax, sbuf, kept,
+                                                       flops, ints WB_STAGER_ARG);
     }
 #endif
     // lane 0 counted the tasks (every lane runs every task) in units of the
@@ -661,13 +675,13 @@ cosx_class_kernel_batch(const CosxArgs* __restrict__ args,
             const int split = Am.cls_split[CLS];
             cosx_class_block<LA, LB, FAR, STAGE, NW>(Am, h ? split : Am.cls_pb[CLS],
                                                      h ? Am.cls_pe[CLS] : split,
-                                                     it >> 1, stab, wstage, rmax, sbuf,
+                                                     it >> 1, 0, stab, wstage, rmax, sbuf,
                                                      kept, flops, ints WB_STAGER_ARG,
                                                      h, it);
         }
 #else
         cosx_class_block<LA, LB, FAR, STAGE, NW>(Am, Am.cls_pb[CLS], Am.cls_pe[CLS],
-                                                 item - item_off[m], stab, wstage,
+                                                 item - item_off[m], 0, stab, wstage,
                                                  rmax, sbuf, kept, flops,
                                                  ints WB_STAGER_ARG);
 #endif

@@ -9,10 +9,10 @@ cudaError_t launch_cosx_f_class(int cls, const CosxArgs& a, int pb, int pe,
                                 bool dual);
 int cosx_f_class_blocks_per_sm(int cls, bool far, size_t smem, bool dual);
 
-template<int LA, int LB, bool FAR, bool STAGE, int NW = 1>
+template<int LA, int LB, bool FAR, bool STAGE, int NW = 1, bool HALF = false>
 static cudaError_t run1(const CosxArgs& a, int pb, int pe, int grid,
                         size_t smem, cudaStream_t s) {
-    auto k = cosx_class_kernel<LA, LB, FAR, STAGE, NW>;
+    auto k = cosx_class_kernel<LA, LB, FAR, STAGE, NW, HALF>;
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(
             k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -53,6 +53,34 @@ static int occ(bool far, size_t smem, bool dual) {
     if (smem)
         return far ? occ1<LA, LB, true, true>(smem) : occ1<LA, LB, false, true>(smem);
     return far ? occ1<LA, LB, true, false>(0) : occ1<LA, LB, false, false>(0);
+}
+
+// two warps per block (the caller has asked cosx_class_halves)
+template<int LA, int LB>
+static cudaError_t run_half(const CosxArgs& a, int pb, int pe, int grid,
+                            cudaStream_t s, bool far, size_t smem, bool dual) {
+    if constexpr (ClassPts<LA, LB, 2>::value == 2)
+        if (dual) return run1<LA, LB, false, true, 2, true>(a, pb, pe, grid, smem, s);
+    if constexpr (ClassPts<LA, LB>::value == 2)
+        if (!dual)
+            return far ? run1<LA, LB, true, true, 1, true>(a, pb, pe, grid, smem, s)
+                       : run1<LA, LB, false, true, 1, true>(a, pb, pe, grid, smem, s);
+    return cudaErrorInvalidValue;
+}
+
+bool cosx_class_halves(int cls, size_t smem, bool dual) {
+    return cls <= 3 && smem > 0 && cosx_class_pts(cls, dual) == 2;
+}
+
+cudaError_t launch_cosx_class_half(int cls, const CosxArgs& a, int pb, int pe, int grid,
+                                   cudaStream_t s, bool far, size_t smem, bool dual) {
+    switch (cls) {
+    case 0: return run_half<0, 0>(a, pb, pe, grid, s, far, smem, dual);
+    case 1: return run_half<1, 0>(a, pb, pe, grid, s, far, smem, dual);
+    case 2: return run_half<1, 1>(a, pb, pe, grid, s, far, smem, dual);
+    case 3: return run_half<2, 0>(a, pb, pe, grid, s, far, smem, dual);
+    default: return cudaErrorInvalidValue;
+    }
 }
 
 cudaError_t launch_cosx_class_range(int cls, const CosxArgs& a, int pb,

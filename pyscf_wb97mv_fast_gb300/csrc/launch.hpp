@@ -39,6 +39,11 @@ inline int64_t grid_stride_blocks(int64_t n, int threads, int ctas_per_sm) {
 cudaError_t launch_cosx_class_range(int cls, const CosxArgs& a, int pb,
                                     int pe, int grid, cudaStream_t s, bool far,
                                     size_t stage_smem, bool dual = false);
+// launch_cosx_class_range with two warps per block, where cosx_class_halves
+// (classes of two points per lane whose records are staged)
+bool cosx_class_halves(int cls, size_t smem, bool dual);
+cudaError_t launch_cosx_class_half(int cls, const CosxArgs& a, int pb, int pe, int grid,
+                                   cudaStream_t s, bool far, size_t smem, bool dual);
 // the batched form: one launch over the class's blocks of nmol molecules
 // (args: nmol device argument blocks; off: nmol + 1 item offsets; work: a
 // zeroed counter; rmax: the largest task record of the class over the
