@@ -1369,7 +1369,7 @@ int wb_cosx_get_k_multi(wb_cosx* h, const double* coords,
                 at<unsigned long long>(workspace, L.counters) + 3 * wb::NCLASS);
             if (r) return fail(r >= 1000 ? WB_ERR_CUBLAS : WB_ERR_CUDA,
                                "ozaki F GEMM failed, code " + std::to_string(r));
-            launches += wb::ozaki_f_launches(nao);
+            launches += wb::ozaki_f_launches(nao, ldt);
         } else {
             // F(g, mu) = sum_l X(g, l) QD(l, mu); QD row-major = col-major QD^T
             WB_CUBLAS(cublasDgemm(h->cublas, CUBLAS_OP_N, CUBLAS_OP_T, (int)ldt,
@@ -1888,7 +1888,7 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
                 at<unsigned long long>(ws, L.counters) + 3 * wb::NCLASS);
             if (r) return fail(r >= 1000 ? WB_ERR_CUBLAS : WB_ERR_CUDA,
                                "ozaki F GEMM failed, code " + std::to_string(r));
-            launches += wb::ozaki_f_launches(nao);
+            launches += wb::ozaki_f_launches(nao, ld);
         } else {
             double* F64 = static_cast<double*>(b->scratch);
             WB_CUBLAS(cublasDgemm(h->cublas, CUBLAS_OP_N, CUBLAS_OP_T, (int)ld, nao, nao,

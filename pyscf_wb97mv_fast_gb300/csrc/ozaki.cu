@@ -26,9 +26,10 @@
 // per-row / per-column maxima; the truncated products (i + j >= S) are
 // below 2^-W of them.
 //
-// The level GEMMs are library GEMMs by default (cuBLAS bf16 GEMMs with FP32
+// The level GEMMs are library GEMMs (cuBLAS bf16 GEMMs with FP32
 // accumulation, one per level) around this file's slicing and combination
-// kernels.  ozaki_set_f_engine(kOzEngineTc) runs the F product on this
+// kernels.  Small F products (ozaki_f_small), or all of them after
+// ozaki_set_f_engine(kOzEngineTc), run on this
 // library's own tensor-core kernel instead (ozaki_tc.cu: TMA, tcgen05 MMAs
 // into TMEM, the level combination fused into its epilogue) -- bitwise the
 // same result; its six or seven exact level accumulators leave room for 64-wide
@@ -405,16 +406,25 @@ void f_rowmax(const double* X, int nao, int64_t ld, int* erow, cudaStream_t s) {
 }
 
 namespace {
-std::atomic<int> g_f_engine{kOzEngineLibrary};
+std::atomic<int> g_f_engine{-1};                // none asked for
 }
 
 void ozaki_set_f_engine(int engine) { g_f_engine.store(engine); }
-int ozaki_get_f_engine() { return g_f_engine.load(); }
+int ozaki_get_f_engine() {
+    return g_f_engine.load() == kOzEngineTc ? kOzEngineTc : kOzEngineLibrary;
+}
+bool ozaki_f_small(int nao, int64_t ld) {
+    return nao <= 64 && (ld + 127) / 128 <= sm_count();
+}
+bool ozaki_f_on_tc(int nao, int64_t ld) {
+    const int e = g_f_engine.load();
+    return e == kOzEngineTc || (e < 0 && ozaki_f_small(nao, ld));
+}
 
 int ozaki_f_gemm(cublasHandle_t hb, const double* X, const double* QD,
                  int nao, int64_t ld, float* F, void* ws, cudaStream_t s,
                  unsigned long long* status) {
-    if (g_f_engine.load() == kOzEngineTc)
+    if (ozaki_f_on_tc(nao, ld))
         return ozaki_f_gemm_tc(X, QD, nao, ld, F, ws, s, status);
     return ozaki_f_gemm_cublas(hb, X, QD, nao, ld, F, ws, s);
 }
@@ -422,7 +432,7 @@ int ozaki_f_gemm(cublasHandle_t hb, const double* X, const double* QD,
 int ozaki_f_gemm64(cublasHandle_t hb, const double* X, const double* QD,
                    int nao, int64_t ld, double* F, void* ws, cudaStream_t s,
                    unsigned long long* status) {
-    if (g_f_engine.load() == kOzEngineTc)
+    if (ozaki_f_on_tc(nao, ld))
         return ozaki_f_gemm_tc64(X, QD, nao, ld, F, ws, s, status);
     return ozaki_f_gemm_cublas64(hb, X, QD, nao, ld, F, ws, s);
 }

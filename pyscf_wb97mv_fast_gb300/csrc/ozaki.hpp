@@ -44,14 +44,22 @@ int ozaki_k_gemm64(cublasHandle_t hb, const double* X, const double* G,
                    int accumulate, double* K, void* ws, cudaStream_t s);
 
 // the two engines of the F product (bitwise the same F): cuBLAS level
-// GEMMs (the default) and this library's tcgen05 kernel
+// GEMMs and this library's tcgen05 kernel; until one is asked for, the kernel
+// where ozaki_f_small, the GEMMs elsewhere
 constexpr int kOzEngineLibrary = 0;
 constexpr int kOzEngineTc = 1;
 void ozaki_set_f_engine(int engine);
-int ozaki_get_f_engine();
-// this library's kernel launches of one F product under the current engine
-inline int ozaki_f_launches(int nao) {
-    return ozaki_get_f_engine() == kOzEngineTc ? 4 : 4 + (ozaki_f_seven_bit(nao) ? 6 : 7);
+int ozaki_get_f_engine();               // kOzEngineLibrary until one is set
+// One column of tiles of the tensor-core kernel (64 AOs) in one wave of CTAs:
+// the level GEMMs are then shorter than the gaps between them.  An F product
+// as called: 48 AOs, 9,928 points 76 -> 42 us, 24 AOs, 5,012 points 78 -> 36;
+// past it the level GEMMs win (96 AOs, 19,325 points 78 us against 83; 192 AOs,
+// 36,475 points 178 against 257).
+bool ozaki_f_small(int nao, int64_t ld);
+bool ozaki_f_on_tc(int nao, int64_t ld);        // under the current engine
+// kernel launches of one F product under the current engine
+inline int ozaki_f_launches(int nao, int64_t ld) {
+    return ozaki_f_on_tc(nao, ld) ? 4 : 4 + (ozaki_f_seven_bit(nao) ? 6 : 7);
 }
 // the same of one K product
 int ozaki_k_launches(int nao, int64_t ld);
