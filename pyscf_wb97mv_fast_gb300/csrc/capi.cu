@@ -911,6 +911,10 @@ struct wb_cosx_batch {
     int* d_order = nullptr;             // NCLASS x stride: costliest first
     int64_t stride = 0;
     bool ordered = false;               // the orders hold a previous run's costs
+    // the class launches of a run, side by side
+    cudaStream_t cstream[wb::NCLASS] = {};
+    cudaEvent_t cdone[wb::NCLASS] = {};
+    cudaEvent_t fork = nullptr;
 };
 
 static int batch_fail(wb_cosx_batch* b, int code) {
@@ -1800,6 +1804,14 @@ int wb_cosx_batch_create(int nmol, wb_cosx* const* handles,
         e = cudaMemcpy(b->d_off, off.data(), sizeof(int) * off.size(),
                        cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return batch_fail(b, cuda_fail(e, "wb_cosx_batch_create"));
+    e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
+    for (int c = 0; c < wb::NCLASS && e == cudaSuccess; ++c) {
+        if (!b->has[c]) continue;
+        e = cudaStreamCreateWithFlags(&b->cstream[c], cudaStreamNonBlocking);
+        if (e == cudaSuccess)
+            e = cudaEventCreateWithFlags(&b->cdone[c], cudaEventDisableTiming);
+    }
+    if (e != cudaSuccess) return batch_fail(b, cuda_fail(e, "wb_cosx_batch_create"));
     // what stays fixed for the plan's life: AO values, grid coordinates
     // (hi / lo), the omega records of both slots
     for (int m = 0; m < nmol; ++m) {
@@ -1906,13 +1918,17 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
         launches += 1;
     }
     // every class: one launch over all molecules (two for the classes
-    // without a two-omega kernel)
+    // without a two-omega kernel), side by side on the batch's own streams so
+    // that the tail of one is filled by the others (clusters of 4 to 17 waters,
+    // coarse grids: 21.4 -> 20.7 ms a run, 26.4 -> 23.4 the first, unordered one)
     WB_CUDA(cudaMemsetAsync(b->d_work, 0, sizeof(int) * 2 * wb::NCLASS, s));
     launches += 1;
+    WB_CUDA(cudaEventRecord(b->fork, s));
     const wb_cosx* h0 = b->h[0];
     for (int i = 0; i < wb::NCLASS; ++i) {
         const int c = b->order[i];
         if (!b->has[c] || b->items[c] == 0) continue;
+        WB_CUDA(cudaStreamWaitEvent(b->cstream[c], b->fork, 0));
         const int want = (b->items[c] + 3) / 4;
         const int* off = b->d_off + (size_t)c * (nmol + 1);
         const int* order = b->ordered ? b->d_order + (size_t)c * b->stride : nullptr;
@@ -1920,8 +1936,8 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
             const int cap = std::max(1, h0->blocks_per_sm2[c]) * h0->nsm;
             WB_CUDA(wb::launch_cosx_class_batch(c, b->d_args, off, nmol,
                                                 b->d_work + 2 * c, b->rmax2[c], order,
-                                                std::max(1, std::min(want, cap)), s,
-                                                false, b->smem2[c], true));
+                                                std::max(1, std::min(want, cap)),
+                                                b->cstream[c], false, b->smem2[c], true));
             launches += 1;
         } else {
             for (int w = 0; w < b->nom; ++w) {
@@ -1929,11 +1945,13 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
                 const int cap = std::max(1, h0->blocks_per_sm[c][far ? 1 : 0]) * h0->nsm;
                 WB_CUDA(wb::launch_cosx_class_batch(
                     c, b->d_args + (size_t)w * nmol, off, nmol, b->d_work + 2 * c + w,
-                    b->rmax[c], order, std::max(1, std::min(want, cap)), s, far,
+                    b->rmax[c], order, std::max(1, std::min(want, cap)), b->cstream[c], far,
                     b->smem[c], false));
                 launches += 1;
             }
         }
+        WB_CUDA(cudaEventRecord(b->cdone[c], b->cstream[c]));
+        WB_CUDA(cudaStreamWaitEvent(s, b->cdone[c], 0));
     }
     {   // the next run takes each class's items costliest first
         wb::BlockOrderArgs P;
@@ -2016,6 +2034,11 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
 
 int wb_cosx_batch_destroy(wb_cosx_batch* b) {
     if (!b) return WB_OK;
+    for (int c = 0; c < wb::NCLASS; ++c) {
+        if (b->cstream[c]) cudaStreamDestroy(b->cstream[c]);
+        if (b->cdone[c]) cudaEventDestroy(b->cdone[c]);
+    }
+    if (b->fork) cudaEventDestroy(b->fork);
     if (b->block) cudaFree(b->block);
     delete b;
     return WB_OK;
