@@ -211,9 +211,10 @@ int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
  * while it lives), the omegas (1 or 2) and tile_tol.  wb_cosx_batch_create
  * evaluates the AO values, the grid coordinates and the omega records
  * once (on `stream`, synchronised before it returns).  The F / K split
- * scratch is one buffer shared by the molecules (they use it one after
- * another): each molecule's workspace needs wb_cosx_batch_workspace_bytes
- * bytes and the scratch the largest *scratch_bytes it reports.  Each
+ * scratch is one buffer shared by the molecules: each molecule's workspace
+ * needs wb_cosx_batch_workspace_bytes bytes and the scratch at least the
+ * largest *scratch_bytes it reports; molecules whose parts fit it together
+ * run their F and K products side by side, the others in turn.  Each
  * wb_cosx_batch_run takes one density per molecule (qd[m], (nao_m,
  * nao_m) row-major) and writes nomega unsymmetrised K matrices per
  * molecule to k_out[m], as wb_cosx_get_k_multi does (omega j at k_out[m]

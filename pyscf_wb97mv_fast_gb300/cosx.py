@@ -681,16 +681,26 @@ class KBuildGraph:
 
 
 def batch_workspace_bytes(engines, npts):
-    """Per-molecule workspace bytes of a CosxBatch and the bytes of its
-    shared scratch."""
+    """Per-molecule workspace bytes of a CosxBatch and the bytes its shared
+    scratch needs at least."""
+    ws, scr = _batch_bytes(engines, npts)
+    return ws, max(scr, default=0)
+
+
+def _batch_bytes(engines, npts):
     lib = _native.lib()
-    ws, scr = [], 0
+    ws, scr = [], []
     for e, n in zip(engines, npts):
         s = _native.ctypes.c_size_t(0)
         ws.append(int(lib.wb_cosx_batch_workspace_bytes(e._h, int(n),
                                                         _native.ctypes.byref(s))))
-        scr = max(scr, int(s.value))
+        scr.append(int(s.value))
     return ws, scr
+
+
+# scratch beyond the largest molecule's is taken up to this, so that small
+# molecules' products run side by side
+BATCH_SCRATCH_BYTES = 1 << 32
 
 
 class CosxBatch:
@@ -715,9 +725,15 @@ class CosxBatch:
         dev = self.engines[0].device
         P = _native.ctypes.c_void_p
         npts = [int(c.shape[0]) for c, _ in self._grids]
-        wsb, scr = batch_workspace_bytes(self.engines, npts)
+        wsb, scr = _batch_bytes(self.engines, npts)
         ws = [e.workspace(b) for e, b in zip(self.engines, wsb)]
-        self._scratch = torch.empty(max(scr, 1), dtype=torch.uint8, device=dev)
+        least = max(scr + [1])
+        try:
+            self._scratch = torch.empty(
+                max(least, min(sum(s + 256 for s in scr), BATCH_SCRATCH_BYTES)),
+                dtype=torch.uint8, device=dev)
+        except torch.cuda.OutOfMemoryError:
+            self._scratch = torch.empty(least, dtype=torch.uint8, device=dev)
         self._hold = ws
         handles = (P * n)(*[e._h.value for e in self.engines])
         coords = (P * n)(*[c.data_ptr() for c, _ in self._grids])

@@ -895,6 +895,7 @@ struct wb_cosx_batch {
     std::vector<void*> ws;
     std::vector<WsLayout> L;
     void* scratch = nullptr;            // the F / K split scratch, shared
+    size_t scratch_bytes = 0;
     bool has[wb::NCLASS] = {};          // some molecule has pairs of the class
     bool dual[wb::NCLASS] = {};         // the two-omega kernel, every molecule
     size_t smem[wb::NCLASS] = {};       // staged single-omega kernel (0: prefetch)
@@ -915,7 +916,51 @@ struct wb_cosx_batch {
     cudaStream_t cstream[wb::NCLASS] = {};
     cudaEvent_t cdone[wb::NCLASS] = {};
     cudaEvent_t fork = nullptr;
+    static constexpr int kLanes = 4;    // molecules side by side (batch_lanes)
+    cudaStream_t lane[kLanes] = {};
+    cudaEvent_t ldone[kLanes] = {};
 };
+
+// body(m, stream, scratch) for the molecules of a run, side by side on the
+// batch's lanes as far as their parts of the scratch fit it together: the F
+// and K products of a small molecule leave most of the device idle, and their
+// launches wait on one another.  With room for one at a time, or with one
+// molecule, in turn on the caller's stream.
+template<typename Body>
+static int batch_lanes(wb_cosx_batch* b, const double* const* qd, cudaStream_t s, Body body) {
+    auto bytes = [&](int m) { return align256(b->L[m].total - b->L[m].oz); };
+    char* const base = static_cast<char*>(b->scratch);
+    for (int m = 0; m < b->nmol;) {
+        int live = 0, end = m;
+        size_t used = 0;
+        for (; end < b->nmol; ++end) {
+            const size_t need = qd[end] ? bytes(end) : 0;
+            if (live && used + need > b->scratch_bytes) break;
+            used += need;
+            live += qd[end] != nullptr;
+        }
+        const bool side = live > 1;
+        if (side) WB_CUDA(cudaEventRecord(b->fork, s));
+        size_t off = 0;
+        int n = 0;
+        for (; m < end; ++m) {
+            cudaStream_t t = s;
+            if (side && qd[m]) {
+                const int q = n++ % wb_cosx_batch::kLanes;
+                t = b->lane[q];
+                if (n <= wb_cosx_batch::kLanes) WB_CUDA(cudaStreamWaitEvent(t, b->fork, 0));
+            }
+            const int st = body(m, t, base + off);
+            if (st != WB_OK) return st;
+            if (qd[m]) off += bytes(m);
+        }
+        for (int q = 0; q < std::min(n, wb_cosx_batch::kLanes); ++q) {
+            WB_CUDA(cudaEventRecord(b->ldone[q], b->lane[q]));
+            WB_CUDA(cudaStreamWaitEvent(s, b->ldone[q], 0));
+        }
+    }
+    return WB_OK;
+}
 
 static int batch_fail(wb_cosx_batch* b, int code) {
     wb_cosx_batch_destroy(b);
@@ -1681,6 +1726,7 @@ int wb_cosx_batch_create(int nmol, wb_cosx* const* handles,
     b->tol = tile_tol;
     b->gemm = flags & 3;
     b->scratch = scratch;
+    b->scratch_bytes = scratch_bytes;
     for (int m = 0; m < nmol; ++m) {
         wb_cosx* h = handles[m];
         if (!h || !coords[m] || !weights[m] || npts[m] < 1 || !workspaces[m])
@@ -1811,6 +1857,11 @@ int wb_cosx_batch_create(int nmol, wb_cosx* const* handles,
         if (e == cudaSuccess)
             e = cudaEventCreateWithFlags(&b->cdone[c], cudaEventDisableTiming);
     }
+    for (int q = 0; q < wb_cosx_batch::kLanes && nmol > 1 && e == cudaSuccess; ++q) {
+        e = cudaStreamCreateWithFlags(&b->lane[q], cudaStreamNonBlocking);
+        if (e == cudaSuccess)
+            e = cudaEventCreateWithFlags(&b->ldone[q], cudaEventDisableTiming);
+    }
     if (e != cudaSuccess) return batch_fail(b, cuda_fail(e, "wb_cosx_batch_create"));
     // what stays fixed for the plan's life: AO values, grid coordinates
     // (hi / lo), the omega records of both slots
@@ -1878,34 +1929,34 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
     int launches = 0;
     const double one = 1.0, zero = 0.0;
     // per molecule: F = fl32(X QD) and the block statistics
-    for (int m = 0; m < nmol; ++m) {
+    int st = batch_lanes(b, qd, s, [&](int m, cudaStream_t t, void* scratch) -> int {
         wb_cosx* h = b->h[m];
         const WsLayout& L = b->L[m];
         void* ws = b->ws[m];
         const int nao = h->hp.nao;
         const int64_t ld = b->ld[m];
-        WB_CUBLAS(cublasSetStream(h->cublas, s));
+        WB_CUBLAS(cublasSetStream(h->cublas, t));
         WB_CUBLAS(cublasSetMathMode(h->cublas, CUBLAS_DEFAULT_MATH));
         if (stats)
             WB_CUDA(cudaMemsetAsync(at<void>(ws, L.counters), 0,
-                                    sizeof(unsigned long long) * kCounterWords, s));
+                                    sizeof(unsigned long long) * kCounterWords, t));
         const double* X = at<double>(ws, L.X);
         float* F32 = at<float>(ws, L.F32);
         if (!qd[m]) {
             // an inactive molecule: F = 0, so its screen keeps no task
-            WB_CUDA(cudaMemsetAsync(F32, 0, sizeof(float) * (size_t)nao * ld, s));
+            WB_CUDA(cudaMemsetAsync(F32, 0, sizeof(float) * (size_t)nao * ld, t));
         } else if (b->gemm == WB_K_GEMM_OZAKI_BF16 && wb::ozaki_f_supported(nao)) {
             const int r = wb::ozaki_f_gemm(
-                h->cublas, X, qd[m], nao, ld, F32, b->scratch, s,
+                h->cublas, X, qd[m], nao, ld, F32, scratch, t,
                 at<unsigned long long>(ws, L.counters) + 3 * wb::NCLASS);
             if (r) return fail(r >= 1000 ? WB_ERR_CUBLAS : WB_ERR_CUDA,
                                "ozaki F GEMM failed, code " + std::to_string(r));
             launches += wb::ozaki_f_launches(nao, ld);
         } else {
-            double* F64 = static_cast<double*>(b->scratch);
+            double* F64 = static_cast<double*>(scratch);
             WB_CUBLAS(cublasDgemm(h->cublas, CUBLAS_OP_N, CUBLAS_OP_T, (int)ld, nao, nao,
                                   &one, X, (int)ld, qd[m], nao, &zero, F64, (int)ld));
-            WB_CUDA(wb::launch_f64_to_f32(F64, F32, (int64_t)nao * ld, s));
+            WB_CUDA(wb::launch_f64_to_f32(F64, F32, (int64_t)nao * ld, t));
             launches += 2;
         }
         wb::BlockStatsOut bo;
@@ -1914,9 +1965,11 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
             bo.msh[k] = at<float>(ws, L.msh[k]);
         }
         WB_CUDA(wb::launch_sub_stats(b->coords[m], b->weights[m], F32, b->npts[m], ld,
-                                     h->hp.nvshell, h->vs_ao0, h->vs_nf, bo, s));
+                                     h->hp.nvshell, h->vs_ao0, h->vs_nf, bo, t));
         launches += 1;
-    }
+        return WB_OK;
+    });
+    if (st != WB_OK) return st;
     // every class: one launch over all molecules (two for the classes
     // without a two-omega kernel), side by side on the batch's own streams so
     // that the tail of one is filled by the others (clusters of 4 to 17 waters,
@@ -1964,9 +2017,10 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
         b->ordered = true;
     }
     // per molecule: G of each slot, then K
-    for (int m = 0; m < nmol; ++m) {
-        if (!qd[m]) continue;
+    st = batch_lanes(b, qd, s, [&](int m, cudaStream_t t, void* scratch) -> int {
+        if (!qd[m]) return WB_OK;
         wb_cosx* h = b->h[m];
+        WB_CUBLAS(cublasSetStream(h->cublas, t));
         const WsLayout& L = b->L[m];
         void* ws = b->ws[m];
         const int nao = h->hp.nao;
@@ -1984,48 +2038,50 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
             gs.gc1[w] = at<float>(ws, gclH[w]);
             gs.G[w] = Gs[w];
         }
-        WB_CUDA(wb::launch_gsum2(gs, b->nom, h->gsrc, nao, ld, s));
+        WB_CUDA(wb::launch_gsum2(gs, b->nom, h->gsrc, nao, ld, t));
         launches += 1;
 #else
         for (int w = 0; w < b->nom; ++w)
-            WB_CUDA(wb::launch_gsum(at<float>(ws, gcl[w]), h->gsrc, nao, ld, Gs[w], s));
+            WB_CUDA(wb::launch_gsum(at<float>(ws, gcl[w]), h->gsrc, nao, ld, Gs[w], t));
         launches += b->nom;
 #endif
         if (b->gemm == WB_K_GEMM_OZAKI_BF16) {
             const float* Gc[2] = {Gs[0], Gs[1]};
             const int r = wb::ozaki_k_gemm_multi(h->cublas, X, Gc, b->nom, b->weights[m],
                                                  nao, ld, b->npts[m], 0, Ks,
-                                                 b->scratch, s, false);
+                                                 scratch, t, false);
             if (r) return fail(r >= 1000 ? WB_ERR_CUBLAS : WB_ERR_CUDA,
                                "ozaki K GEMM failed, code " + std::to_string(r));
             launches += wb::ozaki_k_launches(nao, ld);
         } else {
-            double* WG = static_cast<double*>(b->scratch);
+            double* WG = static_cast<double*>(scratch);
             for (int w = 0; w < b->nom; ++w) {
                 WB_CUDA(wb::launch_weight_g(Gs[w], b->weights[m], b->npts[m], ld, nao,
-                                            WG, s));
+                                            WG, t));
                 WB_CUBLAS(cublasDgemm(h->cublas, CUBLAS_OP_T, CUBLAS_OP_N, nao, nao,
                                       (int)ld, &one, WG, (int)ld, X, (int)ld, &zero,
                                       Ks[w], nao));
                 launches += 2;
             }
         }
-    }
+        return WB_OK;
+    });
+    if (st != WB_OK) return st;
     if (!stats) return WB_OK;
     std::memset(stats, 0, sizeof(*stats));
     for (int m = 0; m < nmol; ++m) {
-        wb_cosx_stats st;
+        wb_cosx_stats one_mol;
         const int r = read_stats(b->h[m], b->ws[m], b->L[m],
                                  b->nom * (b->ld[m] / 32) * (int64_t)b->h[m]->hp.npairs,
-                                 s, &st, 0);
+                                 s, &one_mol, 0);
         if (r != WB_OK) return r;
-        stats->tasks_total += st.tasks_total;
-        stats->tasks_kept += st.tasks_kept;
-        stats->integrals += st.integrals;
-        stats->model_flops += st.model_flops;
+        stats->tasks_total += one_mol.tasks_total;
+        stats->tasks_kept += one_mol.tasks_kept;
+        stats->integrals += one_mol.integrals;
+        stats->model_flops += one_mol.model_flops;
         for (int c = 0; c < wb::NCLASS; ++c) {
-            stats->tasks_kept_class[c] += st.tasks_kept_class[c];
-            stats->model_flops_class[c] += st.model_flops_class[c];
+            stats->tasks_kept_class[c] += one_mol.tasks_kept_class[c];
+            stats->model_flops_class[c] += one_mol.model_flops_class[c];
         }
     }
     stats->kernel_launches = launches;
@@ -2037,6 +2093,10 @@ int wb_cosx_batch_destroy(wb_cosx_batch* b) {
     for (int c = 0; c < wb::NCLASS; ++c) {
         if (b->cstream[c]) cudaStreamDestroy(b->cstream[c]);
         if (b->cdone[c]) cudaEventDestroy(b->cdone[c]);
+    }
+    for (int q = 0; q < wb_cosx_batch::kLanes; ++q) {
+        if (b->lane[q]) cudaStreamDestroy(b->lane[q]);
+        if (b->ldone[q]) cudaEventDestroy(b->ldone[q]);
     }
     if (b->fork) cudaEventDestroy(b->fork);
     if (b->block) cudaFree(b->block);
