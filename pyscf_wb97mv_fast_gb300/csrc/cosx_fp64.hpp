@@ -57,13 +57,14 @@ struct CosxF64Args {
 cudaError_t launch_f64_records(int npp, const double* P, const double* p,
                                const double* pref, const double* alpha, double omega,
                                double* rec, cudaStream_t s);
-// Ranges that the pairs of a block are split into.  One warp a block leaves
-// the FP64 pipe idle on grids of fewer than some 16 blocks an SM and in the
-// last blocks of larger ones (an FP64 Fock build of 4 waters, 591 blocks: 21.2
-// -> 18.0 ms with the leaner Boys function).  Ranges beyond 8 cost more screening than they gain.
+// Ranges that the pairs of a block are split into: some six items for each of
+// an SM's 16 warps, so that neither a short grid nor the last items of a class
+// leave warps without work.  FP64 K of 8 waters (192 AOs, 70,478 points) 2
+// ranges 51.8 ms, 4 48.0, 7 46.7; gradient of 8 waters (36,369 points) 4 ranges
+// 58.1 ms, 13 53.6, of C4H10 in TZVP (21,512) 6 73.8, 22 70.3.
 inline int f64_segments(int64_t nblk, int nsm) {
-    const int64_t n = (24 * (int64_t)nsm + nblk - 1) / (nblk > 0 ? nblk : 1);
-    return (int)(n < 1 ? 1 : n > 8 ? 8 : n);
+    const int64_t n = (96 * (int64_t)nsm + nblk - 1) / (nblk > 0 ? nblk : 1);
+    return (int)(n < 1 ? 1 : n > 32 ? 32 : n);
 }
 // G[0] += the other nseg - 1 ranges, in order; n elements each
 cudaError_t launch_f64_segment_sum(double* G, int64_t n, int nseg, cudaStream_t s);

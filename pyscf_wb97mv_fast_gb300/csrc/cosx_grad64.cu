@@ -39,7 +39,7 @@
 // reduction in the task would cost 30 FP64 instructions.  The columns are
 // weighted with -w_g / 2 and summed in a fixed order at the end, so the
 // result is bitwise reproducible.  Measured (whole call): 8 waters, 36,369
-// points 370 -> 58 ms; C4H10 in TZVP, 21,512 points 692 -> 74 ms.
+// points 370 -> 54 ms; C4H10 in TZVP, 21,512 points 692 -> 70 ms.
 #include "cosx_fp64.cuh"
 #include "cosx_grad64.hpp"
 

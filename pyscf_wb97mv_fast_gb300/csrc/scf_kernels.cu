@@ -515,7 +515,7 @@ __device__ __forceinline__ typename HartreeTraits<F64>::Real hartree_pp(
 // kernel for all of them held the registers of the largest and a switch in
 // its inner loop).  The FP64 form is bound by the FP64 pipe and arranged as
 // the FP64 class kernels (cosx_fp64.cuh); the FP32 form by the latency of its
-// loads and instruction issue.  8 waters, 70,479 points, FP32: 6.0 -> 3.5 ms; 4
+// loads and instruction issue.  8 waters, 70,479 points, FP32: 6.0 -> 2.6 ms; 4
 // waters, 18,912 points, FP64: 6.9 -> 3.4 ms.
 template<bool F64, int L>
 __global__ void __launch_bounds__(HartreeTraits<F64>::kThreads, HartreeTraits<F64>::kCtas)
