@@ -924,6 +924,11 @@ struct wb_cosx_batch {
     int* d_order = nullptr;             // NCLASS x stride: costliest first
     int64_t stride = 0;
     bool ordered = false;               // the orders hold a previous run's costs
+    // molecules of more blocks than fill the device on their own run their
+    // own class launches: the batched kernels keep the argument blocks in shared
+    // memory and registers where those have them in the constant bank (four of
+    // 30 waters: 140.6 ms a run batched, 120.9 so)
+    std::vector<char> alone;
     // the class launches of a run, side by side
     cudaStream_t cstream[wb::NCLASS] = {};
     cudaEvent_t cdone[wb::NCLASS] = {};
@@ -1815,13 +1820,24 @@ int wb_cosx_batch_create(int nmol, wb_cosx* const* handles,
         }
         args[m] = a;
         args[nmol + m] = bb;
+        // ten blocks of 64 points an SM; the same kernel variants in both forms
+        bool alone = b->ld[m] >= 640 * (int64_t)h->nsm && (nomega == 1 || h->dual_ok);
+        for (int c = 0; c < wb::NCLASS && nomega == 2; ++c)
+            alone = alone && (!b->has[c] || h->dual_cls[c] == b->dual[c]);
+        b->alone.push_back(alone);
+        if (alone) {        // the orders' arrays, so that a run allocates nothing
+            const bool single[wb::NCLASS] = {};
+            const int st = block_order_args(h, b->ld[m], a,
+                                            nomega == 2 ? h->dual_cls : single, s);
+            if (st != WB_OK) return batch_fail(b, st);
+        }
     }
     for (int c = 0; c < wb::NCLASS; ++c) {
         int* o = off.data() + (size_t)c * (nmol + 1);
         for (int m = 0; m < nmol; ++m) {
             const wb_cosx* h = b->h[m];
             int n = 0;
-            if (h->hp.cls[c].pair_end > h->hp.cls[c].pair_begin) {
+            if (!b->alone[m] && h->hp.cls[c].pair_end > h->hp.cls[c].pair_begin) {
                 const int pc = b->dual[c] ? h->pts2[c] : h->pts[c];
                 n = (WB_COSX_SPLIT ? 2 : 1) * args[m].nblk[pc == 4 ? 2 : pc - 1];
             }
@@ -1982,6 +1998,19 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
         return WB_OK;
     });
     if (st != WB_OK) return st;
+    for (int m = 0; m < nmol; ++m) {
+        if (!b->alone[m] || !qd[m]) continue;
+        const WsLayout& L = b->L[m];
+        void* ws = b->ws[m];
+        float* F32 = at<float>(ws, L.F32);
+        st = b->nom == 2
+                 ? run_g_classes_dual(b->h[m], b->npts[m], b->ld[m], F32, at<float>(ws, L.G32),
+                                      at<float>(ws, L.G32b), b->om[0], b->om[1], b->tol, ws, L,
+                                      s, &launches)
+                 : run_g_classes(b->h[m], b->npts[m], b->ld[m], F32, at<float>(ws, L.G32),
+                                 b->om[0], b->tol, ws, L, s, &launches);
+        if (st != WB_OK) return st;
+    }
     // every class: one launch over all molecules (two for the classes
     // without a two-omega kernel), side by side on the batch's own streams so
     // that the tail of one is filled by the others (clusters of 4 to 17 waters,
@@ -2050,12 +2079,15 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
             gs.gc1[w] = at<float>(ws, gclH[w]);
             gs.G[w] = Gs[w];
         }
-        WB_CUDA(wb::launch_gsum2(gs, b->nom, h->gsrc, nao, ld, t));
-        launches += 1;
+        if (!b->alone[m]) {
+            WB_CUDA(wb::launch_gsum2(gs, b->nom, h->gsrc, nao, ld, t));
+            launches += 1;
+        }
 #else
-        for (int w = 0; w < b->nom; ++w)
+        for (int w = 0; w < b->nom && !b->alone[m]; ++w) {
             WB_CUDA(wb::launch_gsum(at<float>(ws, gcl[w]), h->gsrc, nao, ld, Gs[w], t));
-        launches += b->nom;
+            launches += 1;
+        }
 #endif
         if (b->gemm == WB_K_GEMM_OZAKI_BF16) {
             const float* Gc[2] = {Gs[0], Gs[1]};

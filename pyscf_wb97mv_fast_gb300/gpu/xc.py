@@ -4,7 +4,8 @@ pyscf_wb97mv_fast/gpu/xc.py:1-201).
 ``gpu_nr_rks(ctx, ni, mol, grids, xc_code, dms, ...) -> (nelec, excsum,
 vmat)`` has NumInt.nr_rks's signature and result for one RKS density and an
 LDA / GGA / MGGA (no laplacian) functional -- the wB97M-V case.  Per tile of
-grid points (the whole grid when it fits):
+grid points (up to four, the host's part of one beside the device's of the
+next):
 
     X      = AO values and gradients (4, nao, ld) FP64      wb_ao_eval_deriv1
     T_d    = fl32(dm^T X_d)  (d = 0, and x, y, z for MGGA)   wb_cosx_ozaki_f
