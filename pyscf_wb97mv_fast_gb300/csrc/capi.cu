@@ -878,9 +878,11 @@ WsLayout64 ws_layout_fp64(const wb_cosx* h, int64_t ld, bool two) {
     L.X = take(sizeof(double) * n);
     L.F64 = take(sizeof(double) * n);
     L.F32 = take(sizeof(float) * n);
-    // (as many as fit 8 GiB)
-    L.nseg = (int)std::max<int64_t>(
-        1, std::min<int64_t>(wb::f64_segments(ld / 32, h->nsm), (int64_t)((8ull << 30) / (8 * n))));
+    // as many copies of G as fit 512 MiB, or three of up to 4 GiB, which leave
+    // this workspace no larger than the mixed form's of the same grid
+    const size_t fit = ((size_t)512 << 20) / (8 * n);
+    L.nseg = std::min(wb::f64_segments(ld / 32, h->nsm),
+                      (int)std::max<size_t>(8 * n <= (size_t)4 << 30 ? 3 : 1, fit));
     L.G64 = take(sizeof(double) * n * L.nseg);
     if (two) L.G64b = take(sizeof(double) * n * L.nseg);
     L.gemm = take(wb::gemm64_bytes(nao64, ld));
