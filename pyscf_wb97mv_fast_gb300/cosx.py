@@ -483,6 +483,8 @@ class CosxEngine:
         (wb_cosx_gemm64_f); X (nao, ld) FP64, ld a multiple of 32."""
         torch = _torch()
         X = device_arg(X, 'X', torch.float64, self.device, (self.nao, None))
+        if X.data_ptr() % 16:                   # the kernels load pairs of points
+            X = X.clone()
         qd = self._dm_arg(qd)
         ld = int(X.shape[1])
         out = torch.empty((self.nao, ld), dtype=torch.float64, device=self.device)
