@@ -745,10 +745,11 @@ __device__ __forceinline__ const double* c2s_ptr() {
 
 __constant__ unsigned long long c_exp2m[64];            // the table of exp_neg
 
-// a < 70, on the integer pipe (a >= 0): a primitive below exp(-70) ~ 4e-31 is
-// zero at FP64 parity with any AO value of order one
+// a < 70, on the integer pipe (a >= 0; false for a NaN of either sign): a
+// primitive below exp(-70) ~ 4e-31 is zero at FP64 parity with any AO value of
+// order one
 __device__ __forceinline__ bool below70(const double a) {
-    return __double2hiint(a) < 0x40518000;
+    return (unsigned)__double2hiint(a) < 0x40518000u;
 }
 
 // The real solid harmonics S_m (NS) of a shell at (dx, dy, dz) and, with D,

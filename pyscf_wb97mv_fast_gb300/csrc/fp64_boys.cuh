@@ -36,7 +36,8 @@ __device__ __forceinline__ double widen(const float f) {
 }
 
 // double -> float, truncated, on the integer pipe; magnitudes below 2^-126
-// give zero (the callers' values stay below 2^127)
+// give zero; what is not below 2^127 (infinities and NaN too) gives some float
+// that its caller does not use
 __device__ __forceinline__ float narrow(const double d) {
     const unsigned hi = (unsigned)__double2hiint(d);
     const unsigned lo = (unsigned)__double2loint(d);
@@ -136,7 +137,10 @@ __device__ __forceinline__ void boys_fast(const double T, const double* tab, dou
     const float tf = narrow(T);
     const unsigned long long* etab =
         reinterpret_cast<const unsigned long long*>(tab + B::kExp);
-    if (__double2hiint(T) < 0x40420000) {            // T < 36
+    // the ranges of T by its high word, unsigned: a NaN of either sign is above
+    // all of them (signed, one with its sign bit set would pick a table row)
+    const unsigned ht = (unsigned)__double2hiint(T);
+    if (ht < 0x40420000u) {                          // T < 36
         const int k = __float2int_rn(tf * 32.0f);
         const double* row = tab + k * B::kStride;
         const float* frow = reinterpret_cast<const float*>(row + 4);
@@ -155,12 +159,17 @@ __device__ __forceinline__ void boys_fast(const double T, const double* tab, dou
             }
         }
     } else {
-        const double y0 = widen(rsqrtf(tf));
-        const double e = fma(-(T * y0), y0, 1.0);
-        const double y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
+        double y;
+        if (ht < 0x47e00000u) {                      // T < 2^127
+            const double y0 = widen(rsqrtf(tf));
+            const double e = fma(-(T * y0), y0, 1.0);
+            y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
+        } else {
+            y = rsqrt(T);                            // infinity: 0, NaN: NaN
+        }
         F[0] = 0.88622692545275801365 * y;
         if constexpr (L > 0) {
-            const double ex = __double2hiint(T) < 0x40518000 ? -exp_neg(T, etab) : 0.0;
+            const double ex = ht < 0x40518000u ? -exp_neg(T, etab) : 0.0;
             const double h = half_of(y * y);
 #pragma unroll
             for (int n = 0; n < L; ++n) F[n + 1] = fma((double)(2 * n + 1), F[n], ex) * h;
