@@ -316,6 +316,9 @@ int wb_cosx_g_multi(wb_cosx* h, const double* coords, const double* weights,
  *   wb_cosx_ozaki_k: k_out (nao, nao) row-major (+)= X^T (w o G) over npts
  *     points, g (nao, ld) FP32.  Replaces K += X.T @ (w64 * G)
  *     (gpu/sgx_k.py:734).
+ * A point or column holding an infinity or NaN gives NaN; so does an F tile
+ * of the tensor-core kernel whose bounded wait ran out, and the screen keeps
+ * the pairs such points meet, so a K build with either holds NaN.
  * Workspace: wb_ozaki_workspace_bytes(nao, ld) bytes. */
 size_t wb_ozaki_workspace_bytes(int nao, int64_t ld);
 int wb_cosx_ozaki_f(wb_cosx* h, const double* x, const double* qd,

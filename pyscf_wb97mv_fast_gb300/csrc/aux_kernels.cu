@@ -164,7 +164,8 @@ cudaError_t launch_grid_prep(const double* coords, int64_t npts, int64_t ld,
 // quarters (the reference's sub-block size), its 64-point halves and the
 // whole block, the FP64 centroid and radius of the valid points (centroid
 // rounded to nearest FP32, radius rounded up) and, for every (virtual)
-// shell, msh = max_g fl32(w_g) sum_{t in shell} |F_tg|.  One pass over F
+// shell, msh = max_g fl32(w_g) sum_{t in shell} |F_tg| (NaN where one of them
+// is).  One pass over F
 // serves the 32-, 64- and 128-point class kernels.  Block b of size 32 * 2^k
 // covers points [b 32 2^k, (b + 1) 32 2^k); blocks past ld are not written.
 __device__ __forceinline__ double warp_sum_d(double v) {
@@ -285,7 +286,7 @@ __global__ void sub_stats_kernel(const BlockStatsOut O,
 #pragma unroll
         for (int q = 0; q < 4; ++q)
             for (int o = 16; o > 0; o >>= 1)
-                acc[q] = fmaxf(acc[q], __shfl_xor_sync(0xffffffffu, acc[q], o));
+                acc[q] = max_nan(acc[q], __shfl_xor_sync(0xffffffffu, acc[q], o));
         if (lane == 0) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -296,10 +297,10 @@ __global__ void sub_stats_kernel(const BlockStatsOut O,
             for (int j = 0; j < 2; ++j) {
                 const int64_t b = (int64_t)blk * 2 + j;
                 if (b * 64 < ld)
-                    O.msh[1][b * nvshell + sh] = fmaxf(acc[2 * j], acc[2 * j + 1]);
+                    O.msh[1][b * nvshell + sh] = max_nan(acc[2 * j], acc[2 * j + 1]);
             }
             O.msh[2][(int64_t)blk * nvshell + sh] =
-                fmaxf(fmaxf(acc[0], acc[1]), fmaxf(acc[2], acc[3]));
+                max_nan(max_nan(acc[0], acc[1]), max_nan(acc[2], acc[3]));
         }
     }
 }
@@ -1242,7 +1243,7 @@ __global__ void screen_mask_kernel(const CosxArgs A, const int lv, const int npa
             const float* ms = A.blk_msh[lv] + (int64_t)blk * A.nvshell;
             kp = screen_pair(A.tol, A.bnd + A.pp_begin[c], A.bpref + A.pp_begin[c],
                              A.blk_cr[lv][blk], A.khdr[k], A.ptau[k],
-                             fmaxf(ms[sh.x], ms[sh.y]));
+                             max_nan(ms[sh.x], ms[sh.y]));
         }
         keep[idx] = kp ? 1 : 0;
     }

@@ -299,7 +299,7 @@ cosx_fp64_kernel(const CosxF64Args A, const int cls, const int pair_begin,
             if (keep && A.tol > 0.0f) {
                 const int2 sh = A.pshell[k];
                 keep = screen_pair(A.tol, bnd, bpref, cr, A.khdr[k], A.ptau[k],
-                                   fmaxf(ms[sh.x], ms[sh.y]));
+                                   max_nan(ms[sh.x], ms[sh.y]));
             }
             unsigned mask = __ballot_sync(0xffffffffu, keep);
             if (keep) {

@@ -316,7 +316,7 @@ __device__ __forceinline__ void cosx_class_block(
             nhl = A.khdr[k];
             ntp = A.ptau[k];
             const int2 sh = A.pshell[k];
-            nfm = fmaxf(ms[sh.x], ms[sh.y]);
+            nfm = max_nan(ms[sh.x], ms[sh.y]);
         }
     }
     for (int c0 = pair_begin; c0 < pair_end; c0 += 32) {
@@ -336,7 +336,7 @@ __device__ __forceinline__ void cosx_class_block(
         bool keep = k < pair_end;
         if (keep && tol > 0.0f)
             keep = screen_pair(tol, bnd, bpref, cr, hl, tp, fm);
-        if (kn < pair_end) nfm = fmaxf(ms[nsh.x], ms[nsh.y]);
+        if (kn < pair_end) nfm = max_nan(ms[nsh.x], ms[nsh.y]);
         unsigned mask = __ballot_sync(0xffffffffu, keep);
         if (!mask) continue;
         int4 hdr = shfl_int4(hl, __ffs(mask) - 1);

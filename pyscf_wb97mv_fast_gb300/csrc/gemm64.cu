@@ -45,7 +45,6 @@ constexpr int kPiece = 4096;             // terms of an exact FP32 sum
 constexpr int kKc = 512;                 // points per chunk of the K product
 constexpr int kGroup = 128;              // chunks in flight
 constexpr int64_t kTile = 65536;         // points per tile of the F product
-constexpr int kNonfinite = 1 << 20;      // exponent of a row that holds one
 
 size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
 // slices are padded to 8 entries: cuBLAS needs 16-byte rows for its

@@ -24,7 +24,7 @@
 // throughout).  Pieces and levels are combined exactly in int64 and
 // scaled once in FP64.  The result carries W = 42 bits relative to the
 // per-row / per-column maxima; the truncated products (i + j >= S) are
-// below 2^-W of them.
+// below 2^-W of them.  A row or column with an infinity or a NaN gives NaN.
 //
 // The level GEMMs are library GEMMs (cuBLAS bf16 GEMMs with FP32
 // accumulation, one per level) around this file's slicing and combination
@@ -150,10 +150,17 @@ __global__ void f_combine_kernel(const float* __restrict__ C, int nao,
         v[0] += level_term<B_, S>(l, c[l].x); v[1] += level_term<B_, S>(l, c[l].y);
         v[2] += level_term<B_, S>(l, c[l].z); v[3] += level_term<B_, S>(l, c[l].w);
     }
-    const T o0 = scaled_ll_to<T>(v[0], er.x + base);
-    const T o1 = scaled_ll_to<T>(v[1], er.y + base);
-    const T o2 = scaled_ll_to<T>(v[2], er.z + base);
-    const T o3 = scaled_ll_to<T>(v[3], er.w + base);
+    T o0 = scaled_ll_to<T>(v[0], er.x + base);
+    T o1 = scaled_ll_to<T>(v[1], er.y + base);
+    T o2 = scaled_ll_to<T>(v[2], er.z + base);
+    T o3 = scaled_ll_to<T>(v[3], er.w + base);
+    if (not_finite(max(max(er.x, er.y), max(er.z, er.w)) + base)) {
+        const T nan = (T)__int_as_float(0x7fc00000);
+        if (not_finite(er.x + base)) o0 = nan;
+        if (not_finite(er.y + base)) o1 = nan;
+        if (not_finite(er.z + base)) o2 = nan;
+        if (not_finite(er.w + base)) o3 = nan;
+    }
     if constexpr (sizeof(T) == 4) {
         *reinterpret_cast<float4*>(F + i) = make_float4(o0, o1, o2, o3);
     } else {
@@ -179,6 +186,10 @@ __global__ void f_combine_kernel(const float* __restrict__ C, int nao,
 // side r at r np (np = gridDim.y).  The CTAs of the first one also slice X,
 // unless slice_x is 0: the X slices and exponents of this tile are then already
 // in A / ex (an earlier omega of the same tile).
+// the constant of scale_word: FP64's bias, and what a chunk's sum is scaled by
+template<int B_, int S>
+constexpr int kScaleK = 1023 - 2 * 400 - 2 * kW + 2 + B_ * (S - 1);
+
 template<typename GT>
 struct KIn {
     const GT* g[8];
@@ -264,8 +275,8 @@ k_slice_kernel(const double* __restrict__ X, const __grid_constant__ KIn<GT> Gs,
     }
     const int e1 = exp_of_hi(mx), e2 = exp_of_hi(mw);
     if (threadIdx.x == 0) {
-        if (dox) ex[(int64_t)c * np + col] = e1;
-        ew[(int64_t)c * nb + boff + col] = e2;
+        if (dox) ex[(int64_t)c * np + col] = scale_word(e1, kScaleK<B_, S>);
+        ew[(int64_t)c * nb + boff + col] = scale_word(e2);
     }
     const int64_t colbase = (int64_t)c * S * KC * np + (int64_t)col * S * KC;
     const int64_t colbase_b = (int64_t)c * S * KC * nb + (int64_t)(boff + col) * S * KC;
@@ -320,23 +331,22 @@ __global__ void k_combine_kernel(const float* __restrict__ C, int nao, int np, i
                     v += level_term<B_, S>(l, __ldg(p));
             return v;
         };
-        auto scale = [&](int c) -> int {
-            return ex[(int64_t)c * np + mu] + ew[(int64_t)c * nb + col] - 2 * kW + 2 +
-                   B_ * (S - 1);
+        auto scale = [&](int c) {
+            return scale_of(ex[(int64_t)c * np + mu], ew[(int64_t)c * nb + col]);
         };
         int c = 0;
         for (; c + U <= nchunk; c += U) {
             long long v[U];
-            int sc[U];
+            double sc[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 v[u] = value(c + u);
                 sc[u] = scale(c + u);
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) acc += (double)v[u] * pow2(sc[u]);
+            for (int u = 0; u < U; ++u) acc += (double)v[u] * sc[u];
         }
-        for (; c < nchunk; ++c) acc += (double)value(c) * pow2(scale(c));
+        for (; c < nchunk; ++c) acc += (double)value(c) * scale(c);
         double* K = Ks.k[col / np];
         const int64_t o = (int64_t)mu * nao + col % np;        // K row-major
         K[o] = accumulate ? K[o] + acc : acc;

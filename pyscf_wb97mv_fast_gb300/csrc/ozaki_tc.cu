@@ -268,7 +268,8 @@ ozaki_f_tc_kernel(const __grid_constant__ CUtensorMap mapA,
                 if (mu < P.nao) {
                     const int sc = er + P.ecol[mu] - 2 * kW + 2 + B_ * (S - 1);
                     P.F[(int64_t)mu * P.ld + g] =
-                        bad ? (T)__int_as_float(0x7fc00000) : scaled_ll_to<T>(acc[q], sc);
+                        bad || not_finite(sc) ? (T)__int_as_float(0x7fc00000)
+                                              : scaled_ll_to<T>(acc[q], sc);
                 }
             }
         }

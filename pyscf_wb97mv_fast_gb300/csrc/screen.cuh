@@ -10,6 +10,16 @@
 
 namespace wb {
 
+// the larger of two block maxima, NaN if either is one
+__device__ __forceinline__ float max_nan(const float a, const float b) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
+
+// A pair is dropped only where its bound is below the tolerance: a NaN among
+// the points' F (a non-finite density, a tensor-core F product that gave up)
+// keeps the pairs it meets, so that it shows in G and K.
 // tp = (tau, tau * sum pref), f = max(msh_A, msh_B) of the block; bnd and
 // bpref start at the class's first primitive pair (hdr.z is class-local)
 __device__ __forceinline__ bool screen_pair(const float tol,
@@ -36,7 +46,7 @@ __device__ __forceinline__ bool screen_pair(const float tol,
             f0 = 0.88622692545f * erff(sqrtf(T)) * rsqrtf(T);
         b += bpref[m] * f0;
     }
-    return tp.x * b * f >= tol;
+    return !(tp.x * b * f < tol);
 }
 
 }  // namespace wb
