@@ -1181,9 +1181,10 @@ def main():
     ap.add_argument('--warmup', type=int, default=3)
     ap.add_argument('--impl', default='ours', choices=['ours', 'reference'])
     ap.add_argument('--gemm', default='ozaki', choices=['ozaki', 'native', 'emulated'])
-    ap.add_argument('--f-engine', default='library', choices=['library', 'tc'],
-                    help="the Ozaki F product: this library's tcgen05 kernel or "
-                         "cuBLAS level GEMMs (bitwise the same F)")
+    ap.add_argument('--f-engine', default='auto', choices=['library', 'tc', 'auto'],
+                    help="the Ozaki F product: this library's tcgen05 kernel, "
+                         "cuBLAS level GEMMs or the kernel for small products "
+                         "only (bitwise the same F)")
     ap.add_argument('--small', action='store_true',
                     help='8 waters / grid level 1 (profiling captures)')
     ap.add_argument('--grid-level', type=int, default=None,

@@ -401,13 +401,16 @@ int wb_rsh_lda_eval(const double* rho, int64_t n, double omega, double cx_sr,
  * cuBLAS bf16 GEMM per level; WB_OZAKI_ENGINE_TC is this library's
  * tensor-core kernel (TMA tile loads, tcgen05 MMAs into TMEM, the exact
  * level combination fused into its epilogue), slower on the bench step
- * (its seven level accumulators allow 64-wide tiles only).  Until one is set
- * (wb_ozaki_get_f_engine: library) F products of up to 64 AOs and one wave of
- * 128-point tiles run on the kernel.  Both give bitwise the same F.  Replaces
+ * (its seven level accumulators allow 64-wide tiles only);
+ * WB_OZAKI_ENGINE_AUTO (the default) runs F products of up to 64 AOs and one
+ * wave of 128-point tiles on the kernel, the others on the library.  All give
+ * bitwise the same F.  wb_ozaki_get_f_engine returns what is set, so that
+ * setting it again restores it.  Replaces
  * no reference call (the reference's F GEMM is one CuPy FP64 matmul,
  * gpu/sgx_k.py:722); returns WB_OK or WB_ERR_INVALID_ARGUMENT. */
 #define WB_OZAKI_ENGINE_LIBRARY 0
 #define WB_OZAKI_ENGINE_TC 1
+#define WB_OZAKI_ENGINE_AUTO 2
 int wb_ozaki_set_f_engine(int engine);
 int wb_ozaki_get_f_engine(void);
 

@@ -55,25 +55,35 @@ def device_out(t, name, dtype, device, shape):
     return t
 
 
-F_ENGINES = {'library': 0, 'tc': 1}
+F_ENGINES = {'library': 0, 'tc': 1, 'auto': 2}
+
+
+class _Auto(str):
+    """What get_f_engine returns under 'auto': the name 'library', which all but
+    the small products run on, that asks for 'auto' when it is set again."""
 
 
 def set_f_engine(name):
     """Engine of the F product of the Ozaki split (process-wide): 'library'
-    (cuBLAS bf16 level GEMMs) or 'tc' (this library's tcgen05 tensor-core
-    kernel with the level combination fused); both give bitwise the same F.
-    Until one is set, 'library' except for small F products (up to 64 AOs and
-    one wave of 128-point tiles).  Returns the previous engine's name."""
+    (cuBLAS bf16 level GEMMs), 'tc' (this library's tcgen05 tensor-core kernel
+    with the level combination fused) or 'auto' (the default: 'tc' for products
+    of up to 64 AOs and one wave of 128-point tiles, 'library' for the others);
+    all give bitwise the same F.  Returns the previous engine, to be given back
+    to this function."""
     if name not in F_ENGINES:
         raise ValueError('F engine must be one of %s' % sorted(F_ENGINES))
     prev = get_f_engine()
-    _native.check(_native.lib().wb_ozaki_set_f_engine(F_ENGINES[name]),
-                  'wb_ozaki_set_f_engine')
+    code = F_ENGINES['auto' if isinstance(name, _Auto) else name]
+    _native.check(_native.lib().wb_ozaki_set_f_engine(code), 'wb_ozaki_set_f_engine')
     return prev
 
 
 def get_f_engine():
+    """The engine that is set, as set_f_engine takes it ('library' under
+    'auto')."""
     code = int(_native.lib().wb_ozaki_get_f_engine())
+    if code == F_ENGINES['auto']:
+        return _Auto('library')
     return {v: k for k, v in F_ENGINES.items()}[code]
 
 

@@ -25,6 +25,10 @@
 #include "ozaki.hpp"
 #include "wb97mv_gb300.h"
 
+static_assert(wb::kOzEngineLibrary == WB_OZAKI_ENGINE_LIBRARY &&
+              wb::kOzEngineTc == WB_OZAKI_ENGINE_TC &&
+              wb::kOzEngineAuto == WB_OZAKI_ENGINE_AUTO, "F engines");
+
 namespace {
 
 thread_local std::string g_err;
@@ -2691,17 +2695,14 @@ int wb_rsh_lda_eval(const double* rho, int64_t n, double omega, double cx_sr, do
 }
 
 int wb_ozaki_set_f_engine(int engine) {
-    if (engine != WB_OZAKI_ENGINE_LIBRARY && engine != WB_OZAKI_ENGINE_TC)
+    if (engine != WB_OZAKI_ENGINE_LIBRARY && engine != WB_OZAKI_ENGINE_TC &&
+        engine != WB_OZAKI_ENGINE_AUTO)
         return fail(WB_ERR_INVALID_ARGUMENT, "wb_ozaki_set_f_engine: unknown engine");
-    wb::ozaki_set_f_engine(engine == WB_OZAKI_ENGINE_TC ? wb::kOzEngineTc
-                                                        : wb::kOzEngineLibrary);
+    wb::ozaki_set_f_engine(engine);
     return WB_OK;
 }
 
-int wb_ozaki_get_f_engine(void) {
-    return wb::ozaki_get_f_engine() == wb::kOzEngineTc ? WB_OZAKI_ENGINE_TC
-                                                       : WB_OZAKI_ENGINE_LIBRARY;
-}
+int wb_ozaki_get_f_engine(void) { return wb::ozaki_get_f_engine(); }
 
 int wb_cosx_ozaki_k(wb_cosx* h, const double* x, const float* g,
                     const double* weights, int64_t npts, int accumulate,

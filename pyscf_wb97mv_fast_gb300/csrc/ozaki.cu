@@ -416,19 +416,17 @@ void f_rowmax(const double* X, int nao, int64_t ld, int* erow, cudaStream_t s) {
 }
 
 namespace {
-std::atomic<int> g_f_engine{-1};                // none asked for
+std::atomic<int> g_f_engine{kOzEngineAuto};
 }
 
 void ozaki_set_f_engine(int engine) { g_f_engine.store(engine); }
-int ozaki_get_f_engine() {
-    return g_f_engine.load() == kOzEngineTc ? kOzEngineTc : kOzEngineLibrary;
-}
+int ozaki_get_f_engine() { return g_f_engine.load(); }
 bool ozaki_f_small(int nao, int64_t ld) {
     return nao <= 64 && (ld + 127) / 128 <= sm_count();
 }
 bool ozaki_f_on_tc(int nao, int64_t ld) {
     const int e = g_f_engine.load();
-    return e == kOzEngineTc || (e < 0 && ozaki_f_small(nao, ld));
+    return e == kOzEngineTc || (e == kOzEngineAuto && ozaki_f_small(nao, ld));
 }
 
 int ozaki_f_gemm(cublasHandle_t hb, const double* X, const double* QD,

@@ -44,12 +44,13 @@ int ozaki_k_gemm64(cublasHandle_t hb, const double* X, const double* G,
                    int accumulate, double* K, void* ws, cudaStream_t s);
 
 // the two engines of the F product (bitwise the same F): cuBLAS level
-// GEMMs and this library's tcgen05 kernel; until one is asked for, the kernel
-// where ozaki_f_small, the GEMMs elsewhere
+// GEMMs and this library's tcgen05 kernel; kOzEngineAuto takes the kernel where
+// ozaki_f_small, the GEMMs elsewhere
 constexpr int kOzEngineLibrary = 0;
 constexpr int kOzEngineTc = 1;
+constexpr int kOzEngineAuto = 2;        // the default
 void ozaki_set_f_engine(int engine);
-int ozaki_get_f_engine();               // kOzEngineLibrary until one is set
+int ozaki_get_f_engine();
 // One column of tiles of the tensor-core kernel (64 AOs) in one wave of CTAs:
 // the level GEMMs are then shorter than the gaps between them.  An F product
 // as called: 48 AOs, 9,928 points 76 -> 42 us, 24 AOs, 5,012 points 78 -> 36;
