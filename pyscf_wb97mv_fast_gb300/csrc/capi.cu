@@ -505,6 +505,39 @@ int block_order_update(wb_cosx* h, const wb::CosxArgs& a, const bool* ran,
     return WB_OK;
 }
 
+// Streams that a call shares its work out to beside its caller's.  Each is joined
+// (the caller's stream waits for it) by join, or where the scope ends: after an
+// error too, nothing may be left running on the caller's buffers, and a capture
+// may not stay forked.
+class SideStreams {
+public:
+    explicit SideStreams(cudaStream_t s) : s_(s) {}
+    SideStreams(const SideStreams&) = delete;
+    SideStreams& operator=(const SideStreams&) = delete;
+    ~SideStreams() { join(); }
+    // t runs from the event `from` of the caller's stream on, joined through done
+    cudaError_t fork(cudaStream_t t, cudaEvent_t from, cudaEvent_t done) {
+        const cudaError_t e = cudaStreamWaitEvent(t, from, 0);
+        if (e == cudaSuccess) side_.push_back({t, done});
+        return e;
+    }
+    cudaError_t join() {
+        cudaError_t first = cudaSuccess;
+        for (const Side& q : side_) {
+            cudaError_t e = cudaEventRecord(q.done, q.stream);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(s_, q.done, 0);
+            if (first == cudaSuccess) first = e;
+        }
+        side_.clear();
+        return first;
+    }
+
+private:
+    struct Side { cudaStream_t stream; cudaEvent_t done; };
+    cudaStream_t s_;
+    std::vector<Side> side_;
+};
+
 // One class launch of want CTAs (four items each), at most cap at a time.  A
 // block's two items are serial chains over half the pairs of the class: where
 // all of them as half blocks fit the device at once (16 warps an SM), the light
@@ -542,6 +575,7 @@ int run_g_classes(wb_cosx* h, int64_t npts_t, int64_t ldt, const float* F,
     // (the class kernels zero their buffers block by block)
     WB_CUDA(cudaMemsetAsync(at<int>(ws, L.work), 0, sizeof(int) * wb::NCLASS, s));
     WB_CUDA(cudaEventRecord(h->fork, s));
+    SideStreams classes(s);
     for (int i = 0; i < wb::NCLASS; ++i) {
         const int c = h->corder[i];
         const wb::ClassRange& r = h->hp.cls[c];
@@ -549,14 +583,13 @@ int run_g_classes(wb_cosx* h, int64_t npts_t, int64_t ldt, const float* F,
         const int lvl = h->pts[c] == 4 ? 2 : h->pts[c] - 1;
         const int want = ((WB_COSX_SPLIT ? 2 : 1) * a.nblk[lvl] + 3) / 4;
         const int cap = std::max(1, h->blocks_per_sm[c][far ? 1 : 0]) * h->nsm;
-        WB_CUDA(cudaStreamWaitEvent(h->cstream[c], h->fork, 0));
+        WB_CUDA(classes.fork(h->cstream[c], h->fork, h->cdone[c]));
         WB_CUDA(launch_class(h, c, a, r, want, cap, h->cstream[c], far, h->stage_smem[c],
                              false));
-        WB_CUDA(cudaEventRecord(h->cdone[c], h->cstream[c]));
-        WB_CUDA(cudaStreamWaitEvent(s, h->cdone[c], 0));
         ran[c] = true;
         *launches += 1;
     }
+    WB_CUDA(classes.join());
     {
         const int st = block_order_update(h, a, ran, single, s, launches);
         if (st != WB_OK) return st;
@@ -597,6 +630,7 @@ int run_g_classes_dual(wb_cosx* h, int64_t npts_t, int64_t ldt, const float* F,
     // (the class kernels zero their buffers block by block)
     WB_CUDA(cudaMemsetAsync(at<int>(ws, L.work), 0, sizeof(int) * 2 * wb::NCLASS, s));
     WB_CUDA(cudaEventRecord(h->fork, s));
+    SideStreams classes(s);
     for (int i = 0; i < wb::NCLASS; ++i) {
         const int c = h->corder[i];
         const wb::ClassRange& r = h->hp.cls[c];
@@ -604,7 +638,7 @@ int run_g_classes_dual(wb_cosx* h, int64_t npts_t, int64_t ldt, const float* F,
         const int pc = h->dual_cls[c] ? h->pts2[c] : h->pts[c];
         const int lvl = pc == 4 ? 2 : pc - 1;
         const int want = ((WB_COSX_SPLIT ? 2 : 1) * a.nblk[lvl] + 3) / 4;
-        WB_CUDA(cudaStreamWaitEvent(h->cstream[c], h->fork, 0));
+        WB_CUDA(classes.fork(h->cstream[c], h->fork, h->cdone[c]));
         if (h->dual_cls[c]) {
             const int cap = std::max(1, h->blocks_per_sm2[c]) * h->nsm;
             WB_CUDA(launch_class(h, c, a, r, want, cap, h->cstream[c], false,
@@ -620,10 +654,9 @@ int run_g_classes_dual(wb_cosx* h, int64_t npts_t, int64_t ldt, const float* F,
                 *launches += 1;
             }
         }
-        WB_CUDA(cudaEventRecord(h->cdone[c], h->cstream[c]));
-        WB_CUDA(cudaStreamWaitEvent(s, h->cdone[c], 0));
         ran[c] = true;
     }
+    WB_CUDA(classes.join());
     {
         const int st = block_order_update(h, a, ran, h->dual_cls, s, launches);
         if (st != WB_OK) return st;
@@ -964,6 +997,7 @@ static int batch_lanes(wb_cosx_batch* b, const double* const* qd, cudaStream_t s
         }
         const bool side = live > 1;
         if (side) WB_CUDA(cudaEventRecord(b->fork, s));
+        SideStreams lanes(s);
         size_t off = 0;
         int n = 0;
         for (; m < end; ++m) {
@@ -971,16 +1005,13 @@ static int batch_lanes(wb_cosx_batch* b, const double* const* qd, cudaStream_t s
             if (side && qd[m]) {
                 const int q = n++ % wb_cosx_batch::kLanes;
                 t = b->lane[q];
-                if (n <= wb_cosx_batch::kLanes) WB_CUDA(cudaStreamWaitEvent(t, b->fork, 0));
+                if (n <= wb_cosx_batch::kLanes) WB_CUDA(lanes.fork(t, b->fork, b->ldone[q]));
             }
             const int st = body(m, t, base + off);
             if (st != WB_OK) return st;
             if (qd[m]) off += bytes(m);
         }
-        for (int q = 0; q < std::min(n, wb_cosx_batch::kLanes); ++q) {
-            WB_CUDA(cudaEventRecord(b->ldone[q], b->lane[q]));
-            WB_CUDA(cudaStreamWaitEvent(s, b->ldone[q], 0));
-        }
+        WB_CUDA(lanes.join());
     }
     return WB_OK;
 }
@@ -1408,21 +1439,17 @@ int wb_cosx_get_k_multi(wb_cosx* h, const double* coords,
     // they are formed on a class stream beside the AO values and F (five
     // small kernels, 40 us of the 420 us build of two waters).
     const bool ahead = nomega == 1 || (nomega == 2 && h->dual_ok);
+    SideStreams records(s);
     if (ahead) {
         const cudaStream_t side = h->cstream[0];
         WB_CUDA(cudaEventRecord(h->fork, s));
-        WB_CUDA(cudaStreamWaitEvent(side, h->fork, 0));
+        WB_CUDA(records.fork(side, h->fork, h->cdone[0]));
         if (nomega == 1)
             st = prepare_omega(h, omegas[0], workspace, L, side);
         else
             st = prepare_omega_dual(h, std::min(omegas[0], omegas[1]),
                                     std::max(omegas[0], omegas[1]), workspace, L, side);
-        // joined in any case: nothing may be left running on the workspace
-        WB_CUDA(cudaEventRecord(h->cdone[0], side));
-        if (st != WB_OK) {
-            WB_CUDA(cudaStreamWaitEvent(s, h->cdone[0], 0));
-            return st;
-        }
+        if (st != WB_OK) return st;
         launches += nomega + 1;
     }
     for (int64_t i0 = 0; i0 < npts; i0 += tile) {
@@ -1454,7 +1481,7 @@ int wb_cosx_get_k_multi(wb_cosx* h, const double* coords,
         if ((st = phase_to(3)) != WB_OK) return st;
         if ((st = tile_prep(h, c, w, nt, ldt, F32, workspace, L, s, &launches)) != WB_OK)
             return st;
-        if (ahead && i0 == 0) WB_CUDA(cudaStreamWaitEvent(s, h->cdone[0], 0));
+        WB_CUDA(records.join());
         // K += X^T (w o G) of omega j from the G in Gsrc; the X slices of
         // this tile serve every omega after the first
         bool x_sliced = false;
@@ -2024,11 +2051,12 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
     WB_CUDA(cudaMemsetAsync(b->d_work, 0, sizeof(int) * 2 * wb::NCLASS, s));
     launches += 1;
     WB_CUDA(cudaEventRecord(b->fork, s));
+    SideStreams classes(s);
     const wb_cosx* h0 = b->h[0];
     for (int i = 0; i < wb::NCLASS; ++i) {
         const int c = b->order[i];
         if (!b->has[c] || b->items[c] == 0) continue;
-        WB_CUDA(cudaStreamWaitEvent(b->cstream[c], b->fork, 0));
+        WB_CUDA(classes.fork(b->cstream[c], b->fork, b->cdone[c]));
         const int want = (b->items[c] + 3) / 4;
         const int* off = b->d_off + (size_t)c * (nmol + 1);
         const int* order = b->ordered ? b->d_order + (size_t)c * b->stride : nullptr;
@@ -2050,9 +2078,8 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
                 launches += 1;
             }
         }
-        WB_CUDA(cudaEventRecord(b->cdone[c], b->cstream[c]));
-        WB_CUDA(cudaStreamWaitEvent(s, b->cdone[c], 0));
     }
+    WB_CUDA(classes.join());
     {   // the next run takes each class's items costliest first
         wb::BlockOrderArgs P;
         P.cost = b->d_cost;
