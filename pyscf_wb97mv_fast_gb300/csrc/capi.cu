@@ -1730,7 +1730,7 @@ int wb_cosx_get_k_fp64(wb_cosx* h, const double* coords, const double* weights,
             if ((st = gemm64_k(h, X, G64s[w], weights, ld, npts, 0, k_out + kk * (j + w), gemm,
                                s)) != WB_OK)
                 return st;
-            launches += wb::gemm64_k_launches(npts);
+            launches += wb::gemm64_k_launches(nao, npts);
         }
     }
     return read_stats(h, workspace, L.base, ntasks, s, stats, launches);

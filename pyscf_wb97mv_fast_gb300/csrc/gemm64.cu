@@ -26,7 +26,10 @@
 // AOs and 10,000 points the fixed 0.11 ms of launches is about the DGEMM's
 // time, so there is no other path.
 //
-// Point tiles (F) and groups of chunks (K) bound the workspace to some GB.
+// Point tiles (F) and groups of chunks (K) bound the workspace: 65,536 points and
+// 128 chunks up to some 700 AOs (3.7 GB at 648), fewer above, where their digits
+// and level planes would pass 4 GiB (at 4,000 AOs 5,400 points, 6 chunks; with
+// the digits of QD 4.6 GB).
 // A row or column with an infinity or a NaN gives NaN, as FP64 arithmetic
 // mostly would; magnitudes from subnormal to the largest double are taken.
 #include <cuda_bf16.h>
@@ -45,6 +48,7 @@ constexpr int kPiece = 4096;             // terms of an exact FP32 sum
 constexpr int kKc = 512;                 // points per chunk of the K product
 constexpr int kGroup = 128;              // chunks in flight
 constexpr int64_t kTile = 65536;         // points per tile of the F product
+constexpr size_t kBudget = (size_t)4 << 30;     // bytes of either
 
 size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
 // slices are padded to 8 entries: cuBLAS needs 16-byte rows for its
@@ -283,15 +287,28 @@ __global__ void combine_chunks_kernel(const float* __restrict__ C, const int nao
     K[o] = add ? K[o] + acc : acc;
 }
 
+// points of a tile and chunks of a group within the budget
+int64_t tile_points(int nao) {
+    const size_t np = pad8(nao);
+    const size_t per = sizeof(int) + 2 * kS * np + sizeof(float) * planes((int)np) * nao;
+    return std::min(kTile, std::max<int64_t>((int64_t)(kBudget / per) / 32 * 32, 32));
+}
+int group_chunks(int nao) {
+    const size_t np = pad8(nao);
+    const size_t per = 2 * (sizeof(int) * np + 2 * kS * kKc * np) +
+                       sizeof(float) * planes(kKc) * np * np;
+    return (int)std::min<size_t>(kGroup, std::max<size_t>(kBudget / per, 1));
+}
+
 size_t f_bytes(int nao, int64_t ld) {
-    const size_t np = pad8(nao), n = (size_t)std::min(ld, kTile);
+    const size_t np = pad8(nao), n = (size_t)std::min(ld, tile_points(nao));
     return al(sizeof(int) * n) + al(sizeof(int) * nao) + al(2 * kS * np * n) +
            al(2 * kS * np * nao) + al(sizeof(float) * planes((int)np) * nao * n);
 }
 
 size_t k_bytes(int nao, int64_t ld) {
     const size_t np = pad8(nao);
-    const size_t nc = (size_t)std::min<int64_t>((ld + kKc - 1) / kKc, kGroup);
+    const size_t nc = (size_t)std::min<int64_t>((ld + kKc - 1) / kKc, group_chunks(nao));
     return 2 * (al(sizeof(int) * nc * np) + al(2 * kS * kKc * nc * np)) +
            al(sizeof(float) * planes(kKc) * nc * np * np);
 }
@@ -301,11 +318,12 @@ size_t k_bytes(int nao, int64_t ld) {
 size_t gemm64_bytes(int nao, int64_t ld) { return std::max(f_bytes(nao, ld), k_bytes(nao, ld)); }
 
 int gemm64_f_launches(int nao, int64_t ld) {
-    return 1 + (int)((ld + kTile - 1) / kTile) * (3 + planes(pad8(nao)));
+    const int64_t tile = tile_points(nao);
+    return 1 + (int)((ld + tile - 1) / tile) * (3 + planes(pad8(nao)));
 }
-int gemm64_k_launches(int64_t npts) {
-    return (int)((npts + (int64_t)kKc * kGroup - 1) / ((int64_t)kKc * kGroup)) *
-           (3 + planes(kKc));
+int gemm64_k_launches(int nao, int64_t npts) {
+    const int64_t group = (int64_t)kKc * group_chunks(nao);
+    return (int)((npts + group - 1) / group) * (3 + planes(kKc));
 }
 
 #define G64_CUBLAS(call)                                          \
@@ -322,7 +340,7 @@ int gemm64_k_launches(int64_t npts) {
 int gemm64_f(cublasHandle_t hb, const double* X, const double* QD, int nao, int64_t ld,
              double* F, void* ws, cudaStream_t s) {
     const int np = pad8(nao);
-    const int64_t nmax = std::min(ld, kTile);
+    const int64_t tile = tile_points(nao), nmax = std::min(ld, tile);
     char* p = static_cast<char*>(ws);
     int* ep = reinterpret_cast<int*>(p); p += al(sizeof(int) * nmax);
     int* ec = reinterpret_cast<int*>(p); p += al(sizeof(int) * nao);
@@ -334,8 +352,8 @@ int gemm64_f(cublasHandle_t hb, const double* X, const double* QD, int nao, int6
     slice_matrix_kernel<<<nao, 256, 0, s>>>(QD, nao, np, ec, B);
     G64_CUDA(cudaGetLastError());
     const float one = 1.0f, zero = 0.0f;
-    for (int64_t g = 0; g < ld; g += kTile) {
-        const int n = (int)std::min(kTile, ld - g);
+    for (int64_t g = 0; g < ld; g += tile) {
+        const int n = (int)std::min(tile, ld - g);
         const dim3 grid((n / 2 + 255) / 256, np);
         point_exponents_kernel<<<(n + 255) / 256, 256, 0, s>>>(X + g, nao, ld, n, ep);
         G64_CUDA(cudaGetLastError());
@@ -361,7 +379,8 @@ int gemm64_k(cublasHandle_t hb, const double* X, const double* G, const double* 
              int64_t ld, int64_t npts, int accumulate, double* K, void* ws, cudaStream_t s) {
     const int np = pad8(nao);
     const int nchunk = (int)((npts + kKc - 1) / kKc);
-    const int gmax = (int)std::min<int64_t>((ld + kKc - 1) / kKc, kGroup);
+    const int group = group_chunks(nao);
+    const int gmax = (int)std::min<int64_t>((ld + kKc - 1) / kKc, group);
     char* p = static_cast<char*>(ws);
     int* ex = reinterpret_cast<int*>(p); p += al(sizeof(int) * (size_t)gmax * np);
     int* eg = reinterpret_cast<int*>(p); p += al(sizeof(int) * (size_t)gmax * np);
@@ -372,8 +391,8 @@ int gemm64_k(cublasHandle_t hb, const double* X, const double* G, const double* 
     float* C = reinterpret_cast<float*>(p);
     const float one = 1.0f, zero = 0.0f;
     const long long slab = (long long)kS * kKc * np, nn = (long long)np * np;
-    for (int c0 = 0; c0 < nchunk; c0 += kGroup) {
-        const int nc = std::min(kGroup, nchunk - c0);
+    for (int c0 = 0; c0 < nchunk; c0 += group) {
+        const int nc = std::min(group, nchunk - c0);
         const dim3 grid(nc, np);
         slice_chunk_kernel<false><<<grid, 256, 0, s>>>(X, w, nao, ld, npts, (int64_t)c0 * kKc,
                                                        ex, A);

@@ -23,6 +23,6 @@ int gemm64_k(cublasHandle_t hb, const double* X, const double* G, const double* 
 
 // kernel launches of one product, the GEMMs among them
 int gemm64_f_launches(int nao, int64_t ld);
-int gemm64_k_launches(int64_t npts);
+int gemm64_k_launches(int nao, int64_t npts);
 
 }  // namespace wb
