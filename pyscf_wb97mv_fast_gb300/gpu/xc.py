@@ -35,13 +35,18 @@ from pyscf_wb97mv_fast_gb300.cosx import CosxEngine, as_molecule
 
 SUPPORTED_XCTYPE = ('LDA', 'GGA', 'MGGA')
 Unsupported = _native.Unsupported
-# points per tile: X, T and G take (32 + 16 + 16) bytes per point and AO
+# points per tile: X and then T or G take 32 + 16 bytes per point and AO (of a
+# meta-GGA) beside the split's scratch
 DEFAULT_TILE_PTS = 1 << 20
 # A grid of at least two tiles of this size is cut into (up to) four, so that
 # the functional of one tile runs on the host while the GPU works on the next:
 # in one piece the GPU waited for it (8 of 32 ms, 16 waters, 233,999 points).
 # Below this size a tile's kernels no longer fill the GPU.
 OVERLAP_TILE_PTS = 1 << 15
+# The next tile's X and T then stand beside this one's X: 80 bytes per point and
+# AO.  Tiles above this share of tile_pts, those that tile_pts itself limits,
+# come one after another, so that no tile_pts takes more memory for it.
+OVERLAP_SHARE = 48 / 80
 
 
 def _torch():
@@ -184,15 +189,16 @@ def gpu_nr_rks(ctx, ni, mol, grids, xc_code, dms, relativity=0, hermi=1,
         rho_h.copy_(rho_d[:, :nt], non_blocking=True)
         arrived = torch.cuda.Event()
         arrived.record()
-        return i0, i1, w, X, int(rho_d.shape[1]), rho_h, arrived
+        return w, X, int(rho_d.shape[1]), rho_h, arrived
 
     tiles = _tiles(n, ctx.tile_pts)
-    ahead = density(*tiles[0]) if tiles else None
-    for k in range(len(tiles)):
-        i0, i1, w, X, ld, rho_h, arrived = ahead
+    overlap = bool(tiles) and tiles[0][1] <= OVERLAP_SHARE * max(32, ctx.tile_pts)
+    ahead = None
+    for k, (i0, i1) in enumerate(tiles):
+        w, X, ld, rho_h, arrived = ahead or density(i0, i1)
         nt = i1 - i0
         # the next tile's kernels are queued before the host waits
-        ahead = density(*tiles[k + 1]) if k + 1 < len(tiles) else None
+        ahead = density(*tiles[k + 1]) if overlap and k + 1 < len(tiles) else None
         arrived.synchronize()
         rho = rho_h.numpy()
         exc, vrho, vsigma, vt = functional.eval(rho)
