@@ -184,6 +184,17 @@ def _add_potential(rho, ind, nlc_pars, fac, F, U, W, exc, vv):
         _native.ptr(exc), _native.ptr(vv), CosxEngine._stream()), 'wb_vv10_potential')
 
 
+def _sum_inputs(kernel, rho, coords, weights, ind, nlc_pars):
+    """What kernel.kernel_sum is given at the points ind: FP32 from one kernel
+    (_points) for Vv10Kernel's own sum, which works on those; for a caller's
+    kernel the coordinates in FP32 and q, W0 and kappa in FP64."""
+    torch = _torch()
+    if getattr(kernel.kernel_sum, '__func__', None) is Vv10Kernel.kernel_sum:
+        return _points(rho, coords, weights, ind, nlc_pars)
+    q, W0, kappa = vv10_pointwise(rho[0, ind], rho[1:4, ind], weights[ind], nlc_pars)[:3]
+    return coords[ind].to(torch.float32), q, W0, kappa
+
+
 class Vv10Context:
     """Per-mf state of the VV10 flow: the native engine (AO tables) and the
     kernel-sum settings."""
@@ -213,12 +224,13 @@ def _prepare_dm(dm, hermi):
     return dm
 
 
-def vv10_prepare(eng, g, D, nlc_pars, gemm='fp64'):
+def vv10_prepare(eng, g, D, nlc_pars, gemm='fp64', kernel=None):
     """The steps of vv10_energy_fock before the double sum (the GGA density
     on the NLC grid g, the threshold and the pointwise terms): a state for
     vv10_finish; st['xyz'], st['q'], st['W0'], st['kappa'] are the double
     sum's inputs (Vv10Kernel.kernel_sum or, for several molecules,
-    kernel_sum_batch).  gemm as in vv10_energy_fock."""
+    kernel_sum_batch; or kernel's kernel_sum, see _sum_inputs).  gemm as in
+    vv10_energy_fock."""
     torch = _torch()
     if gemm not in ('fp64', 'split64', 'fp32'):
         raise ValueError("gemm must be 'fp64', 'split64' or 'fp32'")
@@ -232,7 +244,8 @@ def vv10_prepare(eng, g, D, nlc_pars, gemm='fp64'):
         T = eng.gemm64_f(g.X[0], D.T)
     rho = eng.gga_rho(g.X, T, n)                          # (4, ld)
     ind = torch.nonzero(rho[0, :n] >= THRESH).squeeze(1)
-    xyz, q, W0, kappa = _points(rho, g.coords, w, ind, nlc_pars)
+    xyz, q, W0, kappa = _sum_inputs(kernel or Vv10Kernel(0.0), rho, g.coords, w, ind,
+                                    nlc_pars)
     return dict(eng=eng, g=g, gemm=gemm, n=n, rho=rho, ind=ind, nlc_pars=nlc_pars,
                 xyz=xyz, q=q, W0=W0, kappa=kappa)
 
@@ -273,8 +286,8 @@ def vv10_energy_fock(eng, g, D, nlc_pars, kernel=None, fp32=False, gemm='fp64'):
       'fp32'    the split with D X rounded once to FP32 and the Fock side
                 from an FP32-rounded G, the SCF's FP32 stages (fp32=True
                 is the same)."""
-    st = vv10_prepare(eng, g, D, nlc_pars, 'fp32' if fp32 else gemm)
     kernel = kernel or Vv10Kernel(0.0)
+    st = vv10_prepare(eng, g, D, nlc_pars, 'fp32' if fp32 else gemm, kernel)
     F, U, W = kernel.kernel_sum(st['xyz'], st['q'], st['W0'], st['kappa'])
     return vv10_finish(st, F, U, W)
 
@@ -305,7 +318,8 @@ def gpu_nr_nlc_vxc(ctx, ni, mol, grids, xc_code, dm, relativity=0, hermi=1,
     vv = torch.zeros_like(rho)          # d/d rho (half of it) and d/d grad
     ind = torch.nonzero(rho0 >= THRESH).squeeze(1)
     for nlc_pars, fac in nlc_coefs:
-        F, U, W = ctx.kernel.kernel_sum(*_points(rho, coords, w, ind, nlc_pars))
+        F, U, W = ctx.kernel.kernel_sum(
+            *_sum_inputs(ctx.kernel, rho, coords, w, ind, nlc_pars))
         _add_potential(rho, ind, nlc_pars, fac, F, U, W, exc, vv)
     # vmat = X0^T (w o G) + its transpose, G = 1/2 v0 X0 + sum_d v_d X_d
     vmat = eng.gemm64_k(X[0], eng.gga_aow(X, vv, n), w)
