@@ -661,6 +661,7 @@ class KBuildGraph:
         torch = _torch()
         self.eng = eng
         self.omegas = tuple(float(w) for w in omegas)
+        coords_rel, weights, _ = eng._grid_args(coords_rel, weights)
         self._coords, self._weights = coords_rel, weights
         self.qd = torch.zeros((eng.nao, eng.nao), dtype=torch.float64,
                               device=eng.device)
@@ -678,6 +679,7 @@ class KBuildGraph:
         with torch.cuda.graph(self.graph, capture_error_mode='thread_local'):
             eng.get_k_multi(coords_rel, weights, self.qd, self.omegas, **args)
             self.out = (self._k + self._k.transpose(1, 2)) * 0.5
+        self._ws = eng._ws      # replayed on, whatever the engine takes later
 
     def run(self, dm):
         """dm (nao, nao) FP64, host or device -> symmetrised K on the device

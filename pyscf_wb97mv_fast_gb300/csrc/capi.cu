@@ -203,6 +203,8 @@ struct wb_cosx {
     float* bcost = nullptr;
     int* border = nullptr;
     int64_t bo_stride = 0, bo_ld = -1;
+    bool bo_captured = false;        // the arrays are a captured build's
+    std::vector<void*> bo_arrays;    // these and outgrown ones, freed with the handle
     int bo_n[wb::NCLASS] = {0};
     // first pair of the second half of each class's blocks (WB_COSX_SPLIT):
     // a run boundary near the middle of the class's model flops
@@ -463,18 +465,32 @@ int block_order_args(wb_cosx* h, int64_t ldt, wb::CosxArgs& a,
                      const bool* dual, cudaStream_t s) {
     if (!WB_COSX_BLOCK_ORDER) return WB_OK;
     const int64_t stride = (WB_COSX_SPLIT ? 2 : 1) * ((ldt + 31) / 32);
-    if (stride > h->bo_stride) {
-        WB_CUDA(cudaStreamSynchronize(s));
-        if (h->bcost) cudaFree(h->bcost);
-        if (h->border) cudaFree(h->border);
-        h->bcost = nullptr;
-        h->border = nullptr;
-        h->bo_stride = 0;
-        WB_CUDA(cudaMalloc(&h->bcost, sizeof(float) * wb::NCLASS * stride));
-        WB_CUDA(cudaMalloc(&h->border, sizeof(int) * wb::NCLASS * stride));
-        h->bo_stride = stride;
+    // A captured build replays on the arrays it was captured with, and its order
+    // is the one that its last replay left there.  So the next build outside a
+    // capture gets arrays of its own, and outgrown ones (of half the size or
+    // less) stay until the handle goes.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    WB_CUDA(cudaStreamIsCapturing(s, &capture));
+    const bool capturing = capture != cudaStreamCaptureStatusNone;
+    const bool taken = h->bo_captured && !capturing;
+    if (stride > h->bo_stride || taken) {
+        const int64_t room = stride > h->bo_stride ? std::max(stride, 2 * h->bo_stride)
+                                                   : h->bo_stride;
+        void *cost = nullptr, *order = nullptr;
+        WB_CUDA(cudaMalloc(&cost, sizeof(float) * wb::NCLASS * room));
+        const cudaError_t e = cudaMalloc(&order, sizeof(int) * wb::NCLASS * room);
+        if (e != cudaSuccess) {
+            cudaFree(cost);
+            return cuda_fail(e, "block order arrays");
+        }
+        h->bo_arrays.push_back(cost);
+        h->bo_arrays.push_back(order);
+        h->bcost = static_cast<float*>(cost);
+        h->border = static_cast<int*>(order);
+        h->bo_stride = room;
         h->bo_ld = -1;
     }
+    h->bo_captured = capturing;
     if (h->bo_ld != ldt) {
         for (int c = 0; c < wb::NCLASS; ++c) h->bo_n[c] = 0;
         h->bo_ld = ldt;
@@ -1298,8 +1314,7 @@ int wb_cosx_destroy(wb_cosx* h) {
     }
     if (h->fork) cudaEventDestroy(h->fork);
     if (h->block) cudaFree(h->block);
-    if (h->bcost) cudaFree(h->bcost);
-    if (h->border) cudaFree(h->border);
+    for (void* q : h->bo_arrays) cudaFree(q);
     if (h->cublas_ws) cudaFree(h->cublas_ws);
     if (h->f64_P) cudaFree(h->f64_P);
     if (h->f64_E) cudaFree(h->f64_E);
