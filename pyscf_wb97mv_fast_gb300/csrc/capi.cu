@@ -534,24 +534,25 @@ public:
     // t runs from the event `from` of the caller's stream on, joined through done
     cudaError_t fork(cudaStream_t t, cudaEvent_t from, cudaEvent_t done) {
         const cudaError_t e = cudaStreamWaitEvent(t, from, 0);
-        if (e == cudaSuccess) side_.push_back({t, done});
+        if (e == cudaSuccess) side_[n_++] = {t, done};
         return e;
     }
     cudaError_t join() {
         cudaError_t first = cudaSuccess;
-        for (const Side& q : side_) {
-            cudaError_t e = cudaEventRecord(q.done, q.stream);
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(s_, q.done, 0);
+        for (int i = 0; i < n_; ++i) {
+            cudaError_t e = cudaEventRecord(side_[i].done, side_[i].stream);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(s_, side_[i].done, 0);
             if (first == cudaSuccess) first = e;
         }
-        side_.clear();
+        n_ = 0;
         return first;
     }
 
 private:
     struct Side { cudaStream_t stream; cudaEvent_t done; };
     cudaStream_t s_;
-    std::vector<Side> side_;
+    int n_ = 0;
+    Side side_[wb::NCLASS];     // at most a class's each, or a batch's lanes
 };
 
 // One class launch of want CTAs (four items each), at most cap at a time.  A
@@ -602,10 +603,10 @@ int run_g_classes(wb_cosx* h, int64_t npts_t, int64_t ldt, const float* F,
         WB_CUDA(classes.fork(h->cstream[c], h->fork, h->cdone[c]));
         WB_CUDA(launch_class(h, c, a, r, want, cap, h->cstream[c], far, h->stage_smem[c],
                              false));
+        WB_CUDA(classes.join());
         ran[c] = true;
         *launches += 1;
     }
-    WB_CUDA(classes.join());
     {
         const int st = block_order_update(h, a, ran, single, s, launches);
         if (st != WB_OK) return st;
@@ -670,9 +671,9 @@ int run_g_classes_dual(wb_cosx* h, int64_t npts_t, int64_t ldt, const float* F,
                 *launches += 1;
             }
         }
+        WB_CUDA(classes.join());
         ran[c] = true;
     }
-    WB_CUDA(classes.join());
     {
         const int st = block_order_update(h, a, ran, h->dual_cls, s, launches);
         if (st != WB_OK) return st;
@@ -2093,8 +2094,8 @@ int wb_cosx_batch_run(wb_cosx_batch* b, const double* const* qd,
                 launches += 1;
             }
         }
+        WB_CUDA(classes.join());
     }
-    WB_CUDA(classes.join());
     {   // the next run takes each class's items costliest first
         wb::BlockOrderArgs P;
         P.cost = b->d_cost;
