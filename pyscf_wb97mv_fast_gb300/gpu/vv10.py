@@ -22,7 +22,8 @@ import math
 import numpy as np
 
 from pyscf_wb97mv_fast_gb300 import _native
-from pyscf_wb97mv_fast_gb300.cosx import CosxEngine, as_molecule, device_arg, device_out
+from pyscf_wb97mv_fast_gb300.cosx import (CosxEngine, as_molecule, device_arg, device_out,
+                                          round32)
 
 THRESH = 1e-8
 Unsupported = _native.Unsupported
@@ -236,17 +237,20 @@ def vv10_prepare(eng, g, D, nlc_pars, gemm='fp64', kernel=None):
         raise ValueError("gemm must be 'fp64', 'split64' or 'fp32'")
     n = g.n
     w = g.weights
+    X = g.X
     if gemm == 'fp32':
-        T = eng.ozaki_f(g.X[0], D)
+        T = eng.ozaki_f(X[0], D)
     elif gemm == 'split64':
-        T = eng.ozaki_f(g.X[0], D, fp64=True)
+        T = eng.ozaki_f(X[0], D, fp64=True)
     else:
-        T = eng.gemm64_f(g.X[0], D.T)
-    rho = eng.gga_rho(g.X, T, n)                          # (4, ld)
+        if int(X.shape[2]) != round32(n):       # a grid padded to another length
+            X = torch.nn.functional.pad(X[:, :, :n], (0, round32(n) - n))
+        T = eng.gemm64_f(X[0], D.T)
+    rho = eng.gga_rho(X, T, n)                            # (4, ld)
     ind = torch.nonzero(rho[0, :n] >= THRESH).squeeze(1)
     xyz, q, W0, kappa = _sum_inputs(kernel or Vv10Kernel(0.0), rho, g.coords, w, ind,
                                     nlc_pars)
-    return dict(eng=eng, g=g, gemm=gemm, n=n, rho=rho, ind=ind, nlc_pars=nlc_pars,
+    return dict(eng=eng, g=g, X=X, gemm=gemm, n=n, rho=rho, ind=ind, nlc_pars=nlc_pars,
                 xyz=xyz, q=q, W0=W0, kappa=kappa)
 
 
@@ -254,19 +258,19 @@ def vv10_finish(st, F, U, W):
     """E_nl and V_nl from a vv10_prepare state and the double sums F, U, W
     of its points."""
     torch = _torch()
-    eng, g, n, ind, rho = (st[k] for k in ('eng', 'g', 'n', 'ind', 'rho'))
-    w = g.weights
+    eng, X, n, ind, rho = (st[k] for k in ('eng', 'X', 'n', 'ind', 'rho'))
+    w = st['g'].weights
     exc = torch.zeros(n, dtype=torch.float64, device=rho.device)
     vv = torch.zeros_like(rho)
     _add_potential(rho, ind, st['nlc_pars'], 1.0, F, U, W, exc, vv)
     e_nl = (rho[0, :n] * w * exc).sum()
     # G = 1/2 v0 X0 + sum_d 2 v1 grad_d X_d, then X0^T (w o G); G FP64, or
     # rounded once to FP32 (gemm 'fp32')
-    G = eng.gga_aow(g.X, vv, n, torch.float32 if st['gemm'] == 'fp32' else None)
+    G = eng.gga_aow(X, vv, n, torch.float32 if st['gemm'] == 'fp32' else None)
     if st['gemm'] == 'fp64':
-        vmat = eng.gemm64_k(g.X[0], G, w)
+        vmat = eng.gemm64_k(X[0], G, w)
     else:
-        vmat = eng.ozaki_k(g.X[0], G, w)
+        vmat = eng.ozaki_k(X[0], G, w)
     return e_nl, vmat + vmat.T
 
 

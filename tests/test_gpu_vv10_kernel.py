@@ -1,6 +1,6 @@
 """A caller's own double sum in the VV10 flows: it is given q, W0 and kappa in
 FP64 (the library's own sum works on FP32 values), and an FP64 one is not
-limited by a rounding before it."""
+limited by a rounding before it.  And AO values of any padding in the FP64 flow."""
 import types
 
 import numpy as np
@@ -86,3 +86,19 @@ def test_nlc_vxc_with_an_fp64_sum(case):
     _check_inputs(eng, g, dm, ctx.kernel.seen[0])
     assert n1 == n0 and abs(e1 - e0) < 1e-6 * abs(e0)
     assert np.max(np.abs(v1 - v0)) < 1e-5 * np.abs(v0).max()
+
+
+@pytest.mark.parametrize('ld', [1500, 1501, 1536, 2048])
+def test_fp64_flow_takes_any_padding(case, ld):
+    """The FP64 flow on AO values padded to another length than the library's:
+    the same numbers."""
+    import torch
+
+    from pyscf_wb97mv_fast_gb300.gpu.vv10 import vv10_energy_fock
+    mol, coords, weights, eng, g, dm, _ = case
+    e0, v0 = vv10_energy_fock(eng, g, dm, PARS)
+    X = torch.zeros((4, mol.nao, ld), dtype=torch.float64, device=eng.device)
+    X[:, :, :g.n] = g.X[:, :, :g.n]
+    other = types.SimpleNamespace(n=g.n, coords=g.coords, weights=g.weights, X=X)
+    e, v = vv10_energy_fock(eng, other, dm, PARS)
+    assert torch.equal(e, e0) and torch.equal(v, v0)
