@@ -344,9 +344,14 @@ int wb_cosx_ozaki_k64(wb_cosx* h, const double* x, const double* g,
                       double* k_out, void* workspace, size_t workspace_bytes,
                       void* stream);
 
-/* The same two products with no less accuracy than an FP64 GEMM (63-bit
- * digits on the bf16 tensor cores; any nao), the GEMMs of the FP64 form and
- * of the FP64 numint flows (gpu/vv10.py:288-297, :315-322):
+/* The same two products at FP64 accuracy (70 and 63 bits of digits on the bf16
+ * tensor cores; any nao), the GEMMs of the FP64 form and of the FP64 numint
+ * flows (gpu/vv10.py:288-297, :315-322).  Entries are exact to some 2^-68 (F) and
+ * 2^-61 (K, per 512 points) of the product of the largest entries of their row
+ * and column, and rounded once: on AO values and densities closer to exact
+ * arithmetic than an FP64 GEMM, entries of 1e-12 of the largest among them
+ * (gemm64.cu has the figures); on matrices whose rows span more than some 60 bits
+ * small entries keep fewer digits than there:
  *   wb_cosx_gemm64_f: f_out (nao, ld) FP64 = X QD;
  *   wb_cosx_gemm64_k: k_out (+)= X^T (w o G), g (nao, ld) FP64, ld = npts
  *     rounded up to 32.

@@ -489,8 +489,9 @@ class CosxEngine:
         return out
 
     def gemm64_f(self, X, qd):
-        """QD^T X (nao, ld) FP64 with no less accuracy than an FP64 GEMM
-        (wb_cosx_gemm64_f); X (nao, ld) FP64, ld a multiple of 32."""
+        """QD^T X (nao, ld) FP64 to some 2^-68 of the largest entries of its
+        point and column, rounded once (wb_cosx_gemm64_f); X (nao, ld) FP64, ld
+        a multiple of 32."""
         torch = _torch()
         X = device_arg(X, 'X', torch.float64, self.device, (self.nao, None))
         if X.data_ptr() % 16:                   # the kernels load pairs of points
@@ -508,9 +509,9 @@ class CosxEngine:
         return out
 
     def gemm64_k(self, X, G, weights):
-        """X^T (w o G) (nao, nao) FP64 with no less accuracy than an FP64
-        GEMM (wb_cosx_gemm64_k); X, G (nao, ld) FP64, ld the number of
-        weights rounded up to 32."""
+        """X^T (w o G) (nao, nao) FP64 to some 2^-61 of the largest entries of
+        its rows in each 512 points (wb_cosx_gemm64_k); X, G (nao, ld) FP64, ld
+        the number of weights rounded up to 32."""
         torch = _torch()
         weights = device_arg(weights, 'weights', torch.float64, self.device, (None,))
         npts = int(weights.shape[0])

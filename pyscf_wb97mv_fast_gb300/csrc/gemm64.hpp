@@ -1,4 +1,4 @@
-// FP64 GEMMs on the bf16 tensor cores with at least FP64 accuracy (gemm64.cu).
+// FP64 GEMMs on the bf16 tensor cores at FP64 accuracy (gemm64.cu).
 #pragma once
 #include <cublas_v2.h>
 #include <cuda_runtime.h>

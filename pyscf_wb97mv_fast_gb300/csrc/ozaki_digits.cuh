@@ -98,20 +98,27 @@ __device__ __forceinline__ unsigned long long biased_q(const double x, const int
     return (int)hi < 0 ? bias - q : bias + q;
 }
 
-// digit i (0 the most significant) of two biased integers, as a pair of bf16:
-// 128 + field is the bit pattern 0x4300 + field, and subtracting 128 + H from
-// it is exact
-template<int B, int S>
-__device__ __forceinline__ unsigned digit_pair(const unsigned long long a,
-                                               const unsigned long long b, const int i) {
+// the digits in the low B bits (of the most significant digit, `first`, B + 1) of
+// two biased words, as a pair of bf16: 128 + field is the bit pattern 0x4300 +
+// field, and subtracting 128 + H from it is exact
+template<int B>
+__device__ __forceinline__ unsigned field_pair(const unsigned a, const unsigned b,
+                                               const bool first) {
     constexpr unsigned H = 1u << (B - 1), M = ((1u << B) - 1u) * 0x10001u;
-    const int sh = B * (S - 1 - i);
-    unsigned t = __byte_perm((unsigned)(a >> sh), (unsigned)(b >> sh), 0x5410);
-    t = i ? (t & M) | 0x43004300u : t + 0x43004300u;    // the first goes up to 2^B
+    unsigned t = __byte_perm(a, b, 0x5410);
+    t = first ? t + 0x43004300u : (t & M) | 0x43004300u;    // the first goes up to 2^B
     const unsigned h = (0x4300u + H) * 0x10001u;
     const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&t),
                                      *reinterpret_cast<const __nv_bfloat162*>(&h));
     return *reinterpret_cast<const unsigned*>(&d);
+}
+
+// digit i (0 the most significant) of two biased integers
+template<int B, int S>
+__device__ __forceinline__ unsigned digit_pair(const unsigned long long a,
+                                               const unsigned long long b, const int i) {
+    const int sh = B * (S - 1 - i);
+    return field_pair<B>((unsigned)(a >> sh), (unsigned)(b >> sh), i == 0);
 }
 
 // A pair of exponents e, f as the scale 2^(e + f + K), K the constant of a
