@@ -294,8 +294,8 @@ class CosxEngine:
     def get_k_fp64(self, coords_rel, weights, qd, omegas, tile_tol=1e-11,
                    out=None, stats=True):
         """The plain FP64 form of get_k_multi: FP64 AO values, F = X QD kept
-        in FP64 (cuBLAS DGEMM), the same screen, G from the FP64 class
-        kernels (accumulated in FP64), K = X^T (w o G) by cuBLAS DGEMM; the
+        in FP64 (as gemm64_f), the same screen, G from the FP64 class
+        kernels (accumulated in FP64), K = X^T (w o G) as gemm64_k; the
         whole grid is one tile.  Returns (len(omegas), nao, nao) FP64 on
         the device, unsymmetrised.  The first call on an engine uploads the
         FP64 pair tables (synchronous)."""

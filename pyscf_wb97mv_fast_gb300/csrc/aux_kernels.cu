@@ -312,7 +312,7 @@ cudaError_t launch_sub_stats(const double* coords, const double* weights,
     const int64_t nblk = (ld + 127) / 128;
     if (nblk <= 0) return cudaSuccess;
     // one warp a CTA while the blocks are fewer than four an SM
-    const int warps = nblk < 4 * 152 ? 1 : 4;
+    const int warps = nblk < 4 * (int64_t)sm_count() ? 1 : 4;
     const dim3 grid((unsigned)((nblk + warps - 1) / warps),
                     (unsigned)std::max(1, (nvshell + kStatsShells - 1) / kStatsShells));
     sub_stats_kernel<<<grid, 32 * warps, 0, s>>>(

@@ -980,10 +980,12 @@ struct wb_cosx_batch {
     int* d_order = nullptr;             // NCLASS x stride: costliest first
     int64_t stride = 0;
     bool ordered = false;               // the orders hold a previous run's costs
-    // molecules of more blocks than fill the device on their own run their
-    // own class launches: the batched kernels keep the argument blocks in shared
-    // memory and registers where those have them in the constant bank (four of
-    // 30 waters: 140.6 ms a run batched, 120.9 so)
+    // molecules of ten 64-point blocks an SM or more, which fill the device on
+    // their own, run their own class launches: the batched kernels keep the
+    // argument blocks in shared memory and registers where those have them in the
+    // constant bank.  Runs of four clusters, batched and so: 8 waters (7.5 blocks
+    // an SM) 10.5 and 11.0 ms, 10 (9.2) 16.7 and 16.2, 12 (11.0) 24.2 and 23.3,
+    // 18 (16.2) 55.3 and 50.5, 30 (26.5) 167 and 152
     std::vector<char> alone;
     // the class launches of a run, side by side
     cudaStream_t cstream[wb::NCLASS] = {};

@@ -30,7 +30,7 @@
 // Eight to sixteen warps an SM fill the pipe, so one CTA an SM with the
 // whole register file and the Boys table in shared memory is enough.
 // Measured on 8 waters (192 AOs, 70,478 points, both omegas), a whole K build:
-// 180 -> 47.9 ms, the class kernels at 82-88 % of the FP64 pipe's issue rate.
+// 180 -> 48.4 ms, the class kernels at 82-88 % of the FP64 pipe's issue rate.
 #pragma once
 #include <algorithm>
 #include <cuda_runtime.h>

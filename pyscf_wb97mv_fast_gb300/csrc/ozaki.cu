@@ -182,14 +182,14 @@ __global__ void f_combine_kernel(const float* __restrict__ C, int nao,
 // (648 AOs, 384,998 points, two G): 3.8 -> 2.4 ms; 1.2 of them had been spent on
 // |x| and G -> FP64 as FP64 instructions.
 // ---------------------------------------------------------------------------
-// gridDim.z right-hand sides: B holds nb columns per chunk, those of right-hand
-// side r at r np (np = gridDim.y).  The CTAs of the first one also slice X,
-// unless slice_x is 0: the X slices and exponents of this tile are then already
-// in A / ex (an earlier omega of the same tile).
 // the constant of scale_word: FP64's bias, and what a chunk's sum is scaled by
 template<int B_, int S>
 constexpr int kScaleK = 1023 - 2 * 400 - 2 * kW + 2 + B_ * (S - 1);
 
+// gridDim.z right-hand sides: B holds nb columns per chunk, those of right-hand
+// side r at r np (np = gridDim.y).  The CTAs of the first one also slice X,
+// unless slice_x is 0: the X slices and exponents of this tile are then already
+// in A / ex (an earlier omega of the same tile).
 template<typename GT>
 struct KIn {
     const GT* g[8];

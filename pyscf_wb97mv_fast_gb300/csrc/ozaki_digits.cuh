@@ -33,11 +33,11 @@ __device__ __forceinline__ unsigned abs_hi(const double x) {
 }
 
 __device__ __forceinline__ int exp_of_hi(const unsigned hi) {
+    if (hi >= 0x7ff00000u) return kNonfinite;
     // smallest e with |x| < 2^e from the high word of |x|, clamped to
     // [-400, 500]: rows whose largest entry is below 2^-400 are zero at this
     // precision, and the clamp keeps every scale factor 2^k of the kernels
     // (|k| <= 2 * 500 + 84) inside the normal FP64 range of pow2()
-    if (hi >= 0x7ff00000u) return kNonfinite;
     const int e = (int)(hi >> 20) - 1022;           // |x| < 2^(ebits-1023+1)
     return e < -400 ? -400 : (e > 500 ? 500 : e);
 }
